@@ -382,10 +382,12 @@ __device__ __forceinline__ void flush_pushes(const ExpandParams& P, const PushCt
     __syncwarp();
 }
 
+// Chunk descriptors a lane writes by itself; a vertex with more is written by the whole warp.
+constexpr int kLaneChunks = 8;
+
 // Called by all 32 lanes together with U candidate slots each; ok[u] marks slots whose relaxation
 // improved vertex v[u]. Vertices below the chunking degree go to the small queue with one
-// warp-aggregated append for all U slots; chunked vertices get their chunk range from one
-// warp-aggregated atomic per slot and the warp writes every chunk descriptor.
+// warp-aggregated append for all U slots, and so do the chunks of chunked vertices.
 template <class Op, bool kClassify, int CH, int U>
 __device__ __forceinline__ void push_batch(const ExpandParams& P, const PushCtx& Q, bool (&ok)[U],
                                            const int (&v)[U], const int (&row)[U], const int2* se_pre = nullptr) {
@@ -485,34 +487,45 @@ __device__ __forceinline__ void push_batch(const ExpandParams& P, const PushCtx&
         __syncwarp();
     }
     if (kClassify) {
+        // Chunked vertices: one reservation for all U slots of all lanes, then every descriptor.
+        int nchl = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) nchl += chunked[u] ? (e[u] - s[u] + CH - 1) / CH : 0;
+        if (!__any_sync(kFullMask, nchl > 0)) return;
+        const int incl = warp_inclusive_scan(nchl);
+        const int total = __shfl_sync(kFullMask, incl, 31);
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(Q.ccount, static_cast<unsigned>(total));
+        base = __shfl_sync(kFullMask, base, 0);
+        if (static_cast<unsigned long long>(base) + total > static_cast<unsigned long long>(P.ws.cap_chunks)) {
+            if (lane == 0) raise_error(P.st, DPG_ERR_CAPACITY, 10);
+            return;
+        }
+        unsigned my_first = base + static_cast<unsigned>(incl - nchl);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            unsigned hm = __ballot_sync(kFullMask, chunked[u]);
-            if (!hm) continue;
-            const int nch = chunked[u] ? (e[u] - s[u] + CH - 1) / CH : 0;
-            const int incl = warp_inclusive_scan(nch);
-            const int total = __shfl_sync(kFullMask, incl, 31);
-            unsigned base = 0;
-            if (lane == 0) base = atomicAdd(Q.ccount, static_cast<unsigned>(total));
-            base = __shfl_sync(kFullMask, base, 0);
-            const unsigned my_first = base + static_cast<unsigned>(incl - nch);
-            if (static_cast<unsigned long long>(base) + total > static_cast<unsigned long long>(P.ws.cap_chunks)) {
-                if (lane == 0) raise_error(P.st, DPG_ERR_CAPACITY, 10);
-                hm = 0u;
+            const int hn = chunked[u] ? (e[u] - s[u] + CH - 1) / CH : 0;
+            if (hn <= kLaneChunks) {
+                for (int c = 0; c < hn; ++c) {
+                    const int k0 = s[u] + c * CH;
+                    __stcg(Q.chunks + my_first + c, make_int4(v[u], k0, min(e[u], k0 + CH), c == 0 ? 1 : 0));
+                }
             }
-            while (hm) {  // the whole warp writes one chunked vertex's descriptors at a time
+            unsigned hm = __ballot_sync(kFullMask, hn > kLaneChunks);
+            while (hm) {  // the whole warp writes one large vertex's descriptors at a time
                 const int src = __ffs(hm) - 1;
                 hm &= hm - 1u;
                 const int hv = __shfl_sync(kFullMask, v[u], src);
                 const int hs = __shfl_sync(kFullMask, s[u], src);
                 const int he = __shfl_sync(kFullMask, e[u], src);
                 const unsigned first = __shfl_sync(kFullMask, my_first, src);
-                const int hn = (he - hs + CH - 1) / CH;
-                for (int c = lane; c < hn; c += 32) {
+                const int wn = (he - hs + CH - 1) / CH;
+                for (int c = lane; c < wn; c += 32) {
                     const int k0 = hs + c * CH;
                     __stcg(Q.chunks + first + c, make_int4(hv, k0, min(he, k0 + CH), c == 0 ? 1 : 0));
                 }
             }
+            my_first += static_cast<unsigned>(hn);
         }
     }
 }
