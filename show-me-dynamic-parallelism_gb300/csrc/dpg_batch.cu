@@ -336,6 +336,7 @@ dpg_status sssp_plan(dpg_batch* b, int32_t nsrc, const std::vector<GroupLaunch>&
         L.off = b->out->off;
         L.adj = b->out->adj;
         L.V = b->V;
+        L.E = b->out->E;
         L.nsrc = nsrc;
         L.dirty[0] = d0;
         L.dirty[1] = d1;

@@ -72,6 +72,7 @@ struct ExpandParams {
     // Multi-source SSSP: non-zero when nsrc is a multiple of 4 and the labels are 16-byte aligned,
     // so a vertex's labels can be read four at a time (relax_mask_vec4).
     int32_t label_vec4;
+    uint32_t min_item_log;  // log2 of the fewest small-queue vertices in a warp item (binned kernels)
 };
 
 // Operator interface of the expansion:
@@ -924,7 +925,12 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
         const int2* qse_cur = p ? P.ws.qse[1] : P.ws.qse[0];
         uint32_t* bmp_cur = p ? P.ws.bmp[1] : P.ws.bmp[0];
         const int4* chunks_cur = p ? P.ws.chunks[1] : P.ws.chunks[0];
-        const unsigned fchunks = (n + 31u) / 32u;
+        // Vertices per warp item of the small queue: 32, or fewer (a power of two, at least
+        // 2^min_item_log) while that still gives every item a warp of its own.
+        unsigned item_log = 5u;
+        if (kBinned)
+            while (item_log > P.min_item_log && (n >> (item_log - 1u)) + nch < nwarps) --item_log;
+        const unsigned fchunks = (n + (1u << item_log) - 1u) >> item_log;
 
         if (kNearFar && split) {
             // Split: still-current entries below the new threshold join the frontier (de-duplicated
@@ -1108,10 +1114,10 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                     continue;
                 }
                 const unsigned chunk = item - hub_items;
-                const unsigned i = chunk * 32u + lane;
+                const unsigned i = (chunk << item_log) + lane;
                 int u = 0, s = 0, d = 0;
                 RV du{};
-                const bool has = i < n;
+                const bool has = i < n && (!kBinned || static_cast<unsigned>(lane) < (1u << item_log));
                 if (has) {
                     u = __ldcg(qv_cur + i);
                     const int2 se = __ldcg(qse_cur + i);
@@ -1307,6 +1313,21 @@ __global__ void barrier_timeout_kernel(DevStatus* st, unsigned long long timeout
     grid_barrier(st, gridDim.x + 1, timeout_ns);
 }
 
+// Fewest small-queue vertices of a warp item when an iteration has more warps than items of 32: the
+// power of two that still gives an item about kItemArcs arcs at the graph's mean degree. An item's
+// time grows with its arcs (an item of 32 R-MAT vertices is five or more dependent relaxation
+// batches; even within one batch every further slot adds scattered loads and atomics to the chain),
+// while the warps past the last item idle. But every item appends to the frontier by itself, on one
+// counter. Same box, start of 32 always against at least 64 / 32 / 8 / 1 arcs: SSSP R-MAT 14 193 ->
+// 119 / 122 / 123 / 124 us, SSSP 4096^2 grid 65.4 -> 65.4 / 53.3 / 53.4 / 55.4 ms, BFS 1501 x 2003
+// grid 17.7 -> 17.7 / 14.8 / 13.0 / 14.3 ms, BFS 4096^2 grid 35.1 ms at 8 against 42.7 at 1.
+constexpr int64_t kItemArcs = 8;
+uint32_t min_item_log(int32_t V, int64_t E) {
+    uint32_t lg = 0;
+    while (lg < 5 && (E << lg) < kItemArcs * V) ++lg;
+    return lg;
+}
+
 // The kernel of a solution id; `wide` selects the kWideBlocks build of the binned and
 // direction-optimizing kernels.
 template <class Op>
@@ -1368,6 +1389,7 @@ cudaError_t run_multi(const MultiExpandLaunch& L, const ExpandWorkspace& ws, Dev
     P.ws = ws;
     P.st = st;
     P.nsrc = L.nsrc;
+    P.min_item_log = min_item_log(L.V, L.E);
     P.dirty[0] = L.dirty[0];
     P.dirty[1] = L.dirty[1];
     P.label_vec4 = (L.nsrc % 4 == 0 && (reinterpret_cast<uintptr_t>(L.label) & 15u) == 0) ? 1 : 0;
@@ -1442,6 +1464,7 @@ cudaError_t launch_expand(const ExpandLaunch& L, const ExpandWorkspace& ws, DevS
     P.mf = diropt ? L.do_mf : nullptr;
     P.nf = diropt ? L.do_nf : nullptr;
     P.E = L.E;
+    P.min_item_log = min_item_log(L.V, L.E);
     const int classify =
         (L.solution == DPG_SOL_GRID || L.solution == DPG_SOL_BINNED || L.solution == DPG_SOL_DIROPT ||
          L.solution == DPG_SOL_NEARFAR) ? 1 : 0;
@@ -1490,6 +1513,7 @@ cudaError_t launch_color(const ExpandLaunch& L, const int32_t* out_off, const in
     P.trace = L.trace;
     P.trace_cap = L.trace_cap;
     P.aux = pending;
+    P.min_item_log = min_item_log(L.V, L.E);
     err = cudaMemsetAsync(ws.qcount, 0, sizeof(uint32_t) * 3, stream);
     if (err == cudaSuccess) err = cudaMemsetAsync(ws.ccount, 0, sizeof(uint32_t) * 3, stream);
     if (err == cudaSuccess) err = cudaMemsetAsync(&st->bar_count, 0, sizeof(unsigned), stream);

@@ -96,6 +96,7 @@ struct MultiExpandLaunch {
     const int2* adj;
     int32_t V;
     int32_t nsrc;
+    int64_t E;
     int32_t* label;
     unsigned long long* dirty[2];
     const int32_t* sources;
