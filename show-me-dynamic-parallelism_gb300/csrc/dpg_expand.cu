@@ -718,6 +718,26 @@ __device__ __forceinline__ void warp_gather(const ExpandParams& P, const PushCtx
     ss[lane] = s;
     sdu[lane] = du;
     __syncwarp();
+    // Small iterations: at most one arc per lane needs one slot, not U (whose idle slots still issue
+    // their loads of arc 0 ahead of the chain). Same box: SSSP 4096^2 grid 53.3 -> 47.0 ms, BFS 1501 x
+    // 2003 grid 12.7 -> 11.7 ms, SSSP R-MAT 14 124 -> 122 us.
+    if (total <= 32) {
+        const int k = lane;
+        const bool a = k < total;
+        int ee = 0;
+        typename Op::RV d1{};
+        if (a) {
+            int r = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (sx[r + step] <= k) r += step;
+            ee = ss[r] + (k - sx[r]);
+            d1 = sdu[r];
+        }
+        relax_one<Op, kClassify, CH>(P, Q, a, ee, d1);
+        __syncwarp();
+        return;
+    }
     constexpr int U = 4;
     for (int base = 0; base < total; base += 32 * U) {
         bool act[U];

@@ -1,0 +1,38 @@
+"""Small frontiers are cut into warp items of 1 to 32 vertices (by the mean degree and the number of idle warps) and
+items of at most 32 arcs take a shorter path: distances and levels must stay those of the oracle at the edges."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import dpg
+
+pytestmark = pytest.mark.gpu
+
+
+def _layers(width: int, degree: int, depth: int, seed: int):
+    """A root over `width` vertices, then `depth` layers of `width` vertices with `degree` random arcs each into the
+    next layer: every frontier is about `width` vertices of `degree` arcs."""
+    rng = np.random.default_rng(seed)
+    V = 1 + width * (depth + 1)
+    src = [np.zeros(width, np.int64)]
+    dst = [1 + np.arange(width)]
+    for k in range(depth):
+        s = np.repeat(1 + k * width + np.arange(width), degree)
+        src.append(s)
+        dst.append(1 + (k + 1) * width + rng.integers(0, width, s.size))
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    return dpg.csr_from_arcs(V, src, dst, rng.integers(0, 50, src.size))
+
+
+# Degrees around 8 and 32 arcs per item and past the hub threshold of 128; widths around 32, one item per warp
+# (3,648 and 4,864 warps) and their doubles.
+@pytest.mark.parametrize("width", [1, 31, 33, 3647, 3649, 4865, 9731])
+@pytest.mark.parametrize("degree", [1, 2, 7, 9, 31, 33, 130])
+def test_layers(ctx, orc, width, degree):
+    g = _layers(width, degree, 3, seed=width * 1000 + degree)
+    dg = dpg.Graph(ctx, g.offsets, g.col, g.weights)
+    want = orc.sssp_dijkstra(g.offsets, g.col, g.weights, 0)
+    for solution in (dpg.SOL_BINNED, dpg.SOL_NEARFAR):
+        assert np.array_equal(dpg.sssp(ctx, dg, 0, solution=solution), want)
+    assert np.array_equal(dpg.bfs(ctx, dg, 0), orc.bfs(g.offsets, g.col, 0))
