@@ -36,3 +36,24 @@ def test_layers(ctx, orc, width, degree):
     for solution in (dpg.SOL_BINNED, dpg.SOL_NEARFAR):
         assert np.array_equal(dpg.sssp(ctx, dg, 0, solution=solution), want)
     assert np.array_equal(dpg.bfs(ctx, dg, 0), orc.bfs(g.offsets, g.col, 0))
+
+
+# Warps going on with their own improvements (near-far, small iterations): chains, rings with shortcuts that improve
+# labels late, rows that do not fit beside another in one arc per lane, thresholds that send everything or nothing to
+# the far pile, zero weights. An iteration cap turns it off; the distances are the same.
+@pytest.mark.parametrize("delta", [1, 60, 10**9])
+@pytest.mark.parametrize("degree", [1, 4, 16, 17, 33])
+def test_warps_go_on_with_their_own_improvements(ctx, orc, degree, delta):
+    rng = np.random.default_rng(degree)
+    V = 6000
+    v = np.arange(V)
+    src = np.concatenate([v[:-1], np.repeat(v, degree), [0, 17]])
+    dst = np.concatenate([v[1:], np.clip(np.repeat(v, degree) + rng.integers(-40, 41, V * degree), 0, V - 1), [V - 1, 17]])
+    w = np.concatenate([rng.integers(0, 3, V - 1), rng.integers(0, 90, V * degree), [2000, 0]])
+    g = dpg.csr_from_arcs(V, src, dst, w)
+    dg = dpg.Graph(ctx, g.offsets, g.col, g.weights)
+    for source in (0, 17, V - 1):
+        want = orc.sssp_dijkstra(g.offsets, g.col, g.weights, source)
+        assert np.array_equal(dpg.sssp(ctx, dg, source, solution=dpg.SOL_NEARFAR, delta=delta), want)
+        capped = dpg.sssp(ctx, dg, source, solution=dpg.SOL_NEARFAR, delta=delta, max_iterations=1 << 30)
+        assert np.array_equal(capped, want)
