@@ -791,7 +791,7 @@ __device__ __forceinline__ void local_relax(const ExpandParams& P, const PushCtx
 
 // Scan-based gather: the warp concatenates the rows of the active lanes and relaxes 32 consecutive
 // edges per step, so every step is a coalesced read whatever the per-row degrees are.
-template <class Op, bool kClassify, int CH, bool kLocal = false>
+template <class Op, bool kClassify, int CH, bool kOneSlot = false, bool kLocal = false>
 __device__ __forceinline__ void warp_gather(const ExpandParams& P, const PushCtx& Q, bool act, int s,
                                             int d, typename Op::RV du, int* sx, int* ss,
                                             typename Op::RV* sdu, unsigned long long& edges,
@@ -808,8 +808,9 @@ __device__ __forceinline__ void warp_gather(const ExpandParams& P, const PushCtx
     __syncwarp();
     // Small iterations: at most one arc per lane needs one slot, not U (whose idle slots still issue
     // their loads of arc 0 ahead of the chain). Same box: SSSP 4096^2 grid 53.3 -> 47.0 ms, BFS 1501 x
-    // 2003 grid 12.7 -> 11.7 ms, SSSP R-MAT 14 124 -> 122 us.
-    if (total <= 32) {
+    // 2003 grid 12.7 -> 11.7 ms. Only in the 3-CTA builds: in the 4-CTA build the second inlined
+    // relaxation cost more in spills than it gave (see kWideBlocks).
+    if (kOneSlot && total <= 32) {
         const int k = lane;
         const bool a = k < total;
         int ee = 0;
@@ -1245,8 +1246,8 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                 if (POL == DPG_SOL_THREAD || POL == DPG_SOL_GRID) {
                     serial_rows<Op, kClassify, CH>(P, Q, has, s, d, du);
                 } else if (kBinned) {
-                    warp_gather<Op, kClassify, CH, kNearFar>(P, Q, has, s, d, du, s_excl[warp], s_start[warp], s_du[warp],
-                                                             my_edges, my_pops);
+                    warp_gather<Op, kClassify, CH, MINB == 0, kNearFar>(P, Q, has, s, d, du, s_excl[warp], s_start[warp],
+                                                                        s_du[warp], my_edges, my_pops);
                 } else {
                     const bool big = has && d >= P.threshold;
                     serial_rows<Op, kClassify, CH>(P, Q, has && !big, s, d, du);
