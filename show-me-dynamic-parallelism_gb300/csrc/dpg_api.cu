@@ -541,8 +541,10 @@ dpg_status run_color(dpg_ctx* c, dpg_graph* g, const dpg_expand_opts* in_opts, i
 // is within 5 % of the binned expansion, and 2x is 15-50 % slower.
 constexpr double kNearFarStep = 32.0;
 // Rounds a warp goes on with the vertices it improved before the grid barrier (local_relax in
-// dpg_expand.cu, with the measurements): 5 and 6 are fastest; past that the scanned arcs grow.
-constexpr int32_t kLocalRounds = 5;
+// dpg_expand.cu, with the measurements): for distances 5 and 6 are fastest, past that the scanned
+// arcs grow; levels hardly ever need a second relaxation, and 32 rounds leave little to gain.
+constexpr int32_t kNearFarRounds = 5;
+constexpr int32_t kLevelRounds = 32;
 
 void fill_expand_defaults(const dpg_expand_opts* in, dpg_expand_opts* o, const dpg_graph* g) {
     if (in) *o = *in;
@@ -602,6 +604,9 @@ dpg_status run_expand(dpg_ctx* c, const dpg_graph* g, int32_t source, const dpg_
     L.timeout_ns = static_cast<unsigned long long>(o.timeout_seconds * 1e9);
     L.trace = c->trace;
     L.trace_cap = c->trace_cap;
+    // A caller's own iteration cap counts grid-wide iterations of one round each.
+    if (o.solution == DPG_SOL_NEARFAR || o.solution == DPG_SOL_DIROPT)
+        L.local_rounds = in_opts && in_opts->max_iterations > 0 ? 0 : bfs ? kLevelRounds : kNearFarRounds;
     if (!bfs && o.solution == DPG_SOL_NEARFAR) {
         // Three piles of E + V {vertex, distance} pairs (at most one current entry per vertex, plus
         // stale ones; an overflow stops the solve with DPG_ERR_CAPACITY).
@@ -614,8 +619,6 @@ dpg_status run_expand(dpg_ctx* c, const dpg_graph* g, int32_t source, const dpg_
         L.far_count = cnt;
         L.far_min = reinterpret_cast<int*>(cnt + 4);
         L.far_cap = cap;
-        // A caller's own iteration cap counts grid-wide iterations of one round each.
-        L.local_rounds = in_opts && in_opts->max_iterations > 0 ? 0 : kLocalRounds;
         const double mw = g->mean_weight > 0 ? g->mean_weight : 1.0;
         L.delta = o.delta > 0 ? o.delta : static_cast<int32_t>(std::max(1.0, std::min(1e9, kNearFarStep * mw)));
     }

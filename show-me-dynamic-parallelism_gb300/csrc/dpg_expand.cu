@@ -72,7 +72,7 @@ struct ExpandParams {
     // Multi-source SSSP: non-zero when nsrc is a multiple of 4 and the labels are 16-byte aligned,
     // so a vertex's labels can be read four at a time (relax_mask_vec4).
     int32_t label_vec4;
-    int32_t local_rounds;   // near-far: see local_relax (0: off)
+    int32_t local_rounds;   // near-far and direction-optimizing: see local_relax (0: off)
     uint32_t min_item_log;  // log2 of the fewest small-queue vertices in a warp item (binned kernels)
 };
 
@@ -95,6 +95,7 @@ struct SsspOp {
     static constexpr bool kMask = false;
     static constexpr int min_blocks(int) { return 3; }
     __device__ __forceinline__ static int row_value(const ExpandParams& P, int u, int) { return __ldcg(P.label + u); }
+    __device__ __forceinline__ static int2 arc(const ExpandParams& P, int e) { return __ldg(P.adj + e); }
     __device__ __forceinline__ static void load_edge(const ExpandParams& P, int e, int du, int& v, int& r,
                                                      int& cand) {
         const int2 a = __ldg(P.adj + e);
@@ -128,6 +129,28 @@ struct BfsOp {
     __device__ __forceinline__ static bool want(int, int, int cur) { return cur == DPG_UNDEFINED_LEVEL; }
     __device__ __forceinline__ static bool commit(const ExpandParams& P, int v, int cand) {
         return atomicCAS(P.label + v, DPG_UNDEFINED_LEVEL, cand) == DPG_UNDEFINED_LEVEL;
+    }
+};
+
+// Breadth-first levels as a label-correcting relaxation with unit weights: the operator of the
+// relaxing part of a high-diameter traversal (see kLocalAfter). Any order of relaxations ends at the
+// same levels.
+struct LevelRelaxOp {
+    using RV = int;
+    static constexpr bool kDedup = true;
+    static constexpr bool kPeek = true;
+    static constexpr bool kMask = false;
+    __device__ __forceinline__ static int row_value(const ExpandParams& P, int u, int) { return __ldcg(P.label + u); }
+    __device__ __forceinline__ static int2 arc(const ExpandParams& P, int e) { return make_int2(__ldg(P.col + e), 1); }
+    __device__ __forceinline__ static void load_edge(const ExpandParams& P, int e, int du, int& v, int& r,
+                                                     int& cand) {
+        v = __ldg(P.col + e);
+        r = v;
+        cand = du + 1;
+    }
+    __device__ __forceinline__ static bool want(int, int cand, int cur) { return cand < cur; }
+    __device__ __forceinline__ static bool commit(const ExpandParams& P, int v, int cand) {
+        return cand < atomicMin(P.label + v, cand);
     }
 };
 
@@ -332,6 +355,7 @@ struct PushCtx {
     // Small iterations (latency-bound): each candidate head's row range is loaded with its label
     // peek, so a push needs no further round trip.
     bool early_rows;
+    bool local;  // the warp goes on with its own improvements (local_relax)
     // The warp's push buffer in shared memory (see flush_pushes) and its share of the frontier
     // statistics, added to mf / nf once per iteration.
     int* buf_v;
@@ -704,9 +728,9 @@ __device__ __forceinline__ void serial_rows(const ExpandParams& P, const PushCtx
     for (int t = 0; t < wmax; ++t) relax_one<Op, kClassify, CH>(P, Q, t < dd, s + t, du);
 }
 
-// Near-far, small iterations: the warp relaxes its arcs (one per lane, arc e of a tail with label du)
-// and then goes on with the vertices it improved below the threshold, as long as their arcs fit in
-// one per lane and for at most P.local_rounds rounds, before what is left joins the next frontier.
+// Small iterations of high-diameter graphs: the warp relaxes its arcs (one per lane, arc e of a tail with label du)
+// and then goes on with the vertices it improved (near-far: below the threshold), as long as their
+// arcs fit in one per lane and for at most P.local_rounds rounds, before what is left joins the next frontier.
 // Labels only decrease, and every improvement is relaxed by the warp that made it or by a later pop,
 // so the distances are the same fixed point whatever the order. A round is a warp's own chain of
 // three round trips (the arc with its tail's label, the head's label with its row range, the
@@ -715,10 +739,12 @@ __device__ __forceinline__ void serial_rows(const ExpandParams& P, const PushCtx
 // ahead on stale distances (4096^2 grid, 8 rounds: 7.3 E arcs scanned against 4.5 E). A reduction
 // without a result in the atomic's place, checked against the label a round later, saved no time
 // and scanned 25 % more. Same box, 4096^2 grid: 48.5 ms without, 30.1 / 28.0 / 26.9 / 26.5 / 26.5 /
-// 25.9 ms with 2 / 3 / 4 / 5 / 6 / 8 rounds; 300 x 301 grid 3.04 -> 1.41 ms with 5.
+// 25.9 ms with 2 / 3 / 4 / 5 / 6 / 8 rounds; 300 x 301 grid 3.04 -> 1.41 ms with 5. Breadth-first
+// levels (LevelRelaxOp), where the scanned arcs stay within 0.4 % of E: 4096^2 grid 35.0 -> 14.4 /
+// 12.9 / 11.7 / 11.5 ms with 5 / 8 / 16 / 32 rounds, 1501 x 2003 grid 12.1 -> 5.0 / 4.5 / 4.1 / 4.0.
 // Improvements at or above the threshold are collected in far_buf and appended at the end (26.5 ->
 // 25.7 ms on the 4096^2 grid).
-template <bool kClassify, int CH>
+template <class Op, bool kClassify, int CH>
 __device__ __forceinline__ void local_relax(const ExpandParams& P, const PushCtx& Q, bool act, int e, int du, int* sx,
                                             int* ss, int* sv, unsigned long long& edges, unsigned long long& pops) {
     const int lane = lane_id();
@@ -744,13 +770,13 @@ __device__ __forceinline__ void local_relax(const ExpandParams& P, const PushCtx
     };
     int tail = 0;  // from round 1 on: the arc's tail
     for (int r = 0;; ++r) {
-        const int2 a = __ldg(P.adj + (act ? e : 0));
+        const int2 a = Op::arc(P, act ? e : 0);
         if (r > 0) du = act ? __ldcg(P.label + tail) : 0;
         const int cand = du + a.y;
         const int cur = __ldcg(P.label + a.x);
         const int2 se = make_int2(__ldg(P.off + a.x), __ldg(P.off + a.x + 1));
-        bool ok = act && cand < cur && cand < atomicMin(P.label + a.x, cand);
-        const bool far = ok && cand >= Q.threshold;
+        bool ok = act && Op::want(a.x, cand, cur) && Op::commit(P, a.x, cand);
+        const bool far = Q.far && ok && cand >= Q.threshold;
         const unsigned fm = __ballot_sync(kFullMask, far);
         if (fm) {
             if (far) {
@@ -766,7 +792,7 @@ __device__ __forceinline__ void local_relax(const ExpandParams& P, const PushCtx
         const bool keep = d > 0 && incl <= 32 && r < P.local_rounds;
         bool push[1] = {ok && !keep};
         const int v[1] = {a.x};
-        push_batch<SsspOp, kClassify, CH, 1>(P, Q, push, v, v, &se);
+        push_batch<Op, kClassify, CH, 1>(P, Q, push, v, v, &se);
         const int total = __reduce_max_sync(kFullMask, keep ? incl : 0);
         if (total == 0) break;
         // Kept lanes come first in the scan, so the others' starts lie at or past `total`.
@@ -824,8 +850,8 @@ __device__ __forceinline__ void warp_gather(const ExpandParams& P, const PushCtx
             d1 = sdu[r];
         }
         if constexpr (kLocal) {
-            if (Q.early_rows && P.local_rounds > 0) {
-                local_relax<kClassify, CH>(P, Q, a, ee, d1, sx, ss, sdu, edges, pops);
+            if (Q.local) {
+                local_relax<Op, kClassify, CH>(P, Q, a, ee, d1, sx, ss, sdu, edges, pops);
                 return;
             }
         }
@@ -886,6 +912,12 @@ __device__ __forceinline__ void warp_row(const ExpandParams& P, const PushCtx& Q
 // more CTAs at every barrier, and the spills), so sparse graphs without hubs keep Op::min_blocks.
 constexpr int kWideBlocks = 4;
 
+// Iteration from which a small frontier's warps go on with their own improvements (local_relax). Early
+// small frontiers are no sign of a high diameter: on a uniform random graph (16 M vertices, 8 arcs
+// each, done in 10 breadth-first levels or 38 near-far iterations) mixing the hops of the first
+// iterations scanned 1.7 E instead of 1.0 E with unit weights, 4.2 ms against 2.2.
+constexpr int kLocalAfter = 32;
+
 template <class Op, int POL, int CH = kHubChunk, int MINB = 0>
 __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) expand_kernel(ExpandParams P) {
     using RV = typename Op::RV;
@@ -932,6 +964,7 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
     // picks the faster direction at every level. Every CTA reads the same counters after the
     // barrier, so all make the same choice.
     bool bottom_up = false;
+    bool relaxing = false;  // from here on levels are relaxed in any order (LevelRelaxOp)
     long long unexplored = kDirOpt ? static_cast<long long>(P.E) : 0;
     // Near-far (Davidson, Baxter, Garland, Owens, "Work-Efficient Parallel GPU Methods for
     // Single-Source Shortest Paths", IPDPS 2014): improvements below the threshold form the next
@@ -995,7 +1028,7 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
             if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(P.st, DPG_ERR_CAPACITY, 2);
             break;
         }
-        if (kDirOpt) {
+        if (kDirOpt && !relaxing) {
             const unsigned long long mf = kCtaCounters ? s_mf : read_mf();
             bottom_up = static_cast<long long>(mf) * 4 > unexplored && static_cast<long long>(mf) > P.V;
             unexplored -= static_cast<long long>(mf);
@@ -1025,16 +1058,20 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
         // ms; on the 4096^2 grid, buffering every iteration cost near-far SSSP 11 %.
         const unsigned long long work = static_cast<unsigned long long>(n) + 256ull * nch + (split ? far_n : 0u);
         const bool buffered = work >= kPushBufferWork || (kDirOpt && bottom_up);
+        // A traversal past kLocalAfter iterations with a small frontier is of a high-diameter graph.
+        const bool local = kCtaCounters && !buffered && j >= kLocalAfter && P.local_rounds > 0;
+        if (kDirOpt && local) relaxing = true;
         // Parity selects are written as ternaries so the pointer pairs stay in registers.
         const PushCtx Q = {p ? P.ws.qv[0] : P.ws.qv[1], p ? P.ws.qse[0] : P.ws.qse[1],
                            P.ws.qcount + (j + 1) % 3, p ? P.ws.bmp[0] : P.ws.bmp[1],
                            p ? P.ws.chunks[0] : P.ws.chunks[1], P.ws.ccount + (j + 1) % 3,
                            p ? P.dirty[0] : P.dirty[1], static_cast<unsigned>(j + 1),
-                           kDirOpt ? P.mf + (j + 1) % 3 : nullptr, kDirOpt ? P.nf + (j + 1) % 3 : nullptr,
+                           kDirOpt && !relaxing ? P.mf + (j + 1) % 3 : nullptr,
+                           kDirOpt && !relaxing ? P.nf + (j + 1) % 3 : nullptr,
                            kNearFar ? P.far[split ? (pile + 1) % 3 : pile] : nullptr,
                            kNearFar ? P.far_count + (split ? (pile + 1) % 3 : pile) : nullptr,
                            kNearFar ? P.far_min + (split ? (pile + 1) % 3 : pile) : nullptr, threshold,
-                           !buffered, buffered ? p_v[warp] : nullptr, buffered ? p_se[warp] : nullptr,
+                           !buffered, local, buffered ? p_v[warp] : nullptr, buffered ? p_se[warp] : nullptr,
                            buffered ? &p_n[warp] : nullptr, &p_mf[warp], &p_nf[warp], p_se[warp]};
         const int32_t* qv_cur = p ? P.ws.qv[1] : P.ws.qv[0];
         const int2* qse_cur = p ? P.ws.qse[1] : P.ws.qse[0];
@@ -1200,6 +1237,8 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                 __syncthreads();
             }
         } else {
+            auto run_items = [&](auto op) {
+            using O = decltype(op);
             const unsigned hub_items = kClassify ? nch : 0u;
             const unsigned total_items = hub_items + fchunks;
             for (unsigned item = gwarp; item < total_items; item += nwarps) {
@@ -1207,9 +1246,9 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                     // Grid-wide consolidation: one chunk (<= 256 arcs) of a chunked vertex.
                     const int4 C = __ldcg(chunks_cur + item);
                     const int v0 = C.x, k0 = C.y, k1 = C.z;
-                    const RV du = Op::row_value(P, v0, j);
+                    const RV du = O::row_value(P, v0, j);
                     if (C.w && lane == 0) {
-                        if (Op::kDedup) __stcg(bmp_cur + (v0 >> 5), 0u);
+                        if (O::kDedup) __stcg(bmp_cur + (v0 >> 5), 0u);
                         my_pops += 1;
                     }
                     if (lane == 0) my_edges += static_cast<unsigned long long>(k1 - k0);
@@ -1224,7 +1263,7 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                             act[u] = ee[u] < k1;
                             dd[u] = du;
                         }
-                        relax_batch<Op, kClassify, CH, U>(P, Q, act, ee, dd);
+                        relax_batch<O, kClassify, CH, U>(P, Q, act, ee, dd);
                     }
                     continue;
                 }
@@ -1238,21 +1277,21 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                     const int2 se = __ldcg(qse_cur + i);
                     s = se.x;
                     d = se.y - se.x;
-                    du = Op::row_value(P, u, j);
-                    if (Op::kDedup) __stcg(bmp_cur + (u >> 5), 0u);
+                    du = O::row_value(P, u, j);
+                    if (O::kDedup) __stcg(bmp_cur + (u >> 5), 0u);
                     my_pops += 1;
                     my_edges += static_cast<unsigned long long>(d);
                 }
                 if (POL == DPG_SOL_THREAD || POL == DPG_SOL_GRID) {
-                    serial_rows<Op, kClassify, CH>(P, Q, has, s, d, du);
+                    serial_rows<O, kClassify, CH>(P, Q, has, s, d, du);
                 } else if (kBinned) {
-                    warp_gather<Op, kClassify, CH, MINB == 0, kNearFar>(P, Q, has, s, d, du, s_excl[warp], s_start[warp],
+                    warp_gather<O, kClassify, CH, kCtaCounters, kNearFar || std::is_same<O, LevelRelaxOp>::value>(P, Q, has, s, d, du, s_excl[warp], s_start[warp],
                                                                         s_du[warp], my_edges, my_pops);
                 } else {
                     const bool big = has && d >= P.threshold;
-                    serial_rows<Op, kClassify, CH>(P, Q, has && !big, s, d, du);
+                    serial_rows<O, kClassify, CH>(P, Q, has && !big, s, d, du);
                     if (POL == DPG_SOL_WARP) {
-                        warp_gather<Op, kClassify, CH>(P, Q, big, s, d, du, s_excl[warp], s_start[warp], s_du[warp], my_edges,
+                        warp_gather<O, kClassify, CH>(P, Q, big, s, d, du, s_excl[warp], s_start[warp], s_du[warp], my_edges,
                                                        my_pops);
                     } else {  // DPG_SOL_NAIVE
                         unsigned bigmask = __ballot_sync(kFullMask, big);
@@ -1262,10 +1301,17 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                             const int bs = __shfl_sync(kFullMask, s, src);
                             const int bd = __shfl_sync(kFullMask, d, src);
                             const RV bdu = shfl_rv(du, src);
-                            warp_row<Op, kClassify, CH>(P, Q, bs, bd, bdu);
+                            warp_row<O, kClassify, CH>(P, Q, bs, bd, bdu);
                         }
                     }
                 }
+            }
+            };
+            if constexpr (kDirOpt && kCtaCounters) {
+                if (relaxing) run_items(LevelRelaxOp{});
+                else run_items(Op{});
+            } else {
+                run_items(Op{});
             }
         }
         flush_pushes(P, Q);
@@ -1582,7 +1628,7 @@ cudaError_t launch_expand(const ExpandLaunch& L, const ExpandWorkspace& ws, DevS
     P.nf = diropt ? L.do_nf : nullptr;
     P.E = L.E;
     P.min_item_log = min_item_log(L.V, L.E);
-    P.local_rounds = nearfar ? L.local_rounds : 0;
+    P.local_rounds = L.local_rounds;
     const int classify =
         (L.solution == DPG_SOL_GRID || L.solution == DPG_SOL_BINNED || L.solution == DPG_SOL_DIROPT ||
          L.solution == DPG_SOL_NEARFAR) ? 1 : 0;

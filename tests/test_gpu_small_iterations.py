@@ -57,3 +57,45 @@ def test_warps_go_on_with_their_own_improvements(ctx, orc, degree, delta):
         assert np.array_equal(dpg.sssp(ctx, dg, source, solution=dpg.SOL_NEARFAR, delta=delta), want)
         capped = dpg.sssp(ctx, dg, source, solution=dpg.SOL_NEARFAR, delta=delta, max_iterations=1 << 30)
         assert np.array_equal(capped, want)
+
+
+def _chain_then(tail: str, seed: int):
+    """A chain of 100 levels with side branches and back arcs (past the iteration from which levels are relaxed in any
+    order), then a grid (long paths of differing length) or a random graph whose frontier grows large."""
+    rng = np.random.default_rng(seed)
+    n = 100
+    src, dst = [np.arange(n)], [np.arange(1, n + 1)]
+    if tail == "grid":
+        rows, cols = 60, 211
+        s, d, _ = dpg.grid_arcs(rows, cols, 1)
+        keep = rng.random(s.size) < 0.85  # holes: shortest paths bend, some vertices are unreachable
+        s, d, V = s[keep] + n, d[keep] + n, n + rows * cols
+    else:
+        V = n + 150_000
+        s, d = rng.integers(n, V, 6 * 150_000), rng.integers(n, V, 6 * 150_000)
+    back = rng.integers(0, n, 50)
+    src += [s, back, back, [n]]
+    dst += [d, np.maximum(back - rng.integers(0, 9, 50), 0), n + rng.integers(0, 20, 50), [n]]
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    return dpg.csr_from_arcs(V, src, dst, rng.integers(0, 9, src.size))
+
+
+@pytest.mark.parametrize("tail", ["grid", "random"])
+@pytest.mark.parametrize("seed", range(4))
+def test_levels_of_long_graphs(ctx, orc, tail, seed):
+    g = _chain_then(tail, seed)
+    dg = dpg.Graph(ctx, g.offsets, g.col, g.weights)
+    for source in (0, 50, 99):
+        want = orc.bfs(g.offsets, g.col, source)
+        assert np.array_equal(dpg.bfs(ctx, dg, source), want)
+        assert np.array_equal(dpg.bfs(ctx, dg, source, max_iterations=1 << 30), want)
+        assert np.array_equal(dpg.sssp(ctx, dg, source), orc.sssp_dijkstra(g.offsets, g.col, g.weights, source))
+
+
+def test_iteration_cap_still_counts_levels(ctx):
+    g = dpg.csr_from_arcs(301, np.arange(300), np.arange(1, 301), np.ones(300))
+    dg = dpg.Graph(ctx, g.offsets, g.col, g.weights)
+    with pytest.raises(dpg.DpgError):
+        dpg.bfs(ctx, dg, 0, max_iterations=200)
+    assert np.array_equal(dpg.bfs(ctx, dg, 0, max_iterations=302), np.arange(301))
+    assert np.array_equal(dpg.bfs(ctx, dg, 0), np.arange(301))
