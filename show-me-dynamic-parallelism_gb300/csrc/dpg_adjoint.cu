@@ -2,15 +2,15 @@
 //
 // No counterpart in the reference (its SpMV, apps/SpMV/src/SpMV_kernel.cu:81-96, multiplies one
 // vector). With nrhs columns stored row-major ([V][nrhs] FP32), every nonzero touches whole rows of
-// 4 * nrhs bytes, so a warp reads each gathered row with coalesced loads (lane j holds columns
-// j, j+32, ...). Rows are cut on the host into items of at most kSpmmSegment nonzeros; items of a
-// split row write partial rows that a fix-up adds in segment order, so sums have a fixed order.
-//   spmm_rows_kernel      Y[row] = sum over the item's nonzeros of val * X[col]   (Y = A X, and
-//                         dX = A^T G when run over the transposed CSR with permuted values)
-//   arc_dot_kernel        dA[e] = <G[row], X[col(e)]>, the warp holding G[row] in registers
-// With nrhs a multiple of 32 and 16-byte aligned row blocks, the group kernels below take over:
-//   spmm_group_kernel     Y = A X with float4 rows split over 8-lane groups
-//   spmv_bwd_group_kernel dX and dA in one pass over the transposed CSR
+// 4 * nrhs bytes.
+//   rows_kernel           Y[row] = sum over the row's nonzeros of val * X[col] (Y = A X), or, over the
+//                         transposed CSR, both gradients in one pass (dX = A^T G and dA). Takes nrhs
+//                         a multiple of 4 with 16-byte aligned row blocks, and any nrhs up to 32.
+//   spmm_rows_kernel      Y = A X for the other shapes, a warp per row
+//   arc_dot_kernel        dA[e] = <G[row], X[col(e)]> for the other shapes
+// Rows of more than kGroupRow nonzeros are listed in a plan (built on the device) as items of at most
+// kSpmmSegment nonzeros; a row of several items writes partial rows that a fix-up adds in segment
+// order. The others are read straight from the offsets. Every sum has a fixed order.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,17 +32,28 @@ __device__ __forceinline__ void load_row(const float* __restrict__ M, int64_t r,
     }
 }
 
-// One warp per item {row, arc begin, arc end, segment or -1}; 4 nonzeros in flight.
+// The warp's k-th job of a plan: the listed items first, then the rows of at most kGroupRow nonzeros
+// (a longer row reads as empty with row -1: its items were listed).
+__device__ __forceinline__ int4 plan_job(const SpmmPlanDev& P, int64_t k) {
+    if (k < P.nitems) return __ldg(P.items + k);
+    const int v = static_cast<int>(k - P.nitems);
+    const int b = __ldg(P.off + v), e = __ldg(P.off + v + 1);
+    return e - b > kGroupRow ? make_int4(-1, 0, 0, -1) : make_int4(v, b, e, -1);
+}
+
+// One warp per job {row, arc begin, arc end, segment or -1}; 4 nonzeros in flight.
 template <int NV>
-__global__ void __launch_bounds__(kBlock) spmm_rows_kernel(const int4* __restrict__ items, int nitems,
+__global__ void __launch_bounds__(kBlock) spmm_rows_kernel(SpmmPlanDev P,
                                                            const int32_t* __restrict__ col, const float* __restrict__ val,
                                                            const float* __restrict__ X, int nrhs, float* __restrict__ Y,
                                                            float* __restrict__ partial) {
     const int lane = threadIdx.x & 31;
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int it = w; it < nitems; it += nw) {
-        const int4 I = __ldg(items + it);
+    const int64_t njobs = static_cast<int64_t>(P.nitems) + P.V;
+    for (int64_t k = w; k < njobs; k += nw) {
+        const int4 I = plan_job(P, k);
+        if (I.x < 0) continue;
         float acc[NV];
 #pragma unroll
         for (int q = 0; q < NV; ++q) acc[q] = 0.0f;
@@ -93,11 +104,15 @@ __global__ void __launch_bounds__(kBlock) spmm_fixup_kernel(const int4* __restri
         float acc[NV];
 #pragma unroll
         for (int q = 0; q < NV; ++q) acc[q] = 0.0f;
-        for (int s = 0; s < H.z; ++s) {
-            float pv[NV];
-            load_row<NV>(partial, H.y + s, nrhs, lane, pv);
+        for (int s0 = 0; s0 < H.z; s0 += 8) {  // 8 partial rows in flight, added in segment order
+            float pv[8][NV];
 #pragma unroll
-            for (int q = 0; q < NV; ++q) acc[q] += pv[q];
+            for (int u = 0; u < 8; ++u) load_row<NV>(partial, H.y + min(s0 + u, H.z - 1), nrhs, lane, pv[u]);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int q = 0; q < NV; ++q)
+                    if (s0 + u < H.z) acc[q] += pv[u][q];
         }
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
@@ -109,14 +124,16 @@ __global__ void __launch_bounds__(kBlock) spmm_fixup_kernel(const int4* __restri
 
 // dA[e] = <G[row], X[col(e)]> for the item's arcs; the warp keeps G[row] in registers.
 template <int NV>
-__global__ void __launch_bounds__(kBlock) arc_dot_kernel(const int4* __restrict__ items, int nitems,
+__global__ void __launch_bounds__(kBlock) arc_dot_kernel(SpmmPlanDev P,
                                                          const int32_t* __restrict__ col, const float* __restrict__ X,
                                                          const float* __restrict__ G, int nrhs, float* __restrict__ dA) {
     const int lane = threadIdx.x & 31;
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int it = w; it < nitems; it += nw) {
-        const int4 I = __ldg(items + it);
+    const int64_t njobs = static_cast<int64_t>(P.nitems) + P.V;
+    for (int64_t k = w; k < njobs; k += nw) {
+        const int4 I = plan_job(P, k);
+        if (I.x < 0) continue;
         float g[NV];
         load_row<NV>(G, I.x, nrhs, lane, g);
         int e = I.y;
@@ -150,20 +167,6 @@ __global__ void __launch_bounds__(kBlock) arc_dot_kernel(const int4* __restrict_
     }
 }
 
-// One right-hand side: dA[e] = G[row] * X[col(e)], lanes across the item's arcs (coalesced).
-__global__ void __launch_bounds__(kBlock) arc_dot1_kernel(const int4* __restrict__ items, int nitems,
-                                                          const int32_t* __restrict__ col, const float* __restrict__ X,
-                                                          const float* __restrict__ G, float* __restrict__ dA) {
-    const int lane = threadIdx.x & 31;
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int it = w; it < nitems; it += nw) {
-        const int4 I = __ldg(items + it);
-        const float g = __ldg(G + I.x);
-        for (int e = I.y + lane; e < I.z; e += 32) dA[e] = g * __ldg(X + __ldg(col + e));
-    }
-}
-
 __global__ void gather_values_kernel(const float* __restrict__ v, const int32_t* __restrict__ idx, int64_t n,
                                      float* __restrict__ out) {
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -171,185 +174,255 @@ __global__ void gather_values_kernel(const float* __restrict__ v, const int32_t*
         out[i] = __ldg(v + __ldg(idx + i));
 }
 
-// ---- group kernels: nrhs a multiple of 32, rows 16-byte aligned --------------------------------------
-// A warp is 4 groups of 8 lanes; a group holds one row of nrhs = 32 * QPL floats as QPL float4 per
-// lane (lane l of the group holds float4 l, l + 8, ...), so each of its loads is 8 consecutive
-// float4 of one row. The 4 groups take 4 different arcs of the warp's item, each group kGroupU
-// arcs deep, so a warp keeps 4 * kGroupU gathered rows in flight. Each group sums its arcs in arc
-// order; the 4 group partials are combined by a fixed butterfly, so sums keep a fixed order.
-#ifndef DPG_GROUP_U
-#define DPG_GROUP_U 4
-#endif
-constexpr int kGroupU = DPG_GROUP_U;
+// ---- rows in groups of lanes -----------------------------------------------------------------------
+// A gathered row of nrhs floats is Q vectors of VEC floats (float4, or single floats for widths and
+// alignments that do not allow it), one per lane of LQ lanes (the power of two from Q up). A group of
+// GL = max(8, LQ) lanes works through rows of its own (at most kGroupRow nonzeros), with 8 / LQ arcs
+// side by side when LQ < 8, A arcs per step, and moves to its next row in the step after the last
+// arc, whatever the other groups do. The indexes of the next step and the offsets of the next row are
+// loaded one step ahead, so a step costs one round trip (the gathered rows). The listed items of
+// longer rows are taken by whole warps, the groups interleaved.
+// Summation order: a lane adds its arcs in order; the groups' (and side-by-side arcs') sums meet in a
+// fixed butterfly.
+struct RowsLaunch {
+    SpmmPlanDev P;
+    const int32_t* col;   // row of `in` that each arc gathers
+    const int32_t* arc;   // backward: index of each arc in val and dA
+    const float* val;
+    const float* in;      // gathered matrix (X, or G for the backward)
+    const float* X;       // backward: dA = <gathered row, X[own row]>
+    int nrhs;
+    float* out;           // Y or dX; null: skip (backward)
+    float* partial;
+    float* dA;            // backward; null: skip
+};
 
-__device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+template <int VEC>
+struct RowVec;
+template <>
+struct RowVec<4> {
+    float4 v;
+    __device__ __forceinline__ static RowVec zero() { return {make_float4(0.f, 0.f, 0.f, 0.f)}; }
+    // Zero unless `on`: one predicated load. As a conditional expression it became a branch whose
+    // zeroing side waited for the loads in flight of the other lanes (R-MAT 22 x 64 backward: 8.5 -> 6.3
+    // ms, with two vectors per lane).
+    __device__ __forceinline__ static RowVec load_if(bool on, const float* p) {
+        RowVec r = zero();
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+            : "+f"(r.v.x), "+f"(r.v.y), "+f"(r.v.z), "+f"(r.v.w) : "l"(p), "r"(static_cast<int>(on)));
+        return r;
+    }
+    __device__ __forceinline__ void store(float* p) const { *reinterpret_cast<float4*>(p) = v; }
+    __device__ __forceinline__ void fma(float a, const RowVec& x) {
+        v.x = fmaf(a, x.v.x, v.x);
+        v.y = fmaf(a, x.v.y, v.y);
+        v.z = fmaf(a, x.v.z, v.z);
+        v.w = fmaf(a, x.v.w, v.w);
+    }
+    __device__ __forceinline__ float dot(const RowVec& x, float d) const {
+        return fmaf(v.w, x.v.w, fmaf(v.z, x.v.z, fmaf(v.y, x.v.y, fmaf(v.x, x.v.x, d))));
+    }
+    __device__ __forceinline__ void add_xor(int m) {
+        v.x += __shfl_xor_sync(kFullMask, v.x, m);
+        v.y += __shfl_xor_sync(kFullMask, v.y, m);
+        v.z += __shfl_xor_sync(kFullMask, v.z, m);
+        v.w += __shfl_xor_sync(kFullMask, v.w, m);
+    }
+};
+template <>
+struct RowVec<1> {
+    float v;
+    __device__ __forceinline__ static RowVec zero() { return {0.f}; }
+    __device__ __forceinline__ static RowVec load_if(bool on, const float* p) {
+        RowVec r = zero();
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+            : "+f"(r.v) : "l"(p), "r"(static_cast<int>(on)));
+        return r;
+    }
+    __device__ __forceinline__ void store(float* p) const { *p = v; }
+    __device__ __forceinline__ void fma(float a, const RowVec& x) { v = fmaf(a, x.v, v); }
+    __device__ __forceinline__ float dot(const RowVec& x, float d) const { return fmaf(v, x.v, d); }
+    __device__ __forceinline__ void add_xor(int m) { v += __shfl_xor_sync(kFullMask, v, m); }
+};
 
-__device__ __forceinline__ void fma4(float4& acc, float a, const float4& x) {
-    acc.x = fmaf(a, x.x, acc.x);
-    acc.y = fmaf(a, x.y, acc.y);
-    acc.z = fmaf(a, x.z, acc.z);
-    acc.w = fmaf(a, x.w, acc.w);
-}
+// CTAs per SM the kernel is compiled for and launched with.
+// Measured on the same box against the kernels before it (a warp per row: a chain of three dependent
+// loads for every row, most of which have fewer than 4 arcs; float4 rows for multiples of 32 only):
+//   Y = A X, 200,003 rows x 16, 20 columns 185 -> 70 us; R-MAT 20 x 1 / 3 / 64 / 100 / 128 columns
+//   678 -> 118, 682 -> 147, 830 -> 631, 1284 -> 1024, 1385 -> 1056 us
+//   backward, 237,987 rows x 32, 1 / 20 columns 445 -> 119, 949 -> 233 us; R-MAT 20 x 32 / 96 columns
+//   997 -> 866, 1851 -> 1711 us; R-MAT 22 x 64 columns 5.78 -> 5.63 ms
+// Gathered vectors in flight per lane and CTAs per SM: 8 vectors, or 3 or 5 CTAs, were slower on most
+// of these (backward R-MAT 22 x 64: 6.0 ms with 8, 6.3 with 3 or 5). More vectors per lane and 8-lane
+// groups for the wide rows (fewer shuffles) were slower too: 6.3 ms, and 1.66 against 1.06 ms for Y = A X
+// with 128 columns.
+constexpr int kRowLoads = 4;
+constexpr int rows_blocks(int vec) { return vec == 1 ? 5 : 4; }
 
-__device__ __forceinline__ float4 shfl_xor4(const float4& v, int m) {
-    return make_float4(__shfl_xor_sync(kFullMask, v.x, m), __shfl_xor_sync(kFullMask, v.y, m),
-                       __shfl_xor_sync(kFullMask, v.z, m), __shfl_xor_sync(kFullMask, v.w, m));
-}
-
-__device__ __forceinline__ void add4(float4& a, const float4& b) {
-    a.x += b.x;
-    a.y += b.y;
-    a.z += b.z;
-    a.w += b.w;
-}
-
-// Y[row] = sum over the item's arcs of val * X[col].
-template <int QPL>
-__global__ void __launch_bounds__(kBlock) spmm_group_kernel(const int4* __restrict__ items, int nitems,
-                                                            const int32_t* __restrict__ col,
-                                                            const float* __restrict__ val,
-                                                            const float* __restrict__ X, int nrhs,
-                                                            float* __restrict__ Y, float* __restrict__ partial) {
-    const int lane = threadIdx.x & 31;
-    const int grp = lane >> 3;
-    const int gl = lane & 7;
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int it = w; it < nitems; it += nw) {
-        const int4 I = __ldg(items + it);
-        float4 acc[QPL];
+// Arc positions are unsigned: near 2^31 nonzeros a step may reach past INT32_MAX.
+// Indexes of one step of a group: lane l holds arcs p + l, p + 8 + l, ... (zero past the end).
+template <int R, bool BWD>
+struct StepIdx {
+    int c[R];
+    int a[R];    // backward: arc
+    float w[R];  // forward: value
+    __device__ __forceinline__ void load(const RowsLaunch& L, unsigned p, unsigned e, int gl) {
 #pragma unroll
-        for (int q = 0; q < QPL; ++q) acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int base = I.y; base < I.z; base += 4 * kGroupU) {
-            int c[kGroupU];
-            float a[kGroupU];
-            bool act[kGroupU];
-#pragma unroll
-            for (int u = 0; u < kGroupU; ++u) {
-                const int t = base + 4 * u + grp;
-                act[u] = t < I.z;
-                c[u] = act[u] ? __ldg(col + t) : 0;
-                a[u] = act[u] ? __ldg(val + t) : 0.0f;
-            }
-            // Slots past the item's end hold zeros (not 0 x a row, which an Inf would turn into NaN).
-            float4 x[kGroupU][QPL];
-#pragma unroll
-            for (int u = 0; u < kGroupU; ++u)
-#pragma unroll
-                for (int q = 0; q < QPL; ++q)
-                    x[u][q] = act[u] ? ld4(X + static_cast<int64_t>(c[u]) * nrhs + 4 * (gl + 8 * q))
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int u = 0; u < kGroupU; ++u)
-#pragma unroll
-                for (int q = 0; q < QPL; ++q) fma4(acc[q], a[u], x[u][q]);
-        }
-#pragma unroll
-        for (int q = 0; q < QPL; ++q) {
-            add4(acc[q], shfl_xor4(acc[q], 8));
-            add4(acc[q], shfl_xor4(acc[q], 16));
-        }
-        if (grp == 0) {
-            float* dst = I.w < 0 ? Y + static_cast<int64_t>(I.x) * nrhs : partial + static_cast<int64_t>(I.w) * nrhs;
-#pragma unroll
-            for (int q = 0; q < QPL; ++q) *reinterpret_cast<float4*>(dst + 4 * (gl + 8 * q)) = acc[q];
+        for (int r = 0; r < R; ++r) {
+            const unsigned t = p + 8 * r + gl;
+            const bool in = t < e;
+            c[r] = in ? __ldg(L.col + t) : 0;
+            if (BWD) a[r] = in ? __ldg(L.arc + t) : 0;
+            else w[r] = in ? __ldg(L.val + t) : 0.0f;
         }
     }
-}
+};
 
-// The adjoint in one pass over the transposed CSR (item = column j of A): G[i] is gathered once per
-// arc i -> j and serves both dX[j] += val * G[i] and dA[arc] = <G[i], X[j]>, with X[j] held in
-// registers (every group holds it). The dot product of an arc is summed by its group (lane-local
-// float4 parts, then a 3-step butterfly) and written by the group's first lane. dX or dA may be
-// skipped (null). Measured on R-MAT 22 with 64 right-hand sides: 5.6 ms against 7.55 ms for the
-// two general kernels (row gather over the transpose, then an arc pass gathering X as well), and
-// 9.3 ms for two group kernels doing the same two passes. CTAs per SM: with 64 right-hand sides
-// (QPL = 2) the kernel takes 80 registers unbounded (3 CTAs); bounded to 4 CTAs (64 registers,
-// 128 bytes of spills) the call went from 5.57 to 5.30 ms on the same box. The other widths keep
-// what they take unbounded (47, 106 and 128 registers).
-template <int QPL>
-__global__ void __launch_bounds__(kBlock, QPL == 1 ? 5 : QPL == 2 ? 4 : 2) spmv_bwd_group_kernel(const int4* __restrict__ items, int nitems,
-                                                                const int32_t* __restrict__ tcol,
-                                                                const int32_t* __restrict__ tarc,
-                                                                const float* __restrict__ val,
-                                                                const float* __restrict__ X,
-                                                                const float* __restrict__ G, int nrhs,
-                                                                float* __restrict__ dX, float* __restrict__ partial,
-                                                                float* __restrict__ dA) {
+template <int VEC, int LQ, bool BWD>
+__global__ void __launch_bounds__(kBlock, rows_blocks(VEC)) rows_kernel(RowsLaunch L) {
+    using V = RowVec<VEC>;
+    constexpr int GL = LQ < 8 ? 8 : LQ;                 // lanes of a group
+    constexpr int NG = 32 / GL;                         // groups of a warp
+    constexpr int AP = LQ < 8 ? 8 / LQ : 1;             // arcs side by side in a group
+    constexpr int NB = 8 / AP;                          // batches of AP arcs in 8 arcs
+    constexpr int R = LQ == 1 ? 4 : LQ == 2 ? 2 : 1;    // index loads per lane and step
+    constexpr int A = 8 * R;                            // arcs per step
+    constexpr int HB = NB < kRowLoads ? NB : kRowLoads;  // gathered vectors in flight per lane
     const int lane = threadIdx.x & 31;
-    const int grp = lane >> 3;
-    const int gl = lane & 7;
+    const int grp = lane / GL, gl = lane & 7, gbase = grp * GL;  // gl: the arc of 8 whose indexes the lane loads
+    const int q0 = lane % LQ, sub = (lane % GL) / LQ;
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int it = w; it < nitems; it += nw) {
-        const int4 I = __ldg(items + it);
-        float4 xj[QPL], acc[QPL];
+    const bool live = q0 < L.nrhs / VEC;
+    V acc, xj;
+
+    auto load_own = [&](int row, bool any) {  // backward: X[row], of a row that has arcs
+        if (!BWD) return;
+        xj = V::load_if(any && L.dA && live, L.X + static_cast<int64_t>(row) * L.nrhs + VEC * q0);
+    };
+    // The arcs [p, min(p + A, e)) of the group.
+    auto step = [&](unsigned p, unsigned e, const StepIdx<R, BWD>& I) {
 #pragma unroll
-        for (int q = 0; q < QPL; ++q) {
-            xj[q] = dA ? ld4(X + static_cast<int64_t>(I.x) * nrhs + 4 * (gl + 8 * q)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        for (int base = I.y; base < I.z; base += 4 * kGroupU) {
-            int r[kGroupU], e[kGroupU];
-            bool act[kGroupU];
+        for (int r = 0; r < R; ++r) {
+            float wv = 0.0f;
+            if (BWD) wv = p + 8 * r + gl < e ? __ldg(L.val + I.a[r]) : 0.0f;
+            else wv = I.w[r];
+            float d[NB];
 #pragma unroll
-            for (int u = 0; u < kGroupU; ++u) {
-                const int t = base + 4 * u + grp;
-                act[u] = t < I.z;
-                r[u] = act[u] ? __ldg(tcol + t) : 0;
-                e[u] = act[u] ? __ldg(tarc + t) : 0;
+            for (int h = 0; h < NB; h += HB) {
+                // Slots past the end load nothing and hold zeros, value and row (an Inf in a row that
+                // no arc touches must not reach 0 * Inf).
+                V x[HB];
+#pragma unroll
+                for (int i = 0; i < HB; ++i) {
+                    const int u = (h + i) * AP + sub;
+                    const int row = __shfl_sync(kFullMask, I.c[r], gbase + u);
+                    const bool in = p + 8 * r + u < e;
+                    x[i] = V::load_if(in && live, L.in + static_cast<int64_t>(row) * L.nrhs + VEC * q0);
+                }
+#pragma unroll
+                for (int i = 0; i < HB; ++i) {
+                    const int u = (h + i) * AP + sub;
+                    const float a = __shfl_sync(kFullMask, wv, gbase + u);
+                    acc.fma(a, x[i]);
+                    if (BWD) d[h + i] = x[i].dot(xj, 0.0f);
+                }
             }
-            float a[kGroupU];
+            if (BWD && L.dA) {
+                // Sum of each arc's dot over its LQ lanes: every exchange halves the arcs a lane still
+                // holds, down to one, whose sum the lanes left then complete.
+                int batch = 0;
 #pragma unroll
-            for (int u = 0; u < kGroupU; ++u) a[u] = act[u] ? __ldg(val + e[u]) : 0.0f;
-            float4 gr[kGroupU][QPL];
+                for (int m = LQ / 2, n = NB / 2; m > 0; m >>= 1, n >>= 1) {
+                    if (n > 0) {
+                        const bool up = (q0 & m) != 0;
+                        if (up) batch += n;
 #pragma unroll
-            for (int u = 0; u < kGroupU; ++u)
-#pragma unroll
-                for (int q = 0; q < QPL; ++q)
-                    gr[u][q] = act[u] ? ld4(G + static_cast<int64_t>(r[u]) * nrhs + 4 * (gl + 8 * q))
-                                      : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (dX) {
-#pragma unroll
-                for (int u = 0; u < kGroupU; ++u)
-#pragma unroll
-                    for (int q = 0; q < QPL; ++q) fma4(acc[q], a[u], gr[u][q]);
-            }
-            if (dA) {
-                float d[kGroupU];
-#pragma unroll
-                for (int u = 0; u < kGroupU; ++u) {
-                    d[u] = 0.0f;
-#pragma unroll
-                    for (int q = 0; q < QPL; ++q) {
-                        d[u] = fmaf(gr[u][q].x, xj[q].x, d[u]);
-                        d[u] = fmaf(gr[u][q].y, xj[q].y, d[u]);
-                        d[u] = fmaf(gr[u][q].z, xj[q].z, d[u]);
-                        d[u] = fmaf(gr[u][q].w, xj[q].w, d[u]);
+                        for (int k = 0; k < n; ++k) {
+                            const float send = up ? d[k] : d[k + n];
+                            const float keep = up ? d[k + n] : d[k];
+                            d[k] = keep + __shfl_xor_sync(kFullMask, send, m);
+                        }
+                    } else {
+                        d[0] += __shfl_xor_sync(kFullMask, d[0], m);
                     }
                 }
-#pragma unroll
-                for (int m = 4; m > 0; m >>= 1)
-#pragma unroll
-                    for (int u = 0; u < kGroupU; ++u) d[u] += __shfl_xor_sync(kFullMask, d[u], m);
-                if (gl == 0) {
-#pragma unroll
-                    for (int u = 0; u < kGroupU; ++u)
-                        if (act[u]) dA[e[u]] = d[u];
-                }
+                const int u = batch * AP + sub;
+                const int arc = __shfl_sync(kFullMask, I.a[r], gbase + u);
+                if (p + 8 * r + u < e && (LQ <= NB || q0 % (LQ / NB) == 0)) L.dA[arc] = d[0];
             }
         }
-        if (!dX) continue;
-#pragma unroll
-        for (int q = 0; q < QPL; ++q) {
-            add4(acc[q], shfl_xor4(acc[q], 8));
-            add4(acc[q], shfl_xor4(acc[q], 16));
+    };
+
+    // Listed items, a warp each.
+    for (int it = w; it < L.P.nitems; it += nw) {
+        const int4 I = __ldg(L.P.items + it);
+        acc = V::zero();
+        load_own(I.x, true);
+        StepIdx<R, BWD> cur, nxt;
+        const unsigned end = I.z;
+        cur.load(L, I.y + grp * A, end, gl);
+        for (unsigned base = I.y; base < end; base += NG * A) {
+            nxt.load(L, base + (NG + grp) * A, end, gl);
+            step(base + grp * A, end, cur);
+            cur = nxt;
         }
-        if (grp == 0) {
-            float* dst = I.w < 0 ? dX + static_cast<int64_t>(I.x) * nrhs : partial + static_cast<int64_t>(I.w) * nrhs;
+        if (!L.out) continue;
 #pragma unroll
-            for (int q = 0; q < QPL; ++q) *reinterpret_cast<float4*>(dst + 4 * (gl + 8 * q)) = acc[q];
+        for (int m = LQ; m < 32; m <<= 1) acc.add_xor(m);
+        if (grp == 0 && sub == 0 && live)
+            acc.store((I.w < 0 ? L.out + static_cast<int64_t>(I.x) * L.nrhs
+                               : L.partial + static_cast<int64_t>(I.w) * L.nrhs) + VEC * q0);
+    }
+
+    // The other rows, a group each. A listed row reads as empty and is not stored.
+    const int64_t ngroups = static_cast<int64_t>(nw) * NG;
+    auto range = [&](int64_t v, unsigned& b, unsigned& e, bool& mine) {
+        mine = v < L.P.V;
+        b = mine ? __ldg(L.P.off + v) : 0;
+        e = mine ? __ldg(L.P.off + v + 1) : 0;
+        if (e - b > kGroupRow) {
+            e = b;
+            mine = false;
         }
+    };
+    int64_t v = static_cast<int64_t>(w) * NG + grp;
+    unsigned p, e, nb, ne;
+    bool mine, nmine;
+    range(v, p, e, mine);
+    range(v + ngroups, nb, ne, nmine);
+    StepIdx<R, BWD> cur, nxt;
+    cur.load(L, p, e, gl);
+    acc = V::zero();
+    load_own(static_cast<int>(v), mine && p < e);
+    while (__any_sync(kFullMask, v < L.P.V)) {
+        const bool last = p + A >= e;
+        nxt.load(L, last ? nb : p + A, last ? ne : e, gl);
+        unsigned nnb = 0, nne = 0;
+        bool nnmine = false;
+        if (last) range(v + 2 * ngroups, nnb, nne, nnmine);
+        step(p, e, cur);
+        if (AP > 1 && __any_sync(kFullMask, last)) {
+            V t = acc;
+#pragma unroll
+            for (int m = LQ; m < 8; m <<= 1) t.add_xor(m);
+            if (last) acc = t;
+        }
+        if (last) {
+            if (mine && L.out && sub == 0 && live) acc.store(L.out + v * L.nrhs + VEC * q0);
+            v += ngroups;
+            p = nb;
+            e = ne;
+            mine = nmine;
+            nb = nnb;
+            ne = nne;
+            nmine = nnmine;
+            acc = V::zero();
+            load_own(static_cast<int>(v), mine && p < e);
+        } else {
+            p += A;
+        }
+        cur = nxt;
     }
 }
 
@@ -358,7 +431,7 @@ cudaError_t run_spmm(const SpmmPlanDev& P, const int32_t* col, const float* val,
                      float* partial, cudaStream_t s, int sm_count, LaunchHook* hook) {
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, s);
-        if (P.nitems > 0) spmm_rows_kernel<NV><<<sm_count * 8, kBlock, 0, s>>>(P.items, P.nitems, col, val, X, nrhs, Y, partial);
+        spmm_rows_kernel<NV><<<sm_count * 8, kBlock, 0, s>>>(P, col, val, X, nrhs, Y, partial);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || P.nhubs == 0) return e;
@@ -373,30 +446,61 @@ template <int NV>
 cudaError_t run_arc_dot(const SpmmPlanDev& P, const int32_t* col, const float* X, const float* G, int nrhs, float* dA,
                         cudaStream_t s, int sm_count, LaunchHook* hook) {
     HookScope hs(hook, DPG_KERNEL_ROWGATHER, s);
-    if (P.nitems > 0) arc_dot_kernel<NV><<<sm_count * 8, kBlock, 0, s>>>(P.items, P.nitems, col, X, G, nrhs, dA);
+    arc_dot_kernel<NV><<<sm_count * 8, kBlock, 0, s>>>(P, col, X, G, nrhs, dA);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-void build_spmm_plan(const int32_t* off, int32_t V, SpmmPlanHost* plan) {
-    plan->items.clear();
-    plan->hubs.clear();
-    plan->nseg = 0;
-    for (int32_t r = 0; r < V; ++r) {
-        const int32_t b = off[r], e = off[r + 1];
-        if (e - b <= kSpmmSegment) {
-            plan->items.push_back(make_int4(r, b, e, -1));
-            continue;
+namespace {
+
+// Rows of more than kGroupRow nonzeros into the item list, the whole warp writing one row's segments
+// at a time. Positions come from atomics: the order of the lists changes nothing in the results.
+__global__ void __launch_bounds__(kBlock) spmm_plan_kernel(const int32_t* __restrict__ off, int32_t V, int4* items,
+                                                           int4* hubs, int32_t* counts) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t v0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; v0 < V; v0 += stride) {
+        const int64_t v = v0 + lane;
+        const int b = v < V ? __ldg(off + v) : 0;
+        const int e = v < V ? __ldg(off + v + 1) : 0;
+        const int d = e - b;
+        const int n = d > kGroupRow ? (d + kSpmmSegment - 1) / kSpmmSegment : 0;
+        int pos = 0, seg = -1;
+        if (n > 0) pos = atomicAdd(counts, n);
+        if (n > 1) {
+            seg = atomicAdd(counts + 2, n);
+            hubs[atomicAdd(counts + 1, 1)] = make_int4(static_cast<int>(v), seg, n, 0);
         }
-        const int32_t nseg = (e - b + kSpmmSegment - 1) / kSpmmSegment;
-        plan->hubs.push_back(make_int4(r, plan->nseg, nseg, 0));
-        for (int32_t k = 0; k < nseg; ++k) {
-            const int32_t sb = b + k * kSpmmSegment;
-            plan->items.push_back(make_int4(r, sb, std::min(e, sb + kSpmmSegment), plan->nseg + k));
+        unsigned m = __ballot_sync(kFullMask, n > 0);
+        while (m) {
+            const int src = __ffs(m) - 1;
+            m &= m - 1u;
+            const int rb = __shfl_sync(kFullMask, b, src), re = __shfl_sync(kFullMask, e, src);
+            const int rn = __shfl_sync(kFullMask, n, src), rp = __shfl_sync(kFullMask, pos, src);
+            const int rs = __shfl_sync(kFullMask, seg, src);
+            for (int k = lane; k < rn; k += 32) {
+                const int sb = rb + k * kSpmmSegment;
+                items[rp + k] = make_int4(static_cast<int>(v0) + src, sb, min(re, sb + kSpmmSegment), rs < 0 ? -1 : rs + k);
+            }
         }
-        plan->nseg += nseg;
     }
+}
+
+}  // namespace
+
+// A listed row of d nonzeros has ceil(d / kSpmmSegment) <= d / kSpmmSegment + 1 items.
+int64_t spmm_plan_max_items(int64_t E) { return E / kSpmmSegment + E / (kGroupRow + 1) + 1; }
+int64_t spmm_plan_max_hubs(int64_t E) { return E / (kSpmmSegment + 1) + 1; }
+
+cudaError_t launch_spmm_plan(const int32_t* off, int32_t V, int4* items, int4* hubs, int32_t* counts, cudaStream_t s,
+                             int sm_count) {
+    const cudaError_t e = cudaMemsetAsync(counts, 0, 3 * sizeof(int32_t), s);
+    if (e != cudaSuccess || V <= 0) return e;
+    const int64_t blocks = (static_cast<int64_t>(V) + kBlock - 1) / kBlock;
+    spmm_plan_kernel<<<static_cast<int>(std::min<int64_t>(blocks, sm_count * 8)), kBlock, 0, s>>>(off, V, items, hubs,
+                                                                                                  counts);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_spmm(const SpmmPlanDev& P, const int32_t* col, const float* val, const float* X, int nrhs, float* Y,
@@ -408,18 +512,14 @@ cudaError_t launch_spmm(const SpmmPlanDev& P, const int32_t* col, const float* v
 
 cudaError_t launch_arc_dot(const SpmmPlanDev& P, const int32_t* col, const float* X, const float* G, int nrhs,
                            float* dA, cudaStream_t s, int sm_count, LaunchHook* hook) {
-    if (nrhs == 1) {
-        HookScope hs(hook, DPG_KERNEL_ROWGATHER, s);
-        if (P.nitems > 0) arc_dot1_kernel<<<sm_count * 8, kBlock, 0, s>>>(P.items, P.nitems, col, X, G, dA);
-        return cudaGetLastError();
-    }
     if (nrhs <= 32) return run_arc_dot<1>(P, col, X, G, nrhs, dA, s, sm_count, hook);
     if (nrhs <= 64) return run_arc_dot<2>(P, col, X, G, nrhs, dA, s, sm_count, hook);
     return run_arc_dot<4>(P, col, X, G, nrhs, dA, s, sm_count, hook);
 }
 
-bool spmm_group_ok(int nrhs, const void* a, const void* b, const void* c, const void* d) {
-    if (nrhs % 32 != 0 || nrhs > 128) return false;
+bool spmm_rows_ok(int nrhs, const void* a, const void* b, const void* c, const void* d) {
+    if (nrhs <= 32) return true;
+    if (nrhs % 4 != 0 || nrhs > 128) return false;
     for (const void* p : {a, b, c, d})
         if (p && reinterpret_cast<uintptr_t>(p) % 16 != 0) return false;
     return true;
@@ -427,63 +527,58 @@ bool spmm_group_ok(int nrhs, const void* a, const void* b, const void* c, const 
 
 namespace {
 
-template <int QPL>
-cudaError_t run_spmm_group(const SpmmPlanDev& P, const int32_t* col, const float* val, const float* X, int nrhs,
-                           float* Y, float* partial, cudaStream_t s, int sm_count, LaunchHook* hook) {
+template <int VEC, int LQ, bool BWD>
+cudaError_t run_rows(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHook* hook) {
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, s);
-        if (P.nitems > 0)
-            spmm_group_kernel<QPL><<<sm_count * 8, kBlock, 0, s>>>(P.items, P.nitems, col, val, X, nrhs, Y, partial);
+        const int64_t need = std::max((static_cast<int64_t>(L.P.V) + 31) / 32, (static_cast<int64_t>(L.P.nitems) + 7) / 8);
+        const int grid = static_cast<int>(std::min<int64_t>(need, static_cast<int64_t>(sm_count) * rows_blocks(VEC)));
+        rows_kernel<VEC, LQ, BWD><<<grid, kBlock, 0, s>>>(L);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || P.nhubs == 0) return e;
-    {
-        HookScope hs(hook, DPG_KERNEL_FIXUP, s);
-        spmm_fixup_kernel<QPL><<<sm_count * 4, kBlock, 0, s>>>(P.hubs, P.nhubs, partial, nrhs, Y);
-    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || L.P.nhubs == 0 || !L.out) return e;
+    HookScope hs(hook, DPG_KERNEL_FIXUP, s);
+    if (L.nrhs <= 32) spmm_fixup_kernel<1><<<sm_count * 4, kBlock, 0, s>>>(L.P.hubs, L.P.nhubs, L.partial, L.nrhs, L.out);
+    else if (L.nrhs <= 64)
+        spmm_fixup_kernel<2><<<sm_count * 4, kBlock, 0, s>>>(L.P.hubs, L.P.nhubs, L.partial, L.nrhs, L.out);
+    else spmm_fixup_kernel<4><<<sm_count * 4, kBlock, 0, s>>>(L.P.hubs, L.P.nhubs, L.partial, L.nrhs, L.out);
     return cudaGetLastError();
 }
 
-template <int QPL>
-cudaError_t run_bwd_group(const SpmmPlanDev& TP, const int32_t* tcol, const int32_t* tarc, const float* val,
-                          const float* X, const float* G, int nrhs, float* dX, float* partial, float* dA,
-                          cudaStream_t s, int sm_count, LaunchHook* hook) {
-    {
-        HookScope hs(hook, DPG_KERNEL_ROWGATHER, s);
-        if (TP.nitems > 0)
-            spmv_bwd_group_kernel<QPL><<<sm_count * 8, kBlock, 0, s>>>(TP.items, TP.nitems, tcol, tarc, val, X, G,
-                                                                       nrhs, dX, partial, dA);
-    }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || TP.nhubs == 0 || !dX) return e;
-    {
-        HookScope hs(hook, DPG_KERNEL_FIXUP, s);
-        spmm_fixup_kernel<QPL><<<sm_count * 4, kBlock, 0, s>>>(TP.hubs, TP.nhubs, partial, nrhs, dX);
-    }
-    return cudaGetLastError();
+template <int VEC, bool BWD>
+cudaError_t pick_rows(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHook* hook) {
+    const int Q = L.nrhs / VEC;
+    if (Q <= 1) return run_rows<VEC, 1, BWD>(L, s, sm_count, hook);
+    if (Q <= 2) return run_rows<VEC, 2, BWD>(L, s, sm_count, hook);
+    if (Q <= 4) return run_rows<VEC, 4, BWD>(L, s, sm_count, hook);
+    if (Q <= 8) return run_rows<VEC, 8, BWD>(L, s, sm_count, hook);
+    if (Q <= 16) return run_rows<VEC, 16, BWD>(L, s, sm_count, hook);
+    return run_rows<VEC, 32, BWD>(L, s, sm_count, hook);
+}
+
+template <bool BWD>
+cudaError_t pick_vec(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHook* hook) {
+    if (L.P.V <= 0) return cudaSuccess;
+    bool vec4 = L.nrhs % 4 == 0;
+    for (const void* p : {static_cast<const void*>(L.in), static_cast<const void*>(L.X), static_cast<const void*>(L.out),
+                          static_cast<const void*>(L.partial)})
+        vec4 = vec4 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
+    return vec4 ? pick_rows<4, BWD>(L, s, sm_count, hook) : pick_rows<1, BWD>(L, s, sm_count, hook);
 }
 
 }  // namespace
 
 cudaError_t launch_spmm_group(const SpmmPlanDev& P, const int32_t* col, const float* val, const float* X, int nrhs,
                               float* Y, float* partial, cudaStream_t s, int sm_count, LaunchHook* hook) {
-    switch (nrhs / 32) {
-        case 1: return run_spmm_group<1>(P, col, val, X, nrhs, Y, partial, s, sm_count, hook);
-        case 2: return run_spmm_group<2>(P, col, val, X, nrhs, Y, partial, s, sm_count, hook);
-        case 3: return run_spmm_group<3>(P, col, val, X, nrhs, Y, partial, s, sm_count, hook);
-        default: return run_spmm_group<4>(P, col, val, X, nrhs, Y, partial, s, sm_count, hook);
-    }
+    const RowsLaunch L = {P, col, nullptr, val, X, nullptr, nrhs, Y, partial, nullptr};
+    return pick_vec<false>(L, s, sm_count, hook);
 }
 
 cudaError_t launch_spmv_bwd_group(const SpmmPlanDev& TP, const int32_t* tcol, const int32_t* tarc, const float* val,
                                   const float* X, const float* G, int nrhs, float* dX, float* partial, float* dA,
                                   cudaStream_t s, int sm_count, LaunchHook* hook) {
-    switch (nrhs / 32) {
-        case 1: return run_bwd_group<1>(TP, tcol, tarc, val, X, G, nrhs, dX, partial, dA, s, sm_count, hook);
-        case 2: return run_bwd_group<2>(TP, tcol, tarc, val, X, G, nrhs, dX, partial, dA, s, sm_count, hook);
-        case 3: return run_bwd_group<3>(TP, tcol, tarc, val, X, G, nrhs, dX, partial, dA, s, sm_count, hook);
-        default: return run_bwd_group<4>(TP, tcol, tarc, val, X, G, nrhs, dX, partial, dA, s, sm_count, hook);
-    }
+    const RowsLaunch L = {TP, tcol, tarc, val, G, X, nrhs, dX, partial, dA};
+    return pick_vec<true>(L, s, sm_count, hook);
 }
 
 cudaError_t launch_gather_values(const float* v, const int32_t* idx, int64_t n, float* out, cudaStream_t s,

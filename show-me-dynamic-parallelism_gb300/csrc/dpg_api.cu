@@ -199,9 +199,10 @@ void graph_free_device(dpg_graph* g) {
         dev_free(g->ctx, p->hubs);
         *p = SpmmPlanDev();
     }
+    dev_free(g->ctx, g->tt_off);
     dev_free(g->ctx, g->tt_col);
     dev_free(g->ctx, g->tt_arc);
-    g->tt_col = g->tt_arc = nullptr;
+    g->tt_off = g->tt_col = g->tt_arc = nullptr;
     g->spmm_ready = g->spmm_t_ready = false;
     g->relabel_ready = false;
     dev_free(g->ctx, g->plan.tiles);
@@ -372,69 +373,66 @@ dpg_status ensure_relabel(dpg_graph* g) {
     return DPG_OK;
 }
 
-dpg_status upload_spmm_plan(dpg_ctx* c, const SpmmPlanHost& hp, SpmmPlanDev* d) {
-    d->nitems = static_cast<int32_t>(hp.items.size());
-    d->nhubs = static_cast<int32_t>(hp.hubs.size());
-    d->nseg = hp.nseg;
-    DPG_CUDA_TRY(dev_alloc(c, &d->items, sizeof(int4) * (hp.items.size() + 1)));
-    DPG_CUDA_TRY(dev_alloc(c, &d->hubs, sizeof(int4) * (hp.hubs.size() + 1)));
-    if (!hp.items.empty())
-        DPG_CUDA_TRY(cudaMemcpyAsync(d->items, hp.items.data(), sizeof(int4) * hp.items.size(), cudaMemcpyHostToDevice,
-                                     c->stream));
-    if (!hp.hubs.empty())
-        DPG_CUDA_TRY(cudaMemcpyAsync(d->hubs, hp.hubs.data(), sizeof(int4) * hp.hubs.size(), cudaMemcpyHostToDevice,
-                                     c->stream));
-    DPG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+// The batched-RHS plan of a CSR on the device: built there into buffers of the sizes that bound it.
+dpg_status build_spmm_plan(dpg_ctx* c, const int32_t* off, int32_t V, int64_t E, SpmmPlanDev* out) {
+    SpmmPlanDev d;
+    d.off = off;
+    d.V = V;
+    dpg_status st = DPG_OK;
+    int32_t* counts = static_cast<int32_t*>(arena(c, S_SPMM_COUNTS, 3 * sizeof(int32_t), &st));
+    if (st != DPG_OK) return st;
+    int32_t h[3] = {0, 0, 0};
+    cudaError_t e = dev_alloc(c, &d.items, sizeof(int4) * static_cast<size_t>(spmm_plan_max_items(E)));
+    if (e == cudaSuccess) e = dev_alloc(c, &d.hubs, sizeof(int4) * static_cast<size_t>(spmm_plan_max_hubs(E)));
+    if (e == cudaSuccess) e = launch_spmm_plan(off, V, d.items, d.hubs, counts, c->stream, c->sm_count);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, counts, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) {
+        dev_free(c, d.items);
+        dev_free(c, d.hubs);
+        return set_error(DPG_ERR_CUDA, std::string("batched-RHS plan: ") + cudaGetErrorString(e));
+    }
+    d.nitems = h[0];
+    d.nhubs = h[1];
+    d.nseg = h[2];
+    *out = d;
     return DPG_OK;
 }
 
 dpg_status ensure_spmm_plan(dpg_graph* g) {
     if (g->spmm_ready) return DPG_OK;
-    SpmmPlanHost hp;
-    build_spmm_plan(g->h_off.data(), g->V, &hp);
-    DPG_TRY(upload_spmm_plan(g->ctx, hp, &g->spmm_plan));
+    DPG_TRY(build_spmm_plan(g->ctx, g->off, g->V, g->E, &g->spmm_plan));
     g->spmm_ready = true;
     return DPG_OK;
 }
 
 // Deterministic transposed CSR with the arc permutation, built on the device in invertGraph order
-// (dpg_transpose.cu); only its offsets come back to the host, for the batched-RHS plan. With
-// need_graph the transposed CSR also becomes a graph of its own (g->tgraph).
+// (dpg_transpose.cu), and its batched-RHS plan. With need_graph the transposed CSR also becomes a
+// graph of its own (g->tgraph).
 dpg_status ensure_spmm_transpose(dpg_graph* g, bool need_graph = false) {
-    if (g->spmm_t_ready && (!need_graph || g->tgraph)) return DPG_OK;
     dpg_ctx* c = g->ctx;
-    const size_t nv = static_cast<size_t>(g->V), ne = static_cast<size_t>(g->E > 0 ? g->E : 1);
-    int32_t* t_off = nullptr;
-    DPG_CUDA_TRY(dev_alloc(c, &t_off, (nv + 1) * 4));
-    cudaError_t e = cudaSuccess;
-    if (!g->tt_col) e = dev_alloc(c, &g->tt_col, ne * 4);
-    if (e == cudaSuccess && !g->tt_arc) e = dev_alloc(c, &g->tt_arc, ne * 4);
-    dpg_status st = DPG_OK;
-    const size_t scratch_bytes = transpose_scratch_bytes(g->V, g->E);
-    void* scratch = e == cudaSuccess ? arena(c, S_TRANSPOSE, scratch_bytes, &st) : nullptr;
-    if (e == cudaSuccess && st == DPG_OK)
-        e = launch_transpose(g->off, g->col, g->V, g->E, t_off, g->tt_col, g->tt_arc, scratch, scratch_bytes,
-                             c->stream, c->sm_count);
-    std::vector<int32_t> h_t_off(nv + 1);
-    if (e == cudaSuccess && st == DPG_OK)
-        e = cudaMemcpyAsync(h_t_off.data(), t_off, (nv + 1) * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess && st == DPG_OK) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess || st != DPG_OK) {
-        dev_free(c, t_off);
-        return st != DPG_OK ? st : set_error(DPG_ERR_CUDA, std::string("device transpose: ") + cudaGetErrorString(e));
-    }
     if (!g->spmm_t_ready) {
-        SpmmPlanHost hp;
-        build_spmm_plan(h_t_off.data(), g->V, &hp);
-        st = upload_spmm_plan(c, hp, &g->spmm_t_plan);
-        if (st == DPG_OK) g->spmm_t_ready = true;
+        const size_t nv = static_cast<size_t>(g->V), ne = static_cast<size_t>(g->E > 0 ? g->E : 1);
+        cudaError_t e = cudaSuccess;
+        if (!g->tt_off) e = dev_alloc(c, &g->tt_off, (nv + 1) * 4);
+        if (e == cudaSuccess && !g->tt_col) e = dev_alloc(c, &g->tt_col, ne * 4);
+        if (e == cudaSuccess && !g->tt_arc) e = dev_alloc(c, &g->tt_arc, ne * 4);
+        dpg_status st = DPG_OK;
+        const size_t scratch_bytes = transpose_scratch_bytes(g->V, g->E);
+        void* scratch = e == cudaSuccess ? arena(c, S_TRANSPOSE, scratch_bytes, &st) : nullptr;
+        if (e == cudaSuccess && st == DPG_OK)
+            e = launch_transpose(g->off, g->col, g->V, g->E, g->tt_off, g->tt_col, g->tt_arc, scratch, scratch_bytes,
+                                 c->stream, c->sm_count);
+        if (st != DPG_OK) return st;
+        if (e != cudaSuccess) return set_error(DPG_ERR_CUDA, std::string("device transpose: ") + cudaGetErrorString(e));
+        DPG_TRY(build_spmm_plan(c, g->tt_off, g->V, g->E, &g->spmm_t_plan));
+        g->spmm_t_ready = true;
     }
-    if (st == DPG_OK && need_graph && !g->tgraph) {
-        st = graph_create_common(c, g->V, g->E, t_off, g->tt_col, nullptr, true, &g->tgraph);
-        if (st == DPG_OK) g->tgraph->relabel = g->relabel;
+    if (need_graph && !g->tgraph) {
+        DPG_TRY(graph_create_common(c, g->V, g->E, g->tt_off, g->tt_col, nullptr, true, &g->tgraph));
+        g->tgraph->relabel = g->relabel;
     }
-    dev_free(c, t_off);
-    return st;
+    return DPG_OK;
 }
 
 dpg_status check_nrhs(int32_t nrhs) {
@@ -1446,7 +1444,7 @@ dpg_status dpg_spmm_f32_dev(dpg_ctx* c, const dpg_graph* gc, const float* d_vals
         arena(c, S_SPMM_PARTIAL, static_cast<size_t>(g->spmm_plan.nseg + 1) * nrhs * 4, &st));
     if (st != DPG_OK) return st;
     c->last_host_iterations = 1;
-    if (spmm_group_ok(nrhs, d_X, d_Y, partial, nullptr))
+    if (spmm_rows_ok(nrhs, d_X, d_Y, partial, nullptr))
         DPG_CUDA_TRY(launch_spmm_group(g->spmm_plan, g->col, d_vals, d_X, nrhs, d_Y, partial, c->stream, c->sm_count,
                                        &c->prof));
     else
@@ -1464,15 +1462,13 @@ dpg_status dpg_spmv_bwd_f32_dev(dpg_ctx* c, const dpg_graph* gc, const float* d_
     if (g->V == 0) return DPG_OK;
     if (!d_G || (d_dA && !d_X) || (g->E > 0 && !d_vals)) return set_error(DPG_ERR_INVALID_ARG, "null vals/X/G");
     c->last_host_iterations = 1;
-    if (spmm_group_ok(nrhs, d_X, d_G, d_dX, nullptr) && (d_dX || d_dA)) {
+    if (spmm_rows_ok(nrhs, d_X, d_G, d_dX, nullptr) && (d_dX || d_dA)) {
         // Both outputs in one pass over the transposed CSR: each arc's row of G is gathered once.
         DPG_TRY(ensure_spmm_transpose(g));
         dpg_status st = DPG_OK;
         float* partial = static_cast<float*>(
             arena(c, S_SPMM_PARTIAL, static_cast<size_t>(g->spmm_t_plan.nseg + 1) * nrhs * 4, &st));
         if (st != DPG_OK) return st;
-        if (!spmm_group_ok(nrhs, partial, nullptr, nullptr, nullptr))
-            return set_error(DPG_ERR_CUDA, "misaligned workspace");
         DPG_CUDA_TRY(launch_spmv_bwd_group(g->spmm_t_plan, g->tt_col, g->tt_arc, d_vals, d_X, d_G, nrhs, d_dX, partial,
                                            d_dA, c->stream, c->sm_count, &c->prof));
         return DPG_OK;

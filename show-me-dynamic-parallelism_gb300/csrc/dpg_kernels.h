@@ -191,25 +191,28 @@ struct RowGatherLaunch {
 };
 
 // ---- batched right-hand sides / SpMV adjoint (dpg_adjoint.cu) -----------------------------------
-constexpr int kSpmmSegment = 512;  // nonzeros per item; longer rows are split and fixed up in order
+constexpr int kSpmmSegment = 512;  // nonzeros per listed item; longer rows are split and fixed up in order
+constexpr int kGroupRow = 64;      // rows of more nonzeros are listed
 
-// Items {row, arc begin, arc end, segment index or -1}; hubs {row, first segment, segments, 0}.
-struct SpmmPlanHost {
-    std::vector<int4> items;
-    std::vector<int4> hubs;
-    int32_t nseg = 0;
-};
+// Items {row, arc begin, arc end, segment index or -1} of the rows of more than kGroupRow nonzeros, in
+// no particular order; hubs {row, first segment, segments, 0}. The other rows are read from off[V+1].
 struct SpmmPlanDev {
+    const int32_t* off = nullptr;
+    int32_t V = 0;
     int4* items = nullptr;
     int32_t nitems = 0;
     int4* hubs = nullptr;
     int32_t nhubs = 0;
     int32_t nseg = 0;
 };
-void build_spmm_plan(const int32_t* off, int32_t V, SpmmPlanHost* plan);
-// The group kernels (8 lanes per row piece, float4 loads) take nrhs a multiple of 32 (up to 128)
-// and 16-byte aligned row blocks; spmm_group_ok says whether the given pointers qualify.
-bool spmm_group_ok(int nrhs, const void* a, const void* b, const void* c, const void* d);
+// Upper bounds of the items and hubs of any CSR of E nonzeros.
+int64_t spmm_plan_max_items(int64_t E);
+int64_t spmm_plan_max_hubs(int64_t E);
+// Fills items and hubs (capacities as above); counts[0..2] receive the items, hubs and segments.
+cudaError_t launch_spmm_plan(const int32_t* off, int32_t V, int4* items, int4* hubs, int32_t* counts, cudaStream_t s,
+                             int sm_count);
+// Whether rows_kernel takes this width and these row blocks (null: not used).
+bool spmm_rows_ok(int nrhs, const void* a, const void* b, const void* c, const void* d);
 cudaError_t launch_spmm_group(const SpmmPlanDev& P, const int32_t* col, const float* val, const float* X, int nrhs,
                               float* Y, float* partial, cudaStream_t s, int sm_count, LaunchHook* hook);
 // One pass over the transposed CSR (plan TP, columns tcol, arc permutation tarc): dX = A^T G and

@@ -84,22 +84,28 @@ __global__ void __launch_bounds__(kBlock) pr_vec_kernel(PrVecLaunch L) {
     }
 }
 
-// dL/dw[e] for the item's arcs e = (u -> col[e]); lanes across arcs.
-__global__ void __launch_bounds__(kBlock) pr_arc_grad_kernel(const int4* __restrict__ items, int nitems,
-                                                             const int32_t* __restrict__ col, const float* __restrict__ r,
-                                                             const float* __restrict__ W, const float* __restrict__ y,
-                                                             const float* __restrict__ lam, float damping,
-                                                             float* __restrict__ grad) {
+// dL/dw[e] of the arcs e = (u -> col[e]): the listed items a warp each, the other rows 8 lanes each.
+__global__ void __launch_bounds__(kBlock) pr_arc_grad_kernel(SpmmPlanDev P, const int32_t* __restrict__ col,
+                                                             const float* __restrict__ r, const float* __restrict__ W,
+                                                             const float* __restrict__ y, const float* __restrict__ lam,
+                                                             float damping, float* __restrict__ grad) {
     const int lane = threadIdx.x & 31;
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int it = w; it < nitems; it += nw) {
-        const int4 I = __ldg(items + it);
-        const float Wu = __ldg(W + I.x);
+    auto arcs = [&](int u, int b, int e, int first, int step) {
+        const float Wu = __ldg(W + u);
         // A row with arcs and W == 0 (all weights zero) is dangling: its arcs get no gradient.
-        const float c = Wu > 0.0f ? damping * __ldg(r + I.x) / Wu : 0.0f;
-        const float q = Wu > 0.0f ? __ldg(y + I.x) / Wu : 0.0f;
-        for (int e = I.y + lane; e < I.z; e += 32) grad[e] = c * (__ldg(lam + __ldg(col + e)) - q);
+        const float c = Wu > 0.0f ? damping * __ldg(r + u) / Wu : 0.0f;
+        const float q = Wu > 0.0f ? __ldg(y + u) / Wu : 0.0f;
+        for (int k = b + first; k < e; k += step) grad[k] = c * (__ldg(lam + __ldg(col + k)) - q);
+    };
+    for (int it = w; it < P.nitems; it += nw) {
+        const int4 I = __ldg(P.items + it);
+        arcs(I.x, I.y, I.z, lane, 32);
+    }
+    for (int64_t u = static_cast<int64_t>(w) * 4 + (lane >> 3); u < P.V; u += static_cast<int64_t>(nw) * 4) {
+        const int b = __ldg(P.off + u), e = __ldg(P.off + u + 1);
+        if (e > b && e - b <= kGroupRow) arcs(static_cast<int>(u), b, e, lane & 7, 8);
     }
 }
 
@@ -123,8 +129,7 @@ cudaError_t launch_pr_arc_grad(const SpmmPlanDev& P, const int32_t* col, const f
                                const float* lam, float damping, float* grad, cudaStream_t s, int sm_count,
                                LaunchHook* hook) {
     HookScope hs(hook, DPG_KERNEL_ROWGATHER, s);
-    if (P.nitems > 0)
-        pr_arc_grad_kernel<<<sm_count * 8, kBlock, 0, s>>>(P.items, P.nitems, col, r, W, y, lam, damping, grad);
+    pr_arc_grad_kernel<<<sm_count * 8, kBlock, 0, s>>>(P, col, r, W, y, lam, damping, grad);
     return cudaGetLastError();
 }
 
