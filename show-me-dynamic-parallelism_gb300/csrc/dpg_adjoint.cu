@@ -187,15 +187,16 @@ __global__ void gather_values_kernel(const float* __restrict__ v, const int32_t*
 struct RowsLaunch {
     SpmmPlanDev P;
     const int32_t* col;   // row of `in` that each arc gathers
-    const int32_t* arc;   // backward: index of each arc in val and dA
-    const float* val;
+    const int32_t* arc;   // kBwdArcs: index of each arc in val and dA
+    const float* val;     // (kForward, kBwdSlots: in the order of col)
     const float* in;      // gathered matrix (X, or G for the backward)
     const float* X;       // backward: dA = <gathered row, X[own row]>
     int nrhs;
     float* out;           // Y or dX; null: skip (backward)
     float* partial;
-    float* dA;            // backward; null: skip
+    float* dA;            // backward; null: skip (kBwdSlots: in the order of col)
 };
+enum RowsMode { kForward, kBwdArcs, kBwdSlots };
 
 template <int VEC>
 struct RowVec;
@@ -261,26 +262,27 @@ constexpr int rows_blocks(int vec) { return vec == 1 ? 5 : 4; }
 
 // Arc positions are unsigned: near 2^31 nonzeros a step may reach past INT32_MAX.
 // Indexes of one step of a group: lane l holds arcs p + l, p + 8 + l, ... (zero past the end).
-template <int R, bool BWD>
+template <int R, int MODE>
 struct StepIdx {
     int c[R];
-    int a[R];    // backward: arc
-    float w[R];  // forward: value
+    int a[R];    // kBwdArcs: arc
+    float w[R];  // else: value
     __device__ __forceinline__ void load(const RowsLaunch& L, unsigned p, unsigned e, int gl) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const unsigned t = p + 8 * r + gl;
             const bool in = t < e;
             c[r] = in ? __ldg(L.col + t) : 0;
-            if (BWD) a[r] = in ? __ldg(L.arc + t) : 0;
+            if (MODE == kBwdArcs) a[r] = in ? __ldg(L.arc + t) : 0;
             else w[r] = in ? __ldg(L.val + t) : 0.0f;
         }
     }
 };
 
-template <int VEC, int LQ, bool BWD>
+template <int VEC, int LQ, int MODE>
 __global__ void __launch_bounds__(kBlock, rows_blocks(VEC)) rows_kernel(RowsLaunch L) {
     using V = RowVec<VEC>;
+    constexpr bool BWD = MODE != kForward;
     constexpr int GL = LQ < 8 ? 8 : LQ;                 // lanes of a group
     constexpr int NG = 32 / GL;                         // groups of a warp
     constexpr int AP = LQ < 8 ? 8 / LQ : 1;             // arcs side by side in a group
@@ -301,11 +303,11 @@ __global__ void __launch_bounds__(kBlock, rows_blocks(VEC)) rows_kernel(RowsLaun
         xj = V::load_if(any && L.dA && live, L.X + static_cast<int64_t>(row) * L.nrhs + VEC * q0);
     };
     // The arcs [p, min(p + A, e)) of the group.
-    auto step = [&](unsigned p, unsigned e, const StepIdx<R, BWD>& I) {
+    auto step = [&](unsigned p, unsigned e, const StepIdx<R, MODE>& I) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             float wv = 0.0f;
-            if (BWD) wv = p + 8 * r + gl < e ? __ldg(L.val + I.a[r]) : 0.0f;
+            if (MODE == kBwdArcs) wv = p + 8 * r + gl < e ? __ldg(L.val + I.a[r]) : 0.0f;
             else wv = I.w[r];
             float d[NB];
 #pragma unroll
@@ -348,7 +350,8 @@ __global__ void __launch_bounds__(kBlock, rows_blocks(VEC)) rows_kernel(RowsLaun
                     }
                 }
                 const int u = batch * AP + sub;
-                const int arc = __shfl_sync(kFullMask, I.a[r], gbase + u);
+                unsigned arc = p + 8 * r + u;
+                if (MODE == kBwdArcs) arc = __shfl_sync(kFullMask, I.a[r], gbase + u);
                 if (p + 8 * r + u < e && (LQ <= NB || q0 % (LQ / NB) == 0)) L.dA[arc] = d[0];
             }
         }
@@ -359,7 +362,7 @@ __global__ void __launch_bounds__(kBlock, rows_blocks(VEC)) rows_kernel(RowsLaun
         const int4 I = __ldg(L.P.items + it);
         acc = V::zero();
         load_own(I.x, true);
-        StepIdx<R, BWD> cur, nxt;
+        StepIdx<R, MODE> cur, nxt;
         const unsigned end = I.z;
         cur.load(L, I.y + grp * A, end, gl);
         for (unsigned base = I.y; base < end; base += NG * A) {
@@ -391,7 +394,7 @@ __global__ void __launch_bounds__(kBlock, rows_blocks(VEC)) rows_kernel(RowsLaun
     bool mine, nmine;
     range(v, p, e, mine);
     range(v + ngroups, nb, ne, nmine);
-    StepIdx<R, BWD> cur, nxt;
+    StepIdx<R, MODE> cur, nxt;
     cur.load(L, p, e, gl);
     acc = V::zero();
     load_own(static_cast<int>(v), mine && p < e);
@@ -423,6 +426,175 @@ __global__ void __launch_bounds__(kBlock, rows_blocks(VEC)) rows_kernel(RowsLaun
             p += A;
         }
         cur = nxt;
+    }
+}
+
+// ---- arc values between CSR order and transposed order -----------------------------------------------
+// A permutation of E values in two passes over blocks of kPermBlock that fit in shared memory, every
+// global access a run: arcs are cut into chunks and transposed slots into buckets of kPermBlock each,
+// and a middle order holds the values by bucket, then chunk. Position i of a chunk (in middle order)
+// is arc arc_in[i] of the chunk and middle position mid[i]; middle position t of a bucket is slot
+// slot_in[t] of the bucket. The chunk pass moves runs of about kPermBlock^2 / E values to or from the
+// middle order, the bucket pass whole blocks. What it replaces: one random 4-byte access per arc, a
+// DRAM line each (45 G/s): the 64-column backward of R-MAT 22 took 5.6 ms with its value reads and
+// gradient writes at random, of which the pass itself is 3.2 ms. Permuting through windows of slots
+// that fit in L2 (one pass, random writes there) took 1.0 ms per permutation, this 0.69 ms; the call
+// went from 5.65 to 4.62 ms (same box).
+constexpr int kPermThreads = 1024;
+
+// slot_of[arc] = transposed slot.
+__global__ void __launch_bounds__(kBlock) invert_kernel(const int32_t* __restrict__ arc, int64_t E, int32_t* slot_of) {
+    for (int64_t p = static_cast<int64_t>(blockIdx.x) * kBlock + threadIdx.x; p < E;
+         p += static_cast<int64_t>(gridDim.x) * kBlock)
+        slot_of[__ldg(arc + p)] = static_cast<int32_t>(p);
+}
+
+// counts[bucket][chunk]: arcs of the chunk whose slot lies in the bucket.
+__global__ void __launch_bounds__(kPermThreads) perm_count_kernel(const int32_t* __restrict__ slot_of, int64_t E,
+                                                                  int nblk, int32_t* __restrict__ counts) {
+    extern __shared__ int s_n[];
+    for (int c = blockIdx.x; c < nblk; c += gridDim.x) {
+        for (int i = threadIdx.x; i < nblk; i += kPermThreads) s_n[i] = 0;
+        __syncthreads();
+        const int64_t e0 = static_cast<int64_t>(c) * kPermBlock;
+        const int n = static_cast<int>(E - e0 < kPermBlock ? E - e0 : kPermBlock);
+        for (int i = threadIdx.x; i < n; i += kPermThreads) atomicAdd(s_n + __ldg(slot_of + e0 + i) / kPermBlock, 1);
+        __syncthreads();
+        for (int i = threadIdx.x; i < nblk; i += kPermThreads) counts[static_cast<int64_t>(i) * nblk + c] = s_n[i];
+        __syncthreads();
+    }
+}
+
+// Sum over the block's threads before this one (kPermThreads threads).
+__device__ __forceinline__ int block_exclusive(int v, int* s_warp) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int incl = warp_inclusive_scan(v);
+    __syncthreads();
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int before = 0;
+    for (int w = 0; w < warp; ++w) before += s_warp[w];
+    return before + incl - v;
+}
+
+// counts[bucket][chunk] becomes the middle position of the run's first value: a bucket's slots fill it
+// exactly, so each row is scanned on its own from bucket * kPermBlock.
+__global__ void __launch_bounds__(kPermThreads) perm_scan_kernel(int nblk, int32_t* __restrict__ counts) {
+    __shared__ int s_warp[32];
+    for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+        int32_t* row = counts + static_cast<int64_t>(b) * nblk;
+        const int per = (nblk + kPermThreads - 1) / kPermThreads;
+        const int lo = min(nblk, static_cast<int>(threadIdx.x) * per), hi = min(nblk, lo + per);
+        int sum = 0;
+        for (int i = lo; i < hi; ++i) sum += row[i];
+        int64_t run = static_cast<int64_t>(b) * kPermBlock + block_exclusive(sum, s_warp);
+        for (int i = lo; i < hi; ++i) {
+            const int v = row[i];
+            row[i] = static_cast<int32_t>(run);
+            run += v;
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kPermThreads) perm_place_kernel(const int32_t* __restrict__ slot_of, int64_t E,
+                                                                  int nblk, const int32_t* __restrict__ starts,
+                                                                  int32_t* __restrict__ mid,
+                                                                  uint16_t* __restrict__ arc_in,
+                                                                  uint16_t* __restrict__ slot_in) {
+    extern __shared__ int s_n[];
+    int* s_first = s_n;         // middle position of the chunk's run in each bucket
+    int* s_next = s_n + nblk;   // next free one
+    __shared__ int s_warp[32];
+    for (int c = blockIdx.x; c < nblk; c += gridDim.x) {
+        const int64_t e0 = static_cast<int64_t>(c) * kPermBlock;
+        const int n = static_cast<int>(E - e0 < kPermBlock ? E - e0 : kPermBlock);
+        // Run lengths again (the starts of the next chunk are those of this one plus its length, but
+        // the last chunk has no next), then each run's first position in the chunk.
+        for (int i = threadIdx.x; i < nblk; i += kPermThreads) s_next[i] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += kPermThreads) atomicAdd(s_next + __ldg(slot_of + e0 + i) / kPermBlock, 1);
+        __syncthreads();
+        const int per = (nblk + kPermThreads - 1) / kPermThreads;
+        const int lo = min(nblk, static_cast<int>(threadIdx.x) * per), hi = min(nblk, lo + per);
+        int sum = 0;
+        for (int b = lo; b < hi; ++b) sum += s_next[b];
+        int local = block_exclusive(sum, s_warp);
+        for (int b = lo; b < hi; ++b) {
+            const int first = starts[static_cast<int64_t>(b) * nblk + c];
+            const int len = s_next[b];
+            s_first[b] = first - local;  // middle position minus position in the chunk, the same for the run
+            s_next[b] = first;
+            local += len;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += kPermThreads) {
+            const int p = __ldg(slot_of + e0 + i);
+            const int b = p / kPermBlock;
+            const int t = atomicAdd(s_next + b, 1);
+            const int64_t k = e0 + (t - s_first[b]);
+            mid[k] = t;
+            arc_in[k] = static_cast<uint16_t>(i);
+            slot_in[t] = static_cast<uint16_t>(p - b * kPermBlock);
+        }
+        __syncthreads();
+    }
+}
+
+// Block by block: the block's linear values into shared memory, then out[mid ? mid[i] : i] = value
+// idx[i] of the block. The next block's values are loaded while this one is written.
+__global__ void __launch_bounds__(kPermThreads) perm_out_kernel(const float* __restrict__ in, int64_t E, int nblk,
+                                                                const uint16_t* __restrict__ idx,
+                                                                const int32_t* __restrict__ mid,
+                                                                float* __restrict__ out) {
+    extern __shared__ float s_v[];
+    constexpr int N = kPermBlock / kPermThreads;
+    float v[N];
+    auto load = [&](int c) {
+        const int64_t e0 = static_cast<int64_t>(c) * kPermBlock;
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            const int64_t e = e0 + q * kPermThreads + threadIdx.x;
+            v[q] = c < nblk && e < E ? __ldcs(in + e) : 0.0f;
+        }
+    };
+    load(blockIdx.x);
+    for (int c = blockIdx.x; c < nblk; c += gridDim.x) {
+#pragma unroll
+        for (int q = 0; q < N; ++q) s_v[q * kPermThreads + threadIdx.x] = v[q];
+        __syncthreads();
+        load(c + gridDim.x);
+        const int64_t e0 = static_cast<int64_t>(c) * kPermBlock;
+#pragma unroll 8
+        for (int q = 0; q < N; ++q) {
+            const int64_t e = e0 + q * kPermThreads + threadIdx.x;
+            if (e < E) out[mid ? __ldcs(mid + e) : e] = s_v[__ldcs(idx + e)];
+        }
+        __syncthreads();
+    }
+}
+
+// The other way: value idx[i] of the block = in[mid ? mid[i] : i], then the block goes out linearly.
+__global__ void __launch_bounds__(kPermThreads) perm_in_kernel(const float* __restrict__ in, int64_t E, int nblk,
+                                                               const uint16_t* __restrict__ idx,
+                                                               const int32_t* __restrict__ mid,
+                                                               float* __restrict__ out) {
+    extern __shared__ float s_v[];
+    constexpr int N = kPermBlock / kPermThreads;
+    for (int c = blockIdx.x; c < nblk; c += gridDim.x) {
+        const int64_t e0 = static_cast<int64_t>(c) * kPermBlock;
+#pragma unroll 16
+        for (int q = 0; q < N; ++q) {
+            const int64_t e = e0 + q * kPermThreads + threadIdx.x;
+            if (e < E) s_v[__ldcs(idx + e)] = __ldcs(in + (mid ? __ldcs(mid + e) : e));
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            const int64_t e = e0 + q * kPermThreads + threadIdx.x;
+            if (e < E) out[e] = s_v[q * kPermThreads + threadIdx.x];
+        }
+        __syncthreads();
     }
 }
 
@@ -527,13 +699,13 @@ bool spmm_rows_ok(int nrhs, const void* a, const void* b, const void* c, const v
 
 namespace {
 
-template <int VEC, int LQ, bool BWD>
+template <int VEC, int LQ, int MODE>
 cudaError_t run_rows(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHook* hook) {
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, s);
         const int64_t need = std::max((static_cast<int64_t>(L.P.V) + 31) / 32, (static_cast<int64_t>(L.P.nitems) + 7) / 8);
         const int grid = static_cast<int>(std::min<int64_t>(need, static_cast<int64_t>(sm_count) * rows_blocks(VEC)));
-        rows_kernel<VEC, LQ, BWD><<<grid, kBlock, 0, s>>>(L);
+        rows_kernel<VEC, LQ, MODE><<<grid, kBlock, 0, s>>>(L);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || L.P.nhubs == 0 || !L.out) return e;
@@ -545,25 +717,25 @@ cudaError_t run_rows(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHo
     return cudaGetLastError();
 }
 
-template <int VEC, bool BWD>
+template <int VEC, int MODE>
 cudaError_t pick_rows(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHook* hook) {
     const int Q = L.nrhs / VEC;
-    if (Q <= 1) return run_rows<VEC, 1, BWD>(L, s, sm_count, hook);
-    if (Q <= 2) return run_rows<VEC, 2, BWD>(L, s, sm_count, hook);
-    if (Q <= 4) return run_rows<VEC, 4, BWD>(L, s, sm_count, hook);
-    if (Q <= 8) return run_rows<VEC, 8, BWD>(L, s, sm_count, hook);
-    if (Q <= 16) return run_rows<VEC, 16, BWD>(L, s, sm_count, hook);
-    return run_rows<VEC, 32, BWD>(L, s, sm_count, hook);
+    if (Q <= 1) return run_rows<VEC, 1, MODE>(L, s, sm_count, hook);
+    if (Q <= 2) return run_rows<VEC, 2, MODE>(L, s, sm_count, hook);
+    if (Q <= 4) return run_rows<VEC, 4, MODE>(L, s, sm_count, hook);
+    if (Q <= 8) return run_rows<VEC, 8, MODE>(L, s, sm_count, hook);
+    if (Q <= 16) return run_rows<VEC, 16, MODE>(L, s, sm_count, hook);
+    return run_rows<VEC, 32, MODE>(L, s, sm_count, hook);
 }
 
-template <bool BWD>
+template <int MODE>
 cudaError_t pick_vec(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHook* hook) {
     if (L.P.V <= 0) return cudaSuccess;
     bool vec4 = L.nrhs % 4 == 0;
     for (const void* p : {static_cast<const void*>(L.in), static_cast<const void*>(L.X), static_cast<const void*>(L.out),
                           static_cast<const void*>(L.partial)})
         vec4 = vec4 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
-    return vec4 ? pick_rows<4, BWD>(L, s, sm_count, hook) : pick_rows<1, BWD>(L, s, sm_count, hook);
+    return vec4 ? pick_rows<4, MODE>(L, s, sm_count, hook) : pick_rows<1, MODE>(L, s, sm_count, hook);
 }
 
 }  // namespace
@@ -571,14 +743,53 @@ cudaError_t pick_vec(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHo
 cudaError_t launch_spmm_group(const SpmmPlanDev& P, const int32_t* col, const float* val, const float* X, int nrhs,
                               float* Y, float* partial, cudaStream_t s, int sm_count, LaunchHook* hook) {
     const RowsLaunch L = {P, col, nullptr, val, X, nullptr, nrhs, Y, partial, nullptr};
-    return pick_vec<false>(L, s, sm_count, hook);
+    return pick_vec<kForward>(L, s, sm_count, hook);
 }
 
 cudaError_t launch_spmv_bwd_group(const SpmmPlanDev& TP, const int32_t* tcol, const int32_t* tarc, const float* val,
                                   const float* X, const float* G, int nrhs, float* dX, float* partial, float* dA,
                                   cudaStream_t s, int sm_count, LaunchHook* hook) {
     const RowsLaunch L = {TP, tcol, tarc, val, G, X, nrhs, dX, partial, dA};
-    return pick_vec<true>(L, s, sm_count, hook);
+    return tarc ? pick_vec<kBwdArcs>(L, s, sm_count, hook) : pick_vec<kBwdSlots>(L, s, sm_count, hook);
+}
+
+size_t perm_scratch_bytes(int64_t E) {
+    const size_t nblk = static_cast<size_t>((E + kPermBlock - 1) / kPermBlock);
+    return 4 * (static_cast<size_t>(E) + nblk * nblk);
+}
+
+cudaError_t launch_build_perm(const int32_t* tarc, int64_t E, void* scratch, const ArcPerm& P, cudaStream_t s,
+                              int sm_count) {
+    const int nblk = static_cast<int>((E + kPermBlock - 1) / kPermBlock);
+    int32_t* slot_of = static_cast<int32_t*>(scratch);
+    int32_t* counts = slot_of + E;
+    cudaError_t e = cudaFuncSetAttribute(perm_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * nblk);
+    if (e != cudaSuccess) return e;
+    invert_kernel<<<sm_count * 8, kBlock, 0, s>>>(tarc, E, slot_of);
+    const int grid = std::min(nblk, sm_count * 2);
+    perm_count_kernel<<<grid, kPermThreads, 4 * nblk, s>>>(slot_of, E, nblk, counts);
+    perm_scan_kernel<<<grid, kPermThreads, 0, s>>>(nblk, counts);
+    perm_place_kernel<<<grid, kPermThreads, 8 * nblk, s>>>(slot_of, E, nblk, counts, P.mid, P.arc_in, P.slot_in);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_permute(const ArcPerm& P, int64_t E, bool to_slots, const float* in, float* tmp, float* out,
+                           cudaStream_t s, int sm_count, LaunchHook* hook) {
+    constexpr int smem = kPermBlock * sizeof(float);
+    const int nblk = static_cast<int>((E + kPermBlock - 1) / kPermBlock);
+    const int grid = std::min(nblk, sm_count);
+    cudaError_t e = cudaFuncSetAttribute(perm_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(perm_in_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    {
+        HookScope hs(hook, DPG_KERNEL_INIT, s);
+        if (to_slots) perm_out_kernel<<<grid, kPermThreads, smem, s>>>(in, E, nblk, P.arc_in, P.mid, tmp);
+        else perm_out_kernel<<<grid, kPermThreads, smem, s>>>(in, E, nblk, P.slot_in, nullptr, tmp);
+    }
+    HookScope hs(hook, DPG_KERNEL_INIT, s);
+    if (to_slots) perm_in_kernel<<<grid, kPermThreads, smem, s>>>(tmp, E, nblk, P.slot_in, nullptr, out);
+    else perm_in_kernel<<<grid, kPermThreads, smem, s>>>(tmp, E, nblk, P.arc_in, P.mid, out);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_gather_values(const float* v, const int32_t* idx, int64_t n, float* out, cudaStream_t s,

@@ -202,6 +202,10 @@ void graph_free_device(dpg_graph* g) {
     dev_free(g->ctx, g->tt_off);
     dev_free(g->ctx, g->tt_col);
     dev_free(g->ctx, g->tt_arc);
+    dev_free(g->ctx, g->tt_perm.mid);
+    dev_free(g->ctx, g->tt_perm.arc_in);
+    dev_free(g->ctx, g->tt_perm.slot_in);
+    g->tt_perm = ArcPerm();
     g->tt_off = g->tt_col = g->tt_arc = nullptr;
     g->spmm_ready = g->spmm_t_ready = false;
     g->relabel_ready = false;
@@ -433,6 +437,42 @@ dpg_status ensure_spmm_transpose(dpg_graph* g, bool need_graph = false) {
         g->tgraph->relabel = g->relabel;
     }
     return DPG_OK;
+}
+
+// Arc values in transposed order for the backward: the permutation and the two arrays. The transposed
+// pass reads val[arc] and writes dA[arc] at random; past the size of the L2 each is a random DRAM line
+// per arc, which bounds the pass. Permuting both, in arc order / permuted: 67 M arcs (268 MB of values)
+// 5.65 / 4.62 ms with 64 columns, 16.8 M arcs (67 MB, about half the L2) 0.865 / 0.850 ms with 32 and
+// 1.73-1.86 / 1.85 ms with 96 columns, 7.6 M arcs 0.23 / 0.38 ms with 20: the line lies at 2^25 arcs, past
+// the L2's 126 MB. False: not worth it, or no memory for it; the pass then works in arc order.
+constexpr int64_t kSlotArcs = 1 << 25;
+bool backward_slots(dpg_graph* g, float** vals_t, float** dA_t) {
+    if (g->E < kSlotArcs || g->E > kPermMaxArcs) return false;
+    dpg_ctx* c = g->ctx;
+    const size_t ne = static_cast<size_t>(g->E);
+    dpg_status st = DPG_OK;
+    *vals_t = static_cast<float*>(arena(c, S_VALS_T, ne * 4, &st));
+    if (st == DPG_OK) *dA_t = static_cast<float*>(arena(c, S_DA_T, ne * 4, &st));
+    if (st == DPG_OK && !g->tt_perm.mid && !g->tt_perm_tried) {
+        g->tt_perm_tried = true;
+        ArcPerm& P = g->tt_perm;
+        void* scratch = arena(c, S_TRANSPOSE, perm_scratch_bytes(g->E), &st);
+        cudaError_t e = st == DPG_OK ? dev_alloc(c, &P.mid, 4 * ne) : cudaErrorMemoryAllocation;
+        if (e == cudaSuccess) e = dev_alloc(c, &P.arc_in, 2 * ne);
+        if (e == cudaSuccess) e = dev_alloc(c, &P.slot_in, 2 * ne);
+        if (e == cudaSuccess) e = launch_build_perm(g->tt_arc, g->E, scratch, P, c->stream, c->sm_count);
+        if (e != cudaSuccess) {
+            dev_free(c, P.mid);
+            dev_free(c, P.arc_in);
+            dev_free(c, P.slot_in);
+            P = ArcPerm();
+        }
+    }
+    if (st != DPG_OK || !g->tt_perm.mid) {
+        cudaGetLastError();  // an allocation that failed is no error of the call
+        return false;
+    }
+    return true;
 }
 
 dpg_status check_nrhs(int32_t nrhs) {
@@ -1469,8 +1509,15 @@ dpg_status dpg_spmv_bwd_f32_dev(dpg_ctx* c, const dpg_graph* gc, const float* d_
         float* partial = static_cast<float*>(
             arena(c, S_SPMM_PARTIAL, static_cast<size_t>(g->spmm_t_plan.nseg + 1) * nrhs * 4, &st));
         if (st != DPG_OK) return st;
-        DPG_CUDA_TRY(launch_spmv_bwd_group(g->spmm_t_plan, g->tt_col, g->tt_arc, d_vals, d_X, d_G, nrhs, d_dX, partial,
-                                           d_dA, c->stream, c->sm_count, &c->prof));
+        float *vals_t = nullptr, *dA_t = nullptr;
+        const bool slots = backward_slots(g, &vals_t, &dA_t);
+        if (slots && d_dX)
+            DPG_CUDA_TRY(launch_permute(g->tt_perm, g->E, true, d_vals, dA_t, vals_t, c->stream, c->sm_count, &c->prof));
+        DPG_CUDA_TRY(launch_spmv_bwd_group(g->spmm_t_plan, g->tt_col, slots ? nullptr : g->tt_arc, slots ? vals_t : d_vals,
+                                           d_X, d_G, nrhs, d_dX, partial, slots && d_dA ? dA_t : d_dA, c->stream,
+                                           c->sm_count, &c->prof));
+        if (slots && d_dA)
+            DPG_CUDA_TRY(launch_permute(g->tt_perm, g->E, false, dA_t, vals_t, d_dA, c->stream, c->sm_count, &c->prof));
         return DPG_OK;
     }
     if (d_dX) {

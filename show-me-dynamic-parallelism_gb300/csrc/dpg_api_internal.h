@@ -31,7 +31,7 @@ namespace dpg_api {
 
 enum Slot {
     S_QV0, S_QV1, S_QSE0, S_QSE1, S_BMP0, S_BMP1, S_CH0, S_CH1, S_QCOUNT, S_CCOUNT, S_LABEL, S_CONTRIB0, S_CONTRIB1, S_RANK0, S_RANK1,
-    S_PARTIAL, S_DPART, S_DFIX, S_DSUM, S_NONSTOP, S_VALS, S_X, S_Y, S_OUTDEG, S_RANKOUT, S_XPERM, S_PENDING, S_SPMM_PARTIAL, S_SPMM_COUNTS, S_VALS_T,
+    S_PARTIAL, S_DPART, S_DFIX, S_DSUM, S_NONSTOP, S_VALS, S_X, S_Y, S_OUTDEG, S_RANKOUT, S_XPERM, S_PENDING, S_SPMM_PARTIAL, S_SPMM_COUNTS, S_VALS_T, S_DA_T,
     S_PRG_W, S_PRG_Y, S_PRG_C, S_PRG_V0, S_PRG_V1, S_PRG_V2, S_PRG_V3, S_PRG_PART, S_PRG_RED, S_PRG_FLAGS,
     S_DIRTY0, S_DIRTY1,
     S_CDP_BUF0, S_CDP_BUF1, S_CDP_WORDS,
@@ -172,6 +172,8 @@ struct dpg_graph {
     int32_t* tt_off = nullptr;
     int32_t* tt_col = nullptr;
     int32_t* tt_arc = nullptr;
+    ArcPerm tt_perm;             // between val / dA and transposed order; built on first use by the backward
+    bool tt_perm_tried = false;  // of large graphs (its absence is no error)
     // The same transposed CSR as a graph of its own (row-gather plan, column renaming), for pull
     // sweeps over in-arcs with permuted arc values; built on first use by the weighted PageRank.
     dpg_graph* tgraph = nullptr;

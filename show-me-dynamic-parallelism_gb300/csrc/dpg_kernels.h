@@ -216,7 +216,8 @@ bool spmm_rows_ok(int nrhs, const void* a, const void* b, const void* c, const v
 cudaError_t launch_spmm_group(const SpmmPlanDev& P, const int32_t* col, const float* val, const float* X, int nrhs,
                               float* Y, float* partial, cudaStream_t s, int sm_count, LaunchHook* hook);
 // One pass over the transposed CSR (plan TP, columns tcol, arc permutation tarc): dX = A^T G and
-// dA[e] = <G[row(e)], X[col(e)]>; either output may be null.
+// dA[e] = <G[row(e)], X[col(e)]>; either output may be null. With tarc null, val and dA are in the
+// order of tcol (transposed slots).
 cudaError_t launch_spmv_bwd_group(const SpmmPlanDev& TP, const int32_t* tcol, const int32_t* tarc, const float* val,
                                   const float* X, const float* G, int nrhs, float* dX, float* partial, float* dA,
                                   cudaStream_t s, int sm_count, LaunchHook* hook);
@@ -227,6 +228,20 @@ cudaError_t launch_spmm(const SpmmPlanDev& P, const int32_t* col, const float* v
 // dA[e] = <G[row(e)][:], X[col[e]][:]>.
 cudaError_t launch_arc_dot(const SpmmPlanDev& P, const int32_t* col, const float* X, const float* G, int nrhs,
                            float* dA, cudaStream_t s, int sm_count, LaunchHook* hook);
+// Permutation of arc values between CSR order and transposed order (dpg_adjoint.cu): E entries each.
+constexpr int32_t kPermBlock = 1 << 15;
+constexpr int64_t kPermMaxArcs = int64_t{1} << 28;  // 8,192 chunks: their run starts fit in shared memory
+struct ArcPerm {
+    int32_t* mid = nullptr;
+    uint16_t* arc_in = nullptr;
+    uint16_t* slot_in = nullptr;
+};
+size_t perm_scratch_bytes(int64_t E);
+cudaError_t launch_build_perm(const int32_t* tarc, int64_t E, void* scratch, const ArcPerm& P, cudaStream_t s,
+                              int sm_count);
+// out[slot] = in[arc] of every arc (to_slots), or out[arc] = in[slot]; tmp holds E floats.
+cudaError_t launch_permute(const ArcPerm& P, int64_t E, bool to_slots, const float* in, float* tmp, float* out,
+                           cudaStream_t s, int sm_count, LaunchHook* hook);
 // out[i] = v[idx[i]].
 cudaError_t launch_gather_values(const float* v, const int32_t* idx, int64_t n, float* out, cudaStream_t s,
                                  int sm_count);

@@ -76,3 +76,32 @@ def test_widths(ctx, graph, nrhs, shift):
     for t in (dA, dA2):
         prod = G64[rows] * X64[g.col]
         close(t, prod.sum(1), np.abs(prod).sum(1))
+
+
+# From 2^25 arcs up the backward permutes the values to transposed order and dA back, in blocks of 32,768: a last block
+# of every kind, and one arc less than the line. dX sums up to about 1,200 products, dA is one product of nrhs = 1.
+@pytest.mark.parametrize("E", [(1 << 25) - 1, 1 << 25, (1 << 25) + 1, (1 << 25) + 32767])
+def test_permuted_values(ctx, E):
+    import torch
+
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(E)
+    V = 40_009
+    row, _ = torch.sort(torch.randint(0, V, (E,), device=dev, generator=gen, dtype=torch.int32))
+    col = torch.randint(0, V, (E,), device=dev, generator=gen, dtype=torch.int32)
+    off = torch.zeros(V + 1, dtype=torch.int32, device=dev)
+    off[1:] = torch.cumsum(torch.bincount(row, minlength=V), 0)
+    vals = torch.rand(E, device=dev, generator=gen)
+    X, G = (torch.rand(V, 1, device=dev, generator=gen) - 0.5 for _ in range(2))
+    dX, dA = torch.empty_like(X), torch.empty_like(vals)
+    torch.cuda.synchronize()
+    dg = dpg.Graph.from_device(ctx, V, E, off.data_ptr(), col.data_ptr())
+    dpg.spmv_bwd_dev(ctx, dg, vals.data_ptr(), 1, X.data_ptr(), G.data_ptr(), dX.data_ptr(), dA.data_ptr())
+    ctx.synchronize()
+    r, c = row.long(), col.long()
+    assert torch.equal(dA, G[r, 0] * X[c, 0])  # one product each, correctly rounded
+    terms = vals.double() * G[r, 0].double()
+    want = torch.zeros(V, dtype=torch.float64, device=dev).index_add_(0, c, terms)
+    size = torch.zeros(V, dtype=torch.float64, device=dev).index_add_(0, c, terms.abs())
+    assert bool(((dX[:, 0].double() - want).abs() <= TOL * size).all())
