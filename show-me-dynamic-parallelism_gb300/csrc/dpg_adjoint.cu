@@ -223,6 +223,12 @@ struct RowVec<4> {
     __device__ __forceinline__ float dot(const RowVec& x, float d) const {
         return fmaf(v.w, x.v.w, fmaf(v.z, x.v.z, fmaf(v.y, x.v.y, fmaf(v.x, x.v.x, d))));
     }
+    __device__ __forceinline__ void add(const RowVec& x) {
+        v.x += x.v.x;
+        v.y += x.v.y;
+        v.z += x.v.z;
+        v.w += x.v.w;
+    }
     __device__ __forceinline__ void add_xor(int m) {
         v.x += __shfl_xor_sync(kFullMask, v.x, m);
         v.y += __shfl_xor_sync(kFullMask, v.y, m);
@@ -243,6 +249,7 @@ struct RowVec<1> {
     __device__ __forceinline__ void store(float* p) const { *p = v; }
     __device__ __forceinline__ void fma(float a, const RowVec& x) { v = fmaf(a, x.v, v); }
     __device__ __forceinline__ float dot(const RowVec& x, float d) const { return fmaf(v, x.v, d); }
+    __device__ __forceinline__ void add(const RowVec& x) { v += x.v; }
     __device__ __forceinline__ void add_xor(int m) { v += __shfl_xor_sync(kFullMask, v, m); }
 };
 
@@ -365,12 +372,19 @@ __global__ void __launch_bounds__(kBlock, rows_blocks(VEC)) rows_kernel(RowsLaun
         StepIdx<R, MODE> cur, nxt;
         const unsigned end = I.z;
         cur.load(L, I.y + grp * A, end, gl);
-        for (unsigned base = I.y; base < end; base += NG * A) {
+        // Every 64 arcs of a lane the sum so far is set aside, which keeps the chain of roundings short.
+        V total = V::zero();
+        for (unsigned base = I.y, k = 1; base < end; base += NG * A, ++k) {
             nxt.load(L, base + (NG + grp) * A, end, gl);
             step(base + grp * A, end, cur);
             cur = nxt;
+            if (k * A % (64 * AP) == 0) {
+                total.add(acc);
+                acc = V::zero();
+            }
         }
         if (!L.out) continue;
+        acc.add(total);
 #pragma unroll
         for (int m = LQ; m < 32; m <<= 1) acc.add_xor(m);
         if (grp == 0 && sub == 0 && live)
