@@ -746,13 +746,14 @@ dpg_status run_pagerank(dpg_ctx* c, dpg_graph* g, const int32_t* d_outdeg, const
     float* init_rank_dst = conv ? rk[0] : (o.iterations == 0 ? d_rank : nullptr);
     DPG_CUDA_TRY(launch_pagerank_init(L, init_rank, init_rank_dst, c->st, c->stream, c->sm_count, &c->prof));
     // With a tolerance the convergence test is pipelined one sweep deep: sweep it+1 is queued before
-    // the host reads sweep it's flag (pinned memory, an event), so the device does not idle on the
-    // read. A sweep queued after the converged one writes only buffers of the other parity (ranks,
+    // the host reads sweep it's flag (written to pinned memory by the sweep's last kernel, behind an
+    // event), so the device does not idle on the read. A sweep queued after the converged one writes only buffers of the other parity (ranks,
     // contributions, dangling sum, flag), so the converged ranks stay where the count says.
     unsigned* hflags = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     if (conv) {
         DPG_TRY(host_words(c, &hflags));
+        DPG_CUDA_TRY(cudaMemsetAsync(nonstop, 0, sizeof(unsigned), c->stream));
         for (cudaEvent_t& e : ev) DPG_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     struct Events {
@@ -772,8 +773,8 @@ dpg_status run_pagerank(dpg_ctx* c, dpg_graph* g, const int32_t* d_outdeg, const
         if (conv) {
             L.rank_prev = rk[it & 1];
             L.rank_out = rk[(it + 1) & 1];
-            L.nonstop = nonstop + (it & 1);
-            DPG_CUDA_TRY(cudaMemsetAsync(L.nonstop, 0, sizeof(unsigned), c->stream));
+            L.nonstop = nonstop;
+            L.host_flag = hflags + 2 + (it & 1);
         } else {
             L.rank_prev = nullptr;
             L.nonstop = nullptr;
@@ -782,8 +783,6 @@ dpg_status run_pagerank(dpg_ctx* c, dpg_graph* g, const int32_t* d_outdeg, const
         DPG_CUDA_TRY(launch_pagerank_sweep(L, c->st, c->stream, c->sm_count, &c->prof));
         ++sweeps;
         if (conv) {
-            DPG_CUDA_TRY(cudaMemcpyAsync(hflags + 2 + (it & 1), L.nonstop, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                                         c->stream));
             DPG_CUDA_TRY(cudaEventRecord(ev[it & 1], c->stream));
             if (pending >= 0) {
                 DPG_CUDA_TRY(cudaEventSynchronize(ev[pending & 1]));
@@ -1047,20 +1046,33 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
     if (adjoint_epsilon > 0 && (!in_opts || in_opts->iterations == 0)) adj_iters = kMaxGradSweeps;
     DPG_TRY(ensure_spmm_transpose(g, true));
     DPG_TRY(ensure_spmm_plan(g));
+    dpg_graph* tg = g->tgraph;
+    for (dpg_graph* p : {g, tg}) {
+        DPG_TRY(ensure_plan(p));
+        if (p->relabel) DPG_TRY(ensure_relabel(p));
+    }
     const size_t nv = static_cast<size_t>(g->V), ne = static_cast<size_t>(g->E > 0 ? g->E : 1);
     const int nb = pr_vec_blocks(c->sm_count);
+    int gb, fb, bt;
+    rowgather_grid(c->sm_count, &gb, &fb, &bt);
     dpg_status st = DPG_OK;
     float* w_t = static_cast<float*>(arena(c, S_VALS_T, ne * 4, &st));
     float* W = static_cast<float*>(arena(c, S_PRG_W, nv * 4, &st));
     float* y = static_cast<float*>(arena(c, S_PRG_Y, nv * 4, &st));
     float* contrib = static_cast<float*>(arena(c, S_PRG_C, nv * 4, &st));
+    float* x[2] = {static_cast<float*>(arena(c, S_PRG_X0, nv * 4, &st)),
+                   static_cast<float*>(arena(c, S_PRG_X1, nv * 4, &st))};
     float* vec[4] = {static_cast<float*>(arena(c, S_PRG_V0, nv * 4, &st)),
                      static_cast<float*>(arena(c, S_PRG_V1, nv * 4, &st)),
                      static_cast<float*>(arena(c, S_PRG_V2, nv * 4, &st)),
                      static_cast<float*>(arena(c, S_PRG_V3, nv * 4, &st))};
+    const int32_t nseg = std::max(g->plan.nseg, tg->plan.nseg);
+    float* partial = static_cast<float*>(arena(c, S_PARTIAL, static_cast<size_t>(nseg + 1) * 4, &st));
+    double* dpart = static_cast<double*>(arena(c, S_DPART, static_cast<size_t>(gb) * (bt / 32) * 8, &st));
+    double* dfix = static_cast<double*>(arena(c, S_DFIX, static_cast<size_t>(fb) * (256 / 32) * 8, &st));
     double* part = static_cast<double*>(arena(c, S_PRG_PART, static_cast<size_t>(nb) * 8, &st));
     double* red = static_cast<double*>(arena(c, S_PRG_RED, 2 * 8, &st));
-    unsigned* flags = static_cast<unsigned*>(arena(c, S_PRG_FLAGS, 16, &st));  // [0] ticket, [1..2] nonstop
+    unsigned* flags = static_cast<unsigned*>(arena(c, S_PRG_FLAGS, 16, &st));  // [0] ticket, [1] nonstop
     if (st != DPG_OK) return st;
     DPG_CUDA_TRY(cudaMemsetAsync(flags, 0, 16, c->stream));
     // Out-weight sums W = A 1 and the weights in transposed-slot order.
@@ -1068,18 +1080,11 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
     DPG_TRY(run_spmv(c, g, d_w, y, W));
     DPG_CUDA_TRY(launch_gather_values(d_w, g->tt_arc, g->E, w_t, c->stream, c->sm_count));
 
-    PrVecLaunch L;
-    memset(&L, 0, sizeof(L));
-    L.V = g->V;
-    L.W = W;
-    L.part = part;
-    L.ticket = flags;
-    L.damping = static_cast<float>(o.damping);
     // The convergence test is pipelined one sweep deep: sweep it+1 is queued before the host reads
-    // sweep it's flag (copied to pinned memory, waited on with an event), so the device does not
-    // idle on the read. When sweep it converged, sweep it+1 is surplus: it wrote only the other
-    // vector, y, the reduction slot and flag of its own parity and (forward) the contributions,
-    // none of which is read afterwards, so stepping the vector swap back restores sweep it's result.
+    // sweep it's flag (written to pinned memory by the sweep's last kernel, behind an event), so the
+    // device does not idle on the read. When sweep it converged, sweep it+1 is surplus: it wrote only
+    // the vectors and the reduction slot of its own parity, none of which is read afterwards, so
+    // stepping the vector swap back restores sweep it's result.
     unsigned* hflags = nullptr;
     DPG_TRY(host_words(c, &hflags));
     cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -1091,71 +1096,91 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
             cudaEventDestroy(e[1]);
         }
     } ev_guard{ev};
-    auto sweeps_until = [&](int mode, int32_t cap, double eps, float** cur, float** nxt, dpg_graph* sg,
-                            const float* vals, const float* x_of_cur, int64_t* done) -> dpg_status {
+    RowGatherLaunch L;
+    memset(&L, 0, sizeof(L));
+    L.partial = partial;
+    L.V = g->V;
+    L.damping = static_cast<float>(o.damping);
+    L.dangling_scale = o.damping / static_cast<double>(g->V);
+    L.dpart = dpart;
+    L.dfix = dfix;
+    L.W = W;
+    // Sweeps over graph sg with arc values vals; `start` is the vector gathered first, in vertex order.
+    // The gathered vectors x[0], x[1] are in sg's renamed order; sweeps leave entries of x that they do
+    // not write (contributions of W == 0) as they were, so both start with the first vector.
+    auto sweeps_until = [&](int32_t cap, double eps, float** cur, float** nxt, dpg_graph* sg, const float* vals,
+                            const float* start, int64_t* done) -> dpg_status {
+        for (float* xb : x) {
+            if (sg->relabel) DPG_CUDA_TRY(launch_gather_by_index(start, sg->inv, sg->V, xb, c->stream, c->sm_count));
+            else DPG_CUDA_TRY(cudaMemcpyAsync(xb, start, nv * 4, cudaMemcpyDeviceToDevice, c->stream));
+        }
+        L.plan = sg->plan;
+        L.off = sg->off;
+        L.col = sg->relabel ? sg->pcol : sg->col;
+        L.perm = sg->relabel ? sg->perm : nullptr;
+        L.hot = hot_entries(c, sg);
+        L.vals = vals;
+        L.epsilon = static_cast<float>(eps);
         // Every loop starts from the reduction its init pass left in red[0].
         int32_t pending = -1;  // sweep whose flag is on its way to the host
         for (int32_t it = 0; it < cap; ++it) {
-            unsigned* dflag = flags + 1 + (it & 1);
-            DPG_TRY(run_spmv(c, sg, vals, x_of_cur ? x_of_cur : *cur, y));
-            L.mode = mode;
-            L.y = y;
-            L.prev = eps > 0 ? *cur : nullptr;
-            L.out = *nxt;
-            L.red_in = red + (it & 1);
-            L.red_out = red + ((it + 1) & 1);
-            L.epsilon = static_cast<float>(eps);
-            L.nonstop = eps > 0 ? dflag : nullptr;
-            if (eps > 0) DPG_CUDA_TRY(cudaMemsetAsync(dflag, 0, 4, c->stream));
-            DPG_CUDA_TRY(launch_pr_vec(L, c->sm_count, c->stream, &c->prof));
+            L.x = x[it & 1];
+            L.y = x[(it + 1) & 1];
+            L.rank_prev = eps > 0 ? *cur : nullptr;
+            L.rank_out = *nxt;
+            L.dsum_in = red + (it & 1);
+            L.dsum_out = red + ((it + 1) & 1);
+            L.nonstop = eps > 0 ? flags + 1 : nullptr;
+            L.host_flag = hflags + (it & 1);
+            DPG_CUDA_TRY(launch_weighted_sweep(L, c->st, c->stream, c->sm_count, &c->prof));
             std::swap(*cur, *nxt);
             ++*done;
             if (eps > 0) {
-                DPG_CUDA_TRY(cudaMemcpyAsync(hflags + (it & 1), dflag, 4, cudaMemcpyDeviceToHost, c->stream));
                 DPG_CUDA_TRY(cudaEventRecord(ev[it & 1], c->stream));
                 if (pending >= 0) {
                     DPG_CUDA_TRY(cudaEventSynchronize(ev[pending & 1]));
-                    if (hflags[pending & 1] == 0) {
+                    if (reinterpret_cast<volatile unsigned*>(hflags)[pending & 1] == 0) {
                         std::swap(*cur, *nxt);
                         --*done;
-                        pending = -1;
+                        pending = it;
                         break;
                     }
                 }
                 pending = it;
             }
         }
+        // The flag words are free again only when the last sweep queued has written its own.
         if (pending >= 0) DPG_CUDA_TRY(cudaEventSynchronize(ev[pending & 1]));
         return DPG_OK;
     };
 
-    // Forward: r in vec[0]/vec[1], contributions r / W in contrib, dangling sum in red[0].
+    // Forward: r in vec[0]/vec[1], contributions r / W first in contrib, dangling sum in red[0].
     float* r_cur = vec[0];
     float* r_nxt = vec[1];
-    L.mode = PRV_FWD_INIT;
-    L.out = r_cur;
-    L.contrib = contrib;
-    L.init_value = o.init_zero ? 0.0f : static_cast<float>(o.total_rank / static_cast<double>(g->V));
-    L.red_out = red;
-    DPG_CUDA_TRY(launch_pr_vec(L, c->sm_count, c->stream, &c->prof));
+    PrInitLaunch I;
+    memset(&I, 0, sizeof(I));
+    I.V = g->V;
+    I.W = W;
+    I.out = r_cur;
+    I.contrib = contrib;
+    I.init_value = o.init_zero ? 0.0f : static_cast<float>(o.total_rank / static_cast<double>(g->V));
+    I.red_out = red;
+    I.part = part;
+    I.ticket = flags;
+    DPG_CUDA_TRY(launch_pr_vec_init(I, c->sm_count, c->stream, &c->prof));
     L.base_const = (1.0 - o.damping) * o.total_rank / static_cast<double>(g->V);
-    L.red_scale = o.damping / static_cast<double>(g->V);
     int64_t fwd = 0, adj = 0;
-    DPG_TRY(sweeps_until(PRV_FWD_SWEEP, fwd_iters, o.epsilon, &r_cur, &r_nxt, g->tgraph, w_t, contrib, &fwd));
+    DPG_TRY(sweeps_until(fwd_iters, o.epsilon, &r_cur, &r_nxt, tg, w_t, contrib, &fwd));
 
     // Adjoint: lambda in vec[2]/vec[3], its sum in red[0].
     float* l_cur = vec[2];
     float* l_nxt = vec[3];
-    L.mode = PRV_ADJ_INIT;
-    L.seed = d_seed;
-    L.out = l_cur;
-    L.prev = nullptr;
-    L.nonstop = nullptr;
-    L.red_out = red;
-    DPG_CUDA_TRY(launch_pr_vec(L, c->sm_count, c->stream, &c->prof));
+    I.seed = d_seed;
+    I.out = l_cur;
+    DPG_CUDA_TRY(launch_pr_vec_init(I, c->sm_count, c->stream, &c->prof));
     L.base_const = 0.0;
-    L.red_scale = o.damping / static_cast<double>(g->V);
-    DPG_TRY(sweeps_until(PRV_ADJ_SWEEP, adj_iters, adjoint_epsilon, &l_cur, &l_nxt, g, d_w, nullptr, &adj));
+    L.seed = d_seed;
+    DPG_TRY(sweeps_until(adj_iters, adjoint_epsilon, &l_cur, &l_nxt, g, d_w, d_seed, &adj));
 
     // q = (A lambda) / W with the final lambda, then the per-arc gradient.
     DPG_TRY(run_spmv(c, g, d_w, l_cur, y));

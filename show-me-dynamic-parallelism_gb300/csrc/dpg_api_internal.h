@@ -32,7 +32,7 @@ namespace dpg_api {
 enum Slot {
     S_QV0, S_QV1, S_QSE0, S_QSE1, S_BMP0, S_BMP1, S_CH0, S_CH1, S_QCOUNT, S_CCOUNT, S_LABEL, S_CONTRIB0, S_CONTRIB1, S_RANK0, S_RANK1,
     S_PARTIAL, S_DPART, S_DFIX, S_DSUM, S_NONSTOP, S_VALS, S_X, S_Y, S_OUTDEG, S_RANKOUT, S_XPERM, S_PENDING, S_SPMM_PARTIAL, S_SPMM_COUNTS, S_VALS_T, S_DA_T,
-    S_PRG_W, S_PRG_Y, S_PRG_C, S_PRG_V0, S_PRG_V1, S_PRG_V2, S_PRG_V3, S_PRG_PART, S_PRG_RED, S_PRG_FLAGS,
+    S_PRG_W, S_PRG_Y, S_PRG_C, S_PRG_X0, S_PRG_X1, S_PRG_V0, S_PRG_V1, S_PRG_V2, S_PRG_V3, S_PRG_PART, S_PRG_RED, S_PRG_FLAGS,
     S_DIRTY0, S_DIRTY1,
     S_CDP_BUF0, S_CDP_BUF1, S_CDP_WORDS,
     S_TRANSPOSE, S_TRANSPOSE_ARC, S_DO_COUNT, S_FAR0, S_FAR1, S_FAR2, S_FAR_COUNT, S_PLANINFO,

@@ -181,7 +181,13 @@ struct RowGatherLaunch {
     double* dpart;          // [gather warps] dangling partials
     double* dfix;           // [fix-up warps] dangling partials
     float epsilon;
-    unsigned* nonstop;      // nullable: set to 1 when some |new-old| > epsilon
+    unsigned* nonstop;      // nullable: set to 1 when some |new-old| > epsilon; the sweep's end copies it
+    unsigned* host_flag;    // to host_flag (pinned host memory) and clears it
+    // Weighted sweeps only: out-weight sums, and the adjoint's seed (null: forward sweep). rank_out is
+    // always written, rank_prev null without a tolerance (relative: epsilon * |new|), dsum the reduced
+    // quantity, y the gathered vector of the next sweep (renamed).
+    const float* W;
+    const float* seed;
     // Batches of graphs (nullable): row v belongs to graph vgraph[v], whose uniform term this sweep
     // is gbase[g] and whose initial rank is ginit[g]. A dangling row then stores its rank in its
     // (never gathered) contribution slot, where the per-graph dangling reduction reads it.
@@ -266,36 +272,22 @@ cudaError_t launch_bfs_cdp(int variant, const int32_t* off, const int32_t* col, 
 
 // ---- weighted PageRank and its edge-weight gradient (dpg_prgrad.cu) ------------------------------
 
-enum PrVecMode {
-    PRV_FWD_INIT = 0,   // r = init_value; contrib = r / W; red_out = sum of r over dangling vertices
-    PRV_FWD_SWEEP = 1,  // r = (base_const + red_scale * red_in) + damping * y; contrib, red_out as above
-    PRV_ADJ_INIT = 2,   // lambda = seed; red_out = sum of lambda
-    PRV_ADJ_SWEEP = 3,  // lambda = seed + (W > 0 ? damping * y / W : red_scale * red_in); red_out = sum
-};
-
-struct PrVecLaunch {
-    int mode;
+// The start of a loop: forward r = init_value, contrib = r / W (0 where W == 0), red_out = sum of r over
+// dangling vertices; adjoint (seed given) lambda = seed, red_out = its sum.
+struct PrInitLaunch {
     int32_t V;
-    const float* y;       // gathered sums of this sweep
     const float* W;       // out-weight sums
-    const float* seed;    // dL/dr (adjoint)
-    const float* prev;    // previous vector for the change test, or null
-    float* out;           // new vector
-    float* contrib;       // forward: out / W, 0 where W == 0
-    const double* red_in; // reduction of the previous vector
+    const float* seed;    // dL/dr (adjoint), null for the forward
+    float* out;           // r or lambda
+    float* contrib;       // forward
     double* red_out;
     double* part;         // pr_vec_blocks(sm_count) partials
     unsigned* ticket;     // zero before the first launch; the last block resets it
-    float damping;
     float init_value;
-    double base_const;
-    double red_scale;
-    float epsilon;
-    unsigned* nonstop;    // set to 1 when some |out - prev| > epsilon * |out| (null: no test)
 };
 
 int pr_vec_blocks(int sm_count);
-cudaError_t launch_pr_vec(const PrVecLaunch& L, int sm_count, cudaStream_t s, LaunchHook* hook);
+cudaError_t launch_pr_vec_init(const PrInitLaunch& L, int sm_count, cudaStream_t s, LaunchHook* hook);
 cudaError_t launch_pr_arc_grad(const SpmmPlanDev& P, const int32_t* col, const float* r, const float* W, const float* y,
                                const float* lam, float damping, float* grad, cudaStream_t s, int sm_count,
                                LaunchHook* hook);
@@ -337,6 +329,10 @@ cudaError_t launch_spmv(const RowGatherLaunch& L, DevStatus* st, cudaStream_t st
 // One PageRank sweep: gather + hub fix-up + dangling reduction into dsum_out.
 cudaError_t launch_pagerank_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream,
                                   int sm_count, LaunchHook* hook);
+// One sweep of the weighted PageRank or of its adjoint (dpg_prgrad.cu): gather over plan / col / vals,
+// epilogue, hub fix-up, and the reduced quantity into dsum_out.
+cudaError_t launch_weighted_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
+                                  LaunchHook* hook);
 // contrib[v] = init / outdeg[v] (0 for dangling), rank_prev[v] = init (nullable), and the
 // dangling mass of the initial vector into dsum_out.
 cudaError_t launch_pagerank_init(const RowGatherLaunch& L, float init_rank, float* rank_prev,

@@ -11,9 +11,9 @@
 //     lambda[u] = s[u] + d / V * sum_t lambda[t]                             (dangling u)
 // and, per arc e = (u -> v), with q[u] = sum_t w[e'] lambda[t] / W[u],
 //     dL/dw[e] = d * r[u] / W[u] * (lambda[v] - q[u]).
-// The sweeps' gathers are the row-gather SpMV (forward over the transposed CSR with permuted
-// weights, adjoint over the graph itself); the kernels here are the vector epilogues between
-// sweeps and the per-arc gradient. Every reduction runs in a fixed order (per-block partials, summed
+// The sweeps are weighted row gathers with these epilogues (kModeWeighted in dpg_rowgather.cu; forward
+// over the transposed CSR with permuted weights, adjoint over the graph itself); the kernels here start
+// the loops and compute the per-arc gradient. Every reduction runs in a fixed order (per-block partials, summed
 // in block order by the last block), so results are bit-reproducible.
 #include <cuda_runtime.h>
 
@@ -36,38 +36,26 @@ __device__ __forceinline__ double block_sum_f64(double v, double* s_warp) {
     return t;  // valid in thread 0
 }
 
-// One vector pass over all V vertices (see PrVecMode). Block b handles vertices b*256+t, stepping by
-// the grid; its partial of the reduced quantity goes to part[b], and the last block to finish adds
-// the partials in block order into red_out.
-__global__ void __launch_bounds__(kBlock) pr_vec_kernel(PrVecLaunch L) {
+// Block b handles vertices b*256+t, stepping by the grid; its partial of the reduced quantity goes to
+// part[b], and the last block to finish adds the partials in block order into red_out.
+__global__ void __launch_bounds__(kBlock) pr_vec_init_kernel(PrInitLaunch L) {
     __shared__ double s_warp[kBlock / 32];
     __shared__ bool s_last;
-    const int mode = L.mode;
-    const bool adjoint = mode == PRV_ADJ_INIT || mode == PRV_ADJ_SWEEP;
-    const bool sweep = mode == PRV_FWD_SWEEP || mode == PRV_ADJ_SWEEP;
-    // Forward: the uniform term (1-d)T/V + dD/V; adjoint: the dangling rows' d/V * sum(lambda).
-    float uniform = 0.0f;
-    if (sweep) uniform = static_cast<float>(L.base_const + L.red_scale * L.red_in[0]);
     double acc = 0.0;
-    bool moved = false;
     for (int64_t v = static_cast<int64_t>(blockIdx.x) * kBlock + threadIdx.x; v < L.V;
          v += static_cast<int64_t>(gridDim.x) * kBlock) {
-        const float Wv = L.W[v];
         float x;
-        if (!adjoint) {
-            x = sweep ? fmaf(L.damping, L.y[v], uniform) : L.init_value;
+        if (!L.seed) {
+            const float Wv = L.W[v];
+            x = L.init_value;
             L.contrib[v] = Wv > 0.0f ? x / Wv : 0.0f;
             if (!(Wv > 0.0f)) acc += x;
         } else {
-            const float s = L.seed[v];
-            if (!sweep) x = s;
-            else x = Wv > 0.0f ? s + L.damping * (L.y[v] / Wv) : s + uniform;
+            x = L.seed[v];
             acc += x;
         }
-        if (L.prev && fabsf(x - L.prev[v]) > L.epsilon * fabsf(x)) moved = true;
         L.out[v] = x;
     }
-    if (L.nonstop && __syncthreads_or(moved) && threadIdx.x == 0) atomicOr(L.nonstop, 1u);
     const double t = block_sum_f64(acc, s_warp);
     if (threadIdx.x == 0) {
         L.part[blockIdx.x] = t;
@@ -119,9 +107,9 @@ __global__ void fill_f32_kernel(float* p, int64_t n, float v) {
 
 int pr_vec_blocks(int sm_count) { return sm_count * 2; }
 
-cudaError_t launch_pr_vec(const PrVecLaunch& L, int sm_count, cudaStream_t s, LaunchHook* hook) {
-    HookScope hs(hook, L.mode == PRV_FWD_INIT || L.mode == PRV_ADJ_INIT ? DPG_KERNEL_INIT : DPG_KERNEL_FIXUP, s);
-    pr_vec_kernel<<<pr_vec_blocks(sm_count), kBlock, 0, s>>>(L);
+cudaError_t launch_pr_vec_init(const PrInitLaunch& L, int sm_count, cudaStream_t s, LaunchHook* hook) {
+    HookScope hs(hook, DPG_KERNEL_INIT, s);
+    pr_vec_init_kernel<<<pr_vec_blocks(sm_count), kBlock, 0, s>>>(L);
     return cudaGetLastError();
 }
 

@@ -59,7 +59,9 @@ constexpr int kFixBatch = 8;  // loads the fix-up issues before it adds them
 constexpr int kPadded = kRowTileItems + kRowTileItems / 32;
 __device__ __forceinline__ int pad(int i) { return i + (i >> 5); }
 
-enum { kModeSpmv = 0, kModePagerank = 1 };
+enum { kModeSpmv = 0, kModePagerank = 1, kModeWeighted = 2 };
+// SpMV and weighted PageRank sweeps multiply by arc values.
+constexpr bool has_vals(int mode) { return mode != kModePagerank; }
 
 // Loads of the streams every tile reads once (columns, SpMV values, out-degrees, renaming slots):
 // read-only for the launch (nc) and kept out of L1 (L1::no_allocate), so the L1 lines are left to
@@ -70,7 +72,7 @@ enum { kModeSpmv = 0, kModePagerank = 1 };
 template <int MODE>
 __device__ __forceinline__ int ld_stream(const int* p) {
     int v;
-    if constexpr (MODE == kModeSpmv) {
+    if constexpr (has_vals(MODE)) {
         asm("{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
             "ld.global.nc.L1::no_allocate.L2::cache_hint.s32 %0, [%1], pol;\n\t}"
             : "=r"(v) : "l"(p));
@@ -82,7 +84,7 @@ __device__ __forceinline__ int ld_stream(const int* p) {
 template <int MODE>
 __device__ __forceinline__ float ld_stream(const float* p) {
     float v;
-    if constexpr (MODE == kModeSpmv) {
+    if constexpr (has_vals(MODE)) {
         asm("{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
             "ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], pol;\n\t}"
             : "=f"(v) : "l"(p));
@@ -95,11 +97,11 @@ __device__ __forceinline__ float ld_stream(const float* p) {
 // PageRank epilogue of one row: new rank, next contribution, dangling mass, convergence flag.
 // od / pos are the row's out-degree and contribution slot (perm[v] with renamed columns).
 __device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, float sum, float base, int od, int pos,
-                                            double& dang) {
+                                            double& dang, bool& moved) {
     if (L.vgraph) base = __ldg(L.gbase + __ldg(L.vgraph + v));
     const float nv = fmaf(L.damping, sum, base);
     if (L.rank_out) L.rank_out[v] = nv;
-    if (L.rank_prev && fabsf(nv - __ldg(L.rank_prev + v)) > L.epsilon) *L.nonstop = 1u;
+    if (L.rank_prev && fabsf(nv - __ldg(L.rank_prev + v)) > L.epsilon) moved = true;
     // Only vertices with out-arcs are ever gathered (they are the columns), so the contribution
     // slot of a dangling vertex is free: a batch parks its rank there for the per-graph reduction.
     // The division runs for every row (by 1 for a dangling one) so a warp's rows do not diverge
@@ -113,8 +115,33 @@ __device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, flo
     }
 }
 
-__device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, float sum, float base, double& dang) {
-    pr_epilogue(L, v, sum, base, __ldg(L.outdeg + v), L.perm ? __ldg(L.perm + v) : v, dang);
+__device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, float sum, float base, double& dang, bool& moved) {
+    pr_epilogue(L, v, sum, base, __ldg(L.outdeg + v), L.perm ? __ldg(L.perm + v) : v, dang, moved);
+}
+
+// Epilogue of one row of a weighted PageRank sweep (dpg_prgrad.cu): forward (no seed) the new rank and
+// its contribution rank / W; adjoint the new lambda, which is also the next gathered vector. x goes to
+// rank_out[v], the gathered vector's entry to y[pos]; `dang` collects the dangling ranks, or all lambdas.
+__device__ __forceinline__ void weighted_epilogue(const RowGatherLaunch& L, int v, float sum, float base, float W,
+                                                  int pos, float seed, float prev, double& dang, bool& moved) {
+    float x;
+    if (!L.seed) {
+        x = fmaf(L.damping, sum, base);
+        if (W > 0.0f) L.y[pos] = x / W;
+        else dang += static_cast<double>(x);
+    } else {
+        x = W > 0.0f ? seed + L.damping * (sum / W) : seed + base;
+        L.y[pos] = x;
+        dang += static_cast<double>(x);
+    }
+    if (L.rank_prev && fabsf(x - prev) > L.epsilon * fabsf(x)) moved = true;
+    L.rank_out[v] = x;
+}
+
+__device__ __forceinline__ void weighted_epilogue(const RowGatherLaunch& L, int v, float sum, float base,
+                                                  double& dang, bool& moved) {
+    weighted_epilogue(L, v, sum, base, __ldg(L.W + v), L.perm ? __ldg(L.perm + v) : v,
+                      L.seed ? __ldg(L.seed + v) : 0.0f, L.rank_prev ? __ldg(L.rank_prev + v) : 0.0f, dang, moved);
 }
 
 __device__ __forceinline__ float pr_base(const RowGatherLaunch& L) {
@@ -126,7 +153,7 @@ __device__ __forceinline__ float pr_base(const RowGatherLaunch& L) {
 // same order as a plain loop would, so the sums are unchanged and each batch costs one round trip.
 template <int MODE>
 __device__ __forceinline__ void fixup_hubs(const RowGatherLaunch& L, int tid, int nthreads, int gwarp, int nwarps,
-                                           int lane, float base, double& dang) {
+                                           int lane, float base, double& dang, bool& moved) {
     // The epilogue inputs (out-degree, contribution slot) are loaded with the partials.
     for (int h = tid; h < L.plan.nhub_small; h += nthreads) {
         const int4 H = __ldg(L.plan.hubs_small + h);
@@ -142,7 +169,8 @@ __device__ __forceinline__ void fixup_hubs(const RowGatherLaunch& L, int tid, in
 #pragma unroll
         for (int s = 0; s < kSmallHubSegs; ++s) acc += p[s];
         if (MODE == kModeSpmv) L.y[H.x] = acc;
-        else pr_epilogue(L, H.x, acc, base, od, pos, dang);
+        else if (MODE == kModeWeighted) weighted_epilogue(L, H.x, acc, base, dang, moved);
+        else pr_epilogue(L, H.x, acc, base, od, pos, dang, moved);
     }
     for (int h = gwarp; h < L.plan.nhub_big; h += nwarps) {
         const int4 H = __ldg(L.plan.hubs_big + h);
@@ -162,7 +190,8 @@ __device__ __forceinline__ void fixup_hubs(const RowGatherLaunch& L, int tid, in
         acc = warp_sum_f32(acc);
         if (lane == 0) {
             if (MODE == kModeSpmv) L.y[H.x] = acc;
-            else pr_epilogue(L, H.x, acc, base, od, pos, dang);
+            else if (MODE == kModeWeighted) weighted_epilogue(L, H.x, acc, base, dang, moved);
+            else pr_epilogue(L, H.x, acc, base, od, pos, dang, moved);
         }
     }
 }
@@ -196,8 +225,10 @@ __device__ __forceinline__ double block_sum_f64(double v) {
 // One step of a warp covers KT consecutive tiles: first every column and epilogue load of all KT
 // tiles, then all their gathers, then the tiles are walked one after the other through the warp's
 // single staging area. A lane thus keeps KT x 8 gathers in flight instead of 8.
-template <int MODE, int KT>
+// CONV: sweeps with a convergence test (rank_prev given).
+template <int MODE, int KT, bool CONV>
 __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
+    if (!CONV) L.rank_prev = nullptr;
     extern __shared__ __align__(16) unsigned char rg_smem[];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -217,8 +248,9 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
     }
     __syncthreads();
     float base = 0.0f;
-    if (MODE == kModePagerank) base = pr_base(L);
+    if (MODE != kModeSpmv) base = pr_base(L);
     double dang = 0.0;
+    bool moved = false;
 
     const int ntiles = L.plan.ntiles;
     // Descriptors and lane walks of the next step are requested one step ahead.
@@ -284,7 +316,7 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             for (int i = 0; i < kIpl; ++i) {
                 const int j = i * 32 + lane;
                 const int c = cols[k][i];
-                if constexpr (MODE == kModeSpmv) {
+                if constexpr (has_vals(MODE)) {
                     const bool hot = c < L.hot;
                     const float hv = s_hot[hot ? c : 0];
                     float gv = 0.0f;
@@ -318,6 +350,16 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             // stores need no predicate; the walk reads only the first nnz of them as nonzeros.
 #pragma unroll
             for (int i = 0; i < kIpl; ++i) val[pad(i * 32 + lane)] = pv[k][i];
+            // Weighted sweeps: the epilogue inputs of the first 32 rows go out ahead of the walk (with
+            // the columns, as PageRank's do, their eight registers do not fit beside the values).
+            float eW = 0.0f, eseed = 0.0f, eprev = 0.0f;
+            int epos = row + lane;
+            if (MODE == kModeWeighted && lane < nrows) {
+                eW = ld_stream<MODE>(L.W + row + lane);
+                if (L.perm) epos = ld_stream<MODE>(L.perm + row + lane);
+                if (L.seed) eseed = ld_stream<MODE>(L.seed + row + lane);
+                if (L.rank_prev) eprev = ld_stream<MODE>(L.rank_prev + row + lane);
+            }
             __syncwarp();
             // Merge-path: lane owns merge items [d0, d1) starting at row r0; the plan's mask says
             // which of them are row ends (emit the open row) and which are nonzeros (take one).
@@ -358,20 +400,26 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
                 const float sum = out[pad(rr)];
                 if (MODE == kModeSpmv) {
                     L.y[row + rr] = sum;
+                } else if (MODE == kModeWeighted) {
+                    if (rr < 32) weighted_epilogue(L, row + rr, sum, base, eW, epos, eseed, eprev, dang, moved);
+                    else weighted_epilogue(L, row + rr, sum, base, dang, moved);
                 } else if (rr < 32) {
-                    pr_epilogue(L, row + rr, sum, base, od0[k], pos0[k], dang);
+                    pr_epilogue(L, row + rr, sum, base, od0[k], pos0[k], dang, moved);
                 } else if (rr < 64) {
-                    pr_epilogue(L, row + rr, sum, base, od1[k], pos1[k], dang);
+                    pr_epilogue(L, row + rr, sum, base, od1[k], pos1[k], dang, moved);
                 } else {
-                    pr_epilogue(L, row + rr, sum, base, dang);
+                    pr_epilogue(L, row + rr, sum, base, dang, moved);
                 }
             }
             __syncwarp();
         }
     }
-    if (MODE == kModePagerank) {
+    if (MODE != kModeSpmv) {
         dang = warp_sum_f64(dang);
         if (lane == 0) L.dpart[gwarp] = dang;
+        // One store per CTA at most: a store per moved row queued up on that one word (700,001 vertices,
+        // 11 M arcs: 50 us per sweep with it, 37 without; weighted sweep of R-MAT 20: 94 and 64 us).
+        if (CONV && __syncthreads_or(moved) && threadIdx.x == 0) *L.nonstop = 1u;
     }
 }
 
@@ -385,10 +433,12 @@ __global__ void __launch_bounds__(kFixBlock) hub_fixup_kernel(RowGatherLaunch L,
     const int gwarp = tid >> 5;
     const int nwarps = nthreads >> 5;
     float base = 0.0f;
-    if (MODE == kModePagerank) base = pr_base(L);
+    if (MODE != kModeSpmv) base = pr_base(L);
     double dang = 0.0;
-    fixup_hubs<MODE>(L, tid, nthreads, gwarp, nwarps, lane, base, dang);
-    if (MODE != kModePagerank) return;
+    bool moved = false;
+    fixup_hubs<MODE>(L, tid, nthreads, gwarp, nwarps, lane, base, dang, moved);
+    if (MODE == kModeSpmv) return;
+    if (L.nonstop && __syncthreads_or(moved) && threadIdx.x == 0) *L.nonstop = 1u;
     // Block b adds its slice of the gather warps' dangling partials to its own rows' (slices in
     // index order), leaves one partial, and the last block to finish adds those in block order.
     const int per = (gather_warps + gridDim.x - 1) / gridDim.x;
@@ -410,6 +460,11 @@ __global__ void __launch_bounds__(kFixBlock) hub_fixup_kernel(RowGatherLaunch L,
     if (threadIdx.x == 0) {
         *L.dsum_out = total;
         st->fix_count = 0u;
+        if (L.nonstop) {  // the sweep's verdict, straight to the host; the flag is clear for the next sweep
+            *reinterpret_cast<volatile unsigned*>(L.host_flag) = *reinterpret_cast<volatile unsigned*>(L.nonstop);
+            *L.nonstop = 0u;
+            __threadfence_system();
+        }
     }
 }
 
@@ -508,11 +563,11 @@ size_t rowgather_staging_bytes() { return sizeof(int) * kWarps * 2 * kPadded; }
 namespace {
 
 // Sets the kernel's dynamic shared-memory limit to what this launch needs (once per size).
-template <int MODE>
+template <int MODE, bool CONV>
 cudaError_t prepare_rowgather(size_t bytes) {
     static size_t configured = 0;
     if (bytes <= configured) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(rowgather_kernel<MODE, MODE == kModeSpmv ? DPG_GATHER_TILES_SPMV : DPG_GATHER_TILES_PR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(rowgather_kernel<MODE, has_vals(MODE) ? DPG_GATHER_TILES_SPMV : DPG_GATHER_TILES_PR, CONV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(bytes));
     if (e == cudaSuccess) configured = bytes;
     return e;
@@ -719,19 +774,19 @@ namespace {
 // A sweep: the gather kernel, then the hub fix-up kernel (which for PageRank also reduces the
 // dangling partials). Folding the fix-up into the gather behind a grid barrier (one cooperative
 // launch) measured only 0.6 % faster on R-MAT 22: the fix-up's round trips stay on the critical path.
-template <int MODE>
+template <int MODE, bool CONV>
 cudaError_t launch_row_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                              LaunchHook* hook) {
-    constexpr int KT = MODE == kModeSpmv ? DPG_GATHER_TILES_SPMV : DPG_GATHER_TILES_PR;
+    constexpr int KT = has_vals(MODE) ? DPG_GATHER_TILES_SPMV : DPG_GATHER_TILES_PR;
     int gb, fb, bt;
     rowgather_grid(sm_count, &gb, &fb, &bt);
     // At least one hot entry: the SpMV gather reads entry 0 for cold columns.
     const size_t smem = rowgather_staging_bytes() + sizeof(float) * static_cast<size_t>(L.hot > 0 ? L.hot : 1);
-    cudaError_t err = prepare_rowgather<MODE>(smem);
+    cudaError_t err = prepare_rowgather<MODE, CONV>(smem);
     if (err != cudaSuccess) return err;
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, stream);
-        rowgather_kernel<MODE, KT><<<gb, bt, smem, stream>>>(L);
+        rowgather_kernel<MODE, KT, CONV><<<gb, bt, smem, stream>>>(L);
     }
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
@@ -747,12 +802,19 @@ cudaError_t launch_row_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream
 
 cudaError_t launch_spmv(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                         LaunchHook* hook) {
-    return launch_row_sweep<kModeSpmv>(L, st, stream, sm_count, hook);
+    return launch_row_sweep<kModeSpmv, false>(L, st, stream, sm_count, hook);
+}
+
+cudaError_t launch_weighted_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
+                                  LaunchHook* hook) {
+    return L.rank_prev ? launch_row_sweep<kModeWeighted, true>(L, st, stream, sm_count, hook)
+                       : launch_row_sweep<kModeWeighted, false>(L, st, stream, sm_count, hook);
 }
 
 cudaError_t launch_pagerank_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                                   LaunchHook* hook) {
-    return launch_row_sweep<kModePagerank>(L, st, stream, sm_count, hook);
+    return L.rank_prev ? launch_row_sweep<kModePagerank, true>(L, st, stream, sm_count, hook)
+                       : launch_row_sweep<kModePagerank, false>(L, st, stream, sm_count, hook);
 }
 
 cudaError_t launch_pagerank_init(const RowGatherLaunch& L, float init_rank, float* rank_prev, DevStatus* st,
@@ -768,6 +830,7 @@ cudaError_t launch_pagerank_init(const RowGatherLaunch& L, float init_rank, floa
     if (err != cudaSuccess) return err;
     // A fix-up pass over no hubs reduces the initial dangling partials into dsum_out.
     RowGatherLaunch F = L;
+    F.nonstop = nullptr;
     F.plan.nhub_small = 0;
     F.plan.nhub_big = 0;
     {
