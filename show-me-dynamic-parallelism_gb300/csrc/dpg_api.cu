@@ -191,6 +191,8 @@ void graph_free_device(dpg_graph* g) {
     dev_free(g->ctx, g->perm);
     dev_free(g->ctx, g->inv);
     dev_free(g->ctx, g->pcol);
+    dev_free(g->ctx, g->items);
+    g->items = nullptr;
     dev_free(g->ctx, g->t_off);
     dev_free(g->ctx, g->t_col);
     g->perm = g->inv = g->pcol = g->t_off = g->t_col = nullptr;
@@ -311,17 +313,17 @@ dpg_status ensure_plan(dpg_graph* g) {
 #ifndef DPG_GATHER_SMEM_KB
 #define DPG_GATHER_SMEM_KB 164
 #endif
-int32_t hot_entries(const dpg_ctx* c, const dpg_graph* g) {
+int32_t hot_entries(const dpg_ctx* c, const dpg_graph* g, bool sweeps) {
     if (!g->relabel) return 0;
     // 1 KB of each carve-out is reserved per CTA by the system.
     const int64_t budget = std::min<int64_t>(c->smem_optin, DPG_GATHER_SMEM_KB * 1024 - 1024);
-    const int64_t room = budget - static_cast<int64_t>(rowgather_staging_bytes());
-    const int64_t cap = room > 0 ? room / 4 : 0;
+    const int64_t room = budget - static_cast<int64_t>(rowgather_staging_bytes(sweeps));
+    const int64_t cap = room > 4 ? room / 4 - 1 : 0;
     return static_cast<int32_t>(cap < g->V ? cap : g->V);
 }
 
-// Builds perm/inv/pcol for the row gathers: column counts, the frequency order (a 33-class stable
-// multi-split) and the renamed column array, all on the device. With relabel_segments (vertex
+// Builds perm/inv for the row gathers: column counts and the frequency order (a 33-class stable
+// multi-split), on the device. With relabel_segments (vertex
 // starts of packed graphs) each segment is ordered on its own (on the host, once per batch), so
 // renamed ids stay inside their graph's range and each graph's gathers stay inside its own slice.
 dpg_status ensure_relabel(dpg_graph* g) {
@@ -333,7 +335,6 @@ dpg_status ensure_relabel(dpg_graph* g) {
     DPG_CUDA_TRY(dev_alloc(c, &counts, nv * 4));
     cudaError_t e = dev_alloc(c, &g->perm, nv * 4);
     if (e == cudaSuccess) e = dev_alloc(c, &g->inv, nv * 4);
-    if (e == cudaSuccess) e = dev_alloc(c, &g->pcol, static_cast<size_t>(g->E > 0 ? g->E : 1) * 4);
     if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, nv * 4, c->stream);
     if (e == cudaSuccess) e = launch_column_histogram(g->col, g->E, counts, c->stream, c->sm_count);
     if (e == cudaSuccess && seg.size() < 2) {
@@ -363,17 +364,52 @@ dpg_status ensure_relabel(dpg_graph* g) {
             if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         }
     }
-    if (e == cudaSuccess) e = launch_relabel_columns(g->col, g->perm, g->E, g->pcol, c->stream, c->sm_count);
     dev_free(c, counts);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         dev_free(c, g->perm);
         dev_free(c, g->inv);
-        dev_free(c, g->pcol);
-        g->perm = g->inv = g->pcol = nullptr;
+        g->perm = g->inv = nullptr;
         return set_error(DPG_ERR_CUDA, std::string("column renaming: ") + cudaGetErrorString(e));
     }
     g->relabel_ready = true;
+    return DPG_OK;
+}
+
+// The renamed columns in CSR order (SpMV).
+dpg_status ensure_pcol(dpg_graph* g) {
+    DPG_TRY(ensure_relabel(g));
+    if (g->pcol || g->V == 0) return DPG_OK;
+    dpg_ctx* c = g->ctx;
+    cudaError_t e = dev_alloc(c, &g->pcol, static_cast<size_t>(g->E > 0 ? g->E : 1) * 4);
+    if (e == cudaSuccess) e = launch_relabel_columns(g->col, g->perm, g->E, g->pcol, c->stream, c->sm_count);
+    if (e != cudaSuccess) {
+        dev_free(c, g->pcol);
+        g->pcol = nullptr;
+        return set_error(DPG_ERR_CUDA, std::string("column renaming: ") + cudaGetErrorString(e));
+    }
+    return DPG_OK;
+}
+
+// The tiles' merge items (PageRank sweeps), with the graph's current choice of renaming.
+dpg_status ensure_items(dpg_graph* g) {
+    DPG_TRY(ensure_plan(g));
+    if (g->relabel) DPG_TRY(ensure_relabel(g));
+    if (g->V == 0 || (g->items && g->items_relabel == g->relabel)) return DPG_OK;
+    dpg_ctx* c = g->ctx;
+    cudaError_t e = cudaSuccess;
+    if (!g->items)
+        e = dev_alloc(c, &g->items, sizeof(int32_t) * kRowTileItems * (static_cast<size_t>(g->plan.ntiles) + 1));
+    // A one-shot graph has its columns renamed already (graph_create_pull).
+    const int32_t* col = g->relabel && g->pcol ? g->pcol : g->col;
+    const int32_t* perm = g->relabel && !g->pcol ? g->perm : nullptr;
+    if (e == cudaSuccess) e = launch_tile_items(g->plan, col, perm, g->items, c->stream, c->sm_count);
+    if (e != cudaSuccess) {
+        dev_free(c, g->items);
+        g->items = nullptr;
+        return set_error(DPG_ERR_CUDA, std::string("merge items: ") + cudaGetErrorString(e));
+    }
+    g->items_relabel = g->relabel;
     return DPG_OK;
 }
 
@@ -697,8 +733,7 @@ dpg_status run_pagerank(dpg_ctx* c, dpg_graph* g, const int32_t* d_outdeg, const
     dpg_pr_opts o;
     DPG_TRY(pr_defaults(in_opts, &o));
     if (g->V == 0) return DPG_OK;
-    DPG_TRY(ensure_plan(g));
-    if (g->relabel) DPG_TRY(ensure_relabel(g));
+    DPG_TRY(ensure_items(g));
     int gb, fb, bt;
     rowgather_grid(c->sm_count, &gb, &fb, &bt);
     dpg_status st = DPG_OK;
@@ -720,11 +755,9 @@ dpg_status run_pagerank(dpg_ctx* c, dpg_graph* g, const int32_t* d_outdeg, const
     RowGatherLaunch L;
     memset(&L, 0, sizeof(L));
     L.plan = g->plan;
-    L.off = g->off;
-    L.col = g->relabel ? g->pcol : g->col;
+    L.items = g->items;
     L.perm = g->relabel ? g->perm : nullptr;
-    L.hot = hot_entries(c, g);
-    L.vals = nullptr;
+    L.hot = hot_entries(c, g, true);
     L.partial = partial;
     L.V = g->V;
     L.outdeg = d_outdeg;
@@ -809,7 +842,7 @@ dpg_status run_spmv(dpg_ctx* c, dpg_graph* g, const float* d_vals, const float* 
     if (g->V == 0) return DPG_OK;
     if (!d_x || !d_y || (g->E > 0 && !d_vals)) return set_error(DPG_ERR_INVALID_ARG, "null vals/x/y");
     DPG_TRY(ensure_plan(g));
-    if (g->relabel) DPG_TRY(ensure_relabel(g));
+    if (g->relabel) DPG_TRY(ensure_pcol(g));
     dpg_status st = DPG_OK;
     float* partial = static_cast<float*>(arena(c, S_PARTIAL, static_cast<size_t>(g->plan.nseg + 1) * 4, &st));
     float* xp = g->relabel ? static_cast<float*>(arena(c, S_XPERM, static_cast<size_t>(g->V) * 4, &st)) : nullptr;
@@ -822,7 +855,7 @@ dpg_status run_spmv(dpg_ctx* c, dpg_graph* g, const float* d_vals, const float* 
     L.col = g->relabel ? g->pcol : g->col;
     L.vals = d_vals;
     L.x = xp ? xp : d_x;
-    L.hot = hot_entries(c, g);
+    L.hot = hot_entries(c, g, false);
     L.y = d_y;
     L.partial = partial;
     L.V = g->V;
@@ -1047,16 +1080,14 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
     DPG_TRY(ensure_spmm_transpose(g, true));
     DPG_TRY(ensure_spmm_plan(g));
     dpg_graph* tg = g->tgraph;
-    for (dpg_graph* p : {g, tg}) {
-        DPG_TRY(ensure_plan(p));
-        if (p->relabel) DPG_TRY(ensure_relabel(p));
-    }
-    const size_t nv = static_cast<size_t>(g->V), ne = static_cast<size_t>(g->E > 0 ? g->E : 1);
+    for (dpg_graph* p : {g, tg}) DPG_TRY(ensure_items(p));
+    const size_t nv = static_cast<size_t>(g->V);
     const int nb = pr_vec_blocks(c->sm_count);
     int gb, fb, bt;
     rowgather_grid(c->sm_count, &gb, &fb, &bt);
     dpg_status st = DPG_OK;
-    float* w_t = static_cast<float*>(arena(c, S_VALS_T, ne * 4, &st));
+    const size_t ntiles = static_cast<size_t>(std::max(g->plan.ntiles, tg->plan.ntiles));
+    float* witems = static_cast<float*>(arena(c, S_PRG_WITEMS, sizeof(float) * kRowTileItems * (ntiles + 1), &st));
     float* W = static_cast<float*>(arena(c, S_PRG_W, nv * 4, &st));
     float* y = static_cast<float*>(arena(c, S_PRG_Y, nv * 4, &st));
     float* contrib = static_cast<float*>(arena(c, S_PRG_C, nv * 4, &st));
@@ -1075,10 +1106,9 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
     unsigned* flags = static_cast<unsigned*>(arena(c, S_PRG_FLAGS, 16, &st));  // [0] ticket, [1] nonstop
     if (st != DPG_OK) return st;
     DPG_CUDA_TRY(cudaMemsetAsync(flags, 0, 16, c->stream));
-    // Out-weight sums W = A 1 and the weights in transposed-slot order.
+    // Out-weight sums W = A 1.
     DPG_CUDA_TRY(launch_fill_f32(y, g->V, 1.0f, c->stream, c->sm_count));
     DPG_TRY(run_spmv(c, g, d_w, y, W));
-    DPG_CUDA_TRY(launch_gather_values(d_w, g->tt_arc, g->E, w_t, c->stream, c->sm_count));
 
     // The convergence test is pipelined one sweep deep: sweep it+1 is queued before the host reads
     // sweep it's flag (written to pinned memory by the sweep's last kernel, behind an event), so the
@@ -1105,21 +1135,22 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
     L.dpart = dpart;
     L.dfix = dfix;
     L.W = W;
-    // Sweeps over graph sg with arc values vals; `start` is the vector gathered first, in vertex order.
+    // Sweeps over graph sg, whose arc k weighs d_w[arc[k]] (arc null: d_w[k]); `start` is the vector
+    // gathered first, in vertex order.
     // The gathered vectors x[0], x[1] are in sg's renamed order; sweeps leave entries of x that they do
     // not write (contributions of W == 0) as they were, so both start with the first vector.
-    auto sweeps_until = [&](int32_t cap, double eps, float** cur, float** nxt, dpg_graph* sg, const float* vals,
-                            const float* start, int64_t* done) -> dpg_status {
+    auto sweeps_until = [&](int32_t cap, double eps, float** cur, float** nxt, dpg_graph* sg,
+                            const int32_t* arc, const float* start, int64_t* done) -> dpg_status {
+        DPG_CUDA_TRY(launch_tile_values(sg->plan, d_w, arc, witems, c->stream, c->sm_count));
         for (float* xb : x) {
             if (sg->relabel) DPG_CUDA_TRY(launch_gather_by_index(start, sg->inv, sg->V, xb, c->stream, c->sm_count));
             else DPG_CUDA_TRY(cudaMemcpyAsync(xb, start, nv * 4, cudaMemcpyDeviceToDevice, c->stream));
         }
         L.plan = sg->plan;
-        L.off = sg->off;
-        L.col = sg->relabel ? sg->pcol : sg->col;
+        L.items = sg->items;
+        L.witems = witems;
         L.perm = sg->relabel ? sg->perm : nullptr;
-        L.hot = hot_entries(c, sg);
-        L.vals = vals;
+        L.hot = hot_entries(c, sg, true);
         L.epsilon = static_cast<float>(eps);
         // Every loop starts from the reduction its init pass left in red[0].
         int32_t pending = -1;  // sweep whose flag is on its way to the host
@@ -1170,7 +1201,7 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
     DPG_CUDA_TRY(launch_pr_vec_init(I, c->sm_count, c->stream, &c->prof));
     L.base_const = (1.0 - o.damping) * o.total_rank / static_cast<double>(g->V);
     int64_t fwd = 0, adj = 0;
-    DPG_TRY(sweeps_until(fwd_iters, o.epsilon, &r_cur, &r_nxt, tg, w_t, contrib, &fwd));
+    DPG_TRY(sweeps_until(fwd_iters, o.epsilon, &r_cur, &r_nxt, tg, g->tt_arc, contrib, &fwd));
 
     // Adjoint: lambda in vec[2]/vec[3], its sum in red[0].
     float* l_cur = vec[2];
@@ -1180,7 +1211,7 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
     DPG_CUDA_TRY(launch_pr_vec_init(I, c->sm_count, c->stream, &c->prof));
     L.base_const = 0.0;
     L.seed = d_seed;
-    DPG_TRY(sweeps_until(adj_iters, adjoint_epsilon, &l_cur, &l_nxt, g, d_w, d_seed, &adj));
+    DPG_TRY(sweeps_until(adj_iters, adjoint_epsilon, &l_cur, &l_nxt, g, nullptr, d_seed, &adj));
 
     // q = (A lambda) / W with the final lambda, then the per-arc gradient.
     DPG_TRY(run_spmv(c, g, d_w, l_cur, y));
@@ -1424,12 +1455,12 @@ dpg_status dpg_graph_hot_cache(dpg_graph* g, int32_t* hot_entries_out, int64_t* 
     if (!g || !g->ctx) return set_error(DPG_ERR_INVALID_ARG, "null graph or destroyed context");
     dpg_ctx* c = g->ctx;
     DPG_TRY(use_device(c));
-    const int32_t hot = hot_entries(c, g);
+    const int32_t hot = hot_entries(c, g, true);
     if (hot_entries_out) *hot_entries_out = hot;
     if (!hot_arcs) return DPG_OK;
     *hot_arcs = 0;
     if (hot == 0 || g->E == 0) return DPG_OK;
-    DPG_TRY(ensure_relabel(g));
+    DPG_TRY(ensure_pcol(g));
     unsigned long long* d = nullptr;
     DPG_CUDA_TRY(cudaMalloc(&d, sizeof(unsigned long long)));
     cudaError_t e = cudaMemsetAsync(d, 0, sizeof(unsigned long long), c->stream);

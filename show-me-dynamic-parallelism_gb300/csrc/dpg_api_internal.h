@@ -32,7 +32,7 @@ namespace dpg_api {
 enum Slot {
     S_QV0, S_QV1, S_QSE0, S_QSE1, S_BMP0, S_BMP1, S_CH0, S_CH1, S_QCOUNT, S_CCOUNT, S_LABEL, S_CONTRIB0, S_CONTRIB1, S_RANK0, S_RANK1,
     S_PARTIAL, S_DPART, S_DFIX, S_DSUM, S_NONSTOP, S_VALS, S_X, S_Y, S_OUTDEG, S_RANKOUT, S_XPERM, S_PENDING, S_SPMM_PARTIAL, S_SPMM_COUNTS, S_VALS_T, S_DA_T,
-    S_PRG_W, S_PRG_Y, S_PRG_C, S_PRG_X0, S_PRG_X1, S_PRG_V0, S_PRG_V1, S_PRG_V2, S_PRG_V3, S_PRG_PART, S_PRG_RED, S_PRG_FLAGS,
+    S_PRG_W, S_PRG_Y, S_PRG_C, S_PRG_X0, S_PRG_X1, S_PRG_WITEMS, S_PRG_V0, S_PRG_V1, S_PRG_V2, S_PRG_V3, S_PRG_PART, S_PRG_RED, S_PRG_FLAGS,
     S_DIRTY0, S_DIRTY1,
     S_CDP_BUF0, S_CDP_BUF1, S_CDP_WORDS,
     S_TRANSPOSE, S_TRANSPOSE_ARC, S_DO_COUNT, S_FAR0, S_FAR1, S_FAR2, S_FAR_COUNT, S_PLANINFO,
@@ -158,7 +158,9 @@ struct dpg_graph {
     bool relabel_ready = false;
     int32_t* perm = nullptr;  // old column id -> new
     int32_t* inv = nullptr;   // new -> old
-    int32_t* pcol = nullptr;  // col[e] renamed
+    int32_t* pcol = nullptr;  // col[e] renamed (SpMV), built on first use
+    int32_t* items = nullptr;  // the tiles' merge items (PageRank sweeps), built on first use; renamed:
+    bool items_relabel = false;
     std::vector<int32_t> relabel_segments;  // optional vertex starts: rename within each segment
     // Transposed CSR (in-arcs), built on first use by colouring.
     int32_t* t_off = nullptr;
@@ -218,7 +220,8 @@ cudaError_t plan_build_launch(const PlanBuild& pb, const int32_t* d_off, int32_t
 dpg_status plan_finish(dpg_graph* g, PlanBuild* pb, const PlanInfo& info);
 void plan_build_free(dpg_ctx* c, PlanBuild* pb);
 dpg_status ensure_relabel(dpg_graph* g);
-int32_t hot_entries(const dpg_ctx* c, const dpg_graph* g);
+dpg_status ensure_items(dpg_graph* g);
+int32_t hot_entries(const dpg_ctx* c, const dpg_graph* g, bool sweeps);
 dpg_status pr_defaults(const dpg_pr_opts* in, dpg_pr_opts* o);
 void batch_orphan(dpg_batch* b);
 dpg_status expand_workspace(dpg_ctx* c, int32_t V, int64_t E, int32_t min_chunked, ExpandWorkspace* wsp);

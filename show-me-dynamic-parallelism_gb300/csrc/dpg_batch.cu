@@ -181,8 +181,7 @@ dpg_status upload(dpg_ctx* c, T** dst, const T* src, size_t count) {
 dpg_status ensure_dslot(dpg_batch* b) {
     if (b->dslot_ready) return DPG_OK;
     dpg_ctx* c = b->ctx;
-    DPG_TRY(ensure_plan(b->in));
-    if (b->in->relabel) DPG_TRY(ensure_relabel(b->in));
+    DPG_TRY(ensure_items(b->in));
     DPG_CUDA_TRY(cudaMalloc(&b->dslot, sizeof(int32_t) * (b->ndang > 0 ? b->ndang : 1)));
     if (b->ndang > 0) {
         if (b->in->relabel) {
@@ -225,7 +224,7 @@ dpg_status pr_buffers(dpg_batch* b, PrBuffers* pb) {
 }
 
 int32_t pr_hot(const dpg_batch* b) {
-    const int32_t cap = hot_entries(b->ctx, b->in);
+    const int32_t cap = hot_entries(b->ctx, b->in, true);
     if (b->tune.pr_hot < 0) return cap;
     return std::min(cap, b->tune.pr_hot);
 }
@@ -241,8 +240,7 @@ dpg_status run_batch_pagerank(dpg_batch* b, const PrBuffers& pb, const dpg_pr_op
     RowGatherLaunch L;
     memset(&L, 0, sizeof(L));
     L.plan = g->plan;
-    L.off = g->off;
-    L.col = g->relabel ? g->pcol : g->col;
+    L.items = g->items;
     L.perm = g->relabel ? g->perm : nullptr;
     L.hot = pr_hot(b);
     L.partial = pb.partial;
@@ -811,7 +809,7 @@ dpg_status dpg_batch_autotune(dpg_ctx* c, dpg_batch* b, int32_t nsrc, const int3
     pr_defaults(nullptr, &o);
     o.iterations = 3;
     float best_pr = 1e30f;
-    const int32_t cap = hot_entries(c, b->in);
+    const int32_t cap = hot_entries(c, b->in, true);
     for (int32_t hot : {0, 4096, 16384, -1}) {
         if (st != DPG_OK) break;
         if (hot > cap) continue;

@@ -162,7 +162,9 @@ struct RowGatherLaunch {
     RowPlanDev plan;
     const int32_t* off;
     const int32_t* col;
-    const float* vals;      // SpMV values; nullptr for PageRank
+    const float* vals;      // SpMV values
+    const int32_t* items;   // sweeps: the merge items of every tile (launch_tile_items)
+    const float* witems;    // weighted sweeps: the arc values in the order of items
     const float* x;         // SpMV x / PageRank contribution in
     int32_t hot;            // x[0, hot) is staged in shared memory (the most gathered renamed columns)
     float* y;               // SpMV y / PageRank contribution out
@@ -321,8 +323,17 @@ cudaError_t launch_tile_lane_starts_dev(const int4* tiles, const int64_t* d_ntil
 
 // Grid shape used by the row-gather kernels (needed to size dpart/dfix).
 void rowgather_grid(int sm_count, int* gather_blocks, int* fix_blocks, int* block_threads);
-// Shared memory the gather kernel needs besides the hot-value cache.
-size_t rowgather_staging_bytes();
+// Shared memory the gather kernel (of the PageRank sweeps, or of SpMV) needs besides the hot-value cache.
+size_t rowgather_staging_bytes(bool sweeps);
+// The merge items of the plan's tiles for the sweeps: 256 per tile, renamed column perm[col[k]] (perm
+// nullable), kItemRowEnd or kItemNone, and arc values vals[arc[k]] (arc nullable) in the same order
+// (0 at the marks).
+constexpr int32_t kItemRowEnd = INT32_MIN;
+constexpr int32_t kItemNone = -1;
+cudaError_t launch_tile_items(const RowPlanDev& plan, const int32_t* col, const int32_t* perm, int32_t* items,
+                              cudaStream_t s, int sm_count);
+cudaError_t launch_tile_values(const RowPlanDev& plan, const float* vals, const int32_t* arc, float* out, cudaStream_t s,
+                               int sm_count);
 
 cudaError_t launch_spmv(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                         LaunchHook* hook);

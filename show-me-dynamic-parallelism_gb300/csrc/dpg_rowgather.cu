@@ -7,10 +7,12 @@
 //
 // Here the rows are cut (on the device, once per graph) into warp tiles of at most 256 merge items
 // (rows + nonzeros):
-//   - a normal tile holds whole rows of degree <= 255; one warp stages the tile's gathered
-//     products in shared memory, each lane walks 8 consecutive merge items (merge-path over row
-//     ends and nonzeros, from a start row and a row-end mask the plan keeps per lane), and a warp
-//     segmented scan joins rows that cross lanes;
+//   - a normal tile holds whole rows of degree <= 255; each lane walks 8 consecutive merge items
+//     (merge-path over row ends and nonzeros), and a warp segmented scan joins rows that cross lanes.
+//     SpMV stages the gathered products in shared memory and walks them with a start row and a row-end
+//     mask that the plan keeps per lane; the sweeps of PageRank read a stream of the merge items
+//     themselves (renamed column or row-end mark), laid out so that a lane's 8 come with two 16-byte
+//     loads, and walk in registers;
 //   - a row of degree > 255 (a hub) is split into 256-nonzero segments whose partial sums are
 //     combined afterwards, in segment order, by the hub fix-up kernel.
 // Every sum has a fixed order, so results are bit-reproducible run to run; no float atomics.
@@ -42,8 +44,8 @@ constexpr int kInitBlock = 256;
 constexpr int kIpl = kRowTileItems / 32;  // merge items per lane
 constexpr int kFixBlock = 256;
 constexpr int kFixBatch = 8;  // loads the fix-up issues before it adds them
-// Tiles a warp carries through one step (see rowgather_kernel), per mode. Measured on R-MAT scale
-// 22 (PageRank sweep, 1024-thread CTAs): what limits the gathers is the L1 left beside the shared
+// Tiles a warp of the SpMV carries through one step. Measured on R-MAT scale 22 with the PageRank sweep
+// that shared this kernel (1024-thread CTAs): what limits the gathers is the L1 left beside the shared
 // memory, where their sectors in flight need lines (the shared-memory budget is set with the
 // hot-cache size, see hot_entries). With a 28 KB L1 one tile per step ran best (0.29 ms per sweep);
 // with 92 KB, two tiles run 0.202 ms against 0.216 ms with one. Fewer warps lose at any setting
@@ -51,19 +53,14 @@ constexpr int kFixBatch = 8;  // loads the fix-up issues before it adds them
 #ifndef DPG_GATHER_TILES_SPMV
 #define DPG_GATHER_TILES_SPMV 2
 #endif
-#ifndef DPG_GATHER_TILES_PR
-#define DPG_GATHER_TILES_PR 2
-#endif
 // Shared-memory index with one pad word per 32: lane l walking items 8l.. then hits 32 distinct banks
 // instead of 4 (an 8-way conflict without the pad).
 constexpr int kPadded = kRowTileItems + kRowTileItems / 32;
 __device__ __forceinline__ int pad(int i) { return i + (i >> 5); }
 
 enum { kModeSpmv = 0, kModePagerank = 1, kModeWeighted = 2 };
-// SpMV and weighted PageRank sweeps multiply by arc values.
-constexpr bool has_vals(int mode) { return mode != kModePagerank; }
 
-// Loads of the streams every tile reads once (columns, SpMV values, out-degrees, renaming slots):
+// Loads of the streams every tile reads once (columns, values, items, epilogue inputs):
 // read-only for the launch (nc) and kept out of L1 (L1::no_allocate), so the L1 lines are left to
 // the scattered gathers of x, which are what a sweep waits on. SpMV also marks them first for
 // eviction from L2, which keeps more of x there. Measured per launch (R-MAT 22; R-MAT 24 for
@@ -72,7 +69,7 @@ constexpr bool has_vals(int mode) { return mode != kModePagerank; }
 template <int MODE>
 __device__ __forceinline__ int ld_stream(const int* p) {
     int v;
-    if constexpr (has_vals(MODE)) {
+    if constexpr (MODE == kModeSpmv) {
         asm("{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
             "ld.global.nc.L1::no_allocate.L2::cache_hint.s32 %0, [%1], pol;\n\t}"
             : "=r"(v) : "l"(p));
@@ -84,13 +81,20 @@ __device__ __forceinline__ int ld_stream(const int* p) {
 template <int MODE>
 __device__ __forceinline__ float ld_stream(const float* p) {
     float v;
-    if constexpr (has_vals(MODE)) {
+    if constexpr (MODE == kModeSpmv) {
         asm("{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
             "ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], pol;\n\t}"
             : "=f"(v) : "l"(p));
     } else {
         asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
     }
+    return v;
+}
+
+// 16 bytes of a stream, zero unless `in`; never kept in L1.
+__device__ __forceinline__ int4 ld_stream4(const int4* p, bool in) {
+    int4 v = make_int4(kItemNone, kItemNone, kItemNone, kItemNone);
+    if (in) asm("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 
@@ -222,22 +226,9 @@ __device__ __forceinline__ double block_sum_f64(double v) {
     return total;
 }
 
-// One step of a warp covers KT consecutive tiles: first every column and epilogue load of all KT
-// tiles, then all their gathers, then the tiles are walked one after the other through the warp's
-// single staging area. A lane thus keeps KT x 8 gathers in flight instead of 8.
-// CONV: sweeps with a convergence test (rank_prev given).
-template <int MODE, int KT, bool CONV>
-__global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
-    if (!CONV) L.rank_prev = nullptr;
-    extern __shared__ __align__(16) unsigned char rg_smem[];
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const int gwarp = blockIdx.x * kWarps + warp;
-    const int nwarps = gridDim.x * kWarps;
-    float* val = reinterpret_cast<float*>(rg_smem) + warp * (2 * kPadded);
-    float* out = val + kPadded;
-    float* s_hot = reinterpret_cast<float*>(rg_smem) + kWarps * 2 * kPadded;
-    // Hot-cache fill, loads issued in batches of 8 (one round trip each instead of one per entry).
+// The hot cache: the first `hot` (most gathered) entries of x, loads issued in batches of 8 (one round
+// trip each instead of one per entry).
+__device__ __forceinline__ void fill_hot(const RowGatherLaunch& L, float* s_hot) {
     for (int i0 = threadIdx.x; i0 < L.hot; i0 += kBlock * 8) {
         float h[8];
 #pragma unroll
@@ -247,10 +238,22 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             if (i0 + kBlock * q < L.hot) s_hot[i0 + kBlock * q] = h[q];
     }
     __syncthreads();
-    float base = 0.0f;
-    if (MODE != kModeSpmv) base = pr_base(L);
-    double dang = 0.0;
-    bool moved = false;
+}
+
+// SpMV. One step of a warp covers KT consecutive tiles: first every column load of all KT tiles, then
+// all their gathers, then the tiles are walked one after the other through the warp's single staging
+// area. A lane thus keeps KT x 8 gathers in flight instead of 8.
+template <int KT>
+__global__ void __launch_bounds__(kBlock) spmv_gather_kernel(RowGatherLaunch L) {
+    extern __shared__ __align__(16) unsigned char rg_smem[];
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int gwarp = blockIdx.x * kWarps + warp;
+    const int nwarps = gridDim.x * kWarps;
+    float* val = reinterpret_cast<float*>(rg_smem) + warp * (2 * kPadded);
+    float* out = val + kPadded;
+    float* s_hot = reinterpret_cast<float*>(rg_smem) + kWarps * 2 * kPadded;
+    fill_hot(L, s_hot);
 
     const int ntiles = L.plan.ntiles;
     // Descriptors and lane walks of the next step are requested one step ahead.
@@ -264,36 +267,19 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
     }
     for (int t0 = gwarp * KT; t0 < ntiles; t0 += nwarps * KT) {
         int4 T[KT];
-        int info[KT], od0[KT], pos0[KT], od1[KT], pos1[KT];
+        int info[KT];
         float pv[KT][kIpl];
-        // Phase 1: columns and the epilogue inputs of the first 32 rows of every tile.
+        // Phase 1: columns.
         int cols[KT][kIpl];
 #pragma unroll
         for (int k = 0; k < KT; ++k) {
             T[k] = Tn[k];
             info[k] = infon[k];
-            const int row = T[k].x, nrows = T[k].y, nb = T[k].z, nnz = T[k].w;
+            const int nb = T[k].z, nnz = T[k].w;
 #pragma unroll
             for (int i = 0; i < kIpl; ++i) {
                 const int j = i * 32 + lane;
-                cols[k][i] = j < nnz ? ld_stream<MODE>(L.col + nb + j) : 0;
-            }
-            // Predicated loads rather than branches, so they go out with the column loads.
-            od0[k] = 0;
-            pos0[k] = 0;
-            od1[k] = 0;
-            pos1[k] = 0;
-            if (MODE == kModePagerank) {
-                const bool in0 = lane < nrows, in1 = lane + 32 < nrows;
-                od0[k] = in0 ? ld_stream<MODE>(L.outdeg + row + lane) : 0;
-                od1[k] = in1 ? ld_stream<MODE>(L.outdeg + row + lane + 32) : 0;
-                if (L.perm) {
-                    pos0[k] = in0 ? ld_stream<MODE>(L.perm + row + lane) : 0;
-                    pos1[k] = in1 ? ld_stream<MODE>(L.perm + row + lane + 32) : 0;
-                } else {
-                    pos0[k] = row + lane;
-                    pos1[k] = row + lane + 32;
-                }
+                cols[k][i] = j < nnz ? ld_stream<kModeSpmv>(L.col + nb + j) : 0;
             }
         }
 #pragma unroll
@@ -302,13 +288,10 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             Tn[k] = t < ntiles ? __ldg(L.plan.tiles + t) : make_int4(0, 0, 0, 0);
             infon[k] = t < ntiles ? __ldg(L.plan.lane_info + t * 32 + lane) : 0;
         }
-        // Phase 2: the gathers of every tile. Both forms keep the hot test a select between a shared
-        // and a global load (written as an if/else it became a divergent branch: PageRank 0.192 ms
-        // per sweep against 0.176 ms). PageRank keeps its gathers under the (almost always warp-
-        // uniform) `j < nnz` test. SpMV issues them with no branch at all, the shared-memory read
-        // unconditional (entry 0 for cold columns; the launch allocates at least one) and the
-        // value load predicated, so the gather and its value load go out together: 204 -> 255 GTEPS
-        // on R-MAT 22. The unconditional shared read costs PageRank 1.4 %, hence the two forms.
+        // Phase 2: the gathers of every tile, with no branch at all: the hot test is a select, the
+        // shared-memory read unconditional (entry 0 for cold columns; the launch allocates at least
+        // one) and the value load predicated, so the gather and its value load go out together: 204 ->
+        // 255 GTEPS on R-MAT 22.
 #pragma unroll
         for (int k = 0; k < KT; ++k) {
             const int nb = T[k].z, nnz = T[k].w;
@@ -316,18 +299,12 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             for (int i = 0; i < kIpl; ++i) {
                 const int j = i * 32 + lane;
                 const int c = cols[k][i];
-                if constexpr (has_vals(MODE)) {
-                    const bool hot = c < L.hot;
-                    const float hv = s_hot[hot ? c : 0];
-                    float gv = 0.0f;
-                    if (!hot) gv = __ldg(L.x + c);
-                    const float a = j < nnz ? ld_stream<MODE>(L.vals + nb + j) : 0.0f;
-                    pv[k][i] = j < nnz ? (hot ? hv : gv) * a : 0.0f;
-                } else {
-                    float v = 0.0f;
-                    if (j < nnz) v = c < L.hot ? s_hot[c] : __ldg(L.x + c);
-                    pv[k][i] = v;
-                }
+                const bool hot = c < L.hot;
+                const float hv = s_hot[hot ? c : 0];
+                float gv = 0.0f;
+                if (!hot) gv = __ldg(L.x + c);
+                const float a = j < nnz ? ld_stream<kModeSpmv>(L.vals + nb + j) : 0.0f;
+                pv[k][i] = j < nnz ? (hot ? hv : gv) * a : 0.0f;
             }
         }
 
@@ -350,16 +327,6 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             // stores need no predicate; the walk reads only the first nnz of them as nonzeros.
 #pragma unroll
             for (int i = 0; i < kIpl; ++i) val[pad(i * 32 + lane)] = pv[k][i];
-            // Weighted sweeps: the epilogue inputs of the first 32 rows go out ahead of the walk (with
-            // the columns, as PageRank's do, their eight registers do not fit beside the values).
-            float eW = 0.0f, eseed = 0.0f, eprev = 0.0f;
-            int epos = row + lane;
-            if (MODE == kModeWeighted && lane < nrows) {
-                eW = ld_stream<MODE>(L.W + row + lane);
-                if (L.perm) epos = ld_stream<MODE>(L.perm + row + lane);
-                if (L.seed) eseed = ld_stream<MODE>(L.seed + row + lane);
-                if (L.rank_prev) eprev = ld_stream<MODE>(L.rank_prev + row + lane);
-            }
             __syncwarp();
             // Merge-path: lane owns merge items [d0, d1) starting at row r0; the plan's mask says
             // which of them are row ends (emit the open row) and which are nonzeros (take one).
@@ -396,31 +363,162 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             const int kin = __shfl_up_sync(kFullMask, key, 1);
             if (lane > 0 && first_emit >= 0 && kin == first_emit) out[pad(first_emit)] += cin;
             __syncwarp();
-            for (int rr = lane; rr < nrows; rr += 32) {
-                const float sum = out[pad(rr)];
-                if (MODE == kModeSpmv) {
-                    L.y[row + rr] = sum;
-                } else if (MODE == kModeWeighted) {
-                    if (rr < 32) weighted_epilogue(L, row + rr, sum, base, eW, epos, eseed, eprev, dang, moved);
-                    else weighted_epilogue(L, row + rr, sum, base, dang, moved);
-                } else if (rr < 32) {
-                    pr_epilogue(L, row + rr, sum, base, od0[k], pos0[k], dang, moved);
-                } else if (rr < 64) {
-                    pr_epilogue(L, row + rr, sum, base, od1[k], pos1[k], dang, moved);
-                } else {
-                    pr_epilogue(L, row + rr, sum, base, dang, moved);
-                }
-            }
+            for (int rr = lane; rr < nrows; rr += 32) L.y[row + rr] = out[pad(rr)];
             __syncwarp();
         }
     }
-    if (MODE != kModeSpmv) {
-        dang = warp_sum_f64(dang);
-        if (lane == 0) L.dpart[gwarp] = dang;
-        // One store per CTA at most: a store per moved row queued up on that one word (700,001 vertices,
-        // 11 M arcs: 50 us per sweep with it, 37 without; weighted sweep of R-MAT 20: 94 and 64 us).
-        if (CONV && __syncthreads_or(moved) && threadIdx.x == 0) *L.nonstop = 1u;
+}
+
+// Sweeps of PageRank and of the weighted PageRank. A lane's 8 merge items of a tile arrive as two
+// 16-byte loads and stay in registers with their gathered values, so only the row sums pass through
+// shared memory; the next tile's items, descriptor and start rows are loaded while this one's gathers
+// are in flight, so a tile costs one round trip.
+// What bounds it: the load-store pipe (a gathered line, or a shared-memory wavefront, per cycle and SM)
+// and the instruction issue. Walking values staged in shared memory took 490 warp instructions per
+// tile, both pipes at 65-69 % (R-MAT 20). Same box, 20 sweeps with the staged walk, two tiles per step /
+// this one with two tiles per step / one / one with its items a step ahead: R-MAT 22 3.54 / 3.29 /
+// 3.19 / 3.15 ms, 608,712 vertices x 16 810 / 723 / 705 / 682 us; gradient of R-MAT 20 10.8 / 9.6 / 9.0 /
+// 8.55 ms. Three tiles per step spill (4.6 ms). Shared-memory budgets (hot cache) of 132 / 164 / 196
+// KB: R-MAT 22 3.23 / 3.16 / 3.31 ms.
+// CONV: sweeps with a convergence test (rank_prev given).
+template <int MODE, bool CONV>
+__global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
+    if (!CONV) L.rank_prev = nullptr;
+    extern __shared__ __align__(16) unsigned char rg_smem[];
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int gwarp = blockIdx.x * kWarps + warp;
+    const int nwarps = gridDim.x * kWarps;
+    float* out = reinterpret_cast<float*>(rg_smem) + warp * kPadded;
+    float* s_hot = reinterpret_cast<float*>(rg_smem) + kWarps * kPadded + 1;
+    if (threadIdx.x == 0) s_hot[-1] = 0.0f;  // what the marks gather
+    fill_hot(L, s_hot);
+    const float base = pr_base(L);
+    double dang = 0.0;
+    bool moved = false;
+
+    const int ntiles = L.plan.ntiles;
+    int2 Tn;          // the next tile: {row, nrows}, start row of the lane, items
+    int infon;
+    int4 qn[kIpl / 4];
+    int4 wn[kIpl / 4];  // weighted: arc values
+    auto fetch = [&](int t) {
+        const bool in = t < ntiles;
+        Tn = in ? __ldg(reinterpret_cast<const int2*>(L.plan.tiles + t)) : make_int2(0, 0);
+        infon = in ? __ldg(L.plan.lane_info + t * 32 + lane) : 0;
+        const int4* src = reinterpret_cast<const int4*>(L.items) + static_cast<int64_t>(t) * (kRowTileItems / 4) + lane;
+#pragma unroll
+        for (int h = 0; h < kIpl / 4; ++h) qn[h] = ld_stream4(src + 32 * h, in);
+        if (MODE == kModeWeighted) {
+            const int4* sw = reinterpret_cast<const int4*>(L.witems) + static_cast<int64_t>(t) * (kRowTileItems / 4) + lane;
+#pragma unroll
+            for (int h = 0; h < kIpl / 4; ++h) wn[h] = ld_stream4(sw + 32 * h, in);
+        }
+    };
+    fetch(gwarp);
+    for (int t = gwarp; t < ntiles; t += nwarps) {
+        const int row = Tn.x, nrows = Tn.y, r0 = infon & 0xFF;
+        int item[kIpl];
+#pragma unroll
+        for (int h = 0; h < kIpl / 4; ++h) {
+            item[4 * h + 0] = qn[h].x;
+            item[4 * h + 1] = qn[h].y;
+            item[4 * h + 2] = qn[h].z;
+            item[4 * h + 3] = qn[h].w;
+        }
+        // Epilogue inputs of the first 32 rows: predicated loads rather than branches.
+        int eod = 0, epos = row + lane;
+        if (MODE == kModePagerank) {
+            eod = lane < nrows ? ld_stream<MODE>(L.outdeg + row + lane) : 0;
+            if (L.perm) epos = lane < nrows ? ld_stream<MODE>(L.perm + row + lane) : 0;
+        }
+        int4 w[kIpl / 4];
+        if (MODE == kModeWeighted) {
+#pragma unroll
+            for (int h = 0; h < kIpl / 4; ++h) w[h] = wn[h];
+        }
+        fetch(t + nwarps);
+        // The gathers. The hot test stays a select between a shared and a global load (written as an
+        // if/else it became a divergent branch: 0.192 ms per sweep against 0.176 on R-MAT 22). Marks are
+        // negative and read the zero in front of the hot cache.
+        float pv[kIpl];
+#pragma unroll
+        for (int i = 0; i < kIpl; ++i) {
+            const int c = item[i];
+            pv[i] = c < L.hot ? s_hot[max(c, -1)] : __ldg(L.x + c);
+        }
+        if (MODE == kModeWeighted) {
+#pragma unroll
+            for (int h = 0; h < kIpl / 4; ++h) {
+                const int4 q = w[h];
+                pv[4 * h + 0] *= __int_as_float(q.x);
+                pv[4 * h + 1] *= __int_as_float(q.y);
+                pv[4 * h + 2] *= __int_as_float(q.z);
+                pv[4 * h + 3] *= __int_as_float(q.w);
+            }
+        }
+        if (nrows < 0) {
+            // Hub segment: lane sums in item order, then a butterfly; the partial goes to the fix-up.
+            float acc = 0.0f;
+#pragma unroll
+            for (int i = 0; i < kIpl; ++i) acc += pv[i];
+            acc = warp_sum_f32(acc);
+            if (lane == 0) L.partial[-(nrows + 1)] = acc;
+            continue;
+        }
+        float eW = 0.0f, eseed = 0.0f, eprev = 0.0f;
+        if (MODE == kModeWeighted && lane < nrows) {
+            eW = ld_stream<MODE>(L.W + row + lane);
+            if (L.perm) epos = ld_stream<MODE>(L.perm + row + lane);
+            if (L.seed) eseed = ld_stream<MODE>(L.seed + row + lane);
+            if (CONV) eprev = ld_stream<MODE>(L.rank_prev + row + lane);
+        }
+        // The lane's items in order: a nonzero is added to the open row, a row end closes it.
+        int r = r0;
+        float acc = 0.0f;
+        bool any_end = false;
+#pragma unroll
+        for (int i = 0; i < kIpl; ++i) {
+            const bool end = item[i] == kItemRowEnd;
+            acc += pv[i];  // marks hold 0
+            if (end) out[pad(r)] = acc;
+            acc = end ? 0.0f : acc;
+            r += end ? 1 : 0;
+            any_end |= end;
+        }
+        // Segmented inclusive scan of the lanes' open partials (key = row still open at lane end).
+        float cv = acc;
+        const int key = r;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float tv = __shfl_up_sync(kFullMask, cv, o);
+            const int tk = __shfl_up_sync(kFullMask, key, o);
+            if (lane >= o && tk == key) cv += tv;
+        }
+        const float cin = __shfl_up_sync(kFullMask, cv, 1);
+        const int kin = __shfl_up_sync(kFullMask, key, 1);
+        // The first row the lane closes is its start row, open in the lanes before it.
+        if (lane > 0 && any_end && kin == r0) out[pad(r0)] += cin;
+        __syncwarp();
+        for (int rr = lane; rr < nrows; rr += 32) {
+            const float sum = out[pad(rr)];
+            const int v = row + rr;
+            if (MODE == kModeWeighted) {
+                if (rr < 32) weighted_epilogue(L, v, sum, base, eW, epos, eseed, eprev, dang, moved);
+                else weighted_epilogue(L, v, sum, base, dang, moved);
+            } else if (rr < 32) {
+                pr_epilogue(L, v, sum, base, eod, epos, dang, moved);
+            } else {
+                pr_epilogue(L, v, sum, base, dang, moved);
+            }
+        }
+        __syncwarp();
     }
+    dang = warp_sum_f64(dang);
+    if (lane == 0) L.dpart[gwarp] = dang;
+    // One store per CTA at most: a store per moved row queued up on that one word (700,001 vertices, 11 M
+    // arcs: 50 us per sweep with it, 37 without; weighted sweep of R-MAT 20: 94 and 64 us).
+    if (CONV && __syncthreads_or(moved) && threadIdx.x == 0) *L.nonstop = 1u;
 }
 
 // The hub fix-up after each gather launch (and, with no hubs, after the initial vector). For
@@ -552,13 +650,78 @@ cudaError_t launch_tile_lane_starts_dev(const int4* tiles, const int64_t* d_ntil
     return cudaGetLastError();
 }
 
+namespace {
+// A tile's 256 merge items (kIpl per lane) in the order of the sweeps' loads: item i of lane l at
+// (i / 4) * 128 + 4 * l + i % 4. Lane l of the tile's warp calls fn(position, nonzero or -1 for a row end
+// or -2 past the tile) for each of its items; a hub segment is all nonzeros.
+template <class F>
+__device__ __forceinline__ void for_tile_items(const int4& T, int info, int lane, F fn) {
+    const int nrows = T.y, nnz = T.w;
+    const int total = nrows < 0 ? nnz : nrows + nnz;
+    int kk = lane * kIpl - (nrows < 0 ? 0 : info & 0xFF);
+#pragma unroll
+    for (int i = 0; i < kIpl; ++i) {
+        const int at = (i >> 2) * 128 + 4 * lane + (i & 3);
+        const bool end = nrows >= 0 && ((info >> (8 + i)) & 1);
+        if (lane * kIpl + i >= total) fn(at, -2);
+        else if (end) fn(at, -1);
+        else fn(at, kk++);
+    }
+}
+
+__global__ void tile_items_kernel(RowPlanDev plan, const int32_t* __restrict__ col, const int32_t* __restrict__ perm,
+                                  int32_t* __restrict__ items) {
+    const int lane = threadIdx.x & 31;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int t = w; t < plan.ntiles; t += nw) {
+        const int4 T = __ldg(plan.tiles + t);
+        int32_t* dst = items + static_cast<int64_t>(t) * kRowTileItems;
+        for_tile_items(T, __ldg(plan.lane_info + t * 32 + lane), lane, [&](int at, int k) {
+            int c = k == -1 ? kItemRowEnd : kItemNone;
+            if (k >= 0) {
+                c = __ldg(col + T.z + k);
+                if (perm) c = __ldg(perm + c);
+            }
+            dst[at] = c;
+        });
+    }
+}
+
+__global__ void tile_values_kernel(RowPlanDev plan, const float* __restrict__ vals, const int32_t* __restrict__ arc,
+                                   float* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int t = w; t < plan.ntiles; t += nw) {
+        const int4 T = __ldg(plan.tiles + t);
+        float* dst = out + static_cast<int64_t>(t) * kRowTileItems;
+        for_tile_items(T, __ldg(plan.lane_info + t * 32 + lane), lane, [&](int at, int k) {
+            dst[at] = k >= 0 ? __ldg(vals + (arc ? __ldg(arc + T.z + k) : T.z + k)) : 0.0f;
+        });
+    }
+}
+}  // namespace
+
+cudaError_t launch_tile_items(const RowPlanDev& plan, const int32_t* col, const int32_t* perm, int32_t* items,
+                              cudaStream_t s, int sm_count) {
+    if (plan.ntiles > 0) tile_items_kernel<<<sm_count * 8, 256, 0, s>>>(plan, col, perm, items);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tile_values(const RowPlanDev& plan, const float* vals, const int32_t* arc, float* out, cudaStream_t s,
+                               int sm_count) {
+    if (plan.ntiles > 0) tile_values_kernel<<<sm_count * 8, 256, 0, s>>>(plan, vals, arc, out);
+    return cudaGetLastError();
+}
+
 void rowgather_grid(int sm_count, int* gather_blocks, int* fix_blocks, int* block_threads) {
     *gather_blocks = sm_count;
     *fix_blocks = sm_count * 2;
     *block_threads = kBlock;
 }
 
-size_t rowgather_staging_bytes() { return sizeof(int) * kWarps * 2 * kPadded; }
+size_t rowgather_staging_bytes(bool sweeps) { return sizeof(float) * kWarps * kPadded * (sweeps ? 1 : 2); }
 
 namespace {
 
@@ -567,8 +730,13 @@ template <int MODE, bool CONV>
 cudaError_t prepare_rowgather(size_t bytes) {
     static size_t configured = 0;
     if (bytes <= configured) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(rowgather_kernel<MODE, has_vals(MODE) ? DPG_GATHER_TILES_SPMV : DPG_GATHER_TILES_PR, CONV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(bytes));
+    cudaError_t e;
+    if constexpr (MODE == kModeSpmv)
+        e = cudaFuncSetAttribute(spmv_gather_kernel<DPG_GATHER_TILES_SPMV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(bytes));
+    else
+        e = cudaFuncSetAttribute(rowgather_kernel<MODE, CONV>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e == cudaSuccess) configured = bytes;
     return e;
 }
@@ -777,16 +945,16 @@ namespace {
 template <int MODE, bool CONV>
 cudaError_t launch_row_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                              LaunchHook* hook) {
-    constexpr int KT = has_vals(MODE) ? DPG_GATHER_TILES_SPMV : DPG_GATHER_TILES_PR;
     int gb, fb, bt;
     rowgather_grid(sm_count, &gb, &fb, &bt);
-    // At least one hot entry: the SpMV gather reads entry 0 for cold columns.
-    const size_t smem = rowgather_staging_bytes() + sizeof(float) * static_cast<size_t>(L.hot > 0 ? L.hot : 1);
+    // At least one hot entry: the SpMV gather reads entry 0 for cold columns, the sweeps keep a zero.
+    const size_t smem = rowgather_staging_bytes(MODE != kModeSpmv) + sizeof(float) * (static_cast<size_t>(L.hot) + 1);
     cudaError_t err = prepare_rowgather<MODE, CONV>(smem);
     if (err != cudaSuccess) return err;
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, stream);
-        rowgather_kernel<MODE, KT, CONV><<<gb, bt, smem, stream>>>(L);
+        if constexpr (MODE == kModeSpmv) spmv_gather_kernel<DPG_GATHER_TILES_SPMV><<<gb, bt, smem, stream>>>(L);
+        else rowgather_kernel<MODE, CONV><<<gb, bt, smem, stream>>>(L);
     }
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
