@@ -196,7 +196,14 @@ struct RowGatherLaunch {
     const int32_t* vgraph;
     const float* gbase;
     const float* ginit;
+    // Hot-cache windows {first tile, first row = first renamed column}, ascending, and per gather CTA
+    // {first tile, its window} with an end entry; nwin 0: tiles strided over all warps, window at 0.
+    const int2* win;
+    int32_t nwin;
+    const int2* cta_first;
 };
+// The windows that start at rows[0] = 0, rows[1], ... (device pointers).
+cudaError_t launch_window_tiles(const RowPlanDev& plan, const int32_t* rows, int nwin, int2* win, cudaStream_t s);
 
 // ---- batched right-hand sides / SpMV adjoint (dpg_adjoint.cu) -----------------------------------
 constexpr int kSpmmSegment = 512;  // nonzeros per listed item; longer rows are split and fixed up in order

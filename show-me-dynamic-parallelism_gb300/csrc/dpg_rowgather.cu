@@ -100,9 +100,10 @@ __device__ __forceinline__ int4 ld_stream4(const int4* p, bool in) {
 
 // PageRank epilogue of one row: new rank, next contribution, dangling mass, convergence flag.
 // od / pos are the row's out-degree and contribution slot (perm[v] with renamed columns).
+// BATCH: packed graphs, `base` being the uniform term of the row's graph.
+template <bool BATCH>
 __device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, float sum, float base, int od, int pos,
                                             double& dang, bool& moved) {
-    if (L.vgraph) base = __ldg(L.gbase + __ldg(L.vgraph + v));
     const float nv = fmaf(L.damping, sum, base);
     if (L.rank_out) L.rank_out[v] = nv;
     if (L.rank_prev && fabsf(nv - __ldg(L.rank_prev + v)) > L.epsilon) moved = true;
@@ -111,7 +112,7 @@ __device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, flo
     // The division runs for every row (by 1 for a dangling one) so a warp's rows do not diverge
     // around it; only the stores and the dangling sum depend on the out-degree.
     const float q = nv / static_cast<float>(od > 0 ? od : 1);
-    if (L.vgraph) {
+    if (BATCH) {
         L.y[pos] = od > 0 ? q : nv;
     } else {
         if (od > 0) L.y[pos] = q;
@@ -119,8 +120,8 @@ __device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, flo
     }
 }
 
-__device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, float sum, float base, double& dang, bool& moved) {
-    pr_epilogue(L, v, sum, base, __ldg(L.outdeg + v), L.perm ? __ldg(L.perm + v) : v, dang, moved);
+__device__ __forceinline__ float batch_base(const RowGatherLaunch& L, int v) {
+    return __ldg(L.gbase + __ldg(L.vgraph + v));
 }
 
 // Epilogue of one row of a weighted PageRank sweep (dpg_prgrad.cu): forward (no seed) the new rank and
@@ -174,7 +175,8 @@ __device__ __forceinline__ void fixup_hubs(const RowGatherLaunch& L, int tid, in
         for (int s = 0; s < kSmallHubSegs; ++s) acc += p[s];
         if (MODE == kModeSpmv) L.y[H.x] = acc;
         else if (MODE == kModeWeighted) weighted_epilogue(L, H.x, acc, base, dang, moved);
-        else pr_epilogue(L, H.x, acc, base, od, pos, dang, moved);
+        else if (L.vgraph) pr_epilogue<true>(L, H.x, acc, batch_base(L, H.x), od, pos, dang, moved);
+        else pr_epilogue<false>(L, H.x, acc, base, od, pos, dang, moved);
     }
     for (int h = gwarp; h < L.plan.nhub_big; h += nwarps) {
         const int4 H = __ldg(L.plan.hubs_big + h);
@@ -195,7 +197,8 @@ __device__ __forceinline__ void fixup_hubs(const RowGatherLaunch& L, int tid, in
         if (lane == 0) {
             if (MODE == kModeSpmv) L.y[H.x] = acc;
             else if (MODE == kModeWeighted) weighted_epilogue(L, H.x, acc, base, dang, moved);
-            else pr_epilogue(L, H.x, acc, base, od, pos, dang, moved);
+            else if (L.vgraph) pr_epilogue<true>(L, H.x, acc, batch_base(L, H.x), od, pos, dang, moved);
+            else pr_epilogue<false>(L, H.x, acc, base, od, pos, dang, moved);
         }
     }
 }
@@ -228,14 +231,14 @@ __device__ __forceinline__ double block_sum_f64(double v) {
 
 // The hot cache: the first `hot` (most gathered) entries of x, loads issued in batches of 8 (one round
 // trip each instead of one per entry).
-__device__ __forceinline__ void fill_hot(const RowGatherLaunch& L, float* s_hot) {
-    for (int i0 = threadIdx.x; i0 < L.hot; i0 += kBlock * 8) {
+__device__ __forceinline__ void fill_hot(const float* __restrict__ x, int hot, float* s_hot) {
+    for (int i0 = threadIdx.x; i0 < hot; i0 += kBlock * 8) {
         float h[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) h[q] = i0 + kBlock * q < L.hot ? __ldg(L.x + i0 + kBlock * q) : 0.0f;
+        for (int q = 0; q < 8; ++q) h[q] = i0 + kBlock * q < hot ? __ldg(x + i0 + kBlock * q) : 0.0f;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
-            if (i0 + kBlock * q < L.hot) s_hot[i0 + kBlock * q] = h[q];
+            if (i0 + kBlock * q < hot) s_hot[i0 + kBlock * q] = h[q];
     }
     __syncthreads();
 }
@@ -253,7 +256,7 @@ __global__ void __launch_bounds__(kBlock) spmv_gather_kernel(RowGatherLaunch L) 
     float* val = reinterpret_cast<float*>(rg_smem) + warp * (2 * kPadded);
     float* out = val + kPadded;
     float* s_hot = reinterpret_cast<float*>(rg_smem) + kWarps * 2 * kPadded;
-    fill_hot(L, s_hot);
+    fill_hot(L.x, L.hot, s_hot);
 
     const int ntiles = L.plan.ntiles;
     // Descriptors and lane walks of the next step are requested one step ahead.
@@ -381,7 +384,13 @@ __global__ void __launch_bounds__(kBlock) spmv_gather_kernel(RowGatherLaunch L) 
 // 8.55 ms. Three tiles per step spill (4.6 ms). Shared-memory budgets (hot cache) of 132 / 164 / 196
 // KB: R-MAT 22 3.23 / 3.16 / 3.31 ms.
 // CONV: sweeps with a convergence test (rank_prev given).
-template <int MODE, bool CONV>
+// BATCH: packed graphs. Each graph's most gathered columns open its own range of columns, so a hot cache
+// of the first ones would serve the first graph alone. Each CTA takes a consecutive run of tiles, and
+// with them the windows of L.win in turn: a window's tiles are those of one graph, or of several small
+// ones that fit in the cache together, and the cache is filled from the window's first column on. A tile
+// that reaches into the next window only misses it. 48 graphs (107 M arcs), same box, per sweep: 0.35 ms
+// with one cache at 0 for all, 0.26 with windows, 0.22 with the epilogue inputs of 64 rows ahead as well.
+template <int MODE, bool CONV, bool BATCH>
 __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
     if (!CONV) L.rank_prev = nullptr;
     extern __shared__ __align__(16) unsigned char rg_smem[];
@@ -392,12 +401,34 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
     float* out = reinterpret_cast<float*>(rg_smem) + warp * kPadded;
     float* s_hot = reinterpret_cast<float*>(rg_smem) + kWarps * kPadded + 1;
     if (threadIdx.x == 0) s_hot[-1] = 0.0f;  // what the marks gather
-    fill_hot(L, s_hot);
-    const float base = pr_base(L);
+    const float base = BATCH ? 0.0f : pr_base(L);
     double dang = 0.0;
     bool moved = false;
 
-    const int ntiles = L.plan.ntiles;
+    // Tiles [first, ntiles) by `step`; BATCH: of the CTA's window, one after the other.
+    int ntiles = L.plan.ntiles, first = gwarp, step = nwarps;
+    int hot = L.hot, hot0 = 0;  // the cache holds columns [hot0, hot0 + hot)
+    int cta_end = 0, w = 0;
+    const bool windows = BATCH && L.nwin > 0;
+    if (windows) {
+        const int2 c0 = __ldg(L.cta_first + blockIdx.x);  // {first tile, its window}
+        first = c0.x;
+        w = c0.y;
+        cta_end = __ldg(L.cta_first + blockIdx.x + 1).x;
+        step = kWarps;
+    } else {
+        fill_hot(L.x, hot, s_hot);
+    }
+    do {
+    if (windows) {
+        if (first >= cta_end) break;
+        const int2 W = __ldg(L.win + w);  // {first tile, first column}
+        ntiles = w + 1 < L.nwin ? min(cta_end, __ldg(L.win + w + 1).x) : cta_end;
+        hot0 = W.y;
+        hot = min(L.hot, L.V - hot0);
+        fill_hot(L.x + hot0, hot, s_hot);
+        first += warp;
+    }
     int2 Tn;          // the next tile: {row, nrows}, start row of the lane, items
     int infon;
     int4 qn[kIpl / 4];
@@ -415,8 +446,8 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             for (int h = 0; h < kIpl / 4; ++h) wn[h] = ld_stream4(sw + 32 * h, in);
         }
     };
-    fetch(gwarp);
-    for (int t = gwarp; t < ntiles; t += nwarps) {
+    fetch(first);
+    for (int t = first; t < ntiles; t += step) {
         const int row = Tn.x, nrows = Tn.y, r0 = infon & 0xFF;
         int item[kIpl];
 #pragma unroll
@@ -426,18 +457,29 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             item[4 * h + 2] = qn[h].z;
             item[4 * h + 3] = qn[h].w;
         }
-        // Epilogue inputs of the first 32 rows: predicated loads rather than branches.
-        int eod = 0, epos = row + lane;
-        if (MODE == kModePagerank) {
-            eod = lane < nrows ? ld_stream<MODE>(L.outdeg + row + lane) : 0;
-            if (L.perm) epos = lane < nrows ? ld_stream<MODE>(L.perm + row + lane) : 0;
+        // Epilogue inputs of the first 32 rows (64 in a batch, whose graphs of 8 arcs per vertex have
+        // about 28 rows per tile): predicated loads rather than branches.
+        constexpr int NE = BATCH ? 2 : 1;
+        int eod[NE], epos[NE], egraph[NE];
+#pragma unroll
+        for (int q = 0; q < NE; ++q) {
+            const int v = row + lane + 32 * q;
+            const bool in = lane + 32 * q < nrows;
+            eod[q] = 0;
+            epos[q] = v;
+            egraph[q] = 0;
+            if (MODE == kModePagerank) {
+                eod[q] = in ? ld_stream<MODE>(L.outdeg + v) : 0;
+                if (L.perm) epos[q] = in ? ld_stream<MODE>(L.perm + v) : 0;
+            }
+            if (BATCH) egraph[q] = in ? ld_stream<MODE>(L.vgraph + v) : 0;
         }
         int4 w[kIpl / 4];
         if (MODE == kModeWeighted) {
 #pragma unroll
             for (int h = 0; h < kIpl / 4; ++h) w[h] = wn[h];
         }
-        fetch(t + nwarps);
+        fetch(t + step);
         // The gathers. The hot test stays a select between a shared and a global load (written as an
         // if/else it became a divergent branch: 0.192 ms per sweep against 0.176 on R-MAT 22). Marks are
         // negative and read the zero in front of the hot cache.
@@ -445,7 +487,12 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
 #pragma unroll
         for (int i = 0; i < kIpl; ++i) {
             const int c = item[i];
-            pv[i] = c < L.hot ? s_hot[max(c, -1)] : __ldg(L.x + c);
+            if (BATCH) {
+                const int d = c < 0 ? -1 : c - hot0;
+                pv[i] = c < 0 || static_cast<unsigned>(d) < static_cast<unsigned>(hot) ? s_hot[d] : __ldg(L.x + c);
+            } else {
+                pv[i] = c < hot ? s_hot[max(c, -1)] : __ldg(L.x + c);
+            }
         }
         if (MODE == kModeWeighted) {
 #pragma unroll
@@ -466,10 +513,13 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             if (lane == 0) L.partial[-(nrows + 1)] = acc;
             continue;
         }
+        float ebase[NE];
+#pragma unroll
+        for (int q = 0; q < NE; ++q) ebase[q] = BATCH ? __ldg(L.gbase + egraph[q]) : base;
         float eW = 0.0f, eseed = 0.0f, eprev = 0.0f;
         if (MODE == kModeWeighted && lane < nrows) {
             eW = ld_stream<MODE>(L.W + row + lane);
-            if (L.perm) epos = ld_stream<MODE>(L.perm + row + lane);
+            if (L.perm) epos[0] = ld_stream<MODE>(L.perm + row + lane);
             if (L.seed) eseed = ld_stream<MODE>(L.seed + row + lane);
             if (CONV) eprev = ld_stream<MODE>(L.rank_prev + row + lane);
         }
@@ -504,16 +554,25 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             const float sum = out[pad(rr)];
             const int v = row + rr;
             if (MODE == kModeWeighted) {
-                if (rr < 32) weighted_epilogue(L, v, sum, base, eW, epos, eseed, eprev, dang, moved);
+                if (rr < 32) weighted_epilogue(L, v, sum, base, eW, epos[0], eseed, eprev, dang, moved);
                 else weighted_epilogue(L, v, sum, base, dang, moved);
             } else if (rr < 32) {
-                pr_epilogue(L, v, sum, base, eod, epos, dang, moved);
+                pr_epilogue<BATCH>(L, v, sum, ebase[0], eod[0], epos[0], dang, moved);
+            } else if (NE > 1 && rr < 64) {
+                pr_epilogue<BATCH>(L, v, sum, ebase[NE - 1], eod[NE - 1], epos[NE - 1], dang, moved);
             } else {
-                pr_epilogue(L, v, sum, base, dang, moved);
+                pr_epilogue<BATCH>(L, v, sum, BATCH ? batch_base(L, v) : base, __ldg(L.outdeg + v),
+                                   L.perm ? __ldg(L.perm + v) : v, dang, moved);
             }
         }
         __syncwarp();
     }
+    if (windows) {
+        __syncthreads();  // the cache is free again
+        first = ntiles;
+        ++w;
+    }
+    } while (windows);
     dang = warp_sum_f64(dang);
     if (lane == 0) L.dpart[gwarp] = dang;
     // One store per CTA at most: a store per moved row queued up on that one word (700,001 vertices, 11 M
@@ -703,6 +762,26 @@ __global__ void tile_values_kernel(RowPlanDev plan, const float* __restrict__ va
 }
 }  // namespace
 
+namespace {
+// win[k].x: first tile of window k, i.e. the first tile whose row is at or past rows[k] (tiles ascend by row).
+__global__ void window_tiles_kernel(RowPlanDev plan, const int32_t* __restrict__ rows, int nwin, int2* win) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nwin; k += gridDim.x * blockDim.x) {
+        int lo = 0, hi = plan.ntiles;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (__ldg(plan.tiles + mid).x < rows[k]) lo = mid + 1;
+            else hi = mid;
+        }
+        win[k] = make_int2(lo, rows[k]);
+    }
+}
+}  // namespace
+
+cudaError_t launch_window_tiles(const RowPlanDev& plan, const int32_t* rows, int nwin, int2* win, cudaStream_t s) {
+    if (nwin > 0) window_tiles_kernel<<<(nwin + 255) / 256, 256, 0, s>>>(plan, rows, nwin, win);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_tile_items(const RowPlanDev& plan, const int32_t* col, const int32_t* perm, int32_t* items,
                               cudaStream_t s, int sm_count) {
     if (plan.ntiles > 0) tile_items_kernel<<<sm_count * 8, 256, 0, s>>>(plan, col, perm, items);
@@ -726,7 +805,7 @@ size_t rowgather_staging_bytes(bool sweeps) { return sizeof(float) * kWarps * kP
 namespace {
 
 // Sets the kernel's dynamic shared-memory limit to what this launch needs (once per size).
-template <int MODE, bool CONV>
+template <int MODE, bool CONV, bool BATCH>
 cudaError_t prepare_rowgather(size_t bytes) {
     static size_t configured = 0;
     if (bytes <= configured) return cudaSuccess;
@@ -735,7 +814,7 @@ cudaError_t prepare_rowgather(size_t bytes) {
         e = cudaFuncSetAttribute(spmv_gather_kernel<DPG_GATHER_TILES_SPMV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(bytes));
     else
-        e = cudaFuncSetAttribute(rowgather_kernel<MODE, CONV>,
+        e = cudaFuncSetAttribute(rowgather_kernel<MODE, CONV, BATCH>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e == cudaSuccess) configured = bytes;
     return e;
@@ -942,19 +1021,19 @@ namespace {
 // A sweep: the gather kernel, then the hub fix-up kernel (which for PageRank also reduces the
 // dangling partials). Folding the fix-up into the gather behind a grid barrier (one cooperative
 // launch) measured only 0.6 % faster on R-MAT 22: the fix-up's round trips stay on the critical path.
-template <int MODE, bool CONV>
+template <int MODE, bool CONV, bool BATCH>
 cudaError_t launch_row_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                              LaunchHook* hook) {
     int gb, fb, bt;
     rowgather_grid(sm_count, &gb, &fb, &bt);
     // At least one hot entry: the SpMV gather reads entry 0 for cold columns, the sweeps keep a zero.
     const size_t smem = rowgather_staging_bytes(MODE != kModeSpmv) + sizeof(float) * (static_cast<size_t>(L.hot) + 1);
-    cudaError_t err = prepare_rowgather<MODE, CONV>(smem);
+    cudaError_t err = prepare_rowgather<MODE, CONV, BATCH>(smem);
     if (err != cudaSuccess) return err;
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, stream);
         if constexpr (MODE == kModeSpmv) spmv_gather_kernel<DPG_GATHER_TILES_SPMV><<<gb, bt, smem, stream>>>(L);
-        else rowgather_kernel<MODE, CONV><<<gb, bt, smem, stream>>>(L);
+        else rowgather_kernel<MODE, CONV, BATCH><<<gb, bt, smem, stream>>>(L);
     }
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
@@ -970,19 +1049,20 @@ cudaError_t launch_row_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream
 
 cudaError_t launch_spmv(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                         LaunchHook* hook) {
-    return launch_row_sweep<kModeSpmv, false>(L, st, stream, sm_count, hook);
+    return launch_row_sweep<kModeSpmv, false, false>(L, st, stream, sm_count, hook);
 }
 
 cudaError_t launch_weighted_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                                   LaunchHook* hook) {
-    return L.rank_prev ? launch_row_sweep<kModeWeighted, true>(L, st, stream, sm_count, hook)
-                       : launch_row_sweep<kModeWeighted, false>(L, st, stream, sm_count, hook);
+    return L.rank_prev ? launch_row_sweep<kModeWeighted, true, false>(L, st, stream, sm_count, hook)
+                       : launch_row_sweep<kModeWeighted, false, false>(L, st, stream, sm_count, hook);
 }
 
 cudaError_t launch_pagerank_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                                   LaunchHook* hook) {
-    return L.rank_prev ? launch_row_sweep<kModePagerank, true>(L, st, stream, sm_count, hook)
-                       : launch_row_sweep<kModePagerank, false>(L, st, stream, sm_count, hook);
+    if (L.vgraph) return launch_row_sweep<kModePagerank, false, true>(L, st, stream, sm_count, hook);
+    return L.rank_prev ? launch_row_sweep<kModePagerank, true, false>(L, st, stream, sm_count, hook)
+                       : launch_row_sweep<kModePagerank, false, false>(L, st, stream, sm_count, hook);
 }
 
 cudaError_t launch_pagerank_init(const RowGatherLaunch& L, float init_rank, float* rank_prev, DevStatus* st,
