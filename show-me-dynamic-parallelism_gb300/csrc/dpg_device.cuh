@@ -85,6 +85,21 @@ __device__ __forceinline__ bool grid_barrier(DevStatus* st, unsigned expected,
     return s_ok != 0;
 }
 
+// Kernels launched with launch_chained (dpg_kernels.h) may start while the kernel before them in the
+// stream still runs: chain_wait returns when that kernel has completed and its writes are in L2, and
+// nothing is written, and nothing that may still change is read, ahead of it. chain_next, called behind
+// the wait, lets the next chained kernel start early; without it, that happens when this kernel ends. In
+// a kernel that was not launched so, chain_wait does nothing.
+// An early start also moves the L1's invalidation ahead of the predecessor's end, so lines that the
+// predecessor loads on the same SM while it runs stay there: what it (or another of its blocks) writes
+// into such a line must be read past the L1 (__ldcg). So only kernels that follow one of this library's
+// own in the same call are chained, and the dangling sum is read so: the fix-up reads the one of the last
+// sweep and writes the one of this sweep in the same line. What a sweep's gather otherwise reads through
+// the L1 (gathered vector, previous ranks, a batch's uniform terms) no kernel loads between the gather's
+// earliest start, when the kernel before it is past its own wait, and the end of the writes to it.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
 __device__ __forceinline__ int warp_inclusive_scan(int v) {

@@ -30,6 +30,23 @@ struct HookScope {
     }
 };
 
+// Launches a kernel that waits for its predecessor itself (chain_wait in dpg_device.cuh), so that its
+// launch and start-up overlap the predecessor's end.
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- frontier expansion (SSSP / BFS) ------------------------------------------------------------
 
 // Arcs per grid-wide chunk: every vertex at or above the chunking degree is cut into chunks of this

@@ -150,7 +150,7 @@ __device__ __forceinline__ void weighted_epilogue(const RowGatherLaunch& L, int 
 }
 
 __device__ __forceinline__ float pr_base(const RowGatherLaunch& L) {
-    return static_cast<float>(L.base_const + L.dangling_scale * __ldg(L.dsum_in));
+    return static_cast<float>(L.base_const + L.dangling_scale * __ldcg(L.dsum_in));
 }
 
 // Hub rows: the segment partials summed in segment order, then the row epilogue. Small hubs go one
@@ -256,7 +256,6 @@ __global__ void __launch_bounds__(kBlock) spmv_gather_kernel(RowGatherLaunch L) 
     float* val = reinterpret_cast<float*>(rg_smem) + warp * (2 * kPadded);
     float* out = val + kPadded;
     float* s_hot = reinterpret_cast<float*>(rg_smem) + kWarps * 2 * kPadded;
-    fill_hot(L.x, L.hot, s_hot);
 
     const int ntiles = L.plan.ntiles;
     // Descriptors and lane walks of the next step are requested one step ahead.
@@ -268,6 +267,7 @@ __global__ void __launch_bounds__(kBlock) spmv_gather_kernel(RowGatherLaunch L) 
         Tn[k] = t < ntiles ? __ldg(L.plan.tiles + t) : make_int4(0, 0, 0, 0);
         infon[k] = t < ntiles ? __ldg(L.plan.lane_info + t * 32 + lane) : 0;
     }
+    fill_hot(L.x, L.hot, s_hot);
     for (int t0 = gwarp * KT; t0 < ntiles; t0 += nwarps * KT) {
         int4 T[KT];
         int info[KT];
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
     float* out = reinterpret_cast<float*>(rg_smem) + warp * kPadded;
     float* s_hot = reinterpret_cast<float*>(rg_smem) + kWarps * kPadded + 1;
     if (threadIdx.x == 0) s_hot[-1] = 0.0f;  // what the marks gather
-    const float base = BATCH ? 0.0f : pr_base(L);
+    float base = 0.0f;
     double dang = 0.0;
     bool moved = false;
 
@@ -416,8 +416,6 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
         w = c0.y;
         cta_end = __ldg(L.cta_first + blockIdx.x + 1).x;
         step = kWarps;
-    } else {
-        fill_hot(L.x, hot, s_hot);
     }
     do {
     if (windows) {
@@ -426,7 +424,6 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
         ntiles = w + 1 < L.nwin ? min(cta_end, __ldg(L.win + w + 1).x) : cta_end;
         hot0 = W.y;
         hot = min(L.hot, L.V - hot0);
-        fill_hot(L.x + hot0, hot, s_hot);
         first += warp;
     }
     int2 Tn;          // the next tile: {row, nrows}, start row of the lane, items
@@ -446,7 +443,10 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             for (int h = 0; h < kIpl / 4; ++h) wn[h] = ld_stream4(sw + 32 * h, in);
         }
     };
-    fetch(first);
+    fetch(first);  // the plan's arrays: fixed, so they may be read ahead of the wait
+    chain_wait();
+    if (!BATCH) base = pr_base(L);
+    fill_hot(L.x + hot0, hot, s_hot);
     for (int t = first; t < ntiles; t += step) {
         const int row = Tn.x, nrows = Tn.y, r0 = infon & 0xFF;
         int item[kIpl];
@@ -589,6 +589,8 @@ __global__ void __launch_bounds__(kFixBlock) hub_fixup_kernel(RowGatherLaunch L,
     const int lane = threadIdx.x & 31;
     const int gwarp = tid >> 5;
     const int nwarps = nthreads >> 5;
+    chain_wait();
+    chain_next();
     float base = 0.0f;
     if (MODE != kModeSpmv) base = pr_base(L);
     double dang = 0.0;
@@ -1018,6 +1020,10 @@ cudaError_t launch_build_row_plan(const int32_t* off, int32_t V, int64_t E, cons
 
 namespace {
 
+// The kernels of a sweep are chained (launch_chained). Same box, 20 sweeps of R-MAT 22 / 608,712 vertices,
+// gradient of R-MAT 20 / 50,001 vertices x 8: unchained 3.13 / 0.70, 8.29 / 2.73 ms; gather and fix-up
+// chained 3.04 / 0.61, 7.62 / 2.20 ms. Letting the fix-up start ahead of the gather's end cost more than
+// it gave (3.15 / 0.72, 8.58 / 2.39 ms).
 // A sweep: the gather kernel, then the hub fix-up kernel (which for PageRank also reduces the
 // dangling partials). Folding the fix-up into the gather behind a grid barrier (one cooperative
 // launch) measured only 0.6 % faster on R-MAT 22: the fix-up's round trips stay on the critical path.
@@ -1032,17 +1038,20 @@ cudaError_t launch_row_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream
     if (err != cudaSuccess) return err;
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, stream);
-        if constexpr (MODE == kModeSpmv) spmv_gather_kernel<DPG_GATHER_TILES_SPMV><<<gb, bt, smem, stream>>>(L);
-        else rowgather_kernel<MODE, CONV, BATCH><<<gb, bt, smem, stream>>>(L);
+        if constexpr (MODE == kModeSpmv) {
+            spmv_gather_kernel<DPG_GATHER_TILES_SPMV><<<gb, bt, smem, stream>>>(L);
+            err = cudaGetLastError();
+        } else {
+            err = launch_chained(rowgather_kernel<MODE, CONV, BATCH>, gb, bt, smem, stream, L);
+        }
     }
-    err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     if (MODE == kModeSpmv && L.plan.nhub_small + L.plan.nhub_big == 0) return cudaSuccess;
     {
         HookScope hs(hook, DPG_KERNEL_FIXUP, stream);
-        hub_fixup_kernel<MODE><<<fb, kFixBlock, 0, stream>>>(L, gb * (bt / 32), st);
+        err = launch_chained(hub_fixup_kernel<MODE>, fb, kFixBlock, 0, stream, L, gb * (bt / 32), st);
     }
-    return cudaGetLastError();
+    return err;
 }
 
 }  // namespace
