@@ -1252,18 +1252,26 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                         my_pops += 1;
                     }
                     if (lane == 0) my_edges += static_cast<unsigned long long>(k1 - k0);
-                    {
-                        constexpr int U = CH / 32;  // the whole chunk in one batch
+                    // The whole chunk in one batch; the multi-source relaxation, whose slots each hold two
+                    // vertices' labels, 128 arcs at a time: 256-arc chunks in one batch took 12.4 ms
+                    // against 9.0 (8 sources on each of 48 graphs, same box); 64 at a time is as fast.
+                    constexpr int U = O::kMask ? 4 : CH / 32;
+                    auto relax = [&](int kb) {
                         bool act[U];
                         int ee[U];
                         RV dd[U];
 #pragma unroll
                         for (int u = 0; u < U; ++u) {
-                            ee[u] = k0 + 32 * u + lane;
+                            ee[u] = kb + 32 * u + lane;
                             act[u] = ee[u] < k1;
                             dd[u] = du;
                         }
                         relax_batch<O, kClassify, CH, U>(P, Q, act, ee, dd);
+                    };
+                    if constexpr (U * 32 == CH) {
+                        relax(k0);
+                    } else {
+                        for (int kb = k0; kb < k1; kb += 32 * U) relax(kb);
                     }
                     continue;
                 }
