@@ -26,6 +26,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <type_traits>
 
@@ -73,6 +74,7 @@ struct ExpandParams {
     // so a vertex's labels can be read four at a time (relax_mask_vec4).
     int32_t label_vec4;
     int32_t local_rounds;   // near-far and direction-optimizing: see local_relax (0: off)
+    int32_t nctas;          // CTAs that take part in the solve (the first ones of the grid)
     uint32_t min_item_log;  // log2 of the fewest small-queue vertices in a warp item (binned kernels)
 };
 
@@ -920,6 +922,7 @@ constexpr int kLocalAfter = 32;
 
 template <class Op, int POL, int CH = kHubChunk, int MINB = 0>
 __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) expand_kernel(ExpandParams P) {
+    if (blockIdx.x >= static_cast<unsigned>(P.nctas)) return;  // see active_blocks
     using RV = typename Op::RV;
     constexpr bool kDirOpt = (POL == DPG_SOL_DIROPT);
     constexpr bool kNearFar = (POL == DPG_SOL_NEARFAR);
@@ -946,7 +949,7 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const unsigned gwarp = blockIdx.x * kWarps + warp;
-    const unsigned nwarps = gridDim.x * kWarps;
+    const unsigned nwarps = P.nctas * kWarps;
     unsigned long long my_edges = 0, my_pops = 0;
     if (threadIdx.x == 0) c_n = 0;
     if (lane == 0) {
@@ -1173,7 +1176,7 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                     push_converged<Op, kClassify, CH>(P, Q, found[r], found[r] ? vv[r] : 0, &ose[r]);
             }
         } else if (POL == DPG_SOL_BLOCK) {
-            const unsigned per_round = gridDim.x * kWarps;
+            const unsigned per_round = P.nctas * kWarps;
             const unsigned rounds = (fchunks + per_round - 1) / per_round;
             for (unsigned r = 0; r < rounds; ++r) {
                 const unsigned chunk = r * per_round + blockIdx.x * kWarps + warp;
@@ -1323,7 +1326,7 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
             }
         }
         flush_pushes(P, Q);
-        if (!grid_barrier(P.st, gridDim.x, P.timeout_ns)) break;
+        if (!grid_barrier(P.st, P.nctas, P.timeout_ns)) break;
         if (kNearFar && split) pile = (pile + 1) % 3;
     }
 
@@ -1499,6 +1502,15 @@ uint32_t min_item_log(int32_t V, int64_t E) {
     return lg;
 }
 
+// CTAs per SM that take part in the solve of a graph of E arcs (the others leave at once): the iterations
+// of small graphs have too few items for all, which then only lengthen the grid barrier. Same box, 4 / 3 /
+// 2 / 1 CTAs per SM launched: SSSP 40 K arcs 107 / 104 / 102 / 95 us, R-MAT 14 (262 K) 123 / 111 / 102 / 111 us,
+// R-MAT 17 (2.1 M) 249 / 235 / 231 / 265 us, 3.2 M arcs 360 / 355 / 375 / 473 us, R-MAT 20 (16.8 M) 503 / 562 /
+// 681 / 995 us; BFS R-MAT 16 (1 M) 67 / 61 / 57 / 54 us. With 4 launched and 2 or 1 left: R-MAT 14 126 -> 114 us,
+// 40 K arcs 107 -> 97, R-MAT 17 256 -> 247, BFS R-MAT 16 67 -> 60. The multi-source kernel keeps all (15 graphs,
+// 1 M arcs: 661 / 665 / 692 / 734 us with its PageRank).
+int active_blocks(int64_t E, int per_sm) { return std::min(per_sm, E < (1 << 17) ? 1 : E < (5 << 19) ? 2 : per_sm); }
+
 // The kernel of a solution id; `wide` selects the kWideBlocks build of the binned and
 // direction-optimizing kernels.
 template <class Op>
@@ -1560,6 +1572,7 @@ cudaError_t run_multi(const MultiExpandLaunch& L, const ExpandWorkspace& ws, Dev
     P.ws = ws;
     P.st = st;
     P.nsrc = L.nsrc;
+    P.nctas = grid;
     P.min_item_log = min_item_log(L.V, L.E);
     P.dirty[0] = L.dirty[0];
     P.dirty[1] = L.dirty[1];
@@ -1636,6 +1649,7 @@ cudaError_t launch_expand(const ExpandLaunch& L, const ExpandWorkspace& ws, DevS
     P.nf = diropt ? L.do_nf : nullptr;
     P.E = L.E;
     P.min_item_log = min_item_log(L.V, L.E);
+    P.nctas = sm_count * (L.solution >= DPG_SOL_BINNED ? active_blocks(L.E, per_sm) : per_sm);
     P.local_rounds = L.local_rounds;
     const int classify =
         (L.solution == DPG_SOL_GRID || L.solution == DPG_SOL_BINNED || L.solution == DPG_SOL_DIROPT ||
@@ -1685,6 +1699,7 @@ cudaError_t launch_color(const ExpandLaunch& L, const int32_t* out_off, const in
     P.trace = L.trace;
     P.trace_cap = L.trace_cap;
     P.aux = pending;
+    P.nctas = grid;
     P.min_item_log = min_item_log(L.V, L.E);
     err = cudaMemsetAsync(ws.qcount, 0, sizeof(uint32_t) * 3, stream);
     if (err == cudaSuccess) err = cudaMemsetAsync(ws.ccount, 0, sizeof(uint32_t) * 3, stream);
