@@ -118,26 +118,32 @@ __global__ void __launch_bounds__(kSplitBlock) split_count_kernel(const int32_t*
         block_hist[static_cast<int64_t>(kClasses - 1 - threadIdx.x) * gridDim.x + blockIdx.x] = s_tot[threadIdx.x];
 }
 
-// Exclusive scan of n ints in place by one block (n is 33 x blocks, a few hundred thousand at most).
+// Exclusive scan of n ints in place by one block (n is 33 x blocks, a few hundred thousand at most): 4
+// consecutive ones per thread and round, warp sums, then the warps' own scan.
 __global__ void __launch_bounds__(1024) split_scan_kernel(int32_t* __restrict__ a, int64_t n) {
-    __shared__ int32_t s_part[1024];
-    __shared__ int32_t s_carry;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
-    for (int64_t base = 0; base < n; base += 1024) {
-        const int64_t i = base + threadIdx.x;
-        const int32_t x = i < n ? a[i] : 0;
-        s_part[threadIdx.x] = x;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {  // Hillis-Steele inclusive scan
-            const int32_t t = threadIdx.x >= o ? s_part[threadIdx.x - o] : 0;
-            __syncthreads();
-            s_part[threadIdx.x] += t;
-            __syncthreads();
+    __shared__ int32_t s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t carry = 0;
+    for (int64_t base = 0; base < n; base += 4096) {
+        const int64_t i = base + 4 * static_cast<int64_t>(threadIdx.x);
+        int32_t x[4], sum = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            x[q] = i + q < n ? a[i + q] : 0;
+            sum += x[q];
         }
-        if (i < n) a[i] = s_carry + s_part[threadIdx.x] - x;
+        const int32_t incl = warp_inclusive_scan(sum);
+        if (lane == 31) s_warp[warp] = incl;
         __syncthreads();
-        if (threadIdx.x == 1023) s_carry += s_part[1023];
+        const int32_t ws = s_warp[lane];
+        const int32_t wi = warp_inclusive_scan(ws);
+        int32_t run = carry + incl - sum + (warp > 0 ? __shfl_sync(0xffffffffu, wi, warp - 1) : 0);
+        carry += __shfl_sync(0xffffffffu, wi, 31);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (i + q < n) a[i + q] = run;
+            run += x[q];
+        }
         __syncthreads();
     }
 }

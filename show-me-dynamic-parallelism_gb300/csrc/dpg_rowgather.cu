@@ -827,20 +827,27 @@ cudaError_t prepare_rowgather(size_t bytes) {
 namespace {
 
 // ---- the row plan, built on the device ------------------------------------------------------------
-// Rows are tiled in fixed ranges of kPlanRange rows, one thread per range, by a greedy walk:
+// Rows are tiled in fixed ranges of kPlanRange rows, one warp per range, by a greedy walk:
 // consecutive rows share a tile while their merge items (rows + nonzeros) fit in kRowTileItems, and
 // a row above kHubRowDegree becomes a hub cut into kRowTileItems segments (segments numbered from 0
 // within the range, then offset by the earlier ranges' counts). A count pass, an exclusive scan of
 // the per-range counts and a write pass produce the tiles in row order, so the plan is the same on
 // every run. Offsets that are negative, decrease or pass E stop their range's walk and set bit 4 of
 // the status flag; the walk never reads past off[V] and every write is checked against the capacity.
+// The warp reads 32 rows at a time and finds the end of the open tile among them with one ballot, so a
+// range takes about as many steps as it has tiles and groups of 32 rows. A thread per range walked
+// 2,048 rows one after the other: 340 and 604 us for the two passes over 700,001 rows x 16 nonzeros, now 35
+// and 45 us (55 and 73 without the next 32 rows loaded ahead).
 constexpr int32_t kPlanRange = 2048;
 constexpr int kPlanBlock = 128;
 
 struct PlanCount {
     int64_t tiles = 0, small = 0, big = 0, segs = 0;
     __device__ void tile(int32_t, int32_t, int32_t, int32_t) { ++tiles; }
-    __device__ void hub(int32_t, int32_t, int32_t nseg) { (nseg <= kSmallHubSegs ? small : big) += 1; }
+    __device__ void hub(int32_t, int32_t, int32_t, int32_t, int32_t nseg) {
+        tiles += nseg;
+        (nseg <= kSmallHubSegs ? small : big) += 1;
+    }
 };
 
 struct PlanWrite {
@@ -849,60 +856,74 @@ struct PlanWrite {
     int4* tiles;
     int4* hubs_small;
     int4* hubs_big;
-    __device__ void tile(int32_t row, int32_t nrows_or_seg, int32_t nb, int32_t nnz) {
-        // nrows_or_seg >= 0: a normal tile of that many rows; < 0: hub segment -(local id + 1).
-        const int32_t y = nrows_or_seg >= 0 ? nrows_or_seg : static_cast<int32_t>(nrows_or_seg - seg_base);
-        if (t < cap_tiles) tiles[t] = make_int4(row, y, nb, nnz);
+    __device__ void tile(int32_t row, int32_t nrows, int32_t nb, int32_t nnz) {
+        if (lane_id() == 0 && t < cap_tiles) tiles[t] = make_int4(row, nrows, nb, nnz);
         ++t;
     }
-    __device__ void hub(int32_t row, int32_t first_seg, int32_t nseg) {
-        const int4 h = make_int4(row, static_cast<int32_t>(seg_base + first_seg), nseg, 0);
+    // Row [a, b) of the nonzeros in nseg segments, the first of them segment `first` of the range.
+    __device__ void hub(int32_t row, int32_t a, int32_t b, int32_t first, int32_t nseg) {
+        for (int32_t k = lane_id(); k < nseg; k += 32) {
+            const int32_t sb = a + k * kRowTileItems;
+            if (t + k < cap_tiles)
+                tiles[t + k] = make_int4(row, static_cast<int32_t>(-(seg_base + first + k + 1)), sb,
+                                         min(kRowTileItems, b - sb));
+        }
+        t += nseg;
+        const int4 h = make_int4(row, static_cast<int32_t>(seg_base + first), nseg, 0);
         if (nseg <= kSmallHubSegs) {
-            if (hs < cap_hubs) hubs_small[hs] = h;
+            if (lane_id() == 0 && hs < cap_hubs) hubs_small[hs] = h;
             ++hs;
         } else {
-            if (hb < cap_hubs) hubs_big[hb] = h;
+            if (lane_id() == 0 && hb < cap_hubs) hubs_big[hb] = h;
             ++hb;
         }
     }
 };
 
-// The greedy walk over rows [r0, r1); returns the number of hub segments, or -1 on bad offsets.
+// The greedy walk of a warp over rows [r0, r1); returns the number of hub segments, or -1 on bad offsets.
 template <class Sink>
 __device__ int32_t plan_range(const int32_t* __restrict__ off, int32_t r0, int32_t r1, int64_t E, Sink& sk) {
-    int32_t cur_row = r0, cur_rows = 0, cur_items = 0, cur_nb = 0, cur_end = 0, segs = 0;
-    int32_t a = __ldg(off + r0);
-    if (a < 0 || a > E) return -1;
-    for (int32_t r = r0; r < r1; ++r) {
-        const int32_t b = __ldg(off + r + 1);
-        if (b < a || b > E) return -1;
-        const int32_t d = b - a;
-        if (d > kHubRowDegree) {
+    const int lane = lane_id();
+    int32_t cur_row = r0, cur_rows = 0, cur_nb = 0, cur_end = 0, segs = 0;  // the open tile, the same in every lane
+    int32_t na = 0, nb = 0;  // the lane's row of the next 32, loaded a step ahead
+    auto fetch = [&](int32_t c) {
+        na = c + lane < r1 ? __ldg(off + c + lane) : 0;
+        nb = c + lane < r1 ? __ldg(off + c + lane + 1) : 0;
+    };
+    fetch(r0);
+    for (int32_t c = r0; c < r1; c += 32) {
+        const int n = min(32, r1 - c);
+        const int32_t r = c + lane;
+        const int32_t a = na, b = nb;
+        fetch(c + 32);
+        if (__any_sync(kFullMask, lane < n && (a < 0 || b < a || b > E))) return -1;
+        const bool hub = lane < n && b - a > kHubRowDegree;
+        int p = 0;  // next row of the 32
+        while (p < n) {
+            if (cur_rows == 0) {
+                cur_row = c + p;
+                cur_nb = __shfl_sync(kFullMask, a, p);
+            }
+            // Rows that do not fit in the open tile; the first of them, or a hub, ends it.
+            const int64_t items = static_cast<int64_t>(b) - cur_nb + (r - cur_row + 1);
+            const unsigned m = __ballot_sync(kFullMask, lane < n && lane >= p && (hub || items > kRowTileItems));
+            const int q = m ? __ffs(m) - 1 : n;
+            if (q > p) {
+                cur_rows += q - p;
+                cur_end = __shfl_sync(kFullMask, b, q - 1);
+            }
+            p = q;
+            if (q == n) break;
             if (cur_rows > 0) sk.tile(cur_row, cur_rows, cur_nb, cur_end - cur_nb);
             cur_rows = 0;
-            cur_items = 0;
-            const int32_t nseg = (d + kRowTileItems - 1) / kRowTileItems;
-            for (int32_t k = 0; k < nseg; ++k) {
-                const int32_t sb = a + k * kRowTileItems;
-                sk.tile(r, -(segs + k + 1), sb, min(kRowTileItems, b - sb));
+            if (__shfl_sync(kFullMask, static_cast<int>(hub), q)) {
+                const int32_t ha = __shfl_sync(kFullMask, a, q), hb = __shfl_sync(kFullMask, b, q);
+                const int32_t nseg = (hb - ha + kRowTileItems - 1) / kRowTileItems;
+                sk.hub(c + q, ha, hb, segs, nseg);
+                segs += nseg;
+                p = q + 1;
             }
-            sk.hub(r, segs, nseg);
-            segs += nseg;
-        } else {
-            if (cur_items + d + 1 > kRowTileItems) {
-                sk.tile(cur_row, cur_rows, cur_nb, cur_end - cur_nb);
-                cur_rows = 0;
-                cur_items = 0;
-            }
-            if (cur_rows == 0) {
-                cur_row = r;
-                cur_nb = a;
-            }
-            ++cur_rows;
-            cur_items += d + 1;
-            cur_end = b;
         }
-        a = b;
     }
     if (cur_rows > 0) sk.tile(cur_row, cur_rows, cur_nb, cur_end - cur_nb);
     return segs;
@@ -916,11 +937,12 @@ __device__ __forceinline__ int32_t range_end(int32_t r0, int32_t V) {
 // counts[4][nranges]: tiles, small hubs, big hubs, segments of each range.
 __global__ void __launch_bounds__(kPlanBlock) plan_count_kernel(const int32_t* __restrict__ off, int32_t V, int64_t E,
                                                                 int64_t* __restrict__ counts, int32_t nranges, int* bad) {
-    const int32_t k = blockIdx.x * kPlanBlock + threadIdx.x;
+    const int32_t k = (blockIdx.x * kPlanBlock + threadIdx.x) >> 5;
     if (k >= nranges) return;
     PlanCount c;
     const int32_t r0 = k * kPlanRange;
     const int32_t segs = plan_range(off, r0, range_end(r0, V), E, c);
+    if (lane_id() != 0) return;
     if (segs < 0) {
         atomicOr(bad, 4);
         c = PlanCount();
@@ -946,14 +968,21 @@ __global__ void __launch_bounds__(1024) plan_scan_kernel(int64_t* counts, int32_
         s_part[q][t] = acc;
     }
     __syncthreads();
-    if (t < 4) {
+    if (t < 128) {  // a warp per row
+        const int q = t >> 5, lane = t & 31;
         int64_t run = 0;
-        for (int i = 0; i < 1024; ++i) {
-            const int64_t v = s_part[t][i];
-            s_part[t][i] = run;
-            run += v;
+        for (int i = lane; i < 1024; i += 32) {
+            const int64_t v = s_part[q][i];
+            int64_t incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t u = __shfl_up_sync(kFullMask, incl, o);
+                if (lane >= o) incl += u;
+            }
+            s_part[q][i] = run + incl - v;
+            run += __shfl_sync(kFullMask, incl, 31);
         }
-        totals[t] = run;
+        if (lane == 0) totals[q] = run;
     }
     __syncthreads();
     for (int q = 0; q < 4; ++q) {
@@ -971,7 +1000,7 @@ __global__ void __launch_bounds__(kPlanBlock) plan_write_kernel(const int32_t* _
                                                                 const int64_t* __restrict__ bases, int32_t nranges,
                                                                 int4* tiles, int64_t cap_tiles, int4* hubs_small,
                                                                 int4* hubs_big, int64_t cap_hubs) {
-    const int32_t k = blockIdx.x * kPlanBlock + threadIdx.x;
+    const int32_t k = (blockIdx.x * kPlanBlock + threadIdx.x) >> 5;
     if (k >= nranges) return;
     PlanWrite w;
     w.t = bases[k];
@@ -1010,7 +1039,7 @@ cudaError_t launch_build_row_plan(const int32_t* off, int32_t V, int64_t E, cons
     const int32_t nr = plan_ranges(V);
     if (nr == 0) return cudaMemsetAsync(totals, 0, 4 * sizeof(int64_t), s);
     int64_t* counts = static_cast<int64_t*>(scratch);
-    const int blocks = (nr + kPlanBlock - 1) / kPlanBlock;
+    const int blocks = (nr + kPlanBlock / 32 - 1) / (kPlanBlock / 32);
     plan_count_kernel<<<blocks, kPlanBlock, 0, s>>>(off, V, E, counts, nr, bad);
     plan_scan_kernel<<<1, 1024, 0, s>>>(counts, nr, totals);
     plan_write_kernel<<<blocks, kPlanBlock, 0, s>>>(off, V, E, counts, nr, tiles, caps.tiles, hubs_small, hubs_big,
