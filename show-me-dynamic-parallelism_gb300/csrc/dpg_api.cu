@@ -855,6 +855,7 @@ dpg_status run_spmv(dpg_ctx* c, dpg_graph* g, const float* d_vals, const float* 
     L.col = g->relabel ? g->pcol : g->col;
     L.vals = d_vals;
     L.x = xp ? xp : d_x;
+    L.chained = xp != nullptr;
     L.hot = hot_entries(c, g, false);
     L.y = d_y;
     L.partial = partial;

@@ -183,6 +183,7 @@ struct RowGatherLaunch {
     const int32_t* items;   // sweeps: the merge items of every tile (launch_tile_items)
     const float* witems;    // weighted sweeps: the arc values in the order of items
     const float* x;         // SpMV x / PageRank contribution in
+    bool chained;           // SpMV: x is written by the kernel before, in the same call (launch_chained)
     int32_t hot;            // x[0, hot) is staged in shared memory (the most gathered renamed columns)
     float* y;               // SpMV y / PageRank contribution out
     float* partial;         // [plan.nseg] hub-segment partial sums

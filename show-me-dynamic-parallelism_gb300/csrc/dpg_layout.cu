@@ -51,6 +51,7 @@ __global__ void relabel_check_columns_kernel(const int32_t* __restrict__ col, co
 
 __global__ void gather_by_index_kernel(const float* __restrict__ x, const int32_t* __restrict__ inv, int32_t V,
                                        float* __restrict__ out) {
+    chain_next();  // launched unchained: whatever it reads is complete
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < V;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x)
         out[i] = __ldg(x + __ldg(inv + i));

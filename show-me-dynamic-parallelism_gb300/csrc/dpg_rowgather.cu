@@ -33,8 +33,8 @@ namespace dpg {
 namespace {
 
 // One CTA per SM: its dynamic shared memory holds the hot-value cache (the first `hot` renamed
-// entries of x, i.e. the most gathered columns) and its warps' tile staging. DPG_GATHER_BLOCK (and
-// the tile counts below) are build-time tuning knobs (DPG_NVCC_EXTRA); the defaults are measured.
+// entries of x, i.e. the most gathered columns) and its warps' tile staging. DPG_GATHER_BLOCK is a
+// build-time tuning knob (DPG_NVCC_EXTRA); the default is measured.
 #ifndef DPG_GATHER_BLOCK
 #define DPG_GATHER_BLOCK 1024
 #endif
@@ -44,15 +44,10 @@ constexpr int kInitBlock = 256;
 constexpr int kIpl = kRowTileItems / 32;  // merge items per lane
 constexpr int kFixBlock = 256;
 constexpr int kFixBatch = 8;  // loads the fix-up issues before it adds them
-// Tiles a warp of the SpMV carries through one step. Measured on R-MAT scale 22 with the PageRank sweep
-// that shared this kernel (1024-thread CTAs): what limits the gathers is the L1 left beside the shared
-// memory, where their sectors in flight need lines (the shared-memory budget is set with the
-// hot-cache size, see hot_entries). With a 28 KB L1 one tile per step ran best (0.29 ms per sweep);
-// with 92 KB, two tiles run 0.202 ms against 0.216 ms with one. Fewer warps lose at any setting
-// (768 threads: 0.245 ms, 512: 0.35 ms), and three tiles would spill at 1024 threads.
-#ifndef DPG_GATHER_TILES_SPMV
-#define DPG_GATHER_TILES_SPMV 2
-#endif
+// What limits the gathers is the L1 left beside the shared memory, where their sectors in flight need
+// lines: the shared-memory budget is set with the hot-cache size (see hot_entries). Fewer warps lose at
+// any setting (an earlier PageRank sweep of R-MAT 22: 0.20 ms with 1,024 threads, 0.245 with 768, 0.35 with
+// 512).
 // Shared-memory index with one pad word per 32: lane l walking items 8l.. then hits 32 distinct banks
 // instead of 4 (an 8-way conflict without the pad).
 constexpr int kPadded = kRowTileItems + kRowTileItems / 32;
@@ -243,10 +238,10 @@ __device__ __forceinline__ void fill_hot(const float* __restrict__ x, int hot, f
     __syncthreads();
 }
 
-// SpMV. One step of a warp covers KT consecutive tiles: first every column load of all KT tiles, then
-// all their gathers, then the tiles are walked one after the other through the warp's single staging
-// area. A lane thus keeps KT x 8 gathers in flight instead of 8.
-template <int KT>
+// SpMV. A warp takes one tile at a time through its staging area; the next tile's columns and values are
+// loaded while this one's gathers are in flight, and the descriptor of the one after that, so a tile costs
+// one round trip. Same box, R-MAT 22: 224 us with two tiles per step and nothing loaded ahead, 206 this way
+// (290 with the values not loaded ahead).
 __global__ void __launch_bounds__(kBlock) spmv_gather_kernel(RowGatherLaunch L) {
     extern __shared__ __align__(16) unsigned char rg_smem[];
     const int warp = threadIdx.x >> 5;
@@ -258,117 +253,106 @@ __global__ void __launch_bounds__(kBlock) spmv_gather_kernel(RowGatherLaunch L) 
     float* s_hot = reinterpret_cast<float*>(rg_smem) + kWarps * 2 * kPadded;
 
     const int ntiles = L.plan.ntiles;
-    // Descriptors and lane walks of the next step are requested one step ahead.
-    int4 Tn[KT];
-    int infon[KT];
+    int4 Tn;  // descriptor and lane walk two tiles ahead, columns and values one tile ahead
+    int infon, cn[kIpl];
+    float an[kIpl];
+    auto fetch_tile = [&](int t) {
+        Tn = t < ntiles ? __ldg(L.plan.tiles + t) : make_int4(0, 0, 0, 0);
+        infon = t < ntiles ? __ldg(L.plan.lane_info + t * 32 + lane) : 0;
+    };
+    auto fetch_values = [&] {
 #pragma unroll
-    for (int k = 0; k < KT; ++k) {
-        const int t = gwarp * KT + k;
-        Tn[k] = t < ntiles ? __ldg(L.plan.tiles + t) : make_int4(0, 0, 0, 0);
-        infon[k] = t < ntiles ? __ldg(L.plan.lane_info + t * 32 + lane) : 0;
-    }
+        for (int i = 0; i < kIpl; ++i) {
+            const int j = i * 32 + lane;
+            cn[i] = j < Tn.w ? ld_stream<kModeSpmv>(L.col + Tn.z + j) : 0;
+            an[i] = j < Tn.w ? ld_stream<kModeSpmv>(L.vals + Tn.z + j) : 0.0f;
+        }
+    };
+    fetch_tile(gwarp);
+    fetch_values();
+    int4 Tc = Tn;
+    int infoc = infon;
+    fetch_tile(gwarp + nwarps);
+    chain_wait();  // only x may still be on its way (the renaming of x, in the same call)
     fill_hot(L.x, L.hot, s_hot);
-    for (int t0 = gwarp * KT; t0 < ntiles; t0 += nwarps * KT) {
-        int4 T[KT];
-        int info[KT];
-        float pv[KT][kIpl];
-        // Phase 1: columns.
-        int cols[KT][kIpl];
+    for (int t0 = gwarp; t0 < ntiles; t0 += nwarps) {
+        const int4 T = Tc;
+        const int info = infoc;
+        int cols[kIpl];
+        float av[kIpl], pv[kIpl];
 #pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            T[k] = Tn[k];
-            info[k] = infon[k];
-            const int nb = T[k].z, nnz = T[k].w;
-#pragma unroll
-            for (int i = 0; i < kIpl; ++i) {
-                const int j = i * 32 + lane;
-                cols[k][i] = j < nnz ? ld_stream<kModeSpmv>(L.col + nb + j) : 0;
-            }
+        for (int i = 0; i < kIpl; ++i) {
+            cols[i] = cn[i];
+            av[i] = an[i];
         }
+        fetch_values();
+        Tc = Tn;
+        infoc = infon;
+        fetch_tile(t0 + 2 * nwarps);
+        // The gathers, with no branch at all: the hot test is a select and the shared-memory read
+        // unconditional (entry 0 for cold columns; the launch allocates at least one).
+        const int row = T.x, nrows = T.y, nnz = T.w;
 #pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            const int t = t0 + nwarps * KT + k;
-            Tn[k] = t < ntiles ? __ldg(L.plan.tiles + t) : make_int4(0, 0, 0, 0);
-            infon[k] = t < ntiles ? __ldg(L.plan.lane_info + t * 32 + lane) : 0;
+        for (int i = 0; i < kIpl; ++i) {
+            const int c = cols[i];
+            const bool hot = c < L.hot;
+            const float hv = s_hot[hot ? c : 0];
+            float gv = 0.0f;
+            if (!hot) gv = __ldg(L.x + c);
+            pv[i] = i * 32 + lane < nnz ? (hot ? hv : gv) * av[i] : 0.0f;
         }
-        // Phase 2: the gathers of every tile, with no branch at all: the hot test is a select, the
-        // shared-memory read unconditional (entry 0 for cold columns; the launch allocates at least
-        // one) and the value load predicated, so the gather and its value load go out together: 204 ->
-        // 255 GTEPS on R-MAT 22.
-#pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            const int nb = T[k].z, nnz = T[k].w;
-#pragma unroll
-            for (int i = 0; i < kIpl; ++i) {
-                const int j = i * 32 + lane;
-                const int c = cols[k][i];
-                const bool hot = c < L.hot;
-                const float hv = s_hot[hot ? c : 0];
-                float gv = 0.0f;
-                if (!hot) gv = __ldg(L.x + c);
-                const float a = j < nnz ? ld_stream<kModeSpmv>(L.vals + nb + j) : 0.0f;
-                pv[k][i] = j < nnz ? (hot ? hv : gv) * a : 0.0f;
-            }
-        }
-
-        // Phase 3: each tile through the staging area.
-#pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            if (t0 + k >= ntiles) break;
-            const int row = T[k].x, nrows = T[k].y, nb = T[k].z, nnz = T[k].w;
-            if (nrows < 0) {
-                // Hub segment: fixed-order lane sums, then a butterfly; partial goes to the fix-up.
-                // Values past the segment's end are 0 (phase 2), so every lane adds all of its own.
-                float acc = 0.0f;
-#pragma unroll
-                for (int i = 0; i < kIpl; ++i) acc += pv[k][i];
-                acc = warp_sum_f32(acc);
-                if (lane == 0) L.partial[-(nrows + 1)] = acc;
-                continue;
-            }
-            // All 8 values are staged (0 past nnz; pad(255) = 262 is inside the 264-entry row), so the
-            // stores need no predicate; the walk reads only the first nnz of them as nonzeros.
-#pragma unroll
-            for (int i = 0; i < kIpl; ++i) val[pad(i * 32 + lane)] = pv[k][i];
-            __syncwarp();
-            // Merge-path: lane owns merge items [d0, d1) starting at row r0; the plan's mask says
-            // which of them are row ends (emit the open row) and which are nonzeros (take one).
-            // r = row ends consumed, kk = nonzeros consumed. The walk is branch-free.
-            const int total = nrows + nnz;
-            const int d0 = min(lane * kIpl, total);
-            const int nlive = min(d0 + kIpl, total) - d0;
-            const unsigned ends = static_cast<unsigned>(info[k]) >> 8;
-            int r = d0 < total ? (info[k] & 0xFF) : nrows;
-            int kk = d0 - r;
+        if (nrows < 0) {
+            // Hub segment: fixed-order lane sums, then a butterfly; partial goes to the fix-up.
+            // Values past the segment's end are 0, so every lane adds all of its own.
             float acc = 0.0f;
-            // Rows advance only at row ends, so the first row the lane closes is its start row.
-            const int first_emit = ends != 0u ? r : -1;
 #pragma unroll
-            for (int i = 0; i < kIpl; ++i) {
-                const bool emit = (ends >> i) & 1u;
-                const bool take = i < nlive && !emit;
-                const float v = val[pad(kk)];  // kk <= nnz <= 255 stays inside the padded row
-                if (emit) out[pad(r)] = acc;
-                acc = take ? acc + v : (emit ? 0.0f : acc);
-                kk += take ? 1 : 0;
-                r += emit ? 1 : 0;
-            }
-            // Segmented inclusive scan of the lanes' open partials (key = row still open at lane end).
-            float cv = acc;
-            const int key = r;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const float tv = __shfl_up_sync(kFullMask, cv, o);
-                const int tk = __shfl_up_sync(kFullMask, key, o);
-                if (lane >= o && tk == key) cv += tv;
-            }
-            const float cin = __shfl_up_sync(kFullMask, cv, 1);
-            const int kin = __shfl_up_sync(kFullMask, key, 1);
-            if (lane > 0 && first_emit >= 0 && kin == first_emit) out[pad(first_emit)] += cin;
-            __syncwarp();
-            for (int rr = lane; rr < nrows; rr += 32) L.y[row + rr] = out[pad(rr)];
-            __syncwarp();
+            for (int i = 0; i < kIpl; ++i) acc += pv[i];
+            acc = warp_sum_f32(acc);
+            if (lane == 0) L.partial[-(nrows + 1)] = acc;
+            continue;
         }
+        // All 8 values are staged (0 past nnz; pad(255) = 262 is inside the 264-entry row), so the
+        // stores need no predicate; the walk reads only the first nnz of them as nonzeros.
+#pragma unroll
+        for (int i = 0; i < kIpl; ++i) val[pad(i * 32 + lane)] = pv[i];
+        __syncwarp();
+        // Merge-path: lane owns merge items [d0, d1) starting at row r0; the plan's mask says
+        // which of them are row ends (emit the open row) and which are nonzeros (take one).
+        // r = row ends consumed, kk = nonzeros consumed. The walk is branch-free.
+        const int total = nrows + nnz;
+        const int d0 = min(lane * kIpl, total);
+        const int nlive = min(d0 + kIpl, total) - d0;
+        const unsigned ends = static_cast<unsigned>(info) >> 8;
+        int r = d0 < total ? (info & 0xFF) : nrows;
+        int kk = d0 - r;
+        float acc = 0.0f;
+        // Rows advance only at row ends, so the first row the lane closes is its start row.
+        const int first_emit = ends != 0u ? r : -1;
+#pragma unroll
+        for (int i = 0; i < kIpl; ++i) {
+            const bool emit = (ends >> i) & 1u;
+            const bool take = i < nlive && !emit;
+            const float v = val[pad(kk)];  // kk <= nnz <= 255 stays inside the padded row
+            if (emit) out[pad(r)] = acc;
+            acc = take ? acc + v : (emit ? 0.0f : acc);
+            kk += take ? 1 : 0;
+            r += emit ? 1 : 0;
+        }
+        // Segmented inclusive scan of the lanes' open partials (key = row still open at lane end).
+        float cv = acc;
+        const int key = r;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float tv = __shfl_up_sync(kFullMask, cv, o);
+            const int tk = __shfl_up_sync(kFullMask, key, o);
+            if (lane >= o && tk == key) cv += tv;
+        }
+        const float cin = __shfl_up_sync(kFullMask, cv, 1);
+        const int kin = __shfl_up_sync(kFullMask, key, 1);
+        if (lane > 0 && first_emit >= 0 && kin == first_emit) out[pad(first_emit)] += cin;
+        __syncwarp();
+        for (int rr = lane; rr < nrows; rr += 32) L.y[row + rr] = out[pad(rr)];
+        __syncwarp();
     }
 }
 
@@ -813,7 +797,7 @@ cudaError_t prepare_rowgather(size_t bytes) {
     if (bytes <= configured) return cudaSuccess;
     cudaError_t e;
     if constexpr (MODE == kModeSpmv)
-        e = cudaFuncSetAttribute(spmv_gather_kernel<DPG_GATHER_TILES_SPMV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(spmv_gather_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(bytes));
     else
         e = cudaFuncSetAttribute(rowgather_kernel<MODE, CONV, BATCH>,
@@ -1068,8 +1052,12 @@ cudaError_t launch_row_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, stream);
         if constexpr (MODE == kModeSpmv) {
-            spmv_gather_kernel<DPG_GATHER_TILES_SPMV><<<gb, bt, smem, stream>>>(L);
-            err = cudaGetLastError();
+            if (L.chained) {
+                err = launch_chained(spmv_gather_kernel, gb, bt, smem, stream, L);
+            } else {
+                spmv_gather_kernel<<<gb, bt, smem, stream>>>(L);
+                err = cudaGetLastError();
+            }
         } else {
             err = launch_chained(rowgather_kernel<MODE, CONV, BATCH>, gb, bt, smem, stream, L);
         }
