@@ -452,8 +452,9 @@ __global__ void __launch_bounds__(kBlock, rows_blocks(VEC)) rows_kernel(RowsLaun
 // middle order, the bucket pass whole blocks. What it replaces: one random 4-byte access per arc, a
 // DRAM line each (45 G/s): the 64-column backward of R-MAT 22 took 5.6 ms with its value reads and
 // gradient writes at random, of which the pass itself is 3.2 ms. Permuting through windows of slots
-// that fit in L2 (one pass, random writes there) took 1.0 ms per permutation, this 0.69 ms; the call
-// went from 5.65 to 4.62 ms (same box).
+// that fit in L2 (one pass, random writes there) took 1.0 ms per permutation, this 0.40 ms; the call
+// went from 5.65 to 4.14 ms. Blocks of 28,672 / 24,576 / 20,480 values, two CTAs per SM: 4.22 / 4.14 / 4.23
+// ms; 32,768 in one CTA with its loads ahead: 4.77 ms (same box).
 constexpr int kPermThreads = 1024;
 
 // slot_of[arc] = transposed slot.
@@ -556,58 +557,40 @@ __global__ void __launch_bounds__(kPermThreads) perm_place_kernel(const int32_t*
 }
 
 // Block by block: the block's linear values into shared memory, then out[mid ? mid[i] : i] = value
-// idx[i] of the block. The next block's values are loaded while this one is written.
-__global__ void __launch_bounds__(kPermThreads) perm_out_kernel(const float* __restrict__ in, int64_t E, int nblk,
-                                                                const uint16_t* __restrict__ idx,
-                                                                const int32_t* __restrict__ mid,
-                                                                float* __restrict__ out) {
+// idx[i] of the block. Two CTAs per SM: while one loads, the other writes.
+__global__ void __launch_bounds__(kPermThreads, 2) perm_out_kernel(const float* __restrict__ in, int64_t E, int nblk,
+                                                                   const uint16_t* __restrict__ idx,
+                                                                   const int32_t* __restrict__ mid,
+                                                                   float* __restrict__ out) {
     extern __shared__ float s_v[];
-    constexpr int N = kPermBlock / kPermThreads;
-    float v[N];
-    auto load = [&](int c) {
-        const int64_t e0 = static_cast<int64_t>(c) * kPermBlock;
-#pragma unroll
-        for (int q = 0; q < N; ++q) {
-            const int64_t e = e0 + q * kPermThreads + threadIdx.x;
-            v[q] = c < nblk && e < E ? __ldcs(in + e) : 0.0f;
-        }
-    };
-    load(blockIdx.x);
     for (int c = blockIdx.x; c < nblk; c += gridDim.x) {
-#pragma unroll
-        for (int q = 0; q < N; ++q) s_v[q * kPermThreads + threadIdx.x] = v[q];
-        __syncthreads();
-        load(c + gridDim.x);
         const int64_t e0 = static_cast<int64_t>(c) * kPermBlock;
-#pragma unroll 8
-        for (int q = 0; q < N; ++q) {
-            const int64_t e = e0 + q * kPermThreads + threadIdx.x;
-            if (e < E) out[mid ? __ldcs(mid + e) : e] = s_v[__ldcs(idx + e)];
-        }
+        const int n = static_cast<int>(E - e0 < kPermBlock ? E - e0 : kPermBlock);
+#pragma unroll 7
+        for (int i = threadIdx.x; i < n; i += kPermThreads) s_v[i] = __ldcs(in + e0 + i);
+        __syncthreads();
+#pragma unroll 7
+        for (int i = threadIdx.x; i < n; i += kPermThreads)
+            out[mid ? __ldcs(mid + e0 + i) : e0 + i] = s_v[__ldcs(idx + e0 + i)];
         __syncthreads();
     }
 }
 
 // The other way: value idx[i] of the block = in[mid ? mid[i] : i], then the block goes out linearly.
-__global__ void __launch_bounds__(kPermThreads) perm_in_kernel(const float* __restrict__ in, int64_t E, int nblk,
-                                                               const uint16_t* __restrict__ idx,
-                                                               const int32_t* __restrict__ mid,
-                                                               float* __restrict__ out) {
+__global__ void __launch_bounds__(kPermThreads, 2) perm_in_kernel(const float* __restrict__ in, int64_t E, int nblk,
+                                                                  const uint16_t* __restrict__ idx,
+                                                                  const int32_t* __restrict__ mid,
+                                                                  float* __restrict__ out) {
     extern __shared__ float s_v[];
-    constexpr int N = kPermBlock / kPermThreads;
     for (int c = blockIdx.x; c < nblk; c += gridDim.x) {
         const int64_t e0 = static_cast<int64_t>(c) * kPermBlock;
-#pragma unroll 16
-        for (int q = 0; q < N; ++q) {
-            const int64_t e = e0 + q * kPermThreads + threadIdx.x;
-            if (e < E) s_v[__ldcs(idx + e)] = __ldcs(in + (mid ? __ldcs(mid + e) : e));
-        }
+        const int n = static_cast<int>(E - e0 < kPermBlock ? E - e0 : kPermBlock);
+#pragma unroll 7
+        for (int i = threadIdx.x; i < n; i += kPermThreads)
+            s_v[__ldcs(idx + e0 + i)] = __ldcs(in + (mid ? __ldcs(mid + e0 + i) : e0 + i));
         __syncthreads();
-#pragma unroll
-        for (int q = 0; q < N; ++q) {
-            const int64_t e = e0 + q * kPermThreads + threadIdx.x;
-            if (e < E) out[e] = s_v[q * kPermThreads + threadIdx.x];
-        }
+#pragma unroll 7
+        for (int i = threadIdx.x; i < n; i += kPermThreads) out[e0 + i] = s_v[i];
         __syncthreads();
     }
 }
@@ -791,7 +774,7 @@ cudaError_t launch_permute(const ArcPerm& P, int64_t E, bool to_slots, const flo
                            cudaStream_t s, int sm_count, LaunchHook* hook) {
     constexpr int smem = kPermBlock * sizeof(float);
     const int nblk = static_cast<int>((E + kPermBlock - 1) / kPermBlock);
-    const int grid = std::min(nblk, sm_count);
+    const int grid = std::min(nblk, 2 * sm_count);
     cudaError_t e = cudaFuncSetAttribute(perm_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(perm_in_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;

@@ -478,7 +478,7 @@ dpg_status ensure_spmm_transpose(dpg_graph* g, bool need_graph = false) {
 // Arc values in transposed order for the backward: the permutation and the two arrays. The transposed
 // pass reads val[arc] and writes dA[arc] at random; past the size of the L2 each is a random DRAM line
 // per arc, which bounds the pass. Permuting both, in arc order / permuted: 67 M arcs (268 MB of values)
-// 5.65 / 4.62 ms with 64 columns, 16.8 M arcs (67 MB, about half the L2) 0.865 / 0.850 ms with 32 and
+// 5.65 / 4.14 ms with 64 columns, 16.8 M arcs (67 MB, about half the L2) 0.865 / 0.850 ms with 32 and
 // 1.73-1.86 / 1.85 ms with 96 columns, 7.6 M arcs 0.23 / 0.38 ms with 20: the line lies at 2^25 arcs, past
 // the L2's 126 MB. False: not worth it, or no memory for it; the pass then works in arc order.
 constexpr int64_t kSlotArcs = 1 << 25;

@@ -262,8 +262,8 @@ cudaError_t launch_spmm(const SpmmPlanDev& P, const int32_t* col, const float* v
 cudaError_t launch_arc_dot(const SpmmPlanDev& P, const int32_t* col, const float* X, const float* G, int nrhs,
                            float* dA, cudaStream_t s, int sm_count, LaunchHook* hook);
 // Permutation of arc values between CSR order and transposed order (dpg_adjoint.cu): E entries each.
-constexpr int32_t kPermBlock = 1 << 15;
-constexpr int64_t kPermMaxArcs = int64_t{1} << 28;  // 8,192 chunks: their run starts fit in shared memory
+constexpr int32_t kPermBlock = 24576;  // 96 KB: two blocks per SM
+constexpr int64_t kPermMaxArcs = int64_t{1} << 28;  // 10,923 chunks: their run starts fit in shared memory
 struct ArcPerm {
     int32_t* mid = nullptr;
     uint16_t* arc_in = nullptr;
