@@ -477,11 +477,13 @@ dpg_status ensure_spmm_transpose(dpg_graph* g, bool need_graph = false) {
 
 // Arc values in transposed order for the backward: the permutation and the two arrays. The transposed
 // pass reads val[arc] and writes dA[arc] at random; past the size of the L2 each is a random DRAM line
-// per arc, which bounds the pass. Permuting both, in arc order / permuted: 67 M arcs (268 MB of values)
-// 5.65 / 4.14 ms with 64 columns, 16.8 M arcs (67 MB, about half the L2) 0.865 / 0.850 ms with 32 and
-// 1.73-1.86 / 1.85 ms with 96 columns, 7.6 M arcs 0.23 / 0.38 ms with 20: the line lies at 2^25 arcs, past
-// the L2's 126 MB. False: not worth it, or no memory for it; the pass then works in arc order.
-constexpr int64_t kSlotArcs = 1 << 25;
+// per arc, which bounds the pass. Permuting both, in arc order / permuted: 67 M arcs 5.65 / 4.14 ms with
+// 64 columns; 30 M 2.32 / 2.00 with 64 and 1.25 / 0.63 with 1; 16.8 M 0.54 / 0.36 with 1, 0.80 / 0.69 with
+// 32, 1.64 / 1.62 with 96; 12 M 0.27 / 0.26 with 1, 0.52 / 0.49 with 32, 1.16 / 1.11 with 128; 8.4 M 0.14 /
+// 0.21 with 1, 0.29 / 0.38 with 32, 0.74 / 0.81 with 100. The line lies just past the crossing, at 12.6 M
+// arcs: values, gradients and slots together are then 151 MB, past the L2's 129 MB. False: not worth it, or
+// no memory for it; the pass then works in arc order.
+constexpr int64_t kSlotArcs = 3 << 22;
 bool backward_slots(dpg_graph* g, float** vals_t, float** dA_t) {
     if (g->E < kSlotArcs || g->E > kPermMaxArcs) return false;
     dpg_ctx* c = g->ctx;
