@@ -75,6 +75,7 @@ struct ExpandParams {
     int32_t label_vec4;
     int32_t local_rounds;   // near-far and direction-optimizing: see local_relax (0: off)
     int32_t nctas;          // CTAs that take part in the solve (the first ones of the grid)
+    int32_t peek_l1;        // single-source SSSP: label peeks may hit the L1 (see kPeekL1)
     uint32_t min_item_log;  // log2 of the fewest small-queue vertices in a warp item (binned kernels)
 };
 
@@ -594,6 +595,14 @@ __device__ __forceinline__ void far_push(const ExpandParams& P, const PushCtx& Q
     }
 }
 
+// Single-source SSSP may read the label peeks through the L1: labels only decrease within a solve, so a line that is a
+// few relaxations old costs an extra atomic at most, and the barrier's acquire drops the lines once per iteration. The
+// host allows it up to kPeekL1 vertices, where the labels are a few times an SM's L1 at most; with more of them nearly
+// every peek misses and pays for the line's allocation. L2 / L1, R-MAT on one box: 5,062 vertices x 8 arcs 100.0 / 97.0
+// us, 2^14 x 16 114.2 / 104.8, 30,001 x 32 177 / 165, 2^16 x 16 209 / 205, 2^17 285 / 282, 10^6 494 / 498, 2^22
+// 1.435 / 1.465 ms, 2^24 4.69 / 4.99.
+constexpr int32_t kPeekL1 = 1 << 17;
+
 // U independent relaxations per lane, issued phase by phase (U adjacency loads, U label loads, U
 // atomics, one batched push) so each warp keeps U memory operations in flight instead of one.
 template <class Op, bool kClassify, int CH, int U>
@@ -661,7 +670,19 @@ __device__ __forceinline__ void relax_batch(const ExpandParams& P, const PushCtx
 #pragma unroll
         for (int u = 0; u < U; ++u) Op::load_edge(P, act[u] ? e[u] : 0, du[u], v[u], row[u], cand[u]);
 #pragma unroll
-        for (int u = 0; u < U; ++u) cur[u] = Op::kPeek ? __ldcg(P.label + v[u]) : 0;
+        for (int u = 0; u < U; ++u) cur[u] = 0;
+        if constexpr (std::is_same_v<Op, SsspOp>) {
+            if (P.peek_l1) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) cur[u] = __ldca(P.label + v[u]);
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u) cur[u] = __ldcg(P.label + v[u]);
+            }
+        } else if constexpr (Op::kPeek) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) cur[u] = __ldcg(P.label + v[u]);
+        }
         if constexpr (U <= 4) {
             if (Q.early_rows) {
                 // Row ranges of every candidate head, issued with the peeks (extra loads for heads
@@ -1573,6 +1594,7 @@ cudaError_t run_multi(const MultiExpandLaunch& L, const ExpandWorkspace& ws, Dev
     P.st = st;
     P.nsrc = L.nsrc;
     P.nctas = grid;
+    P.peek_l1 = 0;
     P.min_item_log = min_item_log(L.V, L.E);
     P.dirty[0] = L.dirty[0];
     P.dirty[1] = L.dirty[1];
@@ -1649,6 +1671,7 @@ cudaError_t launch_expand(const ExpandLaunch& L, const ExpandWorkspace& ws, DevS
     P.nf = diropt ? L.do_nf : nullptr;
     P.E = L.E;
     P.min_item_log = min_item_log(L.V, L.E);
+    P.peek_l1 = L.V <= kPeekL1;
     P.nctas = sm_count * (L.solution >= DPG_SOL_BINNED ? active_blocks(L.E, per_sm) : per_sm);
     P.local_rounds = L.local_rounds;
     const int classify =
@@ -1700,6 +1723,7 @@ cudaError_t launch_color(const ExpandLaunch& L, const int32_t* out_off, const in
     P.trace_cap = L.trace_cap;
     P.aux = pending;
     P.nctas = grid;
+    P.peek_l1 = 0;
     P.min_item_log = min_item_log(L.V, L.E);
     err = cudaMemsetAsync(ws.qcount, 0, sizeof(uint32_t) * 3, stream);
     if (err == cudaSuccess) err = cudaMemsetAsync(ws.ccount, 0, sizeof(uint32_t) * 3, stream);
