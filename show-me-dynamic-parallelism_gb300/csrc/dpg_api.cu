@@ -621,6 +621,13 @@ constexpr double kNearFarStep = 32.0;
 // arcs grow; levels hardly ever need a second relaxation, and 32 rounds leave little to gain.
 constexpr int32_t kNearFarRounds = 5;
 constexpr int32_t kLevelRounds = 32;
+// Vertices and arcs from which SSSP on graphs with hubs climbs a ladder of thresholds (kLadderPhases in dpg_expand.cu):
+// below, the few more iterations of each phase cost more than the arcs that are not scanned again. Without / with:
+// 10^6 vertices x 8 arcs 396 / 420 us, 100,000 x 32 174 / 229, 300,000 x 32 340 / 368, 500,000 x 32 427 / 477; then
+// 650,000 x 16 559 / 489, 650,000 x 32 544 / 518, 10^6 x 16 519 / 418, 1.2 M x 8 616 / 607, 2 M x 8 569 / 476,
+// 6 M x 8 1.07 / 0.85 ms, 3 M x 32 2.18 / 1.27.
+constexpr int32_t kLadderVertices = 650000;
+constexpr int64_t kLadderArcs = 10000000;
 
 void fill_expand_defaults(const dpg_expand_opts* in, dpg_expand_opts* o, const dpg_graph* g) {
     if (in) *o = *in;
@@ -654,7 +661,8 @@ dpg_status run_expand(dpg_ctx* c, const dpg_graph* g, int32_t source, const dpg_
     // The default id asks for the GB300 choice; for SSSP (bottom-up steps are BFS only) that is
     // near-far on graphs without hubs and of low mean degree (road-like, grids: 4096^2 grid 68 ms
     // against 167 ms binned), and the binned expansion otherwise (R-MAT: near-far only ties it).
-    if (!bfs && o.solution == DPG_SOL_DIROPT)
+    const bool pick = !bfs && o.solution == DPG_SOL_DIROPT;
+    if (pick)
         o.solution = (g->weighted && g->max_degree < o.hub_threshold && g->E <= 8 * static_cast<int64_t>(g->V))
                          ? DPG_SOL_NEARFAR
                          : DPG_SOL_BINNED;
@@ -683,6 +691,13 @@ dpg_status run_expand(dpg_ctx* c, const dpg_graph* g, int32_t source, const dpg_
     // A caller's own iteration cap counts grid-wide iterations of one round each.
     if (o.solution == DPG_SOL_NEARFAR || o.solution == DPG_SOL_DIROPT)
         L.local_rounds = in_opts && in_opts->max_iterations > 0 ? 0 : bfs ? kLevelRounds : kNearFarRounds;
+    // A caller's own solution or iteration cap keeps the plain order of relaxations. The ladder's phases may together
+    // take more iterations than the vertices a path can have.
+    if (pick && o.solution == DPG_SOL_BINNED && !(in_opts && in_opts->max_iterations > 0) && g->V >= kLadderVertices &&
+        g->E >= kLadderArcs) {
+        L.ladder = static_cast<int32_t>(std::max(1.0, std::min(1e8, g->mean_weight / 64)));
+        L.max_iter = static_cast<int32_t>(std::min<int64_t>(INT32_MAX, (static_cast<int64_t>(g->V) + 3) * 8));
+    }
     if (!bfs && o.solution == DPG_SOL_NEARFAR) {
         // Three piles of E + V {vertex, distance} pairs (at most one current entry per vertex, plus
         // stale ones; an overflow stops the solve with DPG_ERR_CAPACITY).

@@ -35,6 +35,23 @@
 namespace dpg {
 namespace {
 
+// Ladder of thresholds for single-source SSSP on large graphs with hubs (binned). Relaxed in plain iterations, the hubs'
+// distances, which are small, improve two or three times after the first, and each time all their arcs are scanned
+// again: R-MAT 24 scanned 2.2 E arcs, nearly all of them out of hubs, though 1 E is enough. From the first large
+// iteration on, only improvements below the threshold are pushed. The others stay in their label, cost no bitmap bit,
+// row range or queue slot, and when the frontier runs dry a sweep over all labels pushes those between the old threshold
+// and the next. A label at or above the threshold has not been expanded since it was set (or, from before the ladder
+// began, is only expanded once more), so the sweeps miss nothing. The last phase has no threshold. Near-far's piles
+// (DPG_SOL_NEARFAR) are for sparse graphs and many thresholds; here every arc's improvement would be appended (R-MAT 24:
+// 8.7 ms or more). A sweep of 16 M labels takes 40-100 us with its pushes, so few thresholds pay: mean weight / 64 (hubs
+// are a few of the smallest weights apart), then 3 and 9 times that. Without / with, one box, 16 arcs per vertex: 2^24
+// 4.83 / 2.82 ms (593 / 301 M arcs scanned, 11.1 / 6.2 M pops), 2^22 1.37 / 0.92 ms, 10^6 515 / 421 us. Other ladders at
+// 2^24 and 10^6, first threshold and steps: 1/64 x 2 x 2 x 2 2.89 ms, 463 us; 1/64 x 4 3.20, 464; 1/32 x 2 x 2 2.85, 459;
+// 1/32 x 1.5 x 1.5 x 1.5 2.78, 464; 1/16 and five steps of 1.5 3.28, 577.
+constexpr int kLadderPhases = 3;
+constexpr int kLadderStep = 3;
+constexpr int kSweep = 16;  // labels a lane reads at a time in a sweep
+
 constexpr int kBlock = 256;
 constexpr int kWarps = kBlock / 32;
 
@@ -75,6 +92,7 @@ struct ExpandParams {
     int32_t label_vec4;
     int32_t local_rounds;   // near-far and direction-optimizing: see local_relax (0: off)
     int32_t nctas;          // CTAs that take part in the solve (the first ones of the grid)
+    int32_t ladder;         // single-source binned SSSP: first threshold (see kLadderPhases; 0: off)
     int32_t peek_l1;        // single-source SSSP: label peeks may hit the L1 (see kPeekL1)
     uint32_t min_item_log;  // log2 of the fewest small-queue vertices in a warp item (binned kernels)
 };
@@ -112,6 +130,11 @@ struct SsspOp {
     __device__ __forceinline__ static bool commit(const ExpandParams& P, int v, int cand) {
         return cand < atomicMin(P.label + v, cand);
     }
+};
+
+// Pushes of a ladder sweep: each vertex comes up once, and nothing else is pushed in its iteration.
+struct SweepOp : SsspOp {
+    static constexpr bool kDedup = false;
 };
 
 struct BfsOp {
@@ -603,6 +626,17 @@ __device__ __forceinline__ void far_push(const ExpandParams& P, const PushCtx& Q
 // 1.435 / 1.465 ms, 2^24 4.69 / 4.99.
 constexpr int32_t kPeekL1 = 1 << 17;
 
+// Improvements at or above the ladder's threshold wait in their label for a sweep (see kLadderPhases).
+template <class Op, int U>
+__device__ __forceinline__ void ladder_cut(const PushCtx& Q, bool (&ok)[U], const int (&cand)[U]) {
+    if constexpr (std::is_same_v<Op, SsspOp>) {
+        if (!Q.far) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) ok[u] = ok[u] && cand[u] < Q.threshold;
+        }
+    }
+}
+
 // U independent relaxations per lane, issued phase by phase (U adjacency loads, U label loads, U
 // atomics, one batched push) so each warp keeps U memory operations in flight instead of one.
 template <class Op, bool kClassify, int CH, int U>
@@ -693,6 +727,7 @@ __device__ __forceinline__ void relax_batch(const ExpandParams& P, const PushCtx
 #pragma unroll
                 for (int u = 0; u < U; ++u)
                     ok[u] = act[u] && Op::want(v[u], cand[u], cur[u]) && Op::commit(P, v[u], cand[u]);
+                ladder_cut<Op>(Q, ok, cand);
                 if (Q.far) {
                     bool far[U];
 #pragma unroll
@@ -709,6 +744,7 @@ __device__ __forceinline__ void relax_batch(const ExpandParams& P, const PushCtx
 #pragma unroll
         for (int u = 0; u < U; ++u)
             ok[u] = act[u] && Op::want(v[u], cand[u], cur[u]) && Op::commit(P, v[u], cand[u]);
+        ladder_cut<Op>(Q, ok, cand);
         if (Q.far) {  // near-far: improvements at or above the threshold wait in the far pile
             bool far[U];
 #pragma unroll
@@ -996,7 +1032,9 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
     // moves past delta and the pile's minimum, and one split step moves the pile's still-current
     // entries below it into the frontier and the rest into the next pile. Piles rotate over three
     // buffers so the one being reset is never the one being read or written.
-    int threshold = kNearFar ? P.delta : 0;
+    constexpr bool kLadder = POL == DPG_SOL_BINNED && std::is_same_v<Op, SsspOp>;
+    int threshold = kNearFar ? P.delta : 0x7FFFFFFF;
+    int phase = kLadder && P.ladder ? 0 : kLadderPhases;  // thresholds left behind; the ladder is off past the last
     int pile = 0;
     int j = 0;
     // The iteration's counters. In the 3-CTA builds (sparse graphs, whose thousands of small
@@ -1047,7 +1085,19 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
             const long long t = max(static_cast<long long>(threshold) + P.delta, static_cast<long long>(fmin) + 1);
             threshold = static_cast<int>(min(t, static_cast<long long>(0x7FFFFFFF)));
         }
-        if (!split && n == 0 && nch == 0) break;
+        if (kLadder && phase == 0 && n + 256ull * nch >= kPushBufferWork) {
+            threshold = P.ladder;
+            phase = 1;
+        }
+        bool sweep = false;
+        int sweep_lo = 0;
+        if (kLadder && n == 0 && nch == 0 && threshold != 0x7FFFFFFF) {
+            sweep = true;
+            sweep_lo = threshold;
+            threshold = phase < kLadderPhases ? threshold * kLadderStep : 0x7FFFFFFF;
+            ++phase;
+        }
+        if (!split && !sweep && n == 0 && nch == 0) break;
         if (j >= P.max_iter) {
             if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(P.st, DPG_ERR_CAPACITY, 2);
             break;
@@ -1080,7 +1130,7 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
         // round trip per iteration. The arcs to relax (vertices plus 256-arc chunks) decide, the
         // same for every CTA. On R-MAT 24 it cut SSSP from 7.6 to 5.6 ms and BFS from 1.70 to 1.16
         // ms; on the 4096^2 grid, buffering every iteration cost near-far SSSP 11 %.
-        const unsigned long long work = static_cast<unsigned long long>(n) + 256ull * nch + (split ? far_n : 0u);
+        const unsigned long long work = static_cast<unsigned long long>(n) + 256ull * nch + (split ? far_n : 0u) + (sweep ? P.V : 0);
         const bool buffered = work >= kPushBufferWork || (kDirOpt && bottom_up);
         // A traversal past kLocalAfter iterations with a small frontier is of a high-diameter graph.
         const bool local = kCtaCounters && !buffered && j >= kLocalAfter && P.local_rounds > 0;
@@ -1108,7 +1158,38 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
             while (item_log > P.min_item_log && (n >> (item_log - 1u)) + nch < nwarps) --item_log;
         const unsigned fchunks = (n + (1u << item_log) - 1u) >> item_log;
 
-        if (kNearFar && split) {
+        if (kLadder && sweep) {
+            // Found vertices are gathered to full warps before they are pushed: a push is a chain of two round trips,
+            // and about one label in thirty qualifies.
+            const int hi = min(threshold, DPG_INF_COST);
+            int* found = s_start[warp];
+            int pend = 0;
+            for (int64_t base = static_cast<int64_t>(gwarp) * (32 * kSweep); base < P.V;
+                 base += static_cast<int64_t>(nwarps) * (32 * kSweep)) {
+                int l[kSweep];
+#pragma unroll
+                for (int u = 0; u < kSweep; ++u)
+                    l[u] = __ldcg(P.label + min(base + 32 * u + lane, static_cast<int64_t>(P.V) - 1));
+#pragma unroll
+                for (int u = 0; u < kSweep; ++u) {
+                    const int64_t x = base + 32 * u + lane;
+                    const bool ok = x < P.V && l[u] >= sweep_lo && l[u] < hi;
+                    const unsigned m = __ballot_sync(kFullMask, ok);
+                    const int pos = pend + __popc(m & ((1u << lane) - 1u));
+                    if (ok && pos < 32) found[pos] = static_cast<int>(x);
+                    pend += __popc(m);
+                    if (pend >= 32) {
+                        __syncwarp();
+                        push_converged<SweepOp, kClassify, CH>(P, Q, true, found[lane]);
+                        __syncwarp();
+                        if (ok && pos >= 32) found[pos - 32] = static_cast<int>(x);
+                        pend -= 32;
+                    }
+                }
+            }
+            __syncwarp();
+            push_converged<SweepOp, kClassify, CH>(P, Q, lane < pend, lane < pend ? found[lane] : 0);
+        } else if (kNearFar && split) {
             // Split: still-current entries below the new threshold join the frontier (de-duplicated
             // by the bitmap), the rest move to the next pile; stale entries are dropped.
             const int2* src = P.far[pile];
@@ -1595,6 +1676,7 @@ cudaError_t run_multi(const MultiExpandLaunch& L, const ExpandWorkspace& ws, Dev
     P.nsrc = L.nsrc;
     P.nctas = grid;
     P.peek_l1 = 0;
+    P.ladder = 0;
     P.min_item_log = min_item_log(L.V, L.E);
     P.dirty[0] = L.dirty[0];
     P.dirty[1] = L.dirty[1];
@@ -1672,6 +1754,7 @@ cudaError_t launch_expand(const ExpandLaunch& L, const ExpandWorkspace& ws, DevS
     P.E = L.E;
     P.min_item_log = min_item_log(L.V, L.E);
     P.peek_l1 = L.V <= kPeekL1;
+    P.ladder = L.ladder;
     P.nctas = sm_count * (L.solution >= DPG_SOL_BINNED ? active_blocks(L.E, per_sm) : per_sm);
     P.local_rounds = L.local_rounds;
     const int classify =
@@ -1724,6 +1807,7 @@ cudaError_t launch_color(const ExpandLaunch& L, const int32_t* out_off, const in
     P.aux = pending;
     P.nctas = grid;
     P.peek_l1 = 0;
+    P.ladder = 0;
     P.min_item_log = min_item_log(L.V, L.E);
     err = cudaMemsetAsync(ws.qcount, 0, sizeof(uint32_t) * 3, stream);
     if (err == cudaSuccess) err = cudaMemsetAsync(ws.ccount, 0, sizeof(uint32_t) * 3, stream);

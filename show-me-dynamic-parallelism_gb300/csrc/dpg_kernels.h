@@ -93,6 +93,7 @@ struct ExpandLaunch {
     int* far_min = nullptr;
     int64_t far_cap = 0;
     int32_t delta = 0;
+    int32_t ladder = 0;        // first threshold of single-source SSSP's ladder (0: off)
     int32_t local_rounds = 0;  // rounds a warp goes on with its own improvements before the grid barrier
     // A graph with hubs or more than 8 arcs per vertex: the binned and direction-optimizing kernels
     // run their build for more CTAs per SM (kWideBlocks in dpg_expand.cu).
