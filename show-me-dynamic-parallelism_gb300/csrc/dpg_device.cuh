@@ -17,7 +17,7 @@ struct DevStatus {
     int error;                     // dpg_status raised on the device
     int error_site;                // small code telling which check fired
     unsigned bar_count;            // grid-barrier word (see grid_barrier); 0 when a launch starts
-    unsigned bar_gen;              // unused
+    int ladder_base;               // smallest distance of a hub when an SSSP ladder begins
     unsigned fix_count;            // last-block ticket of the hub fix-up kernel
     unsigned pad0;
     unsigned long long iterations; // statistics of the last persistent launch

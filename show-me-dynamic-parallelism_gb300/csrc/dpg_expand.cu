@@ -37,17 +37,20 @@ namespace {
 
 // Ladder of thresholds for single-source SSSP on large graphs with hubs (binned). Relaxed in plain iterations, the hubs'
 // distances, which are small, improve two or three times after the first, and each time all their arcs are scanned
-// again: R-MAT 24 scanned 2.2 E arcs, nearly all of them out of hubs, though 1 E is enough. From the first large
-// iteration on, only improvements below the threshold are pushed. The others stay in their label, cost no bitmap bit,
-// row range or queue slot, and when the frontier runs dry a sweep over all labels pushes those between the old threshold
-// and the next. A label at or above the threshold has not been expanded since it was set (or, from before the ladder
-// began, is only expanded once more), so the sweeps miss nothing. The last phase has no threshold. Near-far's piles
-// (DPG_SOL_NEARFAR) are for sparse graphs and many thresholds; here every arc's improvement would be appended (R-MAT 24:
-// 8.7 ms or more). A sweep of 16 M labels takes 40-100 us with its pushes, so few thresholds pay: mean weight / 64 (hubs
-// are a few of the smallest weights apart), then 3 and 9 times that. Without / with, one box, 16 arcs per vertex: 2^24
-// 4.83 / 2.82 ms (593 / 301 M arcs scanned, 11.1 / 6.2 M pops), 2^22 1.37 / 0.92 ms, 10^6 515 / 421 us. Other ladders at
-// 2^24 and 10^6, first threshold and steps: 1/64 x 2 x 2 x 2 2.89 ms, 463 us; 1/64 x 4 3.20, 464; 1/32 x 2 x 2 2.85, 459;
-// 1/32 x 1.5 x 1.5 x 1.5 2.78, 464; 1/16 and five steps of 1.5 3.28, 577.
+// again: R-MAT 24 scans 2 to 4 E arcs by source, nearly all of them out of hubs, though 1 E is enough. At the first large
+// iteration the nearest hub of the frontier gives a base distance (one more barrier); from then on only vertices below
+// the threshold are expanded and pushed. The others stay in their label, cost no bitmap bit, row range or queue slot, and
+// when the frontier runs dry a sweep over all labels pushes those between the old threshold and the next. A label at or
+// above the threshold has not been expanded since it was set (or, from before the ladder began, is only expanded once
+// more), so the sweeps miss nothing. The last phase has no threshold. Counted from 0 instead of from the nearest hub,
+// the thresholds were passed before the first hub was reached from most sources. Near-far's piles (DPG_SOL_NEARFAR) are
+// for sparse graphs and many thresholds; here every arc's improvement would be appended (R-MAT 24: 8.7 ms or more). A
+// sweep of 16 M labels takes 40-100 us with its pushes, so few thresholds pay: mean weight / 64 (hubs are a few of the
+// smallest weights apart), then 3 and 9 times that. Without / with, one box, 16 arcs per vertex, from a hub: 2^24 4.83 /
+// 2.82 ms (593 / 290 M arcs scanned, 11.1 / 6.1 M pops), 2^22 1.37 / 0.92 ms, 10^6 515 / 421 us; from random sources of
+// 2^24 2.0-4.1 E / 1.07-1.73 E arcs scanned. Other ladders at 2^24 and 10^6, first threshold and steps (counted from 0):
+// 1/64 x 2 x 2 x 2 2.89 ms, 463 us; 1/64 x 4 3.20, 464; 1/32 x 2 x 2 2.85, 459; 1/32 x 1.5 x 1.5 x 1.5 2.78, 464; 1/16 and
+// five steps of 1.5 3.28, 577.
 constexpr int kLadderPhases = 3;
 constexpr int kLadderStep = 3;
 constexpr int kSweep = 16;  // labels a lane reads at a time in a sweep
@@ -1035,6 +1038,8 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
     constexpr bool kLadder = POL == DPG_SOL_BINNED && std::is_same_v<Op, SsspOp>;
     int threshold = kNearFar ? P.delta : 0x7FFFFFFF;
     int phase = kLadder && P.ladder ? 0 : kLadderPhases;  // thresholds left behind; the ladder is off past the last
+    int ladder_base = 0;
+    int step = P.ladder;
     int pile = 0;
     int j = 0;
     // The iteration's counters. In the 3-CTA builds (sparse graphs, whose thousands of small
@@ -1085,8 +1090,16 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
             const long long t = max(static_cast<long long>(threshold) + P.delta, static_cast<long long>(fmin) + 1);
             threshold = static_cast<int>(min(t, static_cast<long long>(0x7FFFFFFF)));
         }
-        if (kLadder && phase == 0 && n + 256ull * nch >= kPushBufferWork) {
-            threshold = P.ladder;
+        if (kLadder && phase == 0 && nch > 0 && n + 256ull * nch >= kPushBufferWork) {
+            // The ladder begins: its thresholds count from the nearest hub of this frontier.
+            int nearest = 0x7FFFFFFF;
+            for (unsigned i = gwarp * 32u + lane; i < nch; i += nwarps * 32u)
+                nearest = min(nearest, __ldcg(P.label + __ldcg(&(p ? P.ws.chunks[1] : P.ws.chunks[0])[i].x)));
+            nearest = __reduce_min_sync(kFullMask, nearest);
+            if (lane == 0 && nearest != 0x7FFFFFFF) atomicMin(&P.st->ladder_base, nearest);
+            if (!grid_barrier(P.st, P.nctas, P.timeout_ns)) break;
+            ladder_base = *reinterpret_cast<const volatile int*>(&P.st->ladder_base);
+            threshold = ladder_base + step;
             phase = 1;
         }
         bool sweep = false;
@@ -1094,7 +1107,8 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
         if (kLadder && n == 0 && nch == 0 && threshold != 0x7FFFFFFF) {
             sweep = true;
             sweep_lo = threshold;
-            threshold = phase < kLadderPhases ? threshold * kLadderStep : 0x7FFFFFFF;
+            step *= kLadderStep;
+            threshold = phase < kLadderPhases ? ladder_base + step : 0x7FFFFFFF;
             ++phase;
         }
         if (!split && !sweep && n == 0 && nch == 0) break;
@@ -1356,6 +1370,9 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                         if (O::kDedup) __stcg(bmp_cur + (v0 >> 5), 0u);
                         my_pops += 1;
                     }
+                    if constexpr (kLadder) {
+                        if (du >= threshold) continue;  // queued before the ladder began: left to a sweep
+                    }
                     if (lane == 0) my_edges += static_cast<unsigned long long>(k1 - k0);
                     // The whole chunk in one batch; the multi-source relaxation, whose slots each hold two
                     // vertices' labels, 128 arcs at a time: 256-arc chunks in one batch took 12.4 ms
@@ -1384,7 +1401,7 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                 const unsigned i = (chunk << item_log) + lane;
                 int u = 0, s = 0, d = 0;
                 RV du{};
-                const bool has = i < n && (!kBinned || static_cast<unsigned>(lane) < (1u << item_log));
+                bool has = i < n && (!kBinned || static_cast<unsigned>(lane) < (1u << item_log));
                 if (has) {
                     u = __ldcg(qv_cur + i);
                     const int2 se = __ldcg(qse_cur + i);
@@ -1393,7 +1410,9 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                     du = O::row_value(P, u, j);
                     if (O::kDedup) __stcg(bmp_cur + (u >> 5), 0u);
                     my_pops += 1;
-                    my_edges += static_cast<unsigned long long>(d);
+                    if constexpr (kLadder) has = du < threshold;
+                    if (has) my_edges += static_cast<unsigned long long>(d);
+                    else d = 0;
                 }
                 if (POL == DPG_SOL_THREAD || POL == DPG_SOL_GRID) {
                     serial_rows<O, kClassify, CH>(P, Q, has, s, d, du);
@@ -1472,6 +1491,7 @@ __global__ void expand_init_kernel(ExpandParams P, int32_t source, int32_t init_
             P.ws.ccount[k] = 0u;
         }
         P.st->bar_count = 0u;
+        P.st->ladder_base = 0x7FFFFFFF;
         P.st->iterations = 0ull;
         P.st->edges = 0ull;
         P.st->pops = 0ull;
