@@ -65,7 +65,7 @@ __global__ void batch_pr_setup_kernel(const int32_t* __restrict__ vstart, int n,
 // block to finish adds each graph's piece partials, a warp per graph.
 __global__ void __launch_bounds__(kBlk) batch_dangling_kernel(const int4* __restrict__ pieces, int npieces,
                                                               const int32_t* __restrict__ dslot,
-                                                              const float* __restrict__ y,
+                                                              const float* y,
                                                               const int32_t* __restrict__ gpiece,
                                                               const int32_t* __restrict__ vstart, int n, double damping,
                                                               double total, double* gpart, float* gbase,

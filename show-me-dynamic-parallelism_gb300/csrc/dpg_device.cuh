@@ -90,9 +90,12 @@ __device__ __forceinline__ bool grid_barrier(DevStatus* st, unsigned expected,
 // nothing is written, and nothing that may still change is read, ahead of it. chain_next, called behind
 // the wait, lets the next chained kernel start early; without it, that happens when this kernel ends. In
 // a kernel that was not launched so, chain_wait does nothing.
+// What the predecessors in the chain write changes during this kernel's lifetime, so it is read by ordinary
+// volatile loads behind the wait (__ldca, __ldcg, ld_live), never through the read-only path (__ldg), which
+// is for what was written before the chain.
 // An early start also moves the L1's invalidation ahead of the predecessor's end, so lines that the
 // predecessor loads on the same SM while it runs stay there: what it (or another of its blocks) writes
-// into such a line must be read past the L1 (__ldcg). So only kernels that follow one of this library's
+// into such a line is read past the L1 (__ldcg). So only kernels that follow one of this library's
 // own in the same call are chained, and the dangling sum is read so: the fix-up reads the one of the last
 // sweep and writes the one of this sweep in the same line. What a sweep's gather otherwise reads through
 // the L1 (gathered vector, previous ranks, a batch's uniform terms) no kernel loads between the gather's

@@ -55,9 +55,10 @@ __device__ __forceinline__ int pad(int i) { return i + (i >> 5); }
 
 enum { kModeSpmv = 0, kModePagerank = 1, kModeWeighted = 2 };
 
-// Loads of the streams every tile reads once (columns, values, items, epilogue inputs):
-// read-only for the launch (nc) and kept out of L1 (L1::no_allocate), so the L1 lines are left to
-// the scattered gathers of x, which are what a sweep waits on. SpMV also marks them first for
+// Loads of the streams every tile reads once (columns, values, items, out-degrees and the like):
+// written before the first kernel of the call's chain starts, so read-only for the launch (nc), and kept
+// out of L1 (L1::no_allocate), so the L1 lines are left to the scattered gathers of x, which are what a
+// sweep waits on. SpMV also marks them first for
 // eviction from L2, which keeps more of x there. Measured per launch (R-MAT 22; R-MAT 24 for
 // PageRank): PageRank 0.1623 -> 0.1603 ms and 0.749 -> 0.720 ms with L1::no_allocate, 0.171 and
 // 0.764 ms with the L2 hint too; SpMV 0.2146 -> 0.2137 ms, and 0.2063 ms with the L2 hint.
@@ -86,7 +87,17 @@ __device__ __forceinline__ float ld_stream(const float* p) {
     return v;
 }
 
-// 16 bytes of a stream, zero unless `in`; never kept in L1.
+// What the kernels before this one in a chain write (the gathered vector, the previous ranks, a batch's
+// uniform terms) may still change after this kernel has started, ahead of chain_wait: it is read by
+// ordinary loads, which the wait orders, never by the read-only path. ld_live stays out of L1.
+__device__ __forceinline__ float ld_live(const float* p) {
+    float v;
+    asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// 16 bytes of a stream; every word -1 unless `in` (kItemNone; a NaN as an arc value, which no tile past
+// the last is walked for). Never kept in L1.
 __device__ __forceinline__ int4 ld_stream4(const int4* p, bool in) {
     int4 v = make_int4(kItemNone, kItemNone, kItemNone, kItemNone);
     if (in) asm("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -101,7 +112,7 @@ __device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, flo
                                             double& dang, bool& moved) {
     const float nv = fmaf(L.damping, sum, base);
     if (L.rank_out) L.rank_out[v] = nv;
-    if (L.rank_prev && fabsf(nv - __ldg(L.rank_prev + v)) > L.epsilon) moved = true;
+    if (L.rank_prev && fabsf(nv - __ldca(L.rank_prev + v)) > L.epsilon) moved = true;
     // Only vertices with out-arcs are ever gathered (they are the columns), so the contribution
     // slot of a dangling vertex is free: a batch parks its rank there for the per-graph reduction.
     // The division runs for every row (by 1 for a dangling one) so a warp's rows do not diverge
@@ -116,7 +127,7 @@ __device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, flo
 }
 
 __device__ __forceinline__ float batch_base(const RowGatherLaunch& L, int v) {
-    return __ldg(L.gbase + __ldg(L.vgraph + v));
+    return __ldca(L.gbase + __ldg(L.vgraph + v));
 }
 
 // Epilogue of one row of a weighted PageRank sweep (dpg_prgrad.cu): forward (no seed) the new rank and
@@ -141,7 +152,7 @@ __device__ __forceinline__ void weighted_epilogue(const RowGatherLaunch& L, int 
 __device__ __forceinline__ void weighted_epilogue(const RowGatherLaunch& L, int v, float sum, float base,
                                                   double& dang, bool& moved) {
     weighted_epilogue(L, v, sum, base, __ldg(L.W + v), L.perm ? __ldg(L.perm + v) : v,
-                      L.seed ? __ldg(L.seed + v) : 0.0f, L.rank_prev ? __ldg(L.rank_prev + v) : 0.0f, dang, moved);
+                      L.seed ? __ldg(L.seed + v) : 0.0f, L.rank_prev ? __ldca(L.rank_prev + v) : 0.0f, dang, moved);
 }
 
 __device__ __forceinline__ float pr_base(const RowGatherLaunch& L) {
@@ -226,11 +237,11 @@ __device__ __forceinline__ double block_sum_f64(double v) {
 
 // The hot cache: the first `hot` (most gathered) entries of x, loads issued in batches of 8 (one round
 // trip each instead of one per entry).
-__device__ __forceinline__ void fill_hot(const float* __restrict__ x, int hot, float* s_hot) {
+__device__ __forceinline__ void fill_hot(const float* x, int hot, float* s_hot) {
     for (int i0 = threadIdx.x; i0 < hot; i0 += kBlock * 8) {
         float h[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) h[q] = i0 + kBlock * q < hot ? __ldg(x + i0 + kBlock * q) : 0.0f;
+        for (int q = 0; q < 8; ++q) h[q] = i0 + kBlock * q < hot ? __ldca(x + i0 + kBlock * q) : 0.0f;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
             if (i0 + kBlock * q < hot) s_hot[i0 + kBlock * q] = h[q];
@@ -298,7 +309,7 @@ __global__ void __launch_bounds__(kBlock) spmv_gather_kernel(RowGatherLaunch L) 
             const bool hot = c < L.hot;
             const float hv = s_hot[hot ? c : 0];
             float gv = 0.0f;
-            if (!hot) gv = __ldg(L.x + c);
+            if (!hot) gv = __ldca(L.x + c);
             pv[i] = i * 32 + lane < nnz ? (hot ? hv : gv) * av[i] : 0.0f;
         }
         if (nrows < 0) {
@@ -473,9 +484,9 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             const int c = item[i];
             if (BATCH) {
                 const int d = c < 0 ? -1 : c - hot0;
-                pv[i] = c < 0 || static_cast<unsigned>(d) < static_cast<unsigned>(hot) ? s_hot[d] : __ldg(L.x + c);
+                pv[i] = c < 0 || static_cast<unsigned>(d) < static_cast<unsigned>(hot) ? s_hot[d] : __ldca(L.x + c);
             } else {
-                pv[i] = c < hot ? s_hot[max(c, -1)] : __ldg(L.x + c);
+                pv[i] = c < hot ? s_hot[max(c, -1)] : __ldca(L.x + c);
             }
         }
         if (MODE == kModeWeighted) {
@@ -499,13 +510,13 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
         }
         float ebase[NE];
 #pragma unroll
-        for (int q = 0; q < NE; ++q) ebase[q] = BATCH ? __ldg(L.gbase + egraph[q]) : base;
+        for (int q = 0; q < NE; ++q) ebase[q] = BATCH ? __ldca(L.gbase + egraph[q]) : base;
         float eW = 0.0f, eseed = 0.0f, eprev = 0.0f;
         if (MODE == kModeWeighted && lane < nrows) {
             eW = ld_stream<MODE>(L.W + row + lane);
             if (L.perm) epos[0] = ld_stream<MODE>(L.perm + row + lane);
             if (L.seed) eseed = ld_stream<MODE>(L.seed + row + lane);
-            if (CONV) eprev = ld_stream<MODE>(L.rank_prev + row + lane);
+            if (CONV) eprev = ld_live(L.rank_prev + row + lane);
         }
         // The lane's items in order: a nonzero is added to the open row, a row end closes it.
         int r = r0;
