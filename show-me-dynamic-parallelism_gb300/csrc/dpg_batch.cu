@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cstring>
 #include <functional>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -134,9 +135,14 @@ struct dpg_batch {
     float* gbase = nullptr;
     float* ginit = nullptr;
     unsigned* ticket = nullptr;
-    int2* win = nullptr;  // hot-cache windows of the PageRank sweeps and the CTAs' first tiles, for win_hot
-    int2* cta_first = nullptr;
-    int32_t nwin = 0, win_hot = -1;
+    // Hot-cache windows of the PageRank sweeps and the CTAs' first tiles, per cache size they were cut for. Kept
+    // for the batch's life (16 bytes per graph and CTA at most): captured sweeps hold their addresses.
+    struct Windows {
+        int2* win = nullptr;
+        int2* cta_first = nullptr;
+        int32_t nwin = 0;
+    };
+    std::map<int32_t, Windows> windows;
     // Sources as label indices v * nsrc + k, k = source number within its graph.
     std::vector<int32_t> h_src;
     int32_t nsrc = 0;
@@ -185,8 +191,12 @@ void batch_free(dpg_batch* b) {
     for (void* p : {static_cast<void*>(b->vstart), static_cast<void*>(b->outdeg), static_cast<void*>(b->vgraph),
                     static_cast<void*>(b->dang), static_cast<void*>(b->dslot), static_cast<void*>(b->pieces),
                     static_cast<void*>(b->gpiece), static_cast<void*>(b->gpart), static_cast<void*>(b->gbase),
-                    static_cast<void*>(b->ginit), static_cast<void*>(b->ticket), static_cast<void*>(b->win), static_cast<void*>(b->cta_first), static_cast<void*>(b->d_src)})
+                    static_cast<void*>(b->ginit), static_cast<void*>(b->ticket), static_cast<void*>(b->d_src)})
         cudaFree(p);
+    for (auto& w : b->windows) {
+        cudaFree(w.second.win);
+        cudaFree(w.second.cta_first);
+    }
 }
 
 template <class T>
@@ -231,20 +241,13 @@ int32_t pr_hot(const dpg_batch* b) {
 constexpr int kWindowTiles = 8;
 dpg_status ensure_windows(dpg_batch* b) {
     const int32_t hot = pr_hot(b);
-    if (b->win_hot == hot) return DPG_OK;
+    if (b->windows.count(hot)) return DPG_OK;
     dpg_ctx* c = b->ctx;
     int gb, fb, bt;
     rowgather_grid(c->sm_count, &gb, &fb, &bt);
-    cudaFree(b->win);
-    cudaFree(b->cta_first);
-    b->win = b->cta_first = nullptr;
-    b->nwin = 0;
-    b->win_hot = -1;
     const int64_t ntiles = b->in->plan.ntiles;
-    if (ntiles < static_cast<int64_t>(kWindowTiles) * gb * (bt / 32)) {
-        b->win_hot = hot;
-        return DPG_OK;
-    }
+    if (ntiles < static_cast<int64_t>(kWindowTiles) * gb * (bt / 32)) return DPG_OK;
+    dpg_batch::Windows W;
     std::vector<int32_t> rows;
     for (int32_t g = 0; g < b->n; ++g) {
         const int32_t v0 = b->h_vstart[g], v1 = b->h_vstart[g + 1];
@@ -253,12 +256,12 @@ dpg_status ensure_windows(dpg_batch* b) {
     const size_t n = rows.size();
     std::vector<int2> win(n), first(static_cast<size_t>(gb) + 1);
     int32_t* d_rows = nullptr;
-    cudaError_t e = cudaMalloc(&b->win, sizeof(int2) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&b->cta_first, sizeof(int2) * first.size());
+    cudaError_t e = cudaMalloc(&W.win, sizeof(int2) * n);
+    if (e == cudaSuccess) e = cudaMalloc(&W.cta_first, sizeof(int2) * first.size());
     if (e == cudaSuccess) e = cudaMalloc(&d_rows, sizeof(int32_t) * n);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_rows, rows.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = launch_window_tiles(b->in->plan, d_rows, static_cast<int>(n), b->win, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(win.data(), b->win, sizeof(int2) * n, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = launch_window_tiles(b->in->plan, d_rows, static_cast<int>(n), W.win, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(win.data(), W.win, sizeof(int2) * n, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e == cudaSuccess) {
         size_t k = 0;
@@ -268,19 +271,23 @@ dpg_status ensure_windows(dpg_batch* b) {
             first[i] = make_int2(t, static_cast<int>(k));
         }
         first[gb] = make_int2(static_cast<int>(ntiles), 0);
-        e = cudaMemcpyAsync(b->cta_first, first.data(), sizeof(int2) * first.size(), cudaMemcpyHostToDevice, c->stream);
+        e = cudaMemcpyAsync(W.cta_first, first.data(), sizeof(int2) * first.size(), cudaMemcpyHostToDevice, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     }
     cudaFree(d_rows);
     if (e != cudaSuccess) {
-        cudaFree(b->win);
-        cudaFree(b->cta_first);
-        b->win = b->cta_first = nullptr;
+        cudaFree(W.win);
+        cudaFree(W.cta_first);
         return set_error(DPG_ERR_CUDA, std::string("hot-cache windows: ") + cudaGetErrorString(e));
     }
-    b->nwin = static_cast<int32_t>(n);
-    b->win_hot = hot;
+    W.nwin = static_cast<int32_t>(n);
+    b->windows[hot] = W;
     return DPG_OK;
+}
+
+dpg_batch::Windows windows_of(const dpg_batch* b, int32_t hot) {
+    const auto it = b->windows.find(hot);
+    return it == b->windows.end() ? dpg_batch::Windows() : it->second;
 }
 
 // Everything the PageRank solve needs that allocates, done before any capture.
@@ -324,9 +331,10 @@ dpg_status run_batch_pagerank(dpg_batch* b, const PrBuffers& pb, const dpg_pr_op
     L.items = g->items;
     L.perm = g->relabel ? g->perm : nullptr;
     L.hot = pr_hot(b);
-    L.win = b->win;
-    L.nwin = b->nwin;
-    L.cta_first = b->cta_first;
+    const dpg_batch::Windows W = windows_of(b, L.hot);
+    L.win = W.win;
+    L.nwin = W.nwin;
+    L.cta_first = W.cta_first;
     L.partial = pb.partial;
     L.V = g->V;
     L.outdeg = b->outdeg;
@@ -774,7 +782,10 @@ dpg_status dpg_batch_run(dpg_ctx* c, dpg_batch* b, int32_t nsrc, const int32_t* 
     put(&o, sizeof(o));
     put(&d_rank, sizeof(d_rank));
     put(&b->tune, sizeof(b->tune));
-    put(&b->win, sizeof(b->win));
+    const dpg_batch::Windows W = windows_of(b, pr_hot(b));
+    put(&W.win, sizeof(W.win));
+    put(&W.cta_first, sizeof(W.cta_first));
+    put(&W.nwin, sizeof(W.nwin));
     put(&b->src_version, sizeof(b->src_version));
     if (!b->exec || key != b->key) {
         if (b->exec) cudaGraphExecDestroy(b->exec);
