@@ -897,9 +897,8 @@ dpg_status dpg_batch_autotune(dpg_ctx* c, dpg_batch* b, int32_t nsrc, const int3
         }
     // Gather hot-cache size: three sweeps per candidate.
     PrBuffers pb;
-    st = pr_buffers(b, &pb);
     float* rank = nullptr;
-    if (st == DPG_OK && cudaMalloc(&rank, sizeof(float) * (b->V > 0 ? b->V : 1)) != cudaSuccess)
+    if (cudaMalloc(&rank, sizeof(float) * (b->V > 0 ? b->V : 1)) != cudaSuccess)
         st = set_error(DPG_ERR_CAPACITY, "autotune rank buffer");
     dpg_pr_opts o;
     pr_defaults(nullptr, &o);
@@ -910,8 +909,9 @@ dpg_status dpg_batch_autotune(dpg_ctx* c, dpg_batch* b, int32_t nsrc, const int3
         if (st != DPG_OK) break;
         if (hot > cap) continue;
         b->tune.pr_hot = hot;
-        run_batch_pagerank(b, pb, o, rank, nullptr);
-        st = check_device(c);
+        st = pr_buffers(b, &pb);  // with the windows of this size
+        if (st == DPG_OK) st = run_batch_pagerank(b, pb, o, rank, nullptr);
+        if (st == DPG_OK) st = check_device(c);
         const float t = st == DPG_OK ? time_ms(c, [&] { return run_batch_pagerank(b, pb, o, rank, nullptr); }, 2, &st)
                                      : 1e30f;
         if (st == DPG_OK && t < best_pr) {
