@@ -191,8 +191,10 @@ void graph_free_device(dpg_graph* g) {
     dev_free(g->ctx, g->perm);
     dev_free(g->ctx, g->inv);
     dev_free(g->ctx, g->pcol);
-    dev_free(g->ctx, g->items);
-    g->items = nullptr;
+    for (int32_t*& it : g->items) {
+        dev_free(g->ctx, it);
+        it = nullptr;
+    }
     dev_free(g->ctx, g->t_off);
     dev_free(g->ctx, g->t_col);
     g->perm = g->inv = g->pcol = g->t_off = g->t_col = nullptr;
@@ -391,25 +393,28 @@ dpg_status ensure_pcol(dpg_graph* g) {
     return DPG_OK;
 }
 
-// The tiles' merge items (PageRank sweeps), with the graph's current choice of renaming.
-dpg_status ensure_items(dpg_graph* g) {
-    DPG_TRY(ensure_plan(g));
-    if (g->relabel) DPG_TRY(ensure_relabel(g));
-    if (g->V == 0 || (g->items && g->items_relabel == g->relabel)) return DPG_OK;
-    dpg_ctx* c = g->ctx;
-    cudaError_t e = cudaSuccess;
-    if (!g->items)
-        e = dev_alloc(c, &g->items, sizeof(int32_t) * kRowTileItems * (static_cast<size_t>(g->plan.ntiles) + 1));
-    // A one-shot graph has its columns renamed already (graph_create_pull).
-    const int32_t* col = g->relabel && g->pcol ? g->pcol : g->col;
-    const int32_t* perm = g->relabel && !g->pcol ? g->perm : nullptr;
-    if (e == cudaSuccess) e = launch_tile_items(g->plan, col, perm, g->items, c->stream, c->sm_count);
-    if (e != cudaSuccess) {
-        dev_free(c, g->items);
-        g->items = nullptr;
-        return set_error(DPG_ERR_CUDA, std::string("merge items: ") + cudaGetErrorString(e));
+// The tiles' merge items (PageRank sweeps) for the graph's current choice of renaming. Each choice has an
+// array of its own: a captured sweep reads the one that it was captured with.
+dpg_status ensure_items(dpg_graph* g, const int32_t** items) {
+    int32_t*& at = g->items[g->relabel ? 1 : 0];
+    if (!at && g->V > 0) {
+        dpg_ctx* c = g->ctx;
+        DPG_TRY(ensure_plan(g));
+        if (g->relabel) DPG_TRY(ensure_relabel(g));
+        // A one-shot graph has its columns renamed already (graph_create_pull).
+        const int32_t* col = g->relabel && g->pcol ? g->pcol : g->col;
+        const int32_t* perm = g->relabel && !g->pcol ? g->perm : nullptr;
+        int32_t* p = nullptr;
+        cudaError_t e =
+            dev_alloc(c, &p, sizeof(int32_t) * kRowTileItems * (static_cast<size_t>(g->plan.ntiles) + 1));
+        if (e == cudaSuccess) e = launch_tile_items(g->plan, col, perm, p, c->stream, c->sm_count);
+        if (e != cudaSuccess) {
+            dev_free(c, p);
+            return set_error(DPG_ERR_CUDA, std::string("merge items: ") + cudaGetErrorString(e));
+        }
+        at = p;
     }
-    g->items_relabel = g->relabel;
+    if (items) *items = at;
     return DPG_OK;
 }
 
@@ -750,7 +755,8 @@ dpg_status run_pagerank(dpg_ctx* c, dpg_graph* g, const int32_t* d_outdeg, const
     dpg_pr_opts o;
     DPG_TRY(pr_defaults(in_opts, &o));
     if (g->V == 0) return DPG_OK;
-    DPG_TRY(ensure_items(g));
+    const int32_t* items = nullptr;
+    DPG_TRY(ensure_items(g, &items));
     int gb, fb, bt;
     rowgather_grid(c->sm_count, &gb, &fb, &bt);
     dpg_status st = DPG_OK;
@@ -772,7 +778,7 @@ dpg_status run_pagerank(dpg_ctx* c, dpg_graph* g, const int32_t* d_outdeg, const
     RowGatherLaunch L;
     memset(&L, 0, sizeof(L));
     L.plan = g->plan;
-    L.items = g->items;
+    L.items = items;
     L.perm = g->relabel ? g->perm : nullptr;
     L.hot = hot_entries(c, g, true);
     L.partial = partial;
@@ -1098,7 +1104,7 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
     DPG_TRY(ensure_spmm_transpose(g, true));
     DPG_TRY(ensure_spmm_plan(g));
     dpg_graph* tg = g->tgraph;
-    for (dpg_graph* p : {g, tg}) DPG_TRY(ensure_items(p));
+    for (dpg_graph* p : {g, tg}) DPG_TRY(ensure_items(p, nullptr));
     const size_t nv = static_cast<size_t>(g->V);
     const int nb = pr_vec_blocks(c->sm_count);
     int gb, fb, bt;
@@ -1165,7 +1171,7 @@ dpg_status run_pagerank_grad(dpg_ctx* c, dpg_graph* g, const float* d_w, const f
             else DPG_CUDA_TRY(cudaMemcpyAsync(xb, start, nv * 4, cudaMemcpyDeviceToDevice, c->stream));
         }
         L.plan = sg->plan;
-        L.items = sg->items;
+        DPG_TRY(ensure_items(sg, &L.items));
         L.witems = witems;
         L.perm = sg->relabel ? sg->perm : nullptr;
         L.hot = hot_entries(c, sg, true);

@@ -159,8 +159,8 @@ struct dpg_graph {
     int32_t* perm = nullptr;  // old column id -> new
     int32_t* inv = nullptr;   // new -> old
     int32_t* pcol = nullptr;  // col[e] renamed (SpMV), built on first use
-    int32_t* items = nullptr;  // the tiles' merge items (PageRank sweeps), built on first use; renamed:
-    bool items_relabel = false;
+    int32_t* items[2] = {nullptr, nullptr};  // the tiles' merge items (PageRank sweeps) without and with the
+                                             // renaming, each built on first use
     std::vector<int32_t> relabel_segments;  // optional vertex starts: rename within each segment
     // Transposed CSR (in-arcs), built on first use by colouring.
     int32_t* t_off = nullptr;
@@ -220,7 +220,8 @@ cudaError_t plan_build_launch(const PlanBuild& pb, const int32_t* d_off, int32_t
 dpg_status plan_finish(dpg_graph* g, PlanBuild* pb, const PlanInfo& info);
 void plan_build_free(dpg_ctx* c, PlanBuild* pb);
 dpg_status ensure_relabel(dpg_graph* g);
-dpg_status ensure_items(dpg_graph* g);
+// The merge items for the graph's choice of renaming (items: nullable).
+dpg_status ensure_items(dpg_graph* g, const int32_t** items);
 int32_t hot_entries(const dpg_ctx* c, const dpg_graph* g, bool sweeps);
 dpg_status pr_defaults(const dpg_pr_opts* in, dpg_pr_opts* o);
 void batch_orphan(dpg_batch* b);

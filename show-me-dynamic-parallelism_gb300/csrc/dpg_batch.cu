@@ -210,7 +210,7 @@ dpg_status upload(dpg_ctx* c, T** dst, const T* src, size_t count) {
 dpg_status ensure_dslot(dpg_batch* b) {
     if (b->dslot_ready) return DPG_OK;
     dpg_ctx* c = b->ctx;
-    DPG_TRY(ensure_items(b->in));
+    DPG_TRY(ensure_items(b->in, nullptr));
     DPG_CUDA_TRY(cudaMalloc(&b->dslot, sizeof(int32_t) * (b->ndang > 0 ? b->ndang : 1)));
     if (b->ndang > 0) {
         if (b->in->relabel) {
@@ -328,7 +328,7 @@ dpg_status run_batch_pagerank(dpg_batch* b, const PrBuffers& pb, const dpg_pr_op
     RowGatherLaunch L;
     memset(&L, 0, sizeof(L));
     L.plan = g->plan;
-    L.items = g->items;
+    L.items = g->items[g->relabel ? 1 : 0];
     L.perm = g->relabel ? g->perm : nullptr;
     L.hot = pr_hot(b);
     const dpg_batch::Windows W = windows_of(b, L.hot);
