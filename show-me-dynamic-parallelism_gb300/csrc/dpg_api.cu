@@ -66,6 +66,46 @@ dpg_status host_words(dpg_ctx* c, unsigned** out) {
     return DPG_OK;
 }
 
+bool capturing(dpg_ctx* c) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) {
+        cudaGetLastError();  // the legacy stream while another one is captured: not capturing itself
+        return false;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// What a graph keeps is built on first use and then read by calls on any stream and by captured ones. So a
+// build is complete when it returns, and while the context's stream is being captured it runs on the aux
+// stream, for the scope of a BuildScope (its allocations and kernels would else belong to the capture).
+struct BuildScope {
+    dpg_ctx* c;
+    cudaStream_t user;
+    cudaError_t e = cudaSuccess;
+    bool off_capture;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // the thread's mode while it is exchanged
+    explicit BuildScope(dpg_ctx* ctx) : c(ctx), user(ctx->stream), off_capture(capturing(ctx)) {
+        if (!off_capture) return;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (!c->aux_stream && (e = cudaStreamCreateWithFlags(&c->aux_stream, cudaStreamNonBlocking)) != cudaSuccess)
+            c->aux_stream = nullptr;
+        else
+            c->stream = c->aux_stream;
+    }
+    ~BuildScope() {
+        c->stream = user;
+        if (off_capture) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    BuildScope(const BuildScope&) = delete;
+    BuildScope& operator=(const BuildScope&) = delete;
+};
+
+// Builds that use the arena's shared buffers cannot leave the stream: refused before they touch anything.
+dpg_status refuse_in_capture(dpg_ctx* c, const char* what) {
+    if (!capturing(c)) return DPG_OK;
+    return set_error(DPG_ERR_CUDA, std::string(what) + " is built by the first call, which cannot be captured");
+}
+
 void* arena(dpg_ctx* c, Slot s, size_t bytes, dpg_status* status) {
     Buf& b = c->bufs[s];
     if (bytes == 0) bytes = 16;
@@ -302,6 +342,7 @@ dpg_status ensure_plan(dpg_graph* g) {
     }
     const dpg_status fs = plan_finish(g, &pb, h);
     if (fs != DPG_OK) plan_build_free(c, &pb);
+    else DPG_CUDA_TRY(cudaStreamSynchronize(c->stream));
     return fs;
 }
 
@@ -380,11 +421,15 @@ dpg_status ensure_relabel(dpg_graph* g) {
 
 // The renamed columns in CSR order (SpMV).
 dpg_status ensure_pcol(dpg_graph* g) {
-    DPG_TRY(ensure_relabel(g));
-    if (g->pcol || g->V == 0) return DPG_OK;
+    if (g->V == 0 || (g->relabel_ready && g->pcol)) return DPG_OK;
     dpg_ctx* c = g->ctx;
+    BuildScope build(c);
+    DPG_CUDA_TRY(build.e);
+    DPG_TRY(ensure_relabel(g));
+    if (g->pcol) return DPG_OK;
     cudaError_t e = dev_alloc(c, &g->pcol, static_cast<size_t>(g->E > 0 ? g->E : 1) * 4);
     if (e == cudaSuccess) e = launch_relabel_columns(g->col, g->perm, g->E, g->pcol, c->stream, c->sm_count);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         dev_free(c, g->pcol);
         g->pcol = nullptr;
@@ -399,6 +444,8 @@ dpg_status ensure_items(dpg_graph* g, const int32_t** items) {
     int32_t*& at = g->items[g->relabel ? 1 : 0];
     if (!at && g->V > 0) {
         dpg_ctx* c = g->ctx;
+        BuildScope build(c);
+        DPG_CUDA_TRY(build.e);
         DPG_TRY(ensure_plan(g));
         if (g->relabel) DPG_TRY(ensure_relabel(g));
         // A one-shot graph has its columns renamed already (graph_create_pull).
@@ -408,6 +455,7 @@ dpg_status ensure_items(dpg_graph* g, const int32_t** items) {
         cudaError_t e =
             dev_alloc(c, &p, sizeof(int32_t) * kRowTileItems * (static_cast<size_t>(g->plan.ntiles) + 1));
         if (e == cudaSuccess) e = launch_tile_items(g->plan, col, perm, p, c->stream, c->sm_count);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) {
             dev_free(c, p);
             return set_error(DPG_ERR_CUDA, std::string("merge items: ") + cudaGetErrorString(e));
@@ -446,6 +494,7 @@ dpg_status build_spmm_plan(dpg_ctx* c, const int32_t* off, int32_t V, int64_t E,
 
 dpg_status ensure_spmm_plan(dpg_graph* g) {
     if (g->spmm_ready) return DPG_OK;
+    DPG_TRY(refuse_in_capture(g->ctx, "the batched-RHS plan"));
     DPG_TRY(build_spmm_plan(g->ctx, g->off, g->V, g->E, &g->spmm_plan));
     g->spmm_ready = true;
     return DPG_OK;
@@ -457,6 +506,7 @@ dpg_status ensure_spmm_plan(dpg_graph* g) {
 dpg_status ensure_spmm_transpose(dpg_graph* g, bool need_graph = false) {
     dpg_ctx* c = g->ctx;
     if (!g->spmm_t_ready) {
+        DPG_TRY(refuse_in_capture(c, "the transposed CSR"));
         const size_t nv = static_cast<size_t>(g->V), ne = static_cast<size_t>(g->E > 0 ? g->E : 1);
         cudaError_t e = cudaSuccess;
         if (!g->tt_off) e = dev_alloc(c, &g->tt_off, (nv + 1) * 4);
@@ -492,11 +542,12 @@ constexpr int64_t kSlotArcs = 3 << 22;
 bool backward_slots(dpg_graph* g, float** vals_t, float** dA_t) {
     if (g->E < kSlotArcs || g->E > kPermMaxArcs) return false;
     dpg_ctx* c = g->ctx;
+    if (!g->tt_perm.mid && (g->tt_perm_tried || capturing(c))) return false;
     const size_t ne = static_cast<size_t>(g->E);
     dpg_status st = DPG_OK;
     *vals_t = static_cast<float*>(arena(c, S_VALS_T, ne * 4, &st));
     if (st == DPG_OK) *dA_t = static_cast<float*>(arena(c, S_DA_T, ne * 4, &st));
-    if (st == DPG_OK && !g->tt_perm.mid && !g->tt_perm_tried) {
+    if (st == DPG_OK && !g->tt_perm.mid) {
         g->tt_perm_tried = true;
         ArcPerm& P = g->tt_perm;
         void* scratch = arena(c, S_TRANSPOSE, perm_scratch_bytes(g->E), &st);
@@ -504,6 +555,7 @@ bool backward_slots(dpg_graph* g, float** vals_t, float** dA_t) {
         if (e == cudaSuccess) e = dev_alloc(c, &P.arc_in, 2 * ne);
         if (e == cudaSuccess) e = dev_alloc(c, &P.slot_in, 2 * ne);
         if (e == cudaSuccess) e = launch_build_perm(g->tt_arc, g->E, scratch, P, c->stream, c->sm_count);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) {
             dev_free(c, P.mid);
             dev_free(c, P.arc_in);

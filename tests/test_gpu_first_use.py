@@ -115,3 +115,97 @@ def test_a_capture_survives_the_other_choice_of_renaming(prob, what, relabel):
             g.set_relabel(other)
             prob.check(what, g)
             _replay(prob, what, graph, out)
+
+
+@pytest.mark.parametrize("what, warm", [("pagerank", "spmv"), ("spmv", "pagerank"), ("pagerank", "pagerank")])
+@pytest.mark.parametrize("mode", ["global", "relaxed"])
+def test_first_use_inside_a_capture(prob, what, warm, mode):
+    """The graph was used by another call, or with the other choice of renaming, and the scratch buffers exist."""
+    import torch
+
+    stream = torch.cuda.Stream()
+    g = prob.graph()
+    with _on(prob.ctx, stream):
+        prob.check(warm, g)
+        if what == warm:
+            g.set_relabel(False)
+        out = prob.out()
+        graph = _capture(prob, what, g, out, stream, mode)
+        prob.check(what, g)  # ahead of the first replay
+        _replay(prob, what, graph, out)
+        g.set_relabel(True)
+        prob.check(what, g)
+        _replay(prob, what, graph, out)
+        del graph
+        prob.check(what, g)
+
+
+@pytest.mark.parametrize("first, then", [("pagerank", "pagerank"), ("pagerank", "spmv"), ("spmv", "spmv")])
+def test_next_call_on_another_stream(prob, first, then):
+    """Ordered behind the first by an event; the first one's stream is busy when it comes."""
+    import torch
+
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    g = prob.graph()
+    o1, o2 = prob.out(), prob.out()
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(20_000_000)
+    prob.ctx.set_stream(a.cuda_stream)
+    prob.call(first, g, o1)
+    ev = torch.cuda.Event()
+    ev.record(a)
+    b.wait_event(ev)
+    with _on(prob.ctx, b):
+        prob.call(then, g, o2)
+    assert torch.equal(o1, prob.want[first]) and torch.equal(o2, prob.want[then])
+
+
+def test_backward_captured_before_and_after_its_permutation(ctx):
+    """Past 12.6 M arcs the backward permutes values through blocks; a capture that comes first works in arc order."""
+    import torch
+
+    V, E, n = 400_009, 12_700_001, 1
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    deg = torch.bincount(torch.randint(0, V, (E,), device="cuda", generator=gen), minlength=V)
+    off = torch.zeros(V + 1, dtype=torch.int32, device="cuda")
+    off[1:] = torch.cumsum(deg, 0)
+    col = torch.randint(0, V, (E,), device="cuda", generator=gen, dtype=torch.int32)
+    vals, X, G = (torch.randn(k, device="cuda", generator=gen) for k in (E, V, V))
+    dX, dA = torch.empty(V, device="cuda"), torch.empty(E, device="cuda")
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with _on(ctx, stream):
+        def bwd(g):
+            dpg.spmv_bwd_dev(ctx, g, vals.data_ptr(), n, X.data_ptr(), G.data_ptr(), dX.data_ptr(), dA.data_ptr())
+
+        def graph_of():
+            return dpg.Graph.from_device(ctx, V, E, off.data_ptr(), col.data_ptr(), None)
+
+        g = graph_of()
+        bwd(g)
+        ctx.synchronize()
+        want = dX.clone(), dA.clone()
+        row = torch.repeat_interleave(torch.arange(V, device="cuda"), deg)
+        assert torch.equal(want[1], G[row] * X[col.long()])
+        late = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(late, stream=stream):
+            bwd(g)
+        for _ in range(2):
+            dX.fill_(7)
+            dA.fill_(7)
+            torch.cuda.synchronize()
+            late.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(dX, want[0]) and torch.equal(dA, want[1])
+            bwd(g)
+            ctx.synchronize()
+        h = graph_of()
+        early = torch.cuda.CUDAGraph()
+        with pytest.raises(dpg.DpgError):  # the transposed CSR is not there yet
+            with torch.cuda.graph(early, stream=stream):
+                bwd(h)
+        torch.cuda.synchronize()
+        bwd(h)
+        ctx.synchronize()
+        assert torch.equal(dX, want[0]) and torch.equal(dA, want[1])
