@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kBlock) spmm_rows_kernel(SpmmPlanDev P,
 #pragma unroll
         for (int q = 0; q < NV; ++q) acc[q] = 0.0f;
         int e = I.y;
-        for (; e + 4 <= I.z; e += 4) {
+        for (; I.z - e >= 4; e += 4) {
             int c[4];
             float a[4];
 #pragma unroll
@@ -133,13 +133,13 @@ __global__ void __launch_bounds__(kBlock) arc_dot1_kernel(SpmmPlanDev P, const i
     for (int64_t k = w; k < P.nitems; k += nw) {
         const int4 I = __ldg(P.items + k);
         const float g = __ldg(G + I.x);
-        for (int e = I.y + lane; e < I.z; e += 32) dA[e] = g * __ldg(X + __ldg(col + e));
+        for (unsigned e = I.y + lane, end = I.z; e < end; e += 32) dA[e] = g * __ldg(X + __ldg(col + e));
     }
     for (int64_t v = w * 4 + (lane >> 3); v < P.V; v += nw * 4) {
-        const int b = __ldg(P.off + v), end = __ldg(P.off + v + 1);
+        const unsigned b = __ldg(P.off + v), end = __ldg(P.off + v + 1);
         if (end - b > kGroupRow) continue;  // its items are listed
         const float g = __ldg(G + v);
-        for (int e = b + (lane & 7); e < end; e += 8) dA[e] = g * __ldg(X + __ldg(col + e));
+        for (unsigned e = b + (lane & 7); e < end; e += 8) dA[e] = g * __ldg(X + __ldg(col + e));
     }
 }
 
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kBlock) arc_dot_kernel(SpmmPlanDev P,
         float g[NV];
         load_row<NV>(G, I.x, nrhs, lane, g);
         int e = I.y;
-        for (; e + 4 <= I.z; e += 4) {
+        for (; I.z - e >= 4; e += 4) {
             float xv[4][NV];
 #pragma unroll
             for (int u = 0; u < 4; ++u) load_row<NV>(X, __ldg(col + e + u), nrhs, lane, xv[u]);
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(kBlock) spmm_plan_kernel(const int32_t* __rest
         const int b = v < V ? __ldg(off + v) : 0;
         const int e = v < V ? __ldg(off + v + 1) : 0;
         const int d = e - b;
-        const int n = d > kGroupRow ? (d + kSpmmSegment - 1) / kSpmmSegment : 0;
+        const int n = d > kGroupRow ? segments_of(d, kSpmmSegment) : 0;
         int pos = 0, seg = -1;
         if (n > 0) pos = atomicAdd(counts, n);
         if (n > 1) {
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(kBlock) spmm_plan_kernel(const int32_t* __rest
             const int rs = __shfl_sync(kFullMask, seg, src);
             for (int k = lane; k < rn; k += 32) {
                 const int sb = rb + k * kSpmmSegment;
-                items[rp + k] = make_int4(static_cast<int>(v0) + src, sb, min(re, sb + kSpmmSegment), rs < 0 ? -1 : rs + k);
+                items[rp + k] = make_int4(static_cast<int>(v0) + src, sb, segment_end(sb, re, kSpmmSegment), rs < 0 ? -1 : rs + k);
             }
         }
     }

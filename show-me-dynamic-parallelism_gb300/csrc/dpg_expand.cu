@@ -546,7 +546,7 @@ __device__ __forceinline__ void push_batch(const ExpandParams& P, const PushCtx&
         // Chunked vertices: one reservation for all U slots of all lanes, then every descriptor.
         int nchl = 0;
 #pragma unroll
-        for (int u = 0; u < U; ++u) nchl += chunked[u] ? (e[u] - s[u] + CH - 1) / CH : 0;
+        for (int u = 0; u < U; ++u) nchl += chunked[u] ? segments_of(e[u] - s[u], CH) : 0;
         if (!__any_sync(kFullMask, nchl > 0)) return;
         const int incl = warp_inclusive_scan(nchl);
         const int total = __shfl_sync(kFullMask, incl, 31);
@@ -560,11 +560,11 @@ __device__ __forceinline__ void push_batch(const ExpandParams& P, const PushCtx&
         unsigned my_first = base + static_cast<unsigned>(incl - nchl);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int hn = chunked[u] ? (e[u] - s[u] + CH - 1) / CH : 0;
+            const int hn = chunked[u] ? segments_of(e[u] - s[u], CH) : 0;
             if (hn <= kLaneChunks) {
                 for (int c = 0; c < hn; ++c) {
                     const int k0 = s[u] + c * CH;
-                    __stcg(Q.chunks + my_first + c, make_int4(v[u], k0, min(e[u], k0 + CH), c == 0 ? 1 : 0));
+                    __stcg(Q.chunks + my_first + c, make_int4(v[u], k0, segment_end(k0, e[u], CH), c == 0 ? 1 : 0));
                 }
             }
             unsigned hm = __ballot_sync(kFullMask, hn > kLaneChunks);
@@ -575,10 +575,10 @@ __device__ __forceinline__ void push_batch(const ExpandParams& P, const PushCtx&
                 const int hs = __shfl_sync(kFullMask, s[u], src);
                 const int he = __shfl_sync(kFullMask, e[u], src);
                 const unsigned first = __shfl_sync(kFullMask, my_first, src);
-                const int wn = (he - hs + CH - 1) / CH;
+                const int wn = segments_of(he - hs, CH);
                 for (int c = lane; c < wn; c += 32) {
                     const int k0 = hs + c * CH;
-                    __stcg(Q.chunks + first + c, make_int4(hv, k0, min(he, k0 + CH), c == 0 ? 1 : 0));
+                    __stcg(Q.chunks + first + c, make_int4(hv, k0, segment_end(k0, he, CH), c == 0 ? 1 : 0));
                 }
             }
             my_first += static_cast<unsigned>(hn);
@@ -1378,14 +1378,15 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                     // vertices' labels, 128 arcs at a time: 256-arc chunks in one batch took 12.4 ms
                     // against 9.0 (8 sources on each of 48 graphs, same box); 64 at a time is as fast.
                     constexpr int U = O::kMask ? 4 : CH / 32;
-                    auto relax = [&](int kb) {
+                    auto relax = [&](unsigned kb) {
                         bool act[U];
                         int ee[U];
                         RV dd[U];
 #pragma unroll
                         for (int u = 0; u < U; ++u) {
-                            ee[u] = kb + 32 * u + lane;
-                            act[u] = ee[u] < k1;
+                            const unsigned at = kb + 32 * u + lane;
+                            ee[u] = static_cast<int>(at);
+                            act[u] = at < static_cast<unsigned>(k1);
                             dd[u] = du;
                         }
                         relax_batch<O, kClassify, CH, U>(P, Q, act, ee, dd);
@@ -1393,7 +1394,7 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
                     if constexpr (U * 32 == CH) {
                         relax(k0);
                     } else {
-                        for (int kb = k0; kb < k1; kb += 32 * U) relax(kb);
+                        for (unsigned kb = k0; kb < static_cast<unsigned>(k1); kb += 32 * U) relax(kb);
                     }
                     continue;
                 }
@@ -1480,10 +1481,10 @@ __global__ void expand_init_kernel(ExpandParams P, int32_t source, int32_t init_
     const int s = P.off[source];
     const int e = P.off[source + 1];
     const bool chunked = classify && e > s && e - s >= P.hub_threshold;
-    const int nch = chunked ? (e - s + kHubChunk - 1) / kHubChunk : 0;
+    const int nch = chunked ? segments_of(e - s, kHubChunk) : 0;
     for (int64_t c = tid; c < nch; c += stride) {
         const int k0 = s + static_cast<int>(c) * kHubChunk;
-        P.ws.chunks[0][c] = make_int4(source, k0, min(e, k0 + kHubChunk), c == 0 ? 1 : 0);
+        P.ws.chunks[0][c] = make_int4(source, k0, segment_end(k0, e, kHubChunk), c == 0 ? 1 : 0);
     }
     if (tid == 0) {
         for (int k = 0; k < 3; ++k) {
@@ -1558,7 +1559,7 @@ __global__ void multi_seed_kernel(ExpandParams P, const int32_t* __restrict__ so
         const int s = P.off[v], e = P.off[v + 1];
         if (e <= s) continue;
         if (e - s >= P.hub_threshold) {
-            const int nch = (e - s + CH - 1) / CH;
+            const int nch = segments_of(e - s, CH);
             const unsigned first = atomicAdd(P.ws.ccount, static_cast<unsigned>(nch));
             if (static_cast<int64_t>(first) + nch > P.ws.cap_chunks) {
                 raise_error(P.st, DPG_ERR_CAPACITY, 12);
@@ -1566,7 +1567,7 @@ __global__ void multi_seed_kernel(ExpandParams P, const int32_t* __restrict__ so
             }
             for (int c = 0; c < nch; ++c) {
                 const int k0 = s + c * CH;
-                P.ws.chunks[0][first + c] = make_int4(v, k0, min(e, k0 + CH), c == 0 ? 1 : 0);
+                P.ws.chunks[0][first + c] = make_int4(v, k0, segment_end(k0, e, CH), c == 0 ? 1 : 0);
             }
         } else {
             const unsigned pos = atomicAdd(P.ws.qcount, 1u);

@@ -913,7 +913,7 @@ __device__ int32_t plan_range(const int32_t* __restrict__ off, int32_t r0, int32
             cur_rows = 0;
             if (__shfl_sync(kFullMask, static_cast<int>(hub), q)) {
                 const int32_t ha = __shfl_sync(kFullMask, a, q), hb = __shfl_sync(kFullMask, b, q);
-                const int32_t nseg = (hb - ha + kRowTileItems - 1) / kRowTileItems;
+                const int32_t nseg = segments_of(hb - ha, kRowTileItems);
                 sk.hub(c + q, ha, hb, segs, nseg);
                 segs += nseg;
                 p = q + 1;
