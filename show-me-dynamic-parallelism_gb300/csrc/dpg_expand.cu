@@ -849,7 +849,7 @@ __device__ __forceinline__ void local_relax(const ExpandParams& P, const PushCtx
             if (nfar > static_cast<unsigned>(kPushBuf - 32)) flush_far();
         }
         ok = ok && !far;
-        const int d = ok ? se.y - se.x : 0;
+        const int d = ok ? kept_degree(se.x, se.y) : 0;
         const int incl = warp_inclusive_scan(d);
         const bool keep = d > 0 && incl <= 32 && r < P.local_rounds;
         bool push[1] = {ok && !keep};

@@ -58,6 +58,10 @@ __host__ __device__ __forceinline__ int segment_end(int b, int e, int len) {
     return end < static_cast<unsigned>(e) ? static_cast<int>(end) : e;
 }
 
+// Degree of the row [b, e) for a scan over a warp that asks whether the rows so far hold at most 32 arcs:
+// longer rows count 33 (the true degrees of several hubs may add up to more than 2^31).
+__host__ __device__ __forceinline__ int kept_degree(int b, int e) { return e - b < 33 ? e - b : 33; }
+
 // ---- frontier expansion (SSSP / BFS) ------------------------------------------------------------
 
 // Arcs per grid-wide chunk: every vertex at or above the chunking degree is cut into chunks of this

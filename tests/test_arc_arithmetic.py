@@ -45,6 +45,24 @@ int main() {
                         return 1;
                     }
                 }
+    // A warp's rows, some of them hubs of a billion arcs: the rows kept are the longest prefix of at most 32 arcs.
+    const int degs[] = {0, 1, 2, 5, 31, 32, 33, 1100000000, 2147483647};
+    unsigned rnd = 1;
+    for (int t = 0; t < 200000; ++t) {
+        int incl = 0;
+        int64_t sum = 0;
+        for (int lane = 0; lane < 32; ++lane) {
+            rnd = rnd * 1664525u + 1013904223u;
+            const int d = degs[(rnd >> 16) % (t % 2 ? 9 : 4)];
+            const int b = static_cast<int>(2147483647 - static_cast<int64_t>(d));
+            incl = static_cast<int>(static_cast<unsigned>(incl) + static_cast<unsigned>(kept_degree(b, b + d)));
+            sum += d;
+            if ((incl <= 32) != (sum <= 32) || (sum <= 32 && incl != sum)) {
+                std::printf("scan at lane %d: %d, %lld\n", lane, incl, (long long)sum);
+                return 1;
+            }
+        }
+    }
     return 0;
 }
 """
