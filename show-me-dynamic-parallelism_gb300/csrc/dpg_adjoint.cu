@@ -786,7 +786,9 @@ cudaError_t launch_build_perm(const int32_t* tarc, int64_t E, void* scratch, con
     const int nblk = static_cast<int>((E + kPermBlock - 1) / kPermBlock);
     int32_t* slot_of = static_cast<int32_t*>(scratch);
     int32_t* counts = slot_of + E;
-    cudaError_t e = cudaFuncSetAttribute(perm_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * nblk);
+    // The limit of the largest permutation, whatever this one takes (two threads may set it at once).
+    constexpr int kMaxBlocks = static_cast<int>((kPermMaxArcs + kPermBlock - 1) / kPermBlock);
+    cudaError_t e = cudaFuncSetAttribute(perm_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kMaxBlocks);
     if (e != cudaSuccess) return e;
     invert_kernel<<<sm_count * 8, kBlock, 0, s>>>(tarc, E, slot_of);
     const int grid = std::min(nblk, sm_count * 2);

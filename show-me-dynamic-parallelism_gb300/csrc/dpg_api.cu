@@ -353,13 +353,9 @@ dpg_status ensure_plan(dpg_graph* g) {
 // flight need L1 lines, and a 28 KB L1 (the 228 KB shared-memory carve-out) capped them well below
 // what 32 warps issue. On R-MAT scale 22 a PageRank sweep took 0.29 ms with every free byte given
 // to the hot cache (31.5 K entries) and 0.202 ms at this budget (16 K entries, 92 KB of L1).
-#ifndef DPG_GATHER_SMEM_KB
-#define DPG_GATHER_SMEM_KB 164
-#endif
 int32_t hot_entries(const dpg_ctx* c, const dpg_graph* g, bool sweeps) {
     if (!g->relabel) return 0;
-    // 1 KB of each carve-out is reserved per CTA by the system.
-    const int64_t budget = std::min<int64_t>(c->smem_optin, DPG_GATHER_SMEM_KB * 1024 - 1024);
+    const int64_t budget = std::min<int64_t>(c->smem_optin, kGatherSmem);
     const int64_t room = budget - static_cast<int64_t>(rowgather_staging_bytes(sweeps));
     const int64_t cap = room > 4 ? room / 4 - 1 : 0;
     return static_cast<int32_t>(cap < g->V ? cap : g->V);

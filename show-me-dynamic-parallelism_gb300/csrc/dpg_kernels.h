@@ -364,6 +364,12 @@ cudaError_t launch_tile_lane_starts_dev(const int4* tiles, const int64_t* d_ntil
 
 // Grid shape used by the row-gather kernels (needed to size dpart/dfix).
 void rowgather_grid(int sm_count, int* gather_blocks, int* fix_blocks, int* block_threads);
+// Dynamic shared memory of a gather CTA at most (see hot_entries in dpg_api.cu); 1 KB of each carve-out is
+// reserved per CTA by the system.
+#ifndef DPG_GATHER_SMEM_KB
+#define DPG_GATHER_SMEM_KB 164
+#endif
+constexpr int kGatherSmem = DPG_GATHER_SMEM_KB * 1024 - 1024;
 // Shared memory the gather kernel (of the PageRank sweeps, or of SpMV) needs besides the hot-value cache.
 size_t rowgather_staging_bytes(bool sweeps);
 // The merge items of the plan's tiles for the sweeps: 256 per tile, renamed column perm[col[k]] (perm

@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "dpg_kernels.h"
 
@@ -801,19 +802,21 @@ size_t rowgather_staging_bytes(bool sweeps) { return sizeof(float) * kWarps * kP
 
 namespace {
 
-// Sets the kernel's dynamic shared-memory limit to what this launch needs (once per size).
+// Lifts the kernel's dynamic shared-memory limit, once per device. Every thread sets the same limit, whatever
+// its launch takes: a limit set to the launch's own size could be lowered by another thread ahead of the launch.
 template <int MODE, bool CONV, bool BATCH>
-cudaError_t prepare_rowgather(size_t bytes) {
-    static size_t configured = 0;
-    if (bytes <= configured) return cudaSuccess;
-    cudaError_t e;
+cudaError_t prepare_rowgather() {
+    static std::atomic<uint64_t> ready{0};
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    const uint64_t bit = uint64_t{1} << (device & 63);
+    if (e != cudaSuccess || (device < 64 && (ready.load() & bit))) return e;
     if constexpr (MODE == kModeSpmv)
-        e = cudaFuncSetAttribute(spmv_gather_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(bytes));
+        e = cudaFuncSetAttribute(spmv_gather_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatherSmem);
     else
-        e = cudaFuncSetAttribute(rowgather_kernel<MODE, CONV, BATCH>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-    if (e == cudaSuccess) configured = bytes;
+        e = cudaFuncSetAttribute(rowgather_kernel<MODE, CONV, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kGatherSmem);
+    if (e == cudaSuccess) ready.fetch_or(bit);
     return e;
 }
 
@@ -1058,7 +1061,7 @@ cudaError_t launch_row_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream
     rowgather_grid(sm_count, &gb, &fb, &bt);
     // At least one hot entry: the SpMV gather reads entry 0 for cold columns, the sweeps keep a zero.
     const size_t smem = rowgather_staging_bytes(MODE != kModeSpmv) + sizeof(float) * (static_cast<size_t>(L.hot) + 1);
-    cudaError_t err = prepare_rowgather<MODE, CONV, BATCH>(smem);
+    cudaError_t err = prepare_rowgather<MODE, CONV, BATCH>();
     if (err != cudaSuccess) return err;
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, stream);
