@@ -75,9 +75,11 @@ bool capturing(dpg_ctx* c) {
     return st != cudaStreamCaptureStatusNone;
 }
 
-// What a graph keeps is built on first use and then read by calls on any stream and by captured ones. So a
-// build is complete when it returns, and while the context's stream is being captured it runs on the aux
-// stream, for the scope of a BuildScope (its allocations and kernels would else belong to the capture).
+// What a graph keeps is built on first use and then read by calls on any stream and by captured ones. A build
+// leaves an event behind it, and after_builds orders a call's stream behind that. While the context's stream
+// is being captured a build runs on the aux stream instead, for the scope of a BuildScope (its allocations
+// and kernels would else belong to the capture), and is waited for. (Waiting for every build on the host cost
+// first calls 150 us: their allocations no longer overlapped the kernels.)
 struct BuildScope {
     dpg_ctx* c;
     cudaStream_t user;
@@ -98,7 +100,36 @@ struct BuildScope {
     }
     BuildScope(const BuildScope&) = delete;
     BuildScope& operator=(const BuildScope&) = delete;
+
+    cudaError_t queued(dpg_graph* g) {
+        if (off_capture) return cudaStreamSynchronize(c->stream);
+        cudaError_t r = cudaSuccess;
+        if (!g->built) r = cudaEventCreateWithFlags(&g->built, cudaEventDisableTiming);
+        if (r == cudaSuccess) r = cudaEventRecord(g->built, c->stream);
+        if (r == cudaSuccess) g->build_pending = true;
+        return r;
+    }
 };
+
+dpg_status after_builds(dpg_graph* g) {
+    if (!g->build_pending) return DPG_OK;
+    dpg_ctx* c = g->ctx;
+    if (capturing(c)) {
+        BuildScope relaxed(c);  // a captured stream cannot wait for an event from outside: the host does
+        DPG_CUDA_TRY(cudaEventSynchronize(g->built));
+        g->build_pending = false;
+        return DPG_OK;
+    }
+    const cudaError_t e = cudaEventQuery(g->built);
+    if (e == cudaSuccess) {
+        g->build_pending = false;
+        return DPG_OK;
+    }
+    if (e != cudaErrorNotReady) DPG_CUDA_TRY(e);
+    cudaGetLastError();
+    DPG_CUDA_TRY(cudaStreamWaitEvent(c->stream, g->built, 0));
+    return DPG_OK;
+}
 
 // Builds that use the arena's shared buffers cannot leave the stream: refused before they touch anything.
 dpg_status refuse_in_capture(dpg_ctx* c, const char* what) {
@@ -219,6 +250,9 @@ dpg_status graph_finish(dpg_ctx* c, dpg_graph* g, const int32_t* d_w_src) {
 }
 
 void graph_free_device(dpg_graph* g) {
+    if (g->built) cudaEventDestroy(g->built);
+    g->built = nullptr;
+    g->build_pending = false;
     if (g->tgraph) {
         if (g->tgraph->ctx) g->tgraph->ctx->graphs.erase(g->tgraph);
         graph_free_device(g->tgraph);
@@ -320,7 +354,10 @@ dpg_status plan_finish(dpg_graph* g, PlanBuild* pb, const PlanInfo& info) {
 
 // The row plan of a graph whose offsets were validated on the host at creation.
 dpg_status ensure_plan(dpg_graph* g) {
+    DPG_TRY(after_builds(g));
     if (g->plan_ready) return DPG_OK;
+    BuildScope build(g->ctx);
+    DPG_CUDA_TRY(build.e);
     dpg_ctx* c = g->ctx;
     dpg_status st = DPG_OK;
     PlanInfo* info = static_cast<PlanInfo*>(arena(c, S_PLANINFO, sizeof(PlanInfo), &st));
@@ -342,7 +379,7 @@ dpg_status ensure_plan(dpg_graph* g) {
     }
     const dpg_status fs = plan_finish(g, &pb, h);
     if (fs != DPG_OK) plan_build_free(c, &pb);
-    else DPG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    else DPG_CUDA_TRY(build.queued(g));
     return fs;
 }
 
@@ -417,6 +454,7 @@ dpg_status ensure_relabel(dpg_graph* g) {
 
 // The renamed columns in CSR order (SpMV).
 dpg_status ensure_pcol(dpg_graph* g) {
+    DPG_TRY(after_builds(g));
     if (g->V == 0 || (g->relabel_ready && g->pcol)) return DPG_OK;
     dpg_ctx* c = g->ctx;
     BuildScope build(c);
@@ -425,7 +463,7 @@ dpg_status ensure_pcol(dpg_graph* g) {
     if (g->pcol) return DPG_OK;
     cudaError_t e = dev_alloc(c, &g->pcol, static_cast<size_t>(g->E > 0 ? g->E : 1) * 4);
     if (e == cudaSuccess) e = launch_relabel_columns(g->col, g->perm, g->E, g->pcol, c->stream, c->sm_count);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) e = build.queued(g);
     if (e != cudaSuccess) {
         dev_free(c, g->pcol);
         g->pcol = nullptr;
@@ -437,6 +475,7 @@ dpg_status ensure_pcol(dpg_graph* g) {
 // The tiles' merge items (PageRank sweeps) for the graph's current choice of renaming. Each choice has an
 // array of its own: a captured sweep reads the one that it was captured with.
 dpg_status ensure_items(dpg_graph* g, const int32_t** items) {
+    DPG_TRY(after_builds(g));
     int32_t*& at = g->items[g->relabel ? 1 : 0];
     if (!at && g->V > 0) {
         dpg_ctx* c = g->ctx;
@@ -451,7 +490,7 @@ dpg_status ensure_items(dpg_graph* g, const int32_t** items) {
         cudaError_t e =
             dev_alloc(c, &p, sizeof(int32_t) * kRowTileItems * (static_cast<size_t>(g->plan.ntiles) + 1));
         if (e == cudaSuccess) e = launch_tile_items(g->plan, col, perm, p, c->stream, c->sm_count);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e == cudaSuccess) e = build.queued(g);
         if (e != cudaSuccess) {
             dev_free(c, p);
             return set_error(DPG_ERR_CUDA, std::string("merge items: ") + cudaGetErrorString(e));
@@ -536,7 +575,7 @@ dpg_status ensure_spmm_transpose(dpg_graph* g, bool need_graph = false) {
 // no memory for it; the pass then works in arc order.
 constexpr int64_t kSlotArcs = 3 << 22;
 bool backward_slots(dpg_graph* g, float** vals_t, float** dA_t) {
-    if (g->E < kSlotArcs || g->E > kPermMaxArcs) return false;
+    if (g->E < kSlotArcs || g->E > kPermMaxArcs || after_builds(g) != DPG_OK) return false;
     dpg_ctx* c = g->ctx;
     if (!g->tt_perm.mid && (g->tt_perm_tried || capturing(c))) return false;
     const size_t ne = static_cast<size_t>(g->E);
@@ -551,7 +590,7 @@ bool backward_slots(dpg_graph* g, float** vals_t, float** dA_t) {
         if (e == cudaSuccess) e = dev_alloc(c, &P.arc_in, 2 * ne);
         if (e == cudaSuccess) e = dev_alloc(c, &P.slot_in, 2 * ne);
         if (e == cudaSuccess) e = launch_build_perm(g->tt_arc, g->E, scratch, P, c->stream, c->sm_count);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e == cudaSuccess) e = BuildScope(c).queued(g);
         if (e != cudaSuccess) {
             dev_free(c, P.mid);
             dev_free(c, P.arc_in);

@@ -159,6 +159,8 @@ struct dpg_graph {
     int32_t* perm = nullptr;  // old column id -> new
     int32_t* inv = nullptr;   // new -> old
     int32_t* pcol = nullptr;  // col[e] renamed (SpMV), built on first use
+    cudaEvent_t built = nullptr;  // behind the last build queued; later calls are ordered behind it
+    bool build_pending = false;   // until it is known to have passed
     int32_t* items[2] = {nullptr, nullptr};  // the tiles' merge items (PageRank sweeps) without and with the
                                              // renaming, each built on first use
     std::vector<int32_t> relabel_segments;  // optional vertex starts: rename within each segment
