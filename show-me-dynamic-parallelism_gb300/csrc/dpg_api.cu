@@ -1551,12 +1551,12 @@ dpg_status dpg_graph_plan_info(dpg_graph* g, int32_t* tiles, int32_t* hubs_small
 }
 
 namespace {
-__global__ void count_below_kernel(const int32_t* __restrict__ col, int64_t E, int32_t bound,
-                                   unsigned long long* count) {
+__global__ void count_below_kernel(const int32_t* __restrict__ col, const int32_t* __restrict__ perm, int64_t E,
+                                   int32_t bound, unsigned long long* count) {
     unsigned long long c = 0;
     for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < E;
          e += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        c += __ldg(col + e) < bound ? 1ull : 0ull;
+        c += __ldg(perm + __ldg(col + e)) < bound ? 1ull : 0ull;
     c = warp_sum_u64(c);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
 }
@@ -1571,12 +1571,12 @@ dpg_status dpg_graph_hot_cache(dpg_graph* g, int32_t* hot_entries_out, int64_t* 
     if (!hot_arcs) return DPG_OK;
     *hot_arcs = 0;
     if (hot == 0 || g->E == 0) return DPG_OK;
-    DPG_TRY(ensure_pcol(g));
+    DPG_TRY(ensure_relabel(g));
     unsigned long long* d = nullptr;
     DPG_CUDA_TRY(cudaMalloc(&d, sizeof(unsigned long long)));
     cudaError_t e = cudaMemsetAsync(d, 0, sizeof(unsigned long long), c->stream);
     if (e == cudaSuccess) {
-        count_below_kernel<<<c->sm_count * 4, 256, 0, c->stream>>>(g->pcol, g->E, hot, d);
+        count_below_kernel<<<c->sm_count * 4, 256, 0, c->stream>>>(g->col, g->perm, g->E, hot, d);
         e = cudaGetLastError();
     }
     unsigned long long h = 0;
