@@ -133,13 +133,13 @@ __global__ void __launch_bounds__(kBlock) arc_dot1_kernel(SpmmPlanDev P, const i
     for (int64_t k = w; k < P.nitems; k += nw) {
         const int4 I = __ldg(P.items + k);
         const float g = __ldg(G + I.x);
-        for (unsigned e = I.y + lane, end = I.z; e < end; e += 32) dA[e] = g * __ldg(X + __ldg(col + e));
+        for (int t = lane; t < I.z - I.y; t += 32) dA[I.y + t] = g * __ldg(X + __ldg(col + I.y + t));
     }
     for (int64_t v = w * 4 + (lane >> 3); v < P.V; v += nw * 4) {
-        const unsigned b = __ldg(P.off + v), end = __ldg(P.off + v + 1);
-        if (end - b > kGroupRow) continue;  // its items are listed
+        const int b = __ldg(P.off + v), n = __ldg(P.off + v + 1) - b;
+        if (n > kGroupRow) continue;  // its items are listed
         const float g = __ldg(G + v);
-        for (unsigned e = b + (lane & 7); e < end; e += 8) dA[e] = g * __ldg(X + __ldg(col + e));
+        for (int t = lane & 7; t < n; t += 8) dA[b + t] = g * __ldg(X + __ldg(col + b + t));
     }
 }
 

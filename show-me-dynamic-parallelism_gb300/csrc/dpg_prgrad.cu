@@ -80,12 +80,12 @@ __global__ void __launch_bounds__(kBlock) pr_arc_grad_kernel(SpmmPlanDev P, cons
     const int lane = threadIdx.x & 31;
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    auto arcs = [&](int u, unsigned b, unsigned e, int first, int step) {
+    auto arcs = [&](int u, int b, int e, int first, int step) {  // at most kSpmmSegment arcs
         const float Wu = __ldg(W + u);
         // A row with arcs and W == 0 (all weights zero) is dangling: its arcs get no gradient.
         const float c = Wu > 0.0f ? damping * __ldg(r + u) / Wu : 0.0f;
         const float q = Wu > 0.0f ? __ldg(y + u) / Wu : 0.0f;
-        for (unsigned k = b + first; k < e; k += step) grad[k] = c * (__ldg(lam + __ldg(col + k)) - q);
+        for (int t = first; t < e - b; t += step) grad[b + t] = c * (__ldg(lam + __ldg(col + b + t)) - q);
     };
     for (int it = w; it < P.nitems; it += nw) {
         const int4 I = __ldg(P.items + it);
