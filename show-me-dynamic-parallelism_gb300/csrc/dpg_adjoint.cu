@@ -91,8 +91,10 @@ __global__ void __launch_bounds__(kBlock) spmm_rows_kernel(SpmmPlanDev P,
     }
 }
 
-// Split rows: Y[row] = sum of its segments' partial rows, in segment order. Warp per split row.
-template <int NV>
+// Split rows: Y[row] = sum of its segments' partial rows, in segment order; with TREE (segments shorter than
+// kSpmmSegment, so more of them) every eight are added as a tree first and eight of those sums set aside, which
+// keeps the chain of roundings shorter than that of segments of kSpmmSegment. Warp per split row.
+template <int NV, bool TREE = false>
 __global__ void __launch_bounds__(kBlock) spmm_fixup_kernel(const int4* __restrict__ hubs, int nhubs,
                                                             const float* __restrict__ partial, int nrhs,
                                                             float* __restrict__ Y) {
@@ -101,23 +103,37 @@ __global__ void __launch_bounds__(kBlock) spmm_fixup_kernel(const int4* __restri
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int h = w; h < nhubs; h += nw) {
         const int4 H = __ldg(hubs + h);
-        float acc[NV];
+        float acc[NV], aside[NV];
 #pragma unroll
-        for (int q = 0; q < NV; ++q) acc[q] = 0.0f;
+        for (int q = 0; q < NV; ++q) acc[q] = aside[q] = 0.0f;
         for (int s0 = 0; s0 < H.z; s0 += 8) {  // 8 partial rows in flight, added in segment order
             float pv[8][NV];
 #pragma unroll
             for (int u = 0; u < 8; ++u) load_row<NV>(partial, H.y + min(s0 + u, H.z - 1), nrhs, lane, pv[u]);
+            if constexpr (TREE) {
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+                for (int q = 0; q < NV; ++q) {
 #pragma unroll
-                for (int q = 0; q < NV; ++q)
-                    if (s0 + u < H.z) acc[q] += pv[u][q];
+                    for (int u = 0; u < 8; ++u)
+                        if (s0 + u >= H.z) pv[u][q] = 0.0f;
+                    acc[q] += ((pv[0][q] + pv[1][q]) + (pv[2][q] + pv[3][q])) + ((pv[4][q] + pv[5][q]) + (pv[6][q] + pv[7][q]));
+                    if (s0 % 64 == 56) {
+                        aside[q] += acc[q];
+                        acc[q] = 0.0f;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+#pragma unroll
+                    for (int q = 0; q < NV; ++q)
+                        if (s0 + u < H.z) acc[q] += pv[u][q];
+            }
         }
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
             const int j = lane + 32 * q;
-            if (j < nrhs) Y[static_cast<int64_t>(H.x) * nrhs + j] = acc[q];
+            if (j < nrhs) Y[static_cast<int64_t>(H.x) * nrhs + j] = TREE ? aside[q] + acc[q] : acc[q];
         }
     }
 }
@@ -646,8 +662,8 @@ namespace {
 
 // Rows of more than kGroupRow nonzeros into the item list, the whole warp writing one row's segments
 // at a time. Positions come from atomics: the order of the lists changes nothing in the results.
-__global__ void __launch_bounds__(kBlock) spmm_plan_kernel(const int32_t* __restrict__ off, int32_t V, int4* items,
-                                                           int4* hubs, int32_t* counts) {
+__global__ void __launch_bounds__(kBlock) spmm_plan_kernel(const int32_t* __restrict__ off, int32_t V, int segment,
+                                                           int4* items, int4* hubs, int32_t* counts) {
     const int lane = threadIdx.x & 31;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t v0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - lane; v0 < V; v0 += stride) {
@@ -655,7 +671,7 @@ __global__ void __launch_bounds__(kBlock) spmm_plan_kernel(const int32_t* __rest
         const int b = v < V ? __ldg(off + v) : 0;
         const int e = v < V ? __ldg(off + v + 1) : 0;
         const int d = e - b;
-        const int n = d > kGroupRow ? segments_of(d, kSpmmSegment) : 0;
+        const int n = d > kGroupRow ? segments_of(d, segment) : 0;
         int pos = 0, seg = -1;
         if (n > 0) pos = atomicAdd(counts, n);
         if (n > 1) {
@@ -670,8 +686,8 @@ __global__ void __launch_bounds__(kBlock) spmm_plan_kernel(const int32_t* __rest
             const int rn = __shfl_sync(kFullMask, n, src), rp = __shfl_sync(kFullMask, pos, src);
             const int rs = __shfl_sync(kFullMask, seg, src);
             for (int k = lane; k < rn; k += 32) {
-                const int sb = rb + k * kSpmmSegment;
-                items[rp + k] = make_int4(static_cast<int>(v0) + src, sb, segment_end(sb, re, kSpmmSegment), rs < 0 ? -1 : rs + k);
+                const int sb = rb + k * segment;
+                items[rp + k] = make_int4(static_cast<int>(v0) + src, sb, segment_end(sb, re, segment), rs < 0 ? -1 : rs + k);
             }
         }
     }
@@ -679,17 +695,30 @@ __global__ void __launch_bounds__(kBlock) spmm_plan_kernel(const int32_t* __rest
 
 }  // namespace
 
-// A listed row of d nonzeros has ceil(d / kSpmmSegment) <= d / kSpmmSegment + 1 items.
-int64_t spmm_plan_max_items(int64_t E) { return E / kSpmmSegment + E / (kGroupRow + 1) + 1; }
-int64_t spmm_plan_max_hubs(int64_t E) { return E / (kSpmmSegment + 1) + 1; }
+// A warp takes the arcs of an item 16 at a time with up to 64 columns and 8 at a time with more, two round trips
+// each, so an item of 512 is a chain of 64 or 128 round trips; in a small matrix that is the whole call, while most
+// warps have nothing. The items are halved until there could be one for each of the 32 warps of every SM.
+// R-MAT, same box, items of 512 / this rule (and the kernels before this layout, of 4 groups per item): backward of
+// 64 columns, 2,048 vertices x 8 37 / 18 us (27), 10,007 x 16 49 / 29 (37), 60,001 x 16 74 / 68 (101); of 128 columns
+// 51 / 22 (27), 57 / 33 (40), 108 / 96 (144); 200,003 x 16 has 512 either way. Narrow widths take 32 to 128 arcs a
+// step, and the longer fix-up costs them more than that: 3 columns, 25,013 x 16 26.6 / 28.7.
+int32_t spmm_short_segment(int64_t E, int sm_count) {
+    int32_t segment = kSpmmSegment;
+    while (segment > kGroupRow && E / segment < static_cast<int64_t>(sm_count) * 32) segment /= 2;
+    return segment;
+}
 
-cudaError_t launch_spmm_plan(const int32_t* off, int32_t V, int4* items, int4* hubs, int32_t* counts, cudaStream_t s,
-                             int sm_count) {
+// A listed row of d nonzeros has ceil(d / segment) <= d / segment + 1 items.
+int64_t spmm_plan_max_items(int64_t E, int32_t segment) { return E / segment + E / (kGroupRow + 1) + 1; }
+int64_t spmm_plan_max_hubs(int64_t E, int32_t segment) { return E / (segment + 1) + 1; }
+
+cudaError_t launch_spmm_plan(const int32_t* off, int32_t V, int32_t segment, int4* items, int4* hubs, int32_t* counts,
+                             cudaStream_t s, int sm_count) {
     const cudaError_t e = cudaMemsetAsync(counts, 0, 3 * sizeof(int32_t), s);
     if (e != cudaSuccess || V <= 0) return e;
     const int64_t blocks = (static_cast<int64_t>(V) + kBlock - 1) / kBlock;
-    spmm_plan_kernel<<<static_cast<int>(std::min<int64_t>(blocks, sm_count * 8)), kBlock, 0, s>>>(off, V, items, hubs,
-                                                                                                  counts);
+    spmm_plan_kernel<<<static_cast<int>(std::min<int64_t>(blocks, sm_count * 8)), kBlock, 0, s>>>(off, V, segment, items,
+                                                                                                  hubs, counts);
     return cudaGetLastError();
 }
 
@@ -723,7 +752,7 @@ bool spmm_rows_ok(int nrhs, const void* a, const void* b, const void* c, const v
 namespace {
 
 template <int VEC, int LQ, int MODE>
-cudaError_t run_rows(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHook* hook) {
+cudaError_t run_rows(const RowsLaunch& L, bool tree, cudaStream_t s, int sm_count, LaunchHook* hook) {
     {
         HookScope hs(hook, DPG_KERNEL_ROWGATHER, s);
         const int64_t need = std::max((static_cast<int64_t>(L.P.V) + 31) / 32, (static_cast<int64_t>(L.P.nitems) + 7) / 8);
@@ -733,32 +762,32 @@ cudaError_t run_rows(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHo
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || L.P.nhubs == 0 || !L.out) return e;
     HookScope hs(hook, DPG_KERNEL_FIXUP, s);
-    if (L.nrhs <= 32) spmm_fixup_kernel<1><<<sm_count * 4, kBlock, 0, s>>>(L.P.hubs, L.P.nhubs, L.partial, L.nrhs, L.out);
-    else if (L.nrhs <= 64)
-        spmm_fixup_kernel<2><<<sm_count * 4, kBlock, 0, s>>>(L.P.hubs, L.P.nhubs, L.partial, L.nrhs, L.out);
-    else spmm_fixup_kernel<4><<<sm_count * 4, kBlock, 0, s>>>(L.P.hubs, L.P.nhubs, L.partial, L.nrhs, L.out);
+    auto fixup = L.nrhs <= 32   ? spmm_fixup_kernel<1>
+                 : L.nrhs <= 64 ? (tree ? spmm_fixup_kernel<2, true> : spmm_fixup_kernel<2>)
+                                : (tree ? spmm_fixup_kernel<4, true> : spmm_fixup_kernel<4>);
+    fixup<<<sm_count * 4, kBlock, 0, s>>>(L.P.hubs, L.P.nhubs, L.partial, L.nrhs, L.out);
     return cudaGetLastError();
 }
 
 template <int VEC, int MODE>
-cudaError_t pick_rows(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHook* hook) {
+cudaError_t pick_rows(const RowsLaunch& L, bool tree, cudaStream_t s, int sm_count, LaunchHook* hook) {
     const int Q = L.nrhs / VEC;
-    if (Q <= 1) return run_rows<VEC, 1, MODE>(L, s, sm_count, hook);
-    if (Q <= 2) return run_rows<VEC, 2, MODE>(L, s, sm_count, hook);
-    if (Q <= 4) return run_rows<VEC, 4, MODE>(L, s, sm_count, hook);
-    if (Q <= 8) return run_rows<VEC, 8, MODE>(L, s, sm_count, hook);
-    if (Q <= 16) return run_rows<VEC, 16, MODE>(L, s, sm_count, hook);
-    return run_rows<VEC, 32, MODE>(L, s, sm_count, hook);
+    if (Q <= 1) return run_rows<VEC, 1, MODE>(L, tree, s, sm_count, hook);
+    if (Q <= 2) return run_rows<VEC, 2, MODE>(L, tree, s, sm_count, hook);
+    if (Q <= 4) return run_rows<VEC, 4, MODE>(L, tree, s, sm_count, hook);
+    if (Q <= 8) return run_rows<VEC, 8, MODE>(L, tree, s, sm_count, hook);
+    if (Q <= 16) return run_rows<VEC, 16, MODE>(L, tree, s, sm_count, hook);
+    return run_rows<VEC, 32, MODE>(L, tree, s, sm_count, hook);
 }
 
 template <int MODE>
-cudaError_t pick_vec(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHook* hook) {
+cudaError_t pick_vec(const RowsLaunch& L, bool tree, cudaStream_t s, int sm_count, LaunchHook* hook) {
     if (L.P.V <= 0) return cudaSuccess;
     bool vec4 = L.nrhs % 4 == 0;
     for (const void* p : {static_cast<const void*>(L.in), static_cast<const void*>(L.X), static_cast<const void*>(L.out),
                           static_cast<const void*>(L.partial)})
         vec4 = vec4 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
-    return vec4 ? pick_rows<4, MODE>(L, s, sm_count, hook) : pick_rows<1, MODE>(L, s, sm_count, hook);
+    return vec4 ? pick_rows<4, MODE>(L, tree, s, sm_count, hook) : pick_rows<1, MODE>(L, tree, s, sm_count, hook);
 }
 
 }  // namespace
@@ -766,14 +795,14 @@ cudaError_t pick_vec(const RowsLaunch& L, cudaStream_t s, int sm_count, LaunchHo
 cudaError_t launch_spmm_group(const SpmmPlanDev& P, const int32_t* col, const float* val, const float* X, int nrhs,
                               float* Y, float* partial, cudaStream_t s, int sm_count, LaunchHook* hook) {
     const RowsLaunch L = {P, col, nullptr, val, X, nullptr, nrhs, Y, partial, nullptr};
-    return pick_vec<kForward>(L, s, sm_count, hook);
+    return pick_vec<kForward>(L, false, s, sm_count, hook);
 }
 
-cudaError_t launch_spmv_bwd_group(const SpmmPlanDev& TP, const int32_t* tcol, const int32_t* tarc, const float* val,
+cudaError_t launch_spmv_bwd_group(const SpmmPlanDev& TP, bool tree, const int32_t* tcol, const int32_t* tarc, const float* val,
                                   const float* X, const float* G, int nrhs, float* dX, float* partial, float* dA,
                                   cudaStream_t s, int sm_count, LaunchHook* hook) {
     const RowsLaunch L = {TP, tcol, tarc, val, G, X, nrhs, dX, partial, dA};
-    return tarc ? pick_vec<kBwdArcs>(L, s, sm_count, hook) : pick_vec<kBwdSlots>(L, s, sm_count, hook);
+    return tarc ? pick_vec<kBwdArcs>(L, tree, s, sm_count, hook) : pick_vec<kBwdSlots>(L, tree, s, sm_count, hook);
 }
 
 size_t perm_scratch_bytes(int64_t E) {

@@ -272,7 +272,7 @@ void graph_free_device(dpg_graph* g) {
     dev_free(g->ctx, g->t_off);
     dev_free(g->ctx, g->t_col);
     g->perm = g->inv = g->pcol = g->t_off = g->t_col = nullptr;
-    for (SpmmPlanDev* p : {&g->spmm_plan, &g->spmm_t_plan}) {
+    for (SpmmPlanDev* p : {&g->spmm_plan, &g->spmm_t_plan, &g->spmm_t_short}) {
         dev_free(g->ctx, p->items);
         dev_free(g->ctx, p->hubs);
         *p = SpmmPlanDev();
@@ -502,7 +502,7 @@ dpg_status ensure_items(dpg_graph* g, const int32_t** items) {
 }
 
 // The batched-RHS plan of a CSR on the device: built there into buffers of the sizes that bound it.
-dpg_status build_spmm_plan(dpg_ctx* c, const int32_t* off, int32_t V, int64_t E, SpmmPlanDev* out) {
+dpg_status build_spmm_plan(dpg_ctx* c, const int32_t* off, int32_t V, int64_t E, int32_t segment, SpmmPlanDev* out) {
     SpmmPlanDev d;
     d.off = off;
     d.V = V;
@@ -510,9 +510,9 @@ dpg_status build_spmm_plan(dpg_ctx* c, const int32_t* off, int32_t V, int64_t E,
     int32_t* counts = static_cast<int32_t*>(arena(c, S_SPMM_COUNTS, 3 * sizeof(int32_t), &st));
     if (st != DPG_OK) return st;
     int32_t h[3] = {0, 0, 0};
-    cudaError_t e = dev_alloc(c, &d.items, sizeof(int4) * static_cast<size_t>(spmm_plan_max_items(E)));
-    if (e == cudaSuccess) e = dev_alloc(c, &d.hubs, sizeof(int4) * static_cast<size_t>(spmm_plan_max_hubs(E)));
-    if (e == cudaSuccess) e = launch_spmm_plan(off, V, d.items, d.hubs, counts, c->stream, c->sm_count);
+    cudaError_t e = dev_alloc(c, &d.items, sizeof(int4) * static_cast<size_t>(spmm_plan_max_items(E, segment)));
+    if (e == cudaSuccess) e = dev_alloc(c, &d.hubs, sizeof(int4) * static_cast<size_t>(spmm_plan_max_hubs(E, segment)));
+    if (e == cudaSuccess) e = launch_spmm_plan(off, V, segment, d.items, d.hubs, counts, c->stream, c->sm_count);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, counts, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
@@ -530,7 +530,7 @@ dpg_status build_spmm_plan(dpg_ctx* c, const int32_t* off, int32_t V, int64_t E,
 dpg_status ensure_spmm_plan(dpg_graph* g) {
     if (g->spmm_ready) return DPG_OK;
     DPG_TRY(refuse_in_capture(g->ctx, "the batched-RHS plan"));
-    DPG_TRY(build_spmm_plan(g->ctx, g->off, g->V, g->E, &g->spmm_plan));
+    DPG_TRY(build_spmm_plan(g->ctx, g->off, g->V, g->E, kSpmmSegment, &g->spmm_plan));
     g->spmm_ready = true;
     return DPG_OK;
 }
@@ -555,13 +555,27 @@ dpg_status ensure_spmm_transpose(dpg_graph* g, bool need_graph = false) {
                                  c->stream, c->sm_count);
         if (st != DPG_OK) return st;
         if (e != cudaSuccess) return set_error(DPG_ERR_CUDA, std::string("device transpose: ") + cudaGetErrorString(e));
-        DPG_TRY(build_spmm_plan(c, g->tt_off, g->V, g->E, &g->spmm_t_plan));
+        DPG_TRY(build_spmm_plan(c, g->tt_off, g->V, g->E, kSpmmSegment, &g->spmm_t_plan));
         g->spmm_t_ready = true;
     }
     if (need_graph && !g->tgraph) {
         DPG_TRY(graph_create_common(c, g->V, g->E, g->tt_off, g->tt_col, nullptr, true, &g->tgraph));
         g->tgraph->relabel = g->relabel;
     }
+    return DPG_OK;
+}
+
+// The plan of the transposed CSR for the backward of nrhs columns (see spmm_short_segment).
+dpg_status backward_plan(dpg_graph* g, int32_t nrhs, const SpmmPlanDev** plan) {
+    dpg_ctx* c = g->ctx;
+    *plan = &g->spmm_t_plan;
+    const int32_t segment = spmm_short_segment(g->E, c->sm_count);
+    if (nrhs <= 32 || segment == kSpmmSegment) return DPG_OK;
+    if (!g->spmm_t_short.items) {
+        if (capturing(c)) return DPG_OK;
+        DPG_TRY(build_spmm_plan(c, g->tt_off, g->V, g->E, segment, &g->spmm_t_short));
+    }
+    *plan = &g->spmm_t_short;
     return DPG_OK;
 }
 
@@ -1675,15 +1689,17 @@ dpg_status dpg_spmv_bwd_f32_dev(dpg_ctx* c, const dpg_graph* gc, const float* d_
     if (!arcs_only && spmm_rows_ok(nrhs, d_X, d_G, d_dX, nullptr) && (d_dX || d_dA)) {
         // Both outputs in one pass over the transposed CSR: each arc's row of G is gathered once.
         DPG_TRY(ensure_spmm_transpose(g));
+        const SpmmPlanDev* plan = nullptr;
+        DPG_TRY(backward_plan(g, nrhs, &plan));
         dpg_status st = DPG_OK;
-        float* partial = static_cast<float*>(
-            arena(c, S_SPMM_PARTIAL, static_cast<size_t>(g->spmm_t_plan.nseg + 1) * nrhs * 4, &st));
+        float* partial =
+            static_cast<float*>(arena(c, S_SPMM_PARTIAL, static_cast<size_t>(plan->nseg + 1) * nrhs * 4, &st));
         if (st != DPG_OK) return st;
         float *vals_t = nullptr, *dA_t = nullptr;
         const bool slots = backward_slots(g, &vals_t, &dA_t);
         if (slots && d_dX)
             DPG_CUDA_TRY(launch_permute(g->tt_perm, g->E, true, d_vals, dA_t, vals_t, c->stream, c->sm_count, &c->prof));
-        DPG_CUDA_TRY(launch_spmv_bwd_group(g->spmm_t_plan, g->tt_col, slots ? nullptr : g->tt_arc, slots ? vals_t : d_vals,
+        DPG_CUDA_TRY(launch_spmv_bwd_group(*plan, plan == &g->spmm_t_short, g->tt_col, slots ? nullptr : g->tt_arc, slots ? vals_t : d_vals,
                                            d_X, d_G, nrhs, d_dX, partial, slots && d_dA ? dA_t : d_dA, c->stream,
                                            c->sm_count, &c->prof));
         if (slots && d_dA)

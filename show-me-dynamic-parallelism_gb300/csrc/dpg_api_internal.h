@@ -173,6 +173,7 @@ struct dpg_graph {
     SpmmPlanDev spmm_plan;
     bool spmm_t_ready = false;
     SpmmPlanDev spmm_t_plan;
+    SpmmPlanDev spmm_t_short;  // of shorter items, for the backward of wide rows on small graphs
     int32_t* tt_off = nullptr;
     int32_t* tt_col = nullptr;
     int32_t* tt_arc = nullptr;

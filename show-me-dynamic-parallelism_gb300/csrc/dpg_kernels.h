@@ -240,7 +240,7 @@ struct RowGatherLaunch {
 cudaError_t launch_window_tiles(const RowPlanDev& plan, const int32_t* rows, int nwin, int2* win, cudaStream_t s);
 
 // ---- batched right-hand sides / SpMV adjoint (dpg_adjoint.cu) -----------------------------------
-constexpr int kSpmmSegment = 512;  // nonzeros per listed item; longer rows are split and fixed up in order
+constexpr int kSpmmSegment = 512;  // nonzeros per listed item at most; longer rows are split and fixed up
 constexpr int kGroupRow = 64;      // rows of more nonzeros are listed
 
 // Items {row, arc begin, arc end, segment index or -1} of the rows of more than kGroupRow nonzeros, in
@@ -254,20 +254,22 @@ struct SpmmPlanDev {
     int32_t nhubs = 0;
     int32_t nseg = 0;
 };
+// Nonzeros per item for the backward of more than 32 columns on a matrix of E nonzeros.
+int32_t spmm_short_segment(int64_t E, int sm_count);
 // Upper bounds of the items and hubs of any CSR of E nonzeros.
-int64_t spmm_plan_max_items(int64_t E);
-int64_t spmm_plan_max_hubs(int64_t E);
+int64_t spmm_plan_max_items(int64_t E, int32_t segment);
+int64_t spmm_plan_max_hubs(int64_t E, int32_t segment);
 // Fills items and hubs (capacities as above); counts[0..2] receive the items, hubs and segments.
-cudaError_t launch_spmm_plan(const int32_t* off, int32_t V, int4* items, int4* hubs, int32_t* counts, cudaStream_t s,
-                             int sm_count);
+cudaError_t launch_spmm_plan(const int32_t* off, int32_t V, int32_t segment, int4* items, int4* hubs, int32_t* counts,
+                             cudaStream_t s, int sm_count);
 // Whether rows_kernel takes this width and these row blocks (null: not used).
 bool spmm_rows_ok(int nrhs, const void* a, const void* b, const void* c, const void* d);
 cudaError_t launch_spmm_group(const SpmmPlanDev& P, const int32_t* col, const float* val, const float* X, int nrhs,
                               float* Y, float* partial, cudaStream_t s, int sm_count, LaunchHook* hook);
 // One pass over the transposed CSR (plan TP, columns tcol, arc permutation tarc): dX = A^T G and
 // dA[e] = <G[row(e)], X[col(e)]>; either output may be null. With tarc null, val and dA are in the
-// order of tcol (transposed slots).
-cudaError_t launch_spmv_bwd_group(const SpmmPlanDev& TP, const int32_t* tcol, const int32_t* tarc, const float* val,
+// order of tcol (transposed slots). `tree`: the plan's items are shorter than kSpmmSegment.
+cudaError_t launch_spmv_bwd_group(const SpmmPlanDev& TP, bool tree, const int32_t* tcol, const int32_t* tarc, const float* val,
                                   const float* X, const float* G, int nrhs, float* dX, float* partial, float* dA,
                                   cudaStream_t s, int sm_count, LaunchHook* hook);
 // Y[row][:] = sum over the row's arcs of val[e] * X[col[e]][:] (row-major [*][nrhs], nrhs <= 128);
