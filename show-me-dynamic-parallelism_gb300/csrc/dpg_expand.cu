@@ -575,7 +575,7 @@ __device__ __forceinline__ void push_batch(const ExpandParams& P, const PushCtx&
                 const int hs = __shfl_sync(kFullMask, s[u], src);
                 const int he = __shfl_sync(kFullMask, e[u], src);
                 const unsigned first = __shfl_sync(kFullMask, my_first, src);
-                const int wn = segments_of(he - hs, CH);
+                const int wn = __shfl_sync(kFullMask, hn, src);
                 for (int c = lane; c < wn; c += 32) {
                     const int k0 = hs + c * CH;
                     __stcg(Q.chunks + first + c, make_int4(hv, k0, segment_end(k0, he, CH), c == 0 ? 1 : 0));
