@@ -718,9 +718,8 @@ dpg_status run_color(dpg_ctx* c, dpg_graph* g, const dpg_expand_opts* in_opts, i
 }
 
 // Near-far threshold step in units of the mean arc weight (see dpg_expand.cu, DPG_SOL_NEARFAR).
-// Measured (2 sources): on the 4096^2 grid (weights 1..1000) SSSP takes 120 ms at 2x the mean
-// weight, 80 at 8x, 67 at 32x, 65 at 64x and 73 at 256x; on R-MAT 22 and 24 (weights 1..255) 32x
-// is within 5 % of the binned expansion, and 2x is 15-50 % slower.
+// Measured (2 sources, with the local rounds): on the 4096^2 grid (weights 1..1000) SSSP takes 41.6 ms at 2x the mean
+// weight, 29.5 at 8x, 25.9 at 32x, 35.2 at 64x and 63.0 at 256x.
 constexpr double kNearFarStep = 32.0;
 // Rounds a warp goes on with the vertices it improved before the grid barrier (local_relax in
 // dpg_expand.cu, with the measurements): for distances 5 and 6 are fastest, past that the scanned
@@ -742,9 +741,9 @@ void fill_expand_defaults(const dpg_expand_opts* in, dpg_expand_opts* o, const d
         o->solution = DPG_SOL_DIROPT;  // BFS: direction-optimizing; SSSP: near-far or binned (run_expand)
     }
     if (o->threshold <= 0) o->threshold = DPG_REF_THRESHOLD;
-    // Degree from which a frontier vertex is cut into grid-wide chunks. Measured on R-MAT 24 (4
-    // sources): SSSP 9.06 ms at 32, 8.14 at 64, 7.81 at 128, 8.08 at 256; BFS (direction-optimizing)
-    // 1.84 / 1.76 / 1.77 / 1.77 ms. At R-MAT 22, SSSP takes 2.59 / 2.28 / 2.35 / 2.36 ms.
+    // Degree from which a frontier vertex is cut into grid-wide chunks. Measured (4 sources, at 32 / 64 / 128 / 256) on
+    // R-MAT 24: SSSP 3.86 / 2.89 / 2.79 / 2.79 ms, BFS (direction-optimizing) 0.78 / 0.74 / 0.76 / 0.76 ms; on R-MAT 22:
+    // SSSP 1.14 / 0.93 / 0.92 / 1.11 ms, BFS 0.25 / 0.24 / 0.24 / 0.25 ms.
     if (o->hub_threshold <= 0) o->hub_threshold = 128;
     if (o->solution == DPG_SOL_GRID) o->hub_threshold = o->threshold;
     if (o->max_iterations <= 0) {
@@ -764,9 +763,9 @@ dpg_status run_expand(dpg_ctx* c, const dpg_graph* g, int32_t source, const dpg_
     fill_expand_defaults(in_opts, &o, g);
     if (o.solution < DPG_SOL_THREAD || o.solution > DPG_SOL_NEARFAR)
         return set_error(DPG_ERR_INVALID_ARG, "unknown solution id");
-    // The default id asks for the GB300 choice; for SSSP (bottom-up steps are BFS only) that is
-    // near-far on graphs without hubs and of low mean degree (road-like, grids: 4096^2 grid 68 ms
-    // against 167 ms binned), and the binned expansion otherwise (R-MAT: near-far only ties it).
+    // The default id asks for the GB300 choice; for SSSP (bottom-up steps are BFS only) that is near-far on graphs
+    // without hubs and of low mean degree (road-like, grids: 4096^2 grid 26 ms against 200 ms binned), and the binned
+    // expansion otherwise (R-MAT 22 and 24: 0.92 and 2.79 ms, near-far 1.63 and 5.68 ms).
     const bool pick = !bfs && o.solution == DPG_SOL_DIROPT;
     if (pick)
         o.solution = (g->weighted && g->max_degree < o.hub_threshold && g->E <= 8 * static_cast<int64_t>(g->V))
@@ -799,8 +798,8 @@ dpg_status run_expand(dpg_ctx* c, const dpg_graph* g, int32_t source, const dpg_
         L.local_rounds = in_opts && in_opts->max_iterations > 0 ? 0 : bfs ? kLevelRounds : kNearFarRounds;
     // A caller's own solution or iteration cap keeps the plain order of relaxations. The ladder's phases may together
     // take more iterations than the vertices a path can have.
-    if (pick && o.solution == DPG_SOL_BINNED && !(in_opts && in_opts->max_iterations > 0) && g->V >= kLadderVertices &&
-        g->E >= kLadderArcs) {
+    if (pick && o.solution == DPG_SOL_BINNED && L.wide && !(in_opts && in_opts->max_iterations > 0) &&
+        g->V >= kLadderVertices && g->E >= kLadderArcs) {  // (binned by choice is wide; only that build has the ladder)
         L.ladder = static_cast<int32_t>(std::max(1.0, std::min(1e8, g->mean_weight / 64)));
         L.max_iter = static_cast<int32_t>(std::min<int64_t>(INT32_MAX, (static_cast<int64_t>(g->V) + 3) * 8));
     }

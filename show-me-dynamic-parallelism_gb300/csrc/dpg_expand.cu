@@ -1035,7 +1035,9 @@ __global__ void __launch_bounds__(kBlock, MINB > 0 ? MINB : Op::min_blocks(CH)) 
     // moves past delta and the pile's minimum, and one split step moves the pile's still-current
     // entries below it into the frontier and the rest into the next pile. Piles rotate over three
     // buffers so the one being reset is never the one being read or written.
-    constexpr bool kLadder = POL == DPG_SOL_BINNED && std::is_same_v<Op, SsspOp>;
+    // Graphs with hubs, where the ladder is used, run the 4-CTA build; in the 3-CTA build its state only cost
+    // spills (binned SSSP on the 4096^2 grid 197 -> 205 ms).
+    constexpr bool kLadder = POL == DPG_SOL_BINNED && std::is_same_v<Op, SsspOp> && MINB > 0;
     int threshold = kNearFar ? P.delta : 0x7FFFFFFF;
     int phase = kLadder && P.ladder ? 0 : kLadderPhases;  // thresholds left behind; the ladder is off past the last
     int ladder_base = 0;
