@@ -76,7 +76,8 @@ typedef struct dpg_expand_opts {
     int32_t solution;        /* dpg_solution; DPG_SOL_DIROPT when the struct pointer is NULL */
     int32_t threshold;       /* consolidation degree threshold; 0 -> DPG_REF_THRESHOLD */
     int32_t hub_threshold;   /* BINNED: degree at which a vertex is expanded grid-wide; 0 -> auto */
-    int32_t max_iterations;  /* 0 -> V + 2 (label-correcting never needs more) */
+    int32_t max_iterations;  /* grid-wide iterations; 0 -> V + 2 (label-correcting never needs more), or 8 (V + 3)
+                                where the default SSSP climbs a ladder of distance thresholds (hubs, large graphs) */
     double timeout_seconds;  /* limit of each grid-barrier wait; 0 -> 10 s */
     int32_t delta;           /* NEARFAR: threshold step; 0 -> 32 x the mean arc weight */
 } dpg_expand_opts;
@@ -90,7 +91,10 @@ typedef struct dpg_pr_opts {
 } dpg_pr_opts;
 
 typedef struct dpg_run_stats {
-    int64_t iterations;      /* frontier iterations (SSSP/BFS) or PageRank sweeps */
+    int64_t iterations;      /* grid-wide frontier iterations (SSSP/BFS) or PageRank sweeps. Not the number of levels of a
+                                default BFS on a sparse graph of high diameter (nor its trace entries): past 32
+                                iterations, warps go on with their own finds between two of them (4096 x 4096 grid:
+                                195 iterations for 5,387 levels). An explicit max_iterations keeps one level each. */
     int64_t edges_scanned;   /* adjacency entries read by the expansion (>= E for label-correcting) */
     int64_t vertices_popped; /* frontier entries processed */
     int32_t grid_blocks;     /* CTAs of the persistent launch */
@@ -121,6 +125,14 @@ dpg_status dpg_graph_create(dpg_ctx* ctx, int32_t V, int64_t E, const int32_t* o
 dpg_status dpg_graph_create_device(dpg_ctx* ctx, int32_t V, int64_t E, const int32_t* d_offsets,
                                    const int32_t* d_col, const int32_t* d_weights, dpg_graph** out);
 dpg_status dpg_graph_destroy(dpg_graph* g);
+/* Device memory beside the CSR. A graph keeps what the first call that needs it builds, until it is destroyed (V
+ * vertices, E arcs): 8 V bytes for the column renaming of SpMV and PageRank; 4 E for SpMV's renamed columns; about
+ * 4 (V + E) for PageRank's merge items, once per choice of dpg_graph_relabel that was used; 4 V + 8 E for the transposed
+ * CSR of the SpMV backward and the PageRank gradient (which keeps both plans of that CSR too), and for a backward
+ * between 12.6 M and 268 M arcs another 8 E for its value permutation. The context keeps scratch of the size of the
+ * largest call, until it is destroyed; such a backward takes 8 E of it, and 4 E + 4 (E / 24576)^2 for the first call
+ * on a graph. If that cannot be had, the backward reads and writes the values in arc order instead.
+ * First calls may be captured into a CUDA graph only where all they build is the renamed columns or the merge items. */
 /* Gather-locality layout for SpMV / PageRank (on by default): column ids are renamed once, by
  * descending frequency, so hot gathered values share cache sectors. Rows and the order of nonzeros in
  * each row are unchanged, so results are bit-identical either way; enable = 0 turns it off. No

@@ -764,7 +764,7 @@ dpg_status run_expand(dpg_ctx* c, const dpg_graph* g, int32_t source, const dpg_
     if (o.solution < DPG_SOL_THREAD || o.solution > DPG_SOL_NEARFAR)
         return set_error(DPG_ERR_INVALID_ARG, "unknown solution id");
     // The default id asks for the GB300 choice; for SSSP (bottom-up steps are BFS only) that is near-far on graphs
-    // without hubs and of low mean degree (road-like, grids: 4096^2 grid 26 ms against 200 ms binned), and the binned
+    // without hubs and of low mean degree (road-like, grids: 4096^2 grid 25 ms against 157 to 220 ms binned), and the binned
     // expansion otherwise (R-MAT 22 and 24: 0.92 and 2.79 ms, near-far 1.63 and 5.68 ms).
     const bool pick = !bfs && o.solution == DPG_SOL_DIROPT;
     if (pick)
@@ -799,7 +799,7 @@ dpg_status run_expand(dpg_ctx* c, const dpg_graph* g, int32_t source, const dpg_
     // A caller's own solution or iteration cap keeps the plain order of relaxations. The ladder's phases may together
     // take more iterations than the vertices a path can have.
     if (pick && o.solution == DPG_SOL_BINNED && L.wide && !(in_opts && in_opts->max_iterations > 0) &&
-        g->V >= kLadderVertices && g->E >= kLadderArcs) {  // (binned by choice is wide; only that build has the ladder)
+        g->V >= kLadderVertices && g->E >= kLadderArcs) {  // (the pick is binned on wide graphs, whose build has the ladder)
         L.ladder = static_cast<int32_t>(std::max(1.0, std::min(1e8, g->mean_weight / 64)));
         L.max_iter = static_cast<int32_t>(std::min<int64_t>(INT32_MAX, (static_cast<int64_t>(g->V) + 3) * 8));
     }
@@ -903,8 +903,9 @@ dpg_status run_pagerank(dpg_ctx* c, dpg_graph* g, const int32_t* d_outdeg, const
     DPG_CUDA_TRY(launch_pagerank_init(L, init_rank, init_rank_dst, c->st, c->stream, c->sm_count, &c->prof));
     // With a tolerance the convergence test is pipelined one sweep deep: sweep it+1 is queued before
     // the host reads sweep it's flag (written to pinned memory by the sweep's last kernel, behind an
-    // event), so the device does not idle on the read. A sweep queued after the converged one writes only buffers of the other parity (ranks,
-    // contributions, dangling sum, flag), so the converged ranks stay where the count says.
+    // event), so the device does not idle on the read. A sweep queued after the converged one writes
+    // only buffers of the other parity (ranks, contributions, dangling sum, flag), so the converged
+    // ranks stay where the count says.
     unsigned* hflags = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     if (conv) {

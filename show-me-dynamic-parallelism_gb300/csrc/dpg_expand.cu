@@ -51,6 +51,9 @@ namespace {
 // 2^24 2.0-4.1 E / 1.07-1.73 E arcs scanned. Other ladders at 2^24 and 10^6, first threshold and steps (counted from 0):
 // 1/64 x 2 x 2 x 2 2.89 ms, 463 us; 1/64 x 4 3.20, 464; 1/32 x 2 x 2 2.85, 459; 1/32 x 1.5 x 1.5 x 1.5 2.78, 464; 1/16 and
 // five steps of 1.5 3.28, 577.
+// What it can cost: regions of high diameter whose distances lie on either side of a threshold are traversed one after
+// another instead of together. Two cores of hubs with chains of 1,500 and a 40 x 1,000 grid behind them, weights 0..2:
+// 3,008 iterations, 22.8 ms without, 4,396 and 29.3 ms with (weights 1..255: no difference).
 constexpr int kLadderPhases = 3;
 constexpr int kLadderStep = 3;
 constexpr int kSweep = 16;  // labels a lane reads at a time in a sweep

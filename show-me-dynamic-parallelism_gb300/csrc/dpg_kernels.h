@@ -388,7 +388,7 @@ cudaError_t launch_spmv(const RowGatherLaunch& L, DevStatus* st, cudaStream_t st
 // One PageRank sweep: gather + hub fix-up + dangling reduction into dsum_out.
 cudaError_t launch_pagerank_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream,
                                   int sm_count, LaunchHook* hook);
-// One sweep of the weighted PageRank or of its adjoint (dpg_prgrad.cu): gather over plan / col / vals,
+// One sweep of the weighted PageRank or of its adjoint (dpg_prgrad.cu): gather over plan / items / witems,
 // epilogue, hub fix-up, and the reduced quantity into dsum_out.
 cudaError_t launch_weighted_sweep(const RowGatherLaunch& L, DevStatus* st, cudaStream_t stream, int sm_count,
                                   LaunchHook* hook);
