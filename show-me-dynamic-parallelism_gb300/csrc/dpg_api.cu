@@ -285,7 +285,7 @@ void graph_free_device(dpg_graph* g) {
     dev_free(g->ctx, g->tt_perm.slot_in);
     g->tt_perm = ArcPerm();
     g->tt_off = g->tt_col = g->tt_arc = nullptr;
-    g->spmm_ready = g->spmm_t_ready = false;
+    g->spmm_ready = g->tt_ready = false;
     g->relabel_ready = false;
     dev_free(g->ctx, g->plan.tiles);
     dev_free(g->ctx, g->plan.lane_info);
@@ -536,12 +536,13 @@ dpg_status ensure_spmm_plan(dpg_graph* g) {
 }
 
 // Deterministic transposed CSR with the arc permutation, built on the device in invertGraph order
-// (dpg_transpose.cu), and its batched-RHS plan. With need_graph the transposed CSR also becomes a
-// graph of its own (g->tgraph).
+// (dpg_transpose.cu). With need_graph it also becomes a graph of its own (g->tgraph).
 dpg_status ensure_spmm_transpose(dpg_graph* g, bool need_graph = false) {
+    DPG_TRY(after_builds(g));
     dpg_ctx* c = g->ctx;
-    if (!g->spmm_t_ready) {
+    if (!g->tt_ready) {
         DPG_TRY(refuse_in_capture(c, "the transposed CSR"));
+        BuildScope build(c);
         const size_t nv = static_cast<size_t>(g->V), ne = static_cast<size_t>(g->E > 0 ? g->E : 1);
         cudaError_t e = cudaSuccess;
         if (!g->tt_off) e = dev_alloc(c, &g->tt_off, (nv + 1) * 4);
@@ -554,29 +555,37 @@ dpg_status ensure_spmm_transpose(dpg_graph* g, bool need_graph = false) {
             e = launch_transpose(g->off, g->col, g->V, g->E, g->tt_off, g->tt_col, g->tt_arc, scratch, scratch_bytes,
                                  c->stream, c->sm_count);
         if (st != DPG_OK) return st;
+        if (e == cudaSuccess) e = build.queued(g);
         if (e != cudaSuccess) return set_error(DPG_ERR_CUDA, std::string("device transpose: ") + cudaGetErrorString(e));
-        DPG_TRY(build_spmm_plan(c, g->tt_off, g->V, g->E, kSpmmSegment, &g->spmm_t_plan));
-        g->spmm_t_ready = true;
+        g->tt_ready = true;
     }
     if (need_graph && !g->tgraph) {
+        DPG_TRY(refuse_in_capture(c, "the transposed graph"));
+        DPG_CUDA_TRY(cudaStreamSynchronize(c->stream));  // its offsets are read on the host
         DPG_TRY(graph_create_common(c, g->V, g->E, g->tt_off, g->tt_col, nullptr, true, &g->tgraph));
         g->tgraph->relabel = g->relabel;
     }
     return DPG_OK;
 }
 
-// The plan of the transposed CSR for the backward of nrhs columns (see spmm_short_segment).
-dpg_status backward_plan(dpg_graph* g, int32_t nrhs, const SpmmPlanDev** plan) {
+// The plan of the transposed CSR for the backward, of items of up to kSpmmSegment nonzeros, or of shorter ones for wide
+// rows on small graphs (see spmm_short_segment; `tree` is then set). Each is built when it is first asked for. Either
+// serves any width, so a call that is captured takes the one that is there.
+dpg_status backward_plan(dpg_graph* g, bool wide, const SpmmPlanDev** plan, bool* tree) {
     dpg_ctx* c = g->ctx;
-    *plan = &g->spmm_t_plan;
-    const int32_t segment = spmm_short_segment(g->E, c->sm_count);
-    if (nrhs <= 32 || segment == kSpmmSegment) return DPG_OK;
-    if (!g->spmm_t_short.items) {
-        if (capturing(c)) return DPG_OK;
-        DPG_TRY(build_spmm_plan(c, g->tt_off, g->V, g->E, segment, &g->spmm_t_short));
+    const int32_t segment = wide ? spmm_short_segment(g->E, c->sm_count) : kSpmmSegment;
+    *tree = segment != kSpmmSegment;
+    const SpmmPlanDev* other = *tree ? &g->spmm_t_plan : &g->spmm_t_short;
+    SpmmPlanDev* p = *tree ? &g->spmm_t_short : &g->spmm_t_plan;
+    *plan = p;
+    if (p->items) return DPG_OK;
+    if (capturing(c) && other->items) {
+        *plan = other;
+        *tree = false;
+        return DPG_OK;
     }
-    *plan = &g->spmm_t_short;
-    return DPG_OK;
+    DPG_TRY(refuse_in_capture(c, "the batched-RHS plan"));
+    return build_spmm_plan(c, g->tt_off, g->V, g->E, segment, p);
 }
 
 // Arc values in transposed order for the backward: the permutation and the two arrays. The transposed
@@ -1690,7 +1699,8 @@ dpg_status dpg_spmv_bwd_f32_dev(dpg_ctx* c, const dpg_graph* gc, const float* d_
         // Both outputs in one pass over the transposed CSR: each arc's row of G is gathered once.
         DPG_TRY(ensure_spmm_transpose(g));
         const SpmmPlanDev* plan = nullptr;
-        DPG_TRY(backward_plan(g, nrhs, &plan));
+        bool tree = false;
+        DPG_TRY(backward_plan(g, nrhs > 32, &plan, &tree));
         dpg_status st = DPG_OK;
         float* partial =
             static_cast<float*>(arena(c, S_SPMM_PARTIAL, static_cast<size_t>(plan->nseg + 1) * nrhs * 4, &st));
@@ -1699,7 +1709,7 @@ dpg_status dpg_spmv_bwd_f32_dev(dpg_ctx* c, const dpg_graph* gc, const float* d_
         const bool slots = backward_slots(g, &vals_t, &dA_t);
         if (slots && d_dX)
             DPG_CUDA_TRY(launch_permute(g->tt_perm, g->E, true, d_vals, dA_t, vals_t, c->stream, c->sm_count, &c->prof));
-        DPG_CUDA_TRY(launch_spmv_bwd_group(*plan, plan == &g->spmm_t_short, g->tt_col, slots ? nullptr : g->tt_arc, slots ? vals_t : d_vals,
+        DPG_CUDA_TRY(launch_spmv_bwd_group(*plan, tree, g->tt_col, slots ? nullptr : g->tt_arc, slots ? vals_t : d_vals,
                                            d_X, d_G, nrhs, d_dX, partial, slots && d_dA ? dA_t : d_dA, c->stream,
                                            c->sm_count, &c->prof));
         if (slots && d_dA)
@@ -1708,13 +1718,16 @@ dpg_status dpg_spmv_bwd_f32_dev(dpg_ctx* c, const dpg_graph* gc, const float* d_
     }
     if (d_dX) {
         DPG_TRY(ensure_spmm_transpose(g));
+        const SpmmPlanDev* plan = nullptr;
+        bool tree = false;
+        DPG_TRY(backward_plan(g, false, &plan, &tree));
         dpg_status st = DPG_OK;
         float* vals_t = static_cast<float*>(arena(c, S_VALS_T, static_cast<size_t>(g->E > 0 ? g->E : 1) * 4, &st));
         float* partial = static_cast<float*>(
-            arena(c, S_SPMM_PARTIAL, static_cast<size_t>(g->spmm_t_plan.nseg + 1) * nrhs * 4, &st));
+            arena(c, S_SPMM_PARTIAL, static_cast<size_t>(plan->nseg + 1) * nrhs * 4, &st));
         if (st != DPG_OK) return st;
         DPG_CUDA_TRY(launch_gather_values(d_vals, g->tt_arc, g->E, vals_t, c->stream, c->sm_count));
-        DPG_CUDA_TRY(launch_spmm(g->spmm_t_plan, g->tt_col, vals_t, d_G, nrhs, d_dX, partial, c->stream, c->sm_count,
+        DPG_CUDA_TRY(launch_spmm(*plan, g->tt_col, vals_t, d_G, nrhs, d_dX, partial, c->stream, c->sm_count,
                                  &c->prof));
     }
     if (d_dA) {

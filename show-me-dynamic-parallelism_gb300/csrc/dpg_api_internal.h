@@ -171,7 +171,7 @@ struct dpg_graph {
     // (tt_*, with tt_arc[p] = the arc that transposed slot p came from), built on first use.
     bool spmm_ready = false;
     SpmmPlanDev spmm_plan;
-    bool spmm_t_ready = false;
+    bool tt_ready = false;
     SpmmPlanDev spmm_t_plan;
     SpmmPlanDev spmm_t_short;  // of shorter items, for the backward of wide rows on small graphs
     int32_t* tt_off = nullptr;

@@ -80,3 +80,38 @@ def test_backward(ctx, E, hub, nrhs):
         ctx.set_stream(None)
     err, err512 = (np.linalg.norm(d - want) / np.linalg.norm(want) for d in (dX, out.cpu().numpy()))
     assert err <= err512 * 1.05 + 1e-9, (err, err512)
+
+
+@pytest.mark.parametrize("nrhs", [1, 3, 32, 36, 64])
+def test_captured_after_a_wide_call(ctx, nrhs):
+    """A graph whose only backward so far was of 64 columns: a captured one of any width takes the plan that is there."""
+    import torch
+
+    g = _graph(60_000, 20_000, 9)
+    rng = np.random.default_rng(4)
+    tv = torch.from_numpy(rng.uniform(0.5, 1.5, g.E).astype(np.float32)).cuda()
+    X, G = (torch.from_numpy(rng.uniform(-1, 1, (g.V, 64)).astype(np.float32)).cuda() for _ in range(2))
+    x, gg = X[:, :nrhs].contiguous(), G[:, :nrhs].contiguous()
+    dX64, dA = torch.empty_like(X), torch.empty(g.E, device="cuda")
+    dX, dAn = torch.full_like(x, -7), torch.full_like(dA, -7)
+    torch.cuda.synchronize()
+    dg = dpg.Graph(ctx, g.offsets, g.col)
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    try:
+        dpg.spmv_bwd_dev(ctx, dg, tv.data_ptr(), 64, X.data_ptr(), G.data_ptr(), dX64.data_ptr(), dA.data_ptr())
+        ctx.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            dpg.spmv_bwd_dev(ctx, dg, tv.data_ptr(), nrhs, x.data_ptr(), gg.data_ptr(), dX.data_ptr(),
+                             dAn.data_ptr())
+        graph.replay()
+        torch.cuda.synchronize()
+    finally:
+        ctx.set_stream(None)
+    A = sp.csr_matrix((tv.cpu().numpy().astype(np.float64), g.col.copy(), g.offsets.copy()), shape=(g.V, g.V))
+    G64 = gg.cpu().numpy().astype(np.float64)
+    assert np.all(np.abs(dX.cpu().numpy() - A.T @ G64) <= TOL * (abs(A).T @ np.abs(G64)))
+    row = np.repeat(np.arange(g.V), np.diff(g.offsets))
+    p = G64[row] * x.cpu().numpy()[g.col]
+    assert np.all(np.abs(dAn.cpu().numpy() - p.sum(1)) <= TOL * np.abs(p).sum(1))
