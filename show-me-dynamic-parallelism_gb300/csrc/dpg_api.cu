@@ -20,8 +20,11 @@ namespace dpg {
 
 thread_local std::string g_last_error;
 
+// A CUDA call that failed (an allocation, say) leaves its error with the runtime, where the next launch of this thread
+// would find it: it is reported here, once.
 dpg_status set_error(dpg_status s, const std::string& msg) {
     g_last_error = msg;
+    if (s == DPG_ERR_CUDA || s == DPG_ERR_CAPACITY) cudaGetLastError();
     return s;
 }
 
@@ -120,7 +123,11 @@ dpg_status after_builds(dpg_graph* g) {
         g->build_pending = false;
         return DPG_OK;
     }
+    // Another thread's capture may forbid queries to threads in the default mode.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     const cudaError_t e = cudaEventQuery(g->built);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     if (e == cudaSuccess) {
         g->build_pending = false;
         return DPG_OK;
