@@ -130,8 +130,8 @@ dpg_status dpg_graph_destroy(dpg_graph* g);
  * 4 (V + E) for PageRank's merge items, once per choice of dpg_graph_relabel that was used; 4 V + 8 E for the transposed
  * CSR of the SpMV backward and the PageRank gradient (which keeps both plans of that CSR too), and for a backward
  * between 12.6 M and 268 M arcs another 8 E for its value permutation. The context keeps scratch of the size of the
- * largest call, until it is destroyed; such a backward takes 8 E of it, and 4 E + 4 (E / 24576)^2 for the first call
- * on a graph. If that cannot be had, the backward reads and writes the values in arc order instead.
+ * largest call, until it is destroyed: about 24 E for the sort that builds a transposed CSR, and 8 E for such a
+ * backward. If the latter, or the permutation, cannot be had, the values are read and written in arc order instead.
  * First calls may be captured into a CUDA graph only where all they build is the renamed columns or the merge items. */
 /* Gather-locality layout for SpMV / PageRank (on by default): column ids are renamed once, by
  * descending frequency, so hot gathered values share cache sectors. Rows and the order of nonzeros in
