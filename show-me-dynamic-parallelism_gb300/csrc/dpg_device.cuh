@@ -91,7 +91,7 @@ __device__ __forceinline__ bool grid_barrier(DevStatus* st, unsigned expected,
 // the wait, lets the next chained kernel start early; without it, that happens when this kernel ends. In
 // a kernel that was not launched so, chain_wait does nothing.
 // What the predecessors in the chain write changes during this kernel's lifetime, so it is read by ordinary
-// volatile loads behind the wait (__ldca, __ldcg, ld_live), never through the read-only path (__ldg), which
+// volatile loads behind the wait (__ldcg, ld_live), never through the read-only path (__ldg), which
 // is for what was written before the chain.
 // An early start also moves the L1's invalidation ahead of the predecessor's end, so lines that the
 // predecessor loads on the same SM while it runs stay there: what it (or another of its blocks) writes

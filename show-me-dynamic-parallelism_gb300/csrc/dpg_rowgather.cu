@@ -90,10 +90,17 @@ __device__ __forceinline__ float ld_stream(const float* p) {
 
 // What the kernels before this one in a chain write (the gathered vector, the previous ranks, a batch's
 // uniform terms) may still change after this kernel has started, ahead of chain_wait: it is read by
-// ordinary loads, which the wait orders, never by the read-only path. ld_live stays out of L1.
+// ordinary loads, which the wait orders, never by the read-only path. ld_live_once stays out of L1. No slower
+// than the read-only path was; __ldca (ld.global.ca) was: PageRank R-MAT 22 3.07 against 3.06 ms, gradient
+// R-MAT 20 7.68 against 7.60 ms.
 __device__ __forceinline__ float ld_live(const float* p) {
     float v;
-    asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_live_once(const float* p) {
+    float v;
+    asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
 
@@ -113,7 +120,7 @@ __device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, flo
                                             double& dang, bool& moved) {
     const float nv = fmaf(L.damping, sum, base);
     if (L.rank_out) L.rank_out[v] = nv;
-    if (L.rank_prev && fabsf(nv - __ldca(L.rank_prev + v)) > L.epsilon) moved = true;
+    if (L.rank_prev && fabsf(nv - ld_live(L.rank_prev + v)) > L.epsilon) moved = true;
     // Only vertices with out-arcs are ever gathered (they are the columns), so the contribution
     // slot of a dangling vertex is free: a batch parks its rank there for the per-graph reduction.
     // The division runs for every row (by 1 for a dangling one) so a warp's rows do not diverge
@@ -128,7 +135,7 @@ __device__ __forceinline__ void pr_epilogue(const RowGatherLaunch& L, int v, flo
 }
 
 __device__ __forceinline__ float batch_base(const RowGatherLaunch& L, int v) {
-    return __ldca(L.gbase + __ldg(L.vgraph + v));
+    return ld_live(L.gbase + __ldg(L.vgraph + v));
 }
 
 // Epilogue of one row of a weighted PageRank sweep (dpg_prgrad.cu): forward (no seed) the new rank and
@@ -153,7 +160,7 @@ __device__ __forceinline__ void weighted_epilogue(const RowGatherLaunch& L, int 
 __device__ __forceinline__ void weighted_epilogue(const RowGatherLaunch& L, int v, float sum, float base,
                                                   double& dang, bool& moved) {
     weighted_epilogue(L, v, sum, base, __ldg(L.W + v), L.perm ? __ldg(L.perm + v) : v,
-                      L.seed ? __ldg(L.seed + v) : 0.0f, L.rank_prev ? __ldca(L.rank_prev + v) : 0.0f, dang, moved);
+                      L.seed ? __ldg(L.seed + v) : 0.0f, L.rank_prev ? ld_live(L.rank_prev + v) : 0.0f, dang, moved);
 }
 
 __device__ __forceinline__ float pr_base(const RowGatherLaunch& L) {
@@ -242,7 +249,7 @@ __device__ __forceinline__ void fill_hot(const float* x, int hot, float* s_hot) 
     for (int i0 = threadIdx.x; i0 < hot; i0 += kBlock * 8) {
         float h[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) h[q] = i0 + kBlock * q < hot ? __ldca(x + i0 + kBlock * q) : 0.0f;
+        for (int q = 0; q < 8; ++q) h[q] = i0 + kBlock * q < hot ? ld_live(x + i0 + kBlock * q) : 0.0f;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
             if (i0 + kBlock * q < hot) s_hot[i0 + kBlock * q] = h[q];
@@ -310,7 +317,7 @@ __global__ void __launch_bounds__(kBlock) spmv_gather_kernel(RowGatherLaunch L) 
             const bool hot = c < L.hot;
             const float hv = s_hot[hot ? c : 0];
             float gv = 0.0f;
-            if (!hot) gv = __ldca(L.x + c);
+            if (!hot) gv = ld_live(L.x + c);
             pv[i] = i * 32 + lane < nnz ? (hot ? hv : gv) * av[i] : 0.0f;
         }
         if (nrows < 0) {
@@ -485,9 +492,9 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
             const int c = item[i];
             if (BATCH) {
                 const int d = c < 0 ? -1 : c - hot0;
-                pv[i] = c < 0 || static_cast<unsigned>(d) < static_cast<unsigned>(hot) ? s_hot[d] : __ldca(L.x + c);
+                pv[i] = c < 0 || static_cast<unsigned>(d) < static_cast<unsigned>(hot) ? s_hot[d] : ld_live(L.x + c);
             } else {
-                pv[i] = c < hot ? s_hot[max(c, -1)] : __ldca(L.x + c);
+                pv[i] = c < hot ? s_hot[max(c, -1)] : ld_live(L.x + c);
             }
         }
         if (MODE == kModeWeighted) {
@@ -511,13 +518,13 @@ __global__ void __launch_bounds__(kBlock) rowgather_kernel(RowGatherLaunch L) {
         }
         float ebase[NE];
 #pragma unroll
-        for (int q = 0; q < NE; ++q) ebase[q] = BATCH ? __ldca(L.gbase + egraph[q]) : base;
+        for (int q = 0; q < NE; ++q) ebase[q] = BATCH ? ld_live(L.gbase + egraph[q]) : base;
         float eW = 0.0f, eseed = 0.0f, eprev = 0.0f;
         if (MODE == kModeWeighted && lane < nrows) {
             eW = ld_stream<MODE>(L.W + row + lane);
             if (L.perm) epos[0] = ld_stream<MODE>(L.perm + row + lane);
             if (L.seed) eseed = ld_stream<MODE>(L.seed + row + lane);
-            if (CONV) eprev = ld_live(L.rank_prev + row + lane);
+            if (CONV) eprev = ld_live_once(L.rank_prev + row + lane);
         }
         // The lane's items in order: a nonzero is added to the open row, a row end closes it.
         int r = r0;
