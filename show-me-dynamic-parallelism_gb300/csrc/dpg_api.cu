@@ -257,7 +257,10 @@ dpg_status graph_finish(dpg_ctx* c, dpg_graph* g, const int32_t* d_w_src) {
 }
 
 void graph_free_device(dpg_graph* g) {
-    if (g->built) cudaEventDestroy(g->built);
+    if (g->built) {
+        cudaEventSynchronize(g->built);  // the context may be on another stream by now
+        cudaEventDestroy(g->built);
+    }
     g->built = nullptr;
     g->build_pending = false;
     if (g->tgraph) {

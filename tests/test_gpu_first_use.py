@@ -162,6 +162,27 @@ def test_next_call_on_another_stream(prob, first, then):
     assert torch.equal(o1, prob.want[first]) and torch.equal(o2, prob.want[then])
 
 
+def test_destroyed_while_its_first_use_is_queued_on_another_stream(prob):
+    """The graph's memory goes back to the context's pool, and the next graph's builds take it, only behind its builds."""
+    import torch
+
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    for what in ("pagerank", "spmv"):
+        out = prob.out()
+        g = prob.graph()
+        with torch.cuda.stream(a):
+            torch.cuda._sleep(20_000_000)
+        prob.ctx.set_stream(a.cuda_stream)
+        prob.call(what, g, out)
+        ev = torch.cuda.Event()
+        ev.record(a)
+        with _on(prob.ctx, b):
+            b.wait_event(ev)  # its sweeps; the builds are the destruction's own affair
+            g.close()
+            prob.check(what, prob.graph())
+        assert torch.equal(out, prob.want[what])
+
+
 def test_backward_captured_before_and_after_its_permutation(ctx):
     """Past 12.6 M arcs the backward permutes values through blocks; a capture that comes first works in arc order."""
     import torch
